@@ -1,0 +1,35 @@
+# SPDX-License-Identifier: MIT
+"""Linears at the sizes where a kernel or a branch of the dispatch can go wrong: edges of tiles,
+remainders, the smallest and largest of a range.  Oracle: the fp32 statement of each op on the same
+bf16 tensors.  Tolerance: the result is rounded once to bf16 (relative error of one rounding at most
+2^-9, rms 2^-9 / sqrt(3) = 1.1e-3) on top of fp32 sums, so rel-L2 stays below 2^-8 = 3.9e-3."""
+import pytest
+import torch
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+TOL = 2.0 ** -8
+
+
+def _bf(*shape, seed, std=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device="cuda") * std).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("m,n,k", [(512, 256, 64), (513, 600, 136), (777, 1032, 512), (1000, 1024, 72),
+                                   (2049, 512, 256), (200, 512, 256), (130, 264, 64)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_token_major_silu_mul(ext, m, n, k, bias):
+    from barlink_sm86_b200 import ops
+    x, w = _bf(m, k, seed=1), _bf(n, k, seed=2, std=k ** -0.5)
+    b = _bf(n, seed=3) if bias else None
+    want = ops.ref.linear(x.float(), w, b, silu_mul=True)
+    assert rel_l2(ops.linear(x, w, b, silu_mul=True), want) < TOL
+    # an output that starts off a 16-byte boundary
+    buf = torch.zeros(m * (n // 2) + 1, dtype=torch.bfloat16, device="cuda")
+    out = buf[1:].view(m, n // 2)
+    ops.linear(x, w, b, silu_mul=True, out=out)
+    assert rel_l2(out, want) < TOL and float(buf[0]) == 0.0
+    torch.cuda.synchronize()
+    assert ext.gemm_error_flag(0) == 0

@@ -21,6 +21,7 @@ SOURCES = [
     "comm_kernels.cu",
     "gemm_kernels.cu",
     "dlin_kernels.cu",
+    "qlin_kernels.cu",
     "ops_kernels.cu",
     "attn_kernels.cu",
     "attn_tc_kernels.cu",

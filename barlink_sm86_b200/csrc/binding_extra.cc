@@ -193,6 +193,95 @@ std::tuple<at::Tensor, at::Tensor> w8_group_scales(const at::Tensor& scales) {
   return {row, rel};
 }
 
+// ---- decode linears on quantised weights: int8 weights against int8 digits of the activations ----
+struct QWeight {
+  const void* w;
+  int src, n, k;
+  int scale_kind;
+  const void* scale;
+  const void* row_scale = nullptr;
+  int group_k = 0;
+  const void* zeros = nullptr;
+};
+// a shape that bl_qlin takes and (three digits) bf16 rows that bl_quant_digits can read
+bool qlin_takes(const at::Tensor& x, int k, bool act_int8) {
+  if (x.size(0) < 1 || x.size(0) > BL_QLIN_MAX_TOKENS || k % 16 != 0) return false;
+  return act_int8 ? k <= 131072
+                  : k <= 32768 && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0;
+}
+// digits = 3: x as it is; digits = 1: x quantised to int8 per token.  want_slabs: fp32 [splits, m, n]
+// when the shape wants a k-split (bias is then the consumer's), else bf16 [m, n].
+at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10::optional<at::Tensor>& bias,
+                    bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
+  const int m = int(x.size(0));
+  at::Tensor xq, xs = at::empty({m}, x.options().dtype(at::kFloat));
+  if (digits == 3) {
+    xq = at::empty({int64_t(bl_quant_digits_bytes(m, q.k))}, x.options().dtype(at::kChar));
+    BL_CHECK(bl_quant_digits(x.data_ptr(), m, int(x.stride(0)), q.k, q.src == 2 ? 1 : 0, xq.data_ptr(), xs.data_ptr(), st,
+                             err, errlen));
+  } else {
+    at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
+    BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
+  }
+  if (bias) {
+    check_bf16x(*bias, "bias");
+    TORCH_CHECK(bias->numel() == q.n, "barlink: bias must have n entries");
+  }
+  if (splits <= 0) {
+    splits = bl_qlin_splits(q.n, q.k, m);
+    // bl_slab_finish stores 16-byte vectors
+    if (!want_slabs && (silu_mul ? q.n % 16 : q.n % 8) != 0) splits = 1;
+  }
+  const int kb = (q.k + 127) / 128, per = (kb + splits - 1) / splits;
+  splits = (kb + per - 1) / per;
+  blQlinArgs a;
+  memset(&a, 0, sizeof(a));
+  a.w = q.w; a.src = q.src; a.n = q.n; a.k = q.k;
+  a.xq = xq.data_ptr(); a.xs = xs.data_ptr();
+  a.m = m; a.digits = digits;
+  a.scale_kind = q.scale_kind; a.scale = q.scale; a.row_scale = q.row_scale; a.group_k = q.group_k; a.zeros = q.zeros;
+  a.splits = splits;
+  a.err_flag = err_flag;
+  at::Tensor slabs, out;
+  if (splits > 1) {
+    slabs = at::empty({splits, m, q.n}, x.options().dtype(at::kFloat));
+    a.slabs = slabs.data_ptr();
+  } else {
+    out = at::empty({m, silu_mul ? q.n / 2 : q.n}, x.options());
+    a.out = out.data_ptr();
+    a.ldo = int(out.size(1));
+    a.bias = bias ? bias->data_ptr() : nullptr;
+    a.silu_mul = silu_mul ? 1 : 0;
+  }
+  BL_CHECK(bl_qlin(&a, st, err, errlen));
+  if (splits == 1) return out;
+  if (want_slabs) return slabs;
+  out = at::empty({m, silu_mul ? q.n / 2 : q.n}, x.options());
+  BL_CHECK(bl_slab_finish(slabs.data_ptr(), splits, m, q.n, bias ? bias->data_ptr() : nullptr, silu_mul ? 1 : 0,
+                          out.data_ptr(), int(out.size(1)), st, err, errlen));
+  return out;
+}
+
+// Decode form of w8a16_linear without a reduction: fp32 slabs [splits, m, n] (scaled, no bias) for the
+// kernel that reads them next, or the bf16 result when the shape wants no k-split.
+at::Tensor w8a16_linear_split(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& scale,
+                              const c10::optional<at::Tensor>& bias, bool act_int8) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1,
+              "barlink: x must be a 2-D bfloat16 CUDA tensor with unit inner stride");
+  TORCH_CHECK(wq.is_cuda() && wq.is_contiguous() && wq.scalar_type() == at::kChar && wq.dim() == 2 &&
+                  wq.size(1) == x.size(1),
+              "barlink: wq must be a contiguous int8 [n, k] CUDA tensor with k = x.shape[1]");
+  check_bf16x(scale, "scale");
+  const int k = int(x.size(1)), n = int(wq.size(0)), dev = x.device().index();
+  TORCH_CHECK(scale.numel() == n, "barlink: scale must have one entry per output channel");
+  TORCH_CHECK(qlin_takes(x, k, act_int8), "barlink: w8a16_linear_split is for 1..", BL_QLIN_MAX_TOKENS, " 16-byte aligned rows, K % 16 == 0");
+  c10::cuda::CUDAGuard guard(x.device());
+  QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
+  return qlin_run(x, act_int8 ? 1 : 3, q, bias, false, 0, true, w8_scratch(dev).err_flag.data_ptr(),
+                  at::cuda::getCurrentCUDAStream(dev).stream());
+}
+
 at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& scale,
                         const c10::optional<at::Tensor>& bias, bool silu_mul, int splits,
                         const c10::optional<at::Tensor>& group_rel, bool act_int8,
@@ -206,7 +295,8 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   const int m = int(x.size(0)), k = int(x.size(1)), n = int(wq.size(0));
   TORCH_CHECK(group_scale || scale.numel() == n, "barlink: scale must have one entry per output channel");
   if (group_scale) {
-    TORCH_CHECK(act_int8 && m <= 64, "barlink: group_scale goes with act_int8 and at most 64 tokens");
+    TORCH_CHECK(!group_rel && m >= 1 && qlin_takes(x, k, act_int8), "barlink: group_scale goes with 1..", BL_QLIN_MAX_TOKENS,
+                " 16-byte aligned rows");
     TORCH_CHECK(group_scale->is_cuda() && group_scale->is_contiguous() && group_scale->scalar_type() == at::kBFloat16 &&
                     group_scale->dim() == 2 && group_scale->size(0) == n && k % group_scale->size(1) == 0 &&
                     (k / group_scale->size(1)) % 128 == 0,
@@ -215,18 +305,34 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   const int dev = x.device().index();
   c10::cuda::CUDAGuard guard(x.device());
   void* st = at::cuda::getCurrentCUDAStream(dev).stream();
-  at::Tensor out = at::empty({m, silu_mul ? n / 2 : n}, x.options());
-  if (m == 0) return out;
+  if (m == 0) return at::empty({0, silu_mul ? n / 2 : n}, x.options());
   if (group_rel) {
     TORCH_CHECK(group_rel->is_cuda() && group_rel->is_contiguous() && group_rel->scalar_type() == at::kHalf &&
                     group_rel->dim() == 2 && group_rel->size(0) == n && k % group_rel->size(1) == 0,
                 "barlink: group_rel must be contiguous float16 [n, k / group] (see w8_group_scales)");
     TORCH_CHECK(m <= 256, "barlink: in-kernel group scales take at most 256 tokens");
   }
+  TORCH_CHECK(!(act_int8 && group_rel), "barlink: int8 activations go with per-channel or group_scale weight scales");
+  // 1..128 tokens: the weights go to the tensor cores as they are (qlin_kernels.cu).  Group scales need
+  // groups of whole 128-wide k-blocks.
+  if (qlin_takes(x, k, act_int8) && (!group_rel || (k / group_rel->size(1)) % 128 == 0)) {
+    QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
+    if (group_scale) {
+      q.scale_kind = BL_QSCALE_BF16_NG;
+      q.scale = group_scale->data_ptr();
+      q.group_k = k / int(group_scale->size(1));
+    } else if (group_rel) {
+      q.scale_kind = BL_QSCALE_F16_NG;
+      q.scale = group_rel->data_ptr();
+      q.row_scale = scale.data_ptr();
+      q.group_k = k / int(group_rel->size(1));
+    }
+    return qlin_run(x, act_int8 ? 1 : 3, q, bias, silu_mul, splits, false, w8_scratch(dev).err_flag.data_ptr(), st);
+  }
+  at::Tensor out = at::empty({m, silu_mul ? n / 2 : n}, x.options());
   if (act_int8) {
     // the reference's numerics (w8a16.cu:37-92 there quantises the activations per token and
     // multiplies int8 by int8): both operands go to the tensor cores as int8
-    TORCH_CHECK(!group_rel, "barlink: int8 activations go with per-channel weight scales");
     TORCH_CHECK(k % 16 == 0, "barlink: int8 activations need K % 16 == 0");
     at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
     at::Tensor xq = at::empty({m, k}, x.options().dtype(at::kChar));
@@ -248,10 +354,6 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
       a.n = n;
       a.k = k;
       a.scale = scale.data_ptr();
-      if (group_scale) {
-        a.group_scale = group_scale->data_ptr();
-        a.group_k = k / int(group_scale->size(1));
-      }
       a.bias = bias ? bias->data_ptr() : nullptr;
       a.out = out.data_ptr();
       a.ldo = silu_mul ? n / 2 : n;
@@ -661,6 +763,8 @@ void bind_extra(py::module_& m) {
   m.def("w8a16_linear", &w8a16_linear, py::arg("x"), py::arg("wq"), py::arg("scale"),
         py::arg("bias") = py::none(), py::arg("silu_mul") = false, py::arg("splits") = 0,
         py::arg("group_rel") = py::none(), py::arg("act_int8") = false, py::arg("group_scale") = py::none());
+  m.def("w8a16_linear_split", &w8a16_linear_split, py::arg("x"), py::arg("wq"), py::arg("scale"),
+        py::arg("bias") = py::none(), py::arg("act_int8") = false);
   m.def("w8_group_scales", &w8_group_scales, py::arg("scales"));
   m.def("w8_error_flag", &w8_error_flag, py::arg("device") = 0);
   m.def("dlin", &dlin, py::arg("x"), py::arg("weight"), py::arg("pro") = "none", py::arg("epi") = "store",

@@ -103,11 +103,6 @@ typedef struct blGemmArgs {
   int i8;
   const void* feat_scale; /* bf16 per output feature, or null */
   const void* tok_scale;  /* fp32 per token, or null */
-  /* i8 with one weight scale per (feature, k-group) instead of feat_scale: bf16 [ra][k / group_k], group_k a
-   * multiple of 128.  Weights-first orientation (swap) and at most 64 tokens only: every k-block gets an
-   * accumulator of its own and the epilogue warps add acc * scale, k-block by k-block; no k-split. */
-  const void* group_scale;
-  int group_k;
 } blGemmArgs;
 int bl_gemm_bf16(const blGemmArgs* a, void* stream, char* err, size_t errlen);
 /* Weights in 16 KiB tiles [ceil(n/128)][ceil(k/64)][128 x 128 B], each tile in the
@@ -123,7 +118,8 @@ int bl_gemm_splits(int n, int k, int tokens);
 /* W8A16: x [m x k] bf16, wq [n x k] int8 (row = output channel), scale [n]
  * bf16 (per channel) or scales [k/group x n] fp32 (group > 0).  out [m x n]
  * bf16.  The int8 tile is widened to bf16 in shared memory inside the main
- * loop and multiplied on the tensor cores. */
+ * loop and multiplied on the tensor cores.  This form serves 129..256 tokens and what bl_qlin does not
+ * take (groups of 64, rows off 16-byte boundaries). */
 typedef struct blW8A16Args {
   const void* x;
   int m, ldx;
@@ -140,11 +136,6 @@ typedef struct blW8A16Args {
   void* counters;
   int n_counters;
   void* err_flag;
-  /* split-K slabs instead of a reduced output (see blGemmArgs.partial_out); the
-   * per-channel scale is applied to every slab */
-  void* partial_out;
-  size_t partial_stride;
-  int partial_splits;
   /* per-group scales applied inside the main loop: group_rel is fp16 [n][k / group_k], each row's
    * group scales divided by that row's largest one, and `scale` then holds the row's largest
    * scale (see bl_w8_group_scales).  group_k must be a multiple of 64.  null = per channel only */
@@ -152,12 +143,9 @@ typedef struct blW8A16Args {
   int group_k;
   /* activations already quantised per token (bl_w8a16_quant_act): xq int8 [m x k] dense and xs fp32
    * [m].  The product then runs as int8 x int8 on the tensor cores (no widening of the weights); x is
-   * ignored, group_rel must be null and partial_out is not supported. */
+   * ignored and group_rel must be null. */
   const void* xq;
   const void* xs;
-  /* with xq: per-group weight scales bf16 [n][k / group_k] (the reference's checkpoint format, group 128)
-   * instead of `scale`; at most 64 tokens, group_k a multiple of 128 */
-  const void* group_scale;
 } blW8A16Args;
 /* scales bf16 [n][groups] -> row_max bf16 [n] and rel fp16 [n][groups] = scale / row_max */
 int bl_w8_group_scales(const void* scales, int n, int groups, void* row_max, void* rel, void* stream, char* err,
@@ -175,6 +163,55 @@ int bl_w8a16_quant_act(const void* x, int m, int k, void* xq, void* xs, void* st
 int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, const void* sw_t, void* out,
                   int m, int n, int k, int splits, void* ws, void* stream, char* err,
                   size_t errlen);
+
+/* ---- decode linears on quantised weights (qlin_kernels.cu) ------------------------------------
+ * y[m, n] = xs[m] * sum over groups of scale * (integer products), 1..BL_QLIN_MAX_TOKENS tokens.
+ * Activations: digits = 1: xq int8 [m x k] and xs as bl_w8a16_quant_act leaves them; digits = 3: the
+ * planes and xs of bl_quant_digits (bf16 activations without loss, see there).
+ * src: 0 int8 [n][k]; 1 int8 [k/16][n][16] (one digit, group scales); 2 GPTQ-v1 int32 [k/8][n] with
+ * `zeros` int32 [k/group_k][n/8] (three digits written with permute = 1).
+ * out bf16 (splits = 1; bias, silu_mul as in blGemmArgs) or slabs fp32 [splits][m][n] (scales applied,
+ * no bias), summed by the next kernel or by bl_slab_finish. */
+enum {
+  BL_QSCALE_BF16_N = 0,  /* bf16 [n] */
+  BL_QSCALE_BF16_NG = 1, /* bf16 [n][k / group_k] */
+  BL_QSCALE_F16_NG = 2,  /* fp16 [n][k / group_k], times row_scale */
+  BL_QSCALE_F32_GN = 3,  /* fp32 [k / group_k][n] */
+  BL_QSCALE_F16_GN = 4   /* fp16 [k / group_k][n] */
+};
+#define BL_QLIN_MAX_TOKENS 128
+typedef struct blQlinArgs {
+  const void* w;
+  int src, n, k;
+  const void* xq;
+  const void* xs;
+  int m, digits;
+  int scale_kind;
+  const void* scale;
+  const void* row_scale; /* bf16 [n] or null */
+  int group_k;           /* a multiple of 128 that divides k */
+  const void* zeros;
+  const void* bias;
+  void* out;
+  int ldo;
+  int silu_mul;
+  void* slabs;
+  int splits;
+  void* err_flag;
+} blQlinArgs;
+int bl_qlin(const blQlinArgs* a, void* stream, char* err, size_t errlen);
+int bl_qlin_splits(int n, int k, int m);  /* k-splits that suit the shape */
+int bl_qlin_tile_tokens(int m);
+/* x [m x k] bf16 (pitch ldx) -> xq int8 [ceil(m/tile)][3][tile][k] (tile = bl_qlin_tile_tokens(m)) and
+ * xs fp32 [m] with x = xs * (d0 + d1 / 2^8 + d2 / 2^16): exact for elements down to 2^-15 of the row's
+ * largest, to 2^-24 of the largest below that.  permute: digits in the order 0 2 4 6 1 3 5 7 of every
+ * eight (packed int4 weights).  K a multiple of 8, at most 32768. */
+int bl_quant_digits(const void* x, int m, int ldx, int k, int permute, void* xq, void* xs, void* stream, char* err,
+                    size_t errlen);
+size_t bl_quant_digits_bytes(int m, int k);
+/* slabs fp32 [nsplit][m][n] -> bf16, + bias, optionally SiLU*mul over interleaved columns */
+int bl_slab_finish(const void* slabs, int nsplit, int m, int n, const void* bias, int silu_mul, void* out, int ldo,
+                   void* stream, char* err, size_t errlen);
 
 /* out = RMSNorm(x (+ residual)) * gamma; when residual is given, x + residual
  * is also written to residual_out (may alias residual). */

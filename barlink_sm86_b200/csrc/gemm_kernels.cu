@@ -219,13 +219,12 @@ __global__ void __launch_bounds__(kGemmThreads, CPS)
   gemm_body<BN, CPS, false>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
 }
 
-// int8 operands (GemmShape::i8 = MODE: 1 plain, 2 per-group weight scales with one accumulator per k-block)
-template <int BN, int MODE>
+// int8 operands (GemmShape::i8)
+template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     k_gemm_i8(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
               GemmShape g, LocalSink<BN> sink, uint64_t hint_a, uint64_t hint_b) {
-  static_assert(MODE == 1 || (MODE == 2 && BN <= 64), "the per-group accumulators live in registers");
-  gemm_body<BN, 1, false, MODE>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
+  gemm_body<BN, 1, false, 1>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
 }
 
 // Epilogue of the split-K decode path: every k-split stores its raw fp32
@@ -511,20 +510,13 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
   g.tiles_b = (a.rb + BN - 1) / BN;
   g.kblocks = (a.k + int(box_cols) - 1) / int(box_cols);
   g.i8 = a.i8 ? 1 : 0;
-  g.gscale_bf = nullptr;
-  if (a.i8 && a.group_scale) {
-    g.i8 = 2;
-    g.gscale_bf = static_cast<const __nv_bfloat16*>(a.group_scale);
-    g.gs_groups = (a.k + a.group_k - 1) / a.group_k;
-    g.gs_kblocks = a.group_k / int(box_cols);
-  }
   const int tiles = g.tiles_a * g.tiles_b;
   const int sms = sm_count();
   // CTAs launched at most (BL_GEMM_WAVE: percent of the resident slots)
   static const int wave = env_int_or("BL_GEMM_WAVE", 100);
   int slots = sms * S::kCtasPerSm * wave / 100;
   if (slots < 1) slots = 1;
-  g.splits = g.i8 == 2 ? 1 : pick_splits(tiles, g.kblocks, slots, splits_want);
+  g.splits = pick_splits(tiles, g.kblocks, slots, splits_want);
   const bool partial = a.partial_out != nullptr || a.peer != nullptr;
   if (partial) {
     if (a.partial_splits < 1 || g.splits > a.partial_splits) g.splits = a.partial_splits;
@@ -553,10 +545,8 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
   g.gate_timeout_ns = a.gate_timeout_ns ? a.gate_timeout_ns : 2000000000ull;
   g.ab_fmt = 1;
   g.gscale = nullptr;
-  if (g.i8 != 2) {
-    g.gs_groups = 0;
-    g.gs_kblocks = 1;
-  }
+  g.gs_groups = 0;
+  g.gs_kblocks = 1;
   g.weights_in_a = a.dynamic_weights ? 2 : (a.swap ? 1 : 0);
   g.ws = static_cast<float*>(a.ws);
   g.counters = static_cast<uint32_t*>(a.counters);
@@ -641,30 +631,16 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
       }
       attr_set = true;
     }
-    bool done = false;
     if (g.i8) {
       using S1 = GemmSmem<BN, 1>;
-      auto go = [&](auto kern) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S1::kBytes);
-        if (e == cudaSuccess)
-          e = launch_k(kern, dim3(grid), dim3(kGemmThreads), size_t(S1::kBytes), st, ta, tb, g, sink,
-                       a.swap ? hint_w : hint_x, a.swap ? hint_x : hint_w);
-      };
-      if (g.i8 == 1) {
-        go(k_gemm_i8<BN, 1>);
-        done = true;
-      } else if constexpr (BN <= 64) {
-        go(k_gemm_i8<BN, 2>);
-        done = true;
-      }
-      if (!done) {
-        set_err(err, errlen, "barlink: per-group int8 scales need a tile of at most 64 tokens");
-        return -1;
-      }
-    }
-    if (!done)
+      e = cudaFuncSetAttribute(k_gemm_i8<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S1::kBytes);
+      if (e == cudaSuccess)
+        e = launch_k(k_gemm_i8<BN>, dim3(grid), dim3(kGemmThreads), size_t(S1::kBytes), st, ta, tb, g, sink,
+                     a.swap ? hint_w : hint_x, a.swap ? hint_x : hint_w);
+    } else {
       e = launch_k(k_gemm<BN, CPS>, dim3(grid), dim3(kGemmThreads), size_t(S::kBytes), st, ta, tb, g,
                    sink, a.swap ? hint_w : hint_x, a.swap ? hint_x : hint_w);
+    }
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -683,14 +659,6 @@ __global__ void __launch_bounds__(GemmSmem<BN, 1, true>::kThreads, 1)
               GemmShape g, LocalSink<BN> sink, uint64_t hint_a, uint64_t hint_b) {
   gemm_body<BN, 1, true>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
 }
-template <int BN>
-__global__ void __launch_bounds__(GemmSmem<BN, 1, true>::kThreads, 1)
-    k_gemm_w8_partial(const __grid_constant__ CUtensorMap tmap_a,
-                      const __grid_constant__ CUtensorMap tmap_b, GemmShape g, PartialSink<BN> sink,
-                      uint64_t hint_a, uint64_t hint_b) {
-  gemm_body<BN, 1, true>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
-}
-
 __global__ void k_w8_dequant(const int8_t* __restrict__ wq, const __nv_bfloat16* __restrict__ scale,
                              __nv_bfloat16* __restrict__ out, int n, int k) {
   pdl_launch_dependents();
@@ -729,19 +697,10 @@ static int launch_w8(const blW8A16Args& a, cudaStream_t st, char* err, size_t er
   g.kblocks = (a.k + kTileK - 1) / kTileK;
   const int tiles = g.tiles_a * g.tiles_b;
   const int sms = sm_count();
-  const bool partial = a.partial_out != nullptr;
-  g.splits = partial ? a.partial_splits : pick_splits(tiles, g.kblocks, sms, a.splits);
-  if (!partial && g.splits > 1) {
+  g.splits = pick_splits(tiles, g.kblocks, sms, a.splits);
+  if (g.splits > 1) {
     const size_t need = size_t(tiles) * g.splits * BN * kTileA * sizeof(float);
     if (!a.ws || a.ws_bytes < need || !a.counters || a.n_counters < tiles) g.splits = 1;
-  }
-  if (partial) {
-    const int per = (g.kblocks + g.splits - 1) / g.splits;
-    if (g.splits < 1 || (g.kblocks + per - 1) / per != g.splits) {
-      set_err(err, errlen, "barlink: %d k-splits do not divide %d k-blocks into non-empty parts", g.splits,
-              g.kblocks);
-      return -1;
-    }
   }
   g.ab_fmt = 1;
   if (a.group_rel) {
@@ -749,7 +708,6 @@ static int launch_w8(const blW8A16Args& a, cudaStream_t st, char* err, size_t er
     g.gs_kblocks = a.group_k / kTileK;
     g.gs_groups = (a.k + a.group_k - 1) / a.group_k;
   }
-  g.direct = partial ? 1 : 0;
   g.weights_in_a = 1;
   g.ws = static_cast<float*>(a.ws);
   g.counters = static_cast<uint32_t*>(a.counters);
@@ -757,52 +715,30 @@ static int launch_w8(const blW8A16Args& a, cudaStream_t st, char* err, size_t er
   g.gate_timeout_ns = 2000000000ull;
   const int units = tiles * g.splits;
   const int grid = units < sms ? units : sms;
+  LocalSink<BN> sink;
+  sink.out = static_cast<__nv_bfloat16*>(a.out);
+  sink.bias = static_cast<const __nv_bfloat16*>(a.bias);
+  sink.residual = nullptr;
+  sink.ldo = a.ldo;
+  sink.ra = a.n;
+  sink.rb = a.m;
+  sink.swap = 1;
+  sink.epi = (a.bias ? 1 : 0) | (a.silu_mul ? 4 : 0);
+  sink.scale = static_cast<const __nv_bfloat16*>(a.scale);
+  sink.xscale = nullptr;
+  fill_push(sink, nullptr);
+  static bool attr = false;
   cudaError_t e;
-  if (partial) {
-    PartialSink<BN> ps;
-    ps.out = static_cast<float*>(a.partial_out);
-    ps.slab = a.partial_stride;
-    ps.ldo = a.ldo;
-    ps.ra = a.n;
-    ps.rb = a.m;
-    ps.swap = 1;
-    ps.scale = static_cast<const __nv_bfloat16*>(a.scale);
-    static bool attr = false;
-    if (!attr) {
-      e = cudaFuncSetAttribute(k_gemm_w8_partial<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
-      if (e != cudaSuccess) {
-        set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
-        return -1;
-      }
-      attr = true;
+  if (!attr) {
+    e = cudaFuncSetAttribute(k_gemm_w8<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+    if (e != cudaSuccess) {
+      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
+      return -1;
     }
-    e = launch_k(k_gemm_w8_partial<BN>, dim3(grid), dim3(S::kThreads), size_t(S::kBytes), st, ta, tb, g, ps,
-                 kHintEvictFirst, kHintEvictLast);
-  } else {
-    LocalSink<BN> sink;
-    sink.out = static_cast<__nv_bfloat16*>(a.out);
-    sink.bias = static_cast<const __nv_bfloat16*>(a.bias);
-    sink.residual = nullptr;
-    sink.ldo = a.ldo;
-    sink.ra = a.n;
-    sink.rb = a.m;
-    sink.swap = 1;
-    sink.epi = (a.bias ? 1 : 0) | (a.silu_mul ? 4 : 0);
-    sink.scale = static_cast<const __nv_bfloat16*>(a.scale);
-    sink.xscale = nullptr;
-    fill_push(sink, nullptr);
-    static bool attr = false;
-    if (!attr) {
-      e = cudaFuncSetAttribute(k_gemm_w8<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
-      if (e != cudaSuccess) {
-        set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
-        return -1;
-      }
-      attr = true;
-    }
-    e = launch_k(k_gemm_w8<BN>, dim3(grid), dim3(S::kThreads), size_t(S::kBytes), st, ta, tb, g, sink,
-                 kHintEvictFirst, kHintEvictLast);
+    attr = true;
   }
+  e = launch_k(k_gemm_w8<BN>, dim3(grid), dim3(S::kThreads), size_t(S::kBytes), st, ta, tb, g, sink,
+               kHintEvictFirst, kHintEvictLast);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: W8A16 launch failed: %s", cudaGetErrorString(e));
@@ -1126,7 +1062,7 @@ static int launch_gemm_pair(const blGemmArgs& a, cudaStream_t st, char* err, siz
 using namespace bl;
 
 extern "C" int bl_w8a16_linear(const blW8A16Args* a, void* stream, char* err, size_t errlen) {
-  if (!a || (!a->x && !a->xq) || !a->wq || (!a->scale && !a->group_scale) || (!a->out && !a->partial_out) || a->m < 1 || a->n < 1 ||
+  if (!a || (!a->x && !a->xq) || !a->wq || !a->scale || !a->out || a->m < 1 || a->n < 1 ||
       a->k < 16 || (a->k & 15)) {
     set_err(err, errlen, "barlink: w8a16_linear needs x, wq, scale, an output, and K a multiple of 16");
     return -1;
@@ -1144,8 +1080,8 @@ extern "C" int bl_w8a16_linear(const blW8A16Args* a, void* stream, char* err, si
   const int bn = a->m <= 16 ? 16 : a->m <= 32 ? 32 : a->m <= 64 ? 64 : a->m <= 128 ? 128 : 256;
   if (a->xq) {
     // int8 activations: the weights go from HBM to the tensor cores as they are
-    if (!a->xs || a->group_rel || a->partial_out) {
-      set_err(err, errlen, "barlink: int8 activations need their per-token scales and a plain output (group scales: group_scale)");
+    if (!a->xs || a->group_rel) {
+      set_err(err, errlen, "barlink: int8 activations need their per-token scales and per-channel weight scales");
       return -1;
     }
     blGemmArgs g;
@@ -1163,12 +1099,7 @@ extern "C" int bl_w8a16_linear(const blW8A16Args* a, void* stream, char* err, si
     g.counters = a->counters; g.n_counters = a->n_counters;
     g.err_flag = a->err_flag;
     g.i8 = 1;
-    if (a->group_scale) {
-      g.group_scale = a->group_scale;
-      g.group_k = a->group_k;
-    } else {
-      g.feat_scale = a->scale;
-    }
+    g.feat_scale = a->scale;
     g.tok_scale = a->xs;
     return bl_gemm_bf16(&g, stream, err, errlen);
   }
@@ -1284,11 +1215,6 @@ extern "C" int bl_gemm_bf16(const blGemmArgs* a, void* stream, char* err, size_t
   }
   if (a->i8 && ((a->k & 15) || a->weight_tiled || a->peer || a->push || a->gate_flags || a->partial_out)) {
     set_err(err, errlen, "barlink: the int8 product needs K a multiple of 16 and plain operands and output");
-    return -1;
-  }
-  if (a->group_scale && (!a->i8 || !a->swap || a->rb > 64 || a->group_k < 128 || (a->group_k & 127) || a->feat_scale ||
-                         (a->bn > 64))) {
-    set_err(err, errlen, "barlink: per-group scales go with the int8 product, weights first, at most 64 tokens, groups of a multiple of 128");
     return -1;
   }
   if (!a->i8 && (a->feat_scale || a->tok_scale)) {

@@ -1,0 +1,742 @@
+// SPDX-License-Identifier: MIT
+//
+// Decode linears (1..128 tokens) on quantised weights:
+//   y[t, n] = xs[t] * sum_g s[n, g] * sum_{k in g} q[n, k] * X[t, k]
+// on tcgen05.mma kind::i8, int8 weights against int8 digits of the activations.
+//
+// What bounds a decode linear is the weight stream from HBM, so nothing but that stream should cost
+// time.  Widening int8 weights to bf16 on the CUDA cores did: 11 instructions per four weights held
+// the kernel to 2.0-2.7 TB/s.  Here the activations are taken apart instead.  A token's bf16 row is
+// scaled by a power of two so that its largest element is just below 1 and written as three base-256
+// digits (k_quant_digits): 23 bits below the row's largest element, so every element down to 2^-15
+// of it is represented exactly and the rest to within 2^-24 of it -- below what fp32 accumulation
+// rounds away.  The weights go from HBM to the tensor core as they are, the three digit planes of
+// all tokens are the N dimension of one MMA, sums are exact int32, and the epilogue puts
+// (d0 + d1 / 2^8 + d2 / 2^16) * xs[t] together.  With activations that the caller quantised to int8
+// (one digit) the same kernel runs with a third of the N.
+//
+// Weight forms (SRC):
+//   kRows    int8 [n][k], TMA tiles of 128 rows x 128 bytes in the 128-byte swizzle
+//   kChunks  int8 [k/16][n][16] (the reference's layout, torch_ext/barlink_sm86/w8a16.cu:94-117): a
+//            16-byte chunk of 128 rows is 2 KiB contiguous and already the tensor core's unswizzled
+//            K-major layout, so a k-block is eight bulk copies
+//   kNibbles int4 GPTQ-v1 (int32 [k/8][n], 8 k per word): four warps turn a raw 8 KiB tile into the
+//            layout of kChunks, seven instructions per eight weights, zero point subtracted; nibbles
+//            come out in the order 0 2 4 6 1 3 5 7 of each eight and k_quant_digits writes the
+//            digits in that order
+// Scales (SC): per output channel, applied by the epilogue; or per group of 128 (a k-block), where
+// every k-block gets a TMEM accumulator of its own and the epilogue warps add acc * scale in fp32.
+//
+// A k-split writes fp32 slabs [split][token][n]; the consumer of the linear sums them as it reads
+// (the norm, RoPE and attention kernels do), or k_slab_finish does with bias / SiLU*mul.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <stdint.h>
+#include <string.h>
+
+#include "bl_ops.h"
+#include "heap.h"
+#include "launch.h"
+#include "ptx.cuh"
+
+namespace bl {
+
+enum { kRows = 0, kChunks = 1, kNibbles = 2 };
+
+constexpr int kQRows = 128;      // weight rows per tile
+constexpr int kQK = 128;         // weights of a row per k-block
+constexpr int kQTileA = kQRows * kQK;
+
+struct QlinShape {
+  int n, m, k;
+  int tiles_a, tiles_b, kblocks, splits;
+  const uint8_t* w;              // kChunks: weights; kNibbles: packed words come through the tensor map
+  const uint32_t* zeros;         // kNibbles: int32 [groups][n/8]
+  const float* xs;               // per token
+  int scale_kind;                // see blQlinArgs
+  const void* scale;
+  const __nv_bfloat16* row_scale;
+  int groups, gk;                // scale groups of a row, k-blocks per group
+  const __nv_bfloat16* bias;
+  __nv_bfloat16* out;
+  int ldo, silu;
+  float* slabs;                  // non-null: fp32 output [split][token][n]
+  uint32_t* err;
+};
+
+template <int SRC, int ND, int TB, bool GROUPED>
+struct QlinCfg {
+  static constexpr int BN = ND * TB;
+  static constexpr int kStageA = SRC == kNibbles ? kQTileA / 2 : kQTileA;
+  static constexpr int kStageB = BN * kQK;
+  static constexpr int kStage = kStageA + kStageB;
+  static constexpr int kA8 = SRC == kNibbles ? 4 : 0;   // expanded tiles in flight
+  // as many bytes in flight as fit: the weight stream is what counts
+  static constexpr int kFit = (226 * 1024 - 2048 - kA8 * kQTileA) / kStage;
+  static constexpr int kStages = kFit > 10 ? 10 : kFit;
+  static constexpr int kSmem = kStages * kStage + kA8 * kQTileA + 2048;
+  // per-group mode hands an accumulator over every k-block: four of them where they fit
+  static constexpr int kAcc = GROUPED && 4 * BN <= 512 ? 4 : 2;
+  static constexpr int kCols = kAcc * BN <= 32 ? 32 : kAcc * BN <= 64 ? 64 : kAcc * BN <= 128 ? 128 : kAcc * BN <= 256 ? 256 : 512;
+  static constexpr int kExpand = SRC == kNibbles ? 256 : 0;
+  static constexpr int kThreads = 192 + kExpand;
+  static_assert(kStages >= 3 && kAcc * BN <= 512 && kStage % 1024 == 0, "stage ring / TMEM do not fit");
+};
+
+// K-major tile of 16-byte chunks [chunk][row][16 B], no swizzle: eight rows of one chunk are a 128-byte
+// core matrix, the next eight rows 128 bytes on (stride byte offset), the next chunk 2048 bytes on
+// (leading byte offset)
+__device__ __forceinline__ uint64_t umma_desc_k_chunks(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>((kQRows * 16) >> 4) << 16;
+  d |= static_cast<uint64_t>(128 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  return d;
+}
+
+template <int SRC, int ND, int TB, bool GROUPED>
+__global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
+    k_qlin(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const QlinShape g) {
+  using S = QlinCfg<SRC, ND, TB, GROUPED>;
+  extern __shared__ uint8_t smem_raw[];
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_raw);
+  uint64_t* empty_bar = full_bar + S::kStages;
+  uint64_t* tfull_bar = empty_bar + S::kStages;
+  uint64_t* tempty_bar = tfull_bar + 4;
+  uint64_t* ready_bar = tempty_bar + 4;   // kNibbles: an expanded tile is ready / free again
+  uint64_t* afree_bar = ready_bar + 4;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(afree_bar + 4);
+  volatile uint32_t* s_abort = tmem_slot + 1;
+  const uint32_t ring = (smem_u32(smem_raw) + 1024u + 1023u) & ~1023u;
+  const uint32_t ring_a8 = ring + S::kStages * S::kStage;
+
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int units = g.tiles_a * g.tiles_b * g.splits;
+  const int kb_per = (g.kblocks + g.splits - 1) / g.splits;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::kStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], SRC == kNibbles ? 1 + 4 : 1);  // MMAs done; int4: the raw tile is free once expanded
+    }
+    for (int a = 0; a < 4; ++a) {
+      mbar_init(&tfull_bar[a], 1);
+      mbar_init(&tempty_bar[a], 128);
+      mbar_init(&ready_bar[a], 4);   // one lane of each of the four warps of an expanding group
+      mbar_init(&afree_bar[a], 1);
+    }
+    *s_abort = 0;
+    mbar_fence_init();
+    if (SRC != kChunks) tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, S::kCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------ producer ------------------------------
+    if (lane == 0) {
+      // bytes of weights a stage receives: the rows of the last tile may run out (bulk copies only;
+      // tensor copies fill with zeros)
+      auto a_bytes = [&](int ta) {
+        return SRC == kChunks ? 8 * 16 * min(kQRows, g.n - ta * kQRows) : S::kStageA;
+      };
+      auto load_a = [&](uint32_t dst, uint64_t* bar, int kb, int ta) {
+        if constexpr (SRC == kRows) {
+          tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), kb * kQK, ta * kQRows, kHintEvictFirst);
+        } else if constexpr (SRC == kNibbles) {
+          tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), ta * kQRows, kb * (kQK / 8), kHintEvictFirst);
+        } else {
+          const uint32_t bytes = 16u * uint32_t(min(kQRows, g.n - ta * kQRows));
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            bulk_load_s(dst + c * (kQRows * 16),
+                        g.w + (size_t(kb * 8 + c) * g.n + size_t(ta) * kQRows) * 16, bytes, smem_u32(bar),
+                        kHintEvictFirst);
+        }
+      };
+      // the first lap of weight tiles is requested before the kernels ahead have finished
+      int pre = 0;
+      for (int u = blockIdx.x; u < units && pre < S::kStages; u += gridDim.x) {
+        const int tile = u / g.splits, sp = u - tile * g.splits, ta = tile / g.tiles_b;
+        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+        for (int kb = kb0; kb < kb1 && pre < S::kStages; ++kb, ++pre) {
+          mbar_expect_tx(&full_bar[pre], a_bytes(ta) + S::kStageB);
+          load_a(ring + pre * S::kStage, &full_bar[pre], kb, ta);
+        }
+      }
+      pdl_wait();
+      int stage = 0, armed = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const int tile = u / g.splits, sp = u - tile * g.splits;
+        const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
+        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (*s_abort && armed >= pre) {
+            ok = false;
+            break;
+          }
+          const uint32_t dst = ring + stage * S::kStage;
+          if (armed >= pre) {
+            if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort)) {
+              ok = false;
+              break;
+            }
+            mbar_expect_tx(&full_bar[stage], a_bytes(ta) + S::kStageB);
+            load_a(dst, &full_bar[stage], kb, ta);
+          }
+          tma_load_2d_hint_s(dst + S::kStageA, &tmap_x, smem_u32(&full_bar[stage]), kb * kQK, tb * S::BN, kHintEvictLast);
+          ++armed;
+          if (++stage == S::kStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+      if (!ok) {
+        // copies still in flight land before the CTA goes away
+        const int n = armed < S::kStages ? armed : S::kStages;
+        int s = stage;
+        uint32_t ph = phase;
+        for (int i = 0; i < n; ++i) {
+          if (--s < 0) {
+            s = S::kStages - 1;
+            ph ^= 1u;
+          }
+          for (uint32_t p = 0; p < (1u << 20); ++p)
+            if (mbar_try_wait(&full_bar[s], ph)) break;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer ----------------------------
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_i8(kQRows, S::BN);
+      int stage = 0, nkb = 0, accs = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+        const int sp = u % g.splits;
+        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+        for (int kb = kb0; kb < kb1; ++kb, ++nkb) {
+          if (GROUPED || kb == kb0) {
+            if (kb != kb0 || u != int(blockIdx.x)) ++accs;
+            if (!mbar_wait_bounded(&tempty_bar[accs % S::kAcc], (uint32_t(accs / S::kAcc) & 1u) ^ 1u, s_abort)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after_sync();
+          }
+          const uint32_t d_tmem = tmem_base + uint32_t((accs % S::kAcc) * S::BN);
+          // int4: the expanding threads have waited for the stage, but the digits are read here too
+          if (!mbar_wait_bounded(&full_bar[stage], phase, s_abort)) {
+            ok = false;
+            break;
+          }
+          if (SRC == kNibbles && !mbar_wait_bounded(&ready_bar[nkb & 3], uint32_t(nkb >> 2) & 1u, s_abort)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t sa = SRC == kNibbles ? ring_a8 + (nkb & 3) * kQTileA : ring + stage * S::kStage;
+          const uint64_t da = SRC == kRows ? umma_desc_k_sw128(sa) : umma_desc_k_chunks(sa);
+          const uint64_t db = umma_desc_k_sw128(ring + stage * S::kStage + S::kStageA);
+          // 32 bytes along K per instruction: +2 (16-byte units) inside a swizzled row, two chunks otherwise
+          constexpr int kStepA = SRC == kRows ? 2 : 2 * (kQRows * 16) / 16;
+#pragma unroll
+          for (int k = 0; k < kQK / 32; ++k)
+            umma_i8_ss(d_tmem, da + uint64_t(kStepA * k), db + uint64_t(2 * k), idesc,
+                       ((!GROUPED && kb > kb0) || k > 0) ? 1u : 0u);
+          if (SRC == kNibbles) umma_commit(&afree_bar[nkb & 3]);
+          umma_commit(&empty_bar[stage]);
+          if (GROUPED || kb + 1 == kb1) umma_commit(&tfull_bar[accs % S::kAcc]);
+          if (++stage == S::kStages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+        }
+      }
+    }
+  } else if (SRC == kNibbles && warp >= 6) {
+    // ------------------------ int4 -> int8 -------------------------------
+    // Two groups of 128 threads take alternate k-blocks; a thread expands one weight row: 16 words in
+    // (consecutive lanes, consecutive words), eight 16-byte chunks out (consecutive lanes,
+    // consecutive chunks): no bank conflicts on either side.
+    const int ct = threadIdx.x - 192, grp = ct >> 7, row = ct & 127;
+    int nkb = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int tile = u / g.splits, sp = u - tile * g.splits;
+      const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+      const int grow = min((tile / g.tiles_b) * kQRows + row, g.n - 1);
+      const uint32_t* zp = g.zeros + (grow >> 3);
+      auto zero_of = [&](int kb) { return (__ldg(zp + size_t(kb / g.gk) * (g.n >> 3)) >> ((grow & 7) * 4)) & 15u; };
+      // this group's k-blocks of the unit: first, first + 2, ...; the zero points are read two ahead
+      const int first = kb0 + ((nkb & 1) != grp ? 1 : 0);
+      uint32_t z0 = first < kb1 ? zero_of(first) : 0u, z1 = first + 2 < kb1 ? zero_of(first + 2) : 0u;
+      for (int kb = first; kb < kb1 && ok; kb += 2) {
+        const int b = nkb + (kb - kb0), stage = b % S::kStages;
+        const uint32_t z = z0;
+        z0 = z1;
+        z1 = kb + 4 < kb1 ? zero_of(kb + 4) : 0u;
+        if (!mbar_wait_bounded(&full_bar[stage], uint32_t(b / S::kStages) & 1u, s_abort) ||
+            !mbar_wait_bounded(&afree_bar[b & 3], (uint32_t(b >> 2) & 1u) ^ 1u, s_abort)) {
+          ok = false;
+          break;
+        }
+        const uint32_t src = ring + stage * S::kStage + row * 4;
+        const uint32_t dst = ring_a8 + (b & 3) * kQTileA + row * 16;
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i]) : "r"(src + i * (kQRows * 4)));
+        // byte = (128 + nibble - zero) without borrow between bytes, then the sign bit flipped
+        const uint32_t zz = z * 0x01010101u;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint32_t o[4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t v = w[2 * c + h];
+            o[2 * h] = (((v & 0x0F0F0F0Fu) | 0x80808080u) - zz) ^ 0x80808080u;
+            o[2 * h + 1] = ((((v >> 4) & 0x0F0F0F0Fu) | 0x80808080u) - zz) ^ 0x80808080u;
+          }
+          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + c * (kQRows * 16)), "r"(o[0]), "r"(o[1]),
+                       "r"(o[2]), "r"(o[3])
+                       : "memory");
+        }
+        fence_proxy_async_smem();  // the tensor core reads what these threads just wrote
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&ready_bar[b & 3]);
+          mbar_arrive(&empty_bar[stage]);  // raw words consumed (the MMAs' commit frees the digits)
+        }
+      }
+      nkb += kb1 - kb0;
+    }
+  } else {
+    // ------------------------------ epilogue ------------------------------
+    const int q = warp & 3, row = q * 32 + lane;
+    pdl_wait();
+    int accs = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int tile = u / g.splits, sp = u - tile * g.splits;
+      const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
+      const int n = ta * kQRows + row, m0 = tb * TB;
+      const bool nok = n < g.n;
+      const int nn = nok ? n : g.n - 1;
+      // one accumulator set read as fp32: columns c0 .. c0+15 of every digit plane put together
+      auto read16 = [&](int acc, int c0, float (&v)[16]) {
+        const uint32_t t = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(acc * S::BN + c0);
+        if constexpr (ND == 1) {
+          uint32_t r[16];
+          tmem_ld_32x16(t, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = float(int32_t(r[i]));
+        } else {
+          uint32_t r0[16], r1[16], r2[16];
+          tmem_ld_32x16(t, r0);
+          tmem_ld_32x16(t + TB, r1);
+          tmem_ld_32x16(t + 2 * TB, r2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            v[i] = fmaf(float(int32_t(r2[i])), 1.f / 65536.f,
+                        fmaf(float(int32_t(r1[i])), 1.f / 256.f, float(int32_t(r0[i]))));
+        }
+      };
+      float rs = 1.f;  // what is left to multiply with once the sums are there
+      float accf[GROUPED ? TB : 1];
+      int done_acc = 0;
+      if constexpr (GROUPED) {
+        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+        auto scale_of = [&](int kb) -> float {
+          if (!nok || kb >= kb1) return 0.f;
+          const int gi = kb / g.gk;
+          switch (g.scale_kind) {
+            case BL_QSCALE_BF16_NG: return __bfloat162float(static_cast<const __nv_bfloat16*>(g.scale)[size_t(n) * g.groups + gi]);
+            case BL_QSCALE_F16_NG: return __half2float(static_cast<const __half*>(g.scale)[size_t(n) * g.groups + gi]);
+            case BL_QSCALE_F32_GN: return __ldg(static_cast<const float*>(g.scale) + size_t(gi) * g.n + n);
+            default: return __half2float(static_cast<const __half*>(g.scale)[size_t(gi) * g.n + n]);
+          }
+        };
+        if (g.row_scale) rs = __bfloat162float(g.row_scale[nn]);
+#pragma unroll
+        for (int i = 0; i < TB; ++i) accf[i] = 0.f;
+        float sq[4];  // scales of the next four k-blocks are on their way while this one is waited for
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sq[i] = scale_of(kb0 + i);
+        for (int kb = kb0; kb < kb1 && ok; kb += 4) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (kb + i >= kb1 || !ok) break;
+            const float sc = sq[i];
+            sq[i] = scale_of(kb + i + 4);
+            const int acc = accs % S::kAcc;
+            if (!mbar_wait_bounded(&tfull_bar[acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) {
+              ok = false;
+              break;
+            }
+            ++accs;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int c0 = 0; c0 < TB; c0 += 16) {
+              float v[16];
+              read16(acc, c0, v);
+#pragma unroll
+              for (int j = 0; j < 16; ++j) accf[c0 + j] = fmaf(v[j], sc, accf[c0 + j]);
+            }
+            tc_fence_before_sync();
+            mbar_arrive(&tempty_bar[acc]);
+          }
+        }
+        if (!ok) break;
+      } else {
+        rs = __bfloat162float(static_cast<const __nv_bfloat16*>(g.scale)[nn]);
+        done_acc = accs % S::kAcc;
+        if (!mbar_wait_bounded(&tfull_bar[done_acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) break;
+        ++accs;
+        tc_fence_after_sync();
+      }
+      const float bv = (nok && g.bias && !g.slabs) ? __bfloat162float(g.bias[n]) : 0.f;
+      float* slab = g.slabs ? g.slabs + size_t(sp) * g.m * g.n : nullptr;
+#pragma unroll
+      for (int c0 = 0; c0 < TB; c0 += 16) {
+        float v[16];
+        if constexpr (GROUPED) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) v[j] = accf[c0 + j];
+        } else {
+          read16(done_acc, c0, v);
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int m = m0 + c0 + j;
+          const bool mok = m < g.m;
+          const float y = v[j] * ((mok ? __ldg(g.xs + m) : 0.f) * rs);
+          if (slab) {
+            if (mok && nok) __stcg(slab + size_t(m) * g.n + n, y);
+          } else if (g.silu) {
+            // even lanes hold gate rows, odd lanes the matching up rows
+            const float mine = y + bv;
+            const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
+            if (mok && nok && !(row & 1))
+              g.out[size_t(m) * g.ldo + (n >> 1)] = __float2bfloat16(mine / (1.f + __expf(-mine)) * other);
+          } else if (mok && nok) {
+            g.out[size_t(m) * g.ldo + n] = __float2bfloat16(y + bv);
+          }
+        }
+      }
+      if constexpr (!GROUPED) {
+        tc_fence_before_sync();
+        mbar_arrive(&tempty_bar[done_acc]);
+      }
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, S::kCols);
+  }
+  if (threadIdx.x == 0 && *s_abort && g.err) *g.err = 1u;
+}
+
+// ---------------------------------------------------------------------------
+// activations -> digits
+// ---------------------------------------------------------------------------
+// x [m][k] bf16 -> xq [ceil(m/tb)][3][tb][k] int8 and xs[m]: x = xs * (d0 + d1/2^8 + d2/2^16).  xs is a
+// power of two chosen from the row's largest element so that d0 fits 8 bits.  One block per token; the
+// row stays in registers between the two passes.
+constexpr int kDigThreads = 512;
+constexpr int kDigVec = 8;   // 16-byte vectors per thread: rows of up to 32768 elements
+__device__ __forceinline__ uint32_t bf16x2_absmax_bits(uint32_t m, uint32_t v) {
+  m = max(m, v & 0x7fffu);
+  return max(m, (v >> 16) & 0x7fffu);
+}
+template <bool PERMUTE>
+__global__ void __launch_bounds__(kDigThreads) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k,
+                                                              int tb, int8_t* __restrict__ xq,
+                                                              float* __restrict__ xs) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ uint32_t s_max[kDigThreads / 32];
+  const int row = blockIdx.x, vecs = k >> 3;
+  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx);
+  uint4 v[kDigVec];
+  uint32_t mx = 0;  // largest |x| as bf16 bits: ordered like the values, NaN above infinity
+#pragma unroll
+  for (int i = 0; i < kDigVec; ++i) {
+    const int c = threadIdx.x + i * kDigThreads;
+    if (c < vecs) {
+      v[i] = xr[c];
+      mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].x), v[i].y);
+      mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].z), v[i].w);
+    }
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = 0;
+#pragma unroll
+  for (int i = 0; i < kDigThreads / 32; ++i) mx = max(mx, s_max[i]);
+  // |x| < 2^ex; a largest element of 255/256 * 2^ex would round up to 128 in the first digit
+  int ex = int(mx >> 7) - 126 + ((mx & 0x7fu) == 0x7fu ? 1 : 0);
+  if (ex < -110) ex = -110;
+  const bool bad = mx >= 0x7f80u;  // infinity or NaN in the row: the whole row of results is NaN
+  const float scale = bad ? 0.f : __uint_as_float(uint32_t(127 + 7 - ex) << 23);
+  if (threadIdx.x == 0)
+    xs[row] = bad ? __uint_as_float(0x7fffffffu) : __uint_as_float(uint32_t(127 - 7 + ex) << 23);
+  int8_t* base = xq + (size_t(row / tb) * 3 * tb + row % tb) * size_t(k);
+#pragma unroll
+  for (int i = 0; i < kDigVec; ++i) {
+    const int c = threadIdx.x + i * kDigThreads;
+    if (c >= vecs) continue;
+    const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+    uint32_t o[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float f = __uint_as_float((j & 1) ? (w[j >> 1] & 0xffff0000u) : (w[j >> 1] << 16));
+      const float y0 = bad ? 0.f : f * scale;
+      // every step leaves a remainder in [-128.5, 127.5) / 256, so that the next digit fits too
+      const float d0 = floorf(y0 + 128.5f / 256.f);
+      const float y1 = (y0 - d0) * 256.f;
+      const float d1 = fminf(floorf(y1 + 128.5f / 256.f), 127.f);
+      const float y2 = (y1 - d1) * 256.f;
+      const float d2 = fminf(rintf(y2), 127.f);
+      const int pos = PERMUTE ? ((j & 1) * 4 + (j >> 1)) : j;
+      const int sh = 8 * (pos & 3);
+      o[0][pos >> 2] |= (uint32_t(int(d0)) & 0xffu) << sh;
+      o[1][pos >> 2] |= (uint32_t(int(d1)) & 0xffu) << sh;
+      o[2][pos >> 2] |= (uint32_t(int(d2)) & 0xffu) << sh;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      *reinterpret_cast<uint2*>(base + size_t(d) * tb * k + size_t(c) * 8) = make_uint2(o[d][0], o[d][1]);
+  }
+}
+
+// fp32 slabs [split][m][n] -> bf16: sum in split order, + bias, optionally SiLU*mul over interleaved
+// (gate, up) columns.  Eight columns per thread.
+__global__ void __launch_bounds__(256) k_slab_finish(const float* __restrict__ slabs, int nsplit, size_t slab, int n,
+                                                     const __nv_bfloat16* __restrict__ bias, int silu,
+                                                     __nv_bfloat16* __restrict__ out, int ldo, size_t total8) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (t >= total8) return;
+  const int per = n >> 3;
+  const size_t m = t / per;
+  const int c = int(t - m * per) * 8;
+  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  sum_slabs8(slabs + m * n + c, slab, nsplit, a);
+  if (bias) {
+    const uint4 b = *reinterpret_cast<const uint4*>(bias + c);
+    const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y), b2 = unpack_bf16x2(b.z), b3 = unpack_bf16x2(b.w);
+    a[0] += b0.x; a[1] += b0.y; a[2] += b1.x; a[3] += b1.y;
+    a[4] += b2.x; a[5] += b2.y; a[6] += b3.x; a[7] += b3.y;
+  }
+  if (silu) {
+    float o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = a[2 * j] / (1.f + __expf(-a[2 * j])) * a[2 * j + 1];
+    *reinterpret_cast<uint2*>(out + m * ldo + (c >> 1)) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+  } else {
+    *reinterpret_cast<uint4*>(out + m * ldo + c) = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]),
+                                                              pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
+  }
+}
+
+template <int SRC, int ND, int TB, bool GROUPED>
+static int launch_qlin(const blQlinArgs& a, cudaStream_t st, char* err, size_t errlen) {
+  using S = QlinCfg<SRC, ND, TB, GROUPED>;
+  CUtensorMap tw, tx;
+  const int tiles_b = (a.m + TB - 1) / TB;
+  // digit planes are laid out tile by tile, dense; single-digit activations are plain rows
+  const uint64_t xrows = ND == 1 ? uint64_t(a.m) : uint64_t(tiles_b) * S::BN;
+  if (make_tmap_kmajor(a.xq, xrows, a.k, a.k, S::BN, 1, &tx, err, errlen, kQK) != 0) return -1;
+  if (SRC == kRows) {
+    if (make_tmap_kmajor(a.w, a.n, a.k, a.k, kQRows, 1, &tw, err, errlen, kQK) != 0) return -1;
+  } else if (SRC == kNibbles) {
+    const DriverApi* d = driver(err, errlen);
+    if (!d) return -1;
+    cuuint64_t dims[2] = {cuuint64_t(a.n), cuuint64_t(a.k / 8)};
+    cuuint64_t strides[1] = {cuuint64_t(a.n) * 4};
+    cuuint32_t box[2] = {kQRows, kQK / 8}, estr[2] = {1, 1};
+    if (d->cuTensorMapEncodeTiled(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(a.w), dims, strides, box,
+                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+      set_err(err, errlen, "barlink: tensor map of the packed int4 weight failed (n %d, k %d)", a.n, a.k);
+      return -1;
+    }
+  } else {
+    tw = tx;  // not used
+  }
+  QlinShape g;
+  memset(&g, 0, sizeof(g));
+  g.n = a.n;
+  g.m = a.m;
+  g.k = a.k;
+  g.tiles_a = (a.n + kQRows - 1) / kQRows;
+  g.tiles_b = tiles_b;
+  g.kblocks = (a.k + kQK - 1) / kQK;
+  g.splits = a.splits;
+  g.w = static_cast<const uint8_t*>(a.w);
+  g.zeros = static_cast<const uint32_t*>(a.zeros);
+  g.xs = static_cast<const float*>(a.xs);
+  g.scale_kind = a.scale_kind;
+  g.scale = a.scale;
+  g.row_scale = static_cast<const __nv_bfloat16*>(a.row_scale);
+  g.gk = GROUPED ? a.group_k / kQK : 1;
+  g.groups = GROUPED ? a.k / a.group_k : 1;
+  g.bias = static_cast<const __nv_bfloat16*>(a.bias);
+  g.out = static_cast<__nv_bfloat16*>(a.out);
+  g.ldo = a.ldo;
+  g.silu = a.silu_mul;
+  g.slabs = static_cast<float*>(a.slabs);
+  g.err = static_cast<uint32_t*>(a.err_flag);
+  const int units = g.tiles_a * g.tiles_b * g.splits;
+  const int grid = units < sm_count() ? units : sm_count();
+  static bool attr[64] = {};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_qlin<SRC, ND, TB, GROUPED>), S::kSmem, attr);
+  if (e == cudaSuccess)
+    e = launch_k(k_qlin<SRC, ND, TB, GROUPED>, dim3(grid), dim3(S::kThreads), size_t(S::kSmem), st, tw, tx, g);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: quantised linear launch failed: %s", cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+template <int SRC, int ND, bool GROUPED>
+static int launch_qlin_tb(const blQlinArgs& a, cudaStream_t st, char* err, size_t errlen) {
+  switch (bl_qlin_tile_tokens(a.m)) {
+    case 16: return launch_qlin<SRC, ND, 16, GROUPED>(a, st, err, errlen);
+    case 32: return launch_qlin<SRC, ND, 32, GROUPED>(a, st, err, errlen);
+    default: return launch_qlin<SRC, ND, 64, GROUPED>(a, st, err, errlen);
+  }
+}
+
+}  // namespace bl
+
+using namespace bl;
+
+extern "C" int bl_qlin_tile_tokens(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : 64; }
+
+// Work is dealt out in units of (row tile, token tile, k-split); the SMs take them lap by lap.  A lap
+// costs its k-blocks plus about two of hand-over, and every split adds a slab to write and to read.
+extern "C" int bl_qlin_splits(int n, int k, int m) {
+  const int tb = bl_qlin_tile_tokens(m);
+  const int tiles = ((n + kQRows - 1) / kQRows) * ((m + tb - 1) / tb), kb = (k + kQK - 1) / kQK, sms = sm_count();
+  int best = 1;
+  double cost = 1e30;
+  for (int s = 1; s <= 16 && s <= kb; ++s) {
+    const int per = (kb + s - 1) / s;
+    if ((kb + per - 1) / per != s) continue;  // an empty split
+    const int laps = (tiles * s + sms - 1) / sms;
+    const double c = laps * (per + 1.0) + (s > 1 ? 2.0 + 0.25 * s : 0.0);
+    if (c < cost - 1e-9) {
+      cost = c;
+      best = s;
+    }
+  }
+  return best;
+}
+
+extern "C" size_t bl_quant_digits_bytes(int m, int k) {
+  const int tb = bl_qlin_tile_tokens(m);
+  return size_t((m + tb - 1) / tb) * 3 * tb * size_t(k);
+}
+
+extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute, void* xq, void* xs, void* stream,
+                               char* err, size_t errlen) {
+  if (!x || !xq || !xs || m < 1 || k < 8 || (k & 7) || k > 8 * kDigVec * kDigThreads || (ldx & 7) ||
+      (reinterpret_cast<uintptr_t>(x) & 15u)) {
+    set_err(err, errlen, "barlink: quant_digits needs 16-byte aligned rows and K a multiple of 8, at most %d",
+            8 * kDigVec * kDigThreads);
+    return -1;
+  }
+  auto go = [&](auto kern) {
+    return launch_k(kern, dim3(m), dim3(kDigThreads), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const __nv_bfloat16*>(x), ldx, k, bl_qlin_tile_tokens(m), static_cast<int8_t*>(xq),
+                    static_cast<float*>(xs));
+  };
+  cudaError_t e = permute ? go(k_quant_digits<true>) : go(k_quant_digits<false>);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: quant_digits launch failed: %s", cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+extern "C" int bl_slab_finish(const void* slabs, int nsplit, int m, int n, const void* bias, int silu_mul, void* out,
+                              int ldo, void* stream, char* err, size_t errlen) {
+  if (!slabs || !out || nsplit < 1 || m < 1 || n < 8 || (n & 7) || (ldo & 7)) {
+    set_err(err, errlen, "barlink: slab_finish needs n and the output pitch in multiples of 8");
+    return -1;
+  }
+  const size_t total8 = size_t(m) * (n / 8);
+  cudaError_t e = launch_k(k_slab_finish, dim3(unsigned((total8 + 255) / 256)), dim3(256), 0,
+                           static_cast<cudaStream_t>(stream), static_cast<const float*>(slabs), nsplit, size_t(m) * n, n,
+                           static_cast<const __nv_bfloat16*>(bias), silu_mul, static_cast<__nv_bfloat16*>(out), ldo,
+                           total8);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: slab_finish launch failed: %s", cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+extern "C" int bl_qlin(const blQlinArgs* a, void* stream, char* err, size_t errlen) {
+  const bool grouped = a && a->scale_kind != BL_QSCALE_BF16_N;
+  if (!a || !a->w || !a->xq || !a->xs || !a->scale || (!a->out && !a->slabs) || a->m < 1 || a->m > BL_QLIN_MAX_TOKENS ||
+      a->n < 1 || a->k < 16 || (a->k & 15) || (a->digits != 1 && a->digits != 3)) {
+    set_err(err, errlen, "barlink: qlin needs weights, activations with 1 or 3 digits, scales, an output, 1..%d tokens and K a multiple of 16",
+            BL_QLIN_MAX_TOKENS);
+    return -1;
+  }
+  // 32-bit sums: |weight| <= 128, |digit| <= 128
+  if (!grouped && a->k > 131072) {
+    set_err(err, errlen, "barlink: qlin sums at most 131072 products per accumulator (k %d)", a->k);
+    return -1;
+  }
+  if (grouped && (a->group_k < kQK || a->group_k % kQK || a->k % a->group_k)) {
+    set_err(err, errlen, "barlink: qlin group sizes are multiples of %d that divide K", kQK);
+    return -1;
+  }
+  if ((a->src == kChunks && (a->k % kQK || a->digits != 1 || !grouped)) ||
+      (a->src == kNibbles && (a->k % kQK || a->digits != 3 || !grouped || !a->zeros || (a->n & 7)))) {
+    set_err(err, errlen, "barlink: qlin: this weight form needs K a multiple of %d and group scales", kQK);
+    return -1;
+  }
+  const int kb = (a->k + kQK - 1) / kQK;
+  const int per = a->splits > 0 ? (kb + a->splits - 1) / a->splits : 0;
+  if (a->splits < 1 || (kb + per - 1) / per != a->splits || (a->splits > 1 && !a->slabs)) {
+    set_err(err, errlen, "barlink: qlin: %d k-splits of %d k-blocks (every split needs one, and slabs to go to)", a->splits, kb);
+    return -1;
+  }
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (a->src == kChunks) return launch_qlin_tb<kChunks, 1, true>(*a, st, err, errlen);
+  if (a->src == kNibbles) return launch_qlin_tb<kNibbles, 3, true>(*a, st, err, errlen);
+  if (grouped)
+    return a->digits == 1 ? launch_qlin_tb<kRows, 1, true>(*a, st, err, errlen)
+                          : launch_qlin_tb<kRows, 3, true>(*a, st, err, errlen);
+  return a->digits == 1 ? launch_qlin_tb<kRows, 1, false>(*a, st, err, errlen)
+                        : launch_qlin_tb<kRows, 3, false>(*a, st, err, errlen);
+}

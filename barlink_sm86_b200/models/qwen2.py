@@ -106,8 +106,10 @@ class W4Weight:
 
 def qlinear(x, w, bias=None, silu_mul=False, split=False):
     """x @ w.T for any stored form of w (plain / tiled bf16, W8Weight, W4Weight).
-    split=True allows the k-split slab output of the bf16 decode GEMM."""
+    split=True allows the k-split slab output of the bf16 and int8 decode linears."""
     if isinstance(w, W8Weight):
+        if split and not silu_mul:
+            return ops.w8a16_linear_split(x, w.wq, w.scale, bias)
         return ops.w8a16_linear(x, w.wq, w.scale, bias, silu_mul)
     if isinstance(w, W4Weight):
         y = ops.w4a16_linear(x, w.qw, w.sc, w.qz, w.group)
@@ -298,9 +300,10 @@ class Qwen2Model:
             else:
                 normed, res = ops.rmsnorm(h, L["ln1"], cfg.eps, res)
             if w.quant != "none":
-                qkv = qlinear(normed, L["wqkv"], L["bqkv"])
-                a = attn_factory(li)(qkv, None)
-                h = qlinear(a, L["wo"])
+                # decode: as below, a k-split leaves fp32 slabs for the next kernel (which adds the bias)
+                qkv = qlinear(normed, L["wqkv"], L["bqkv"], split=split_k)
+                a = attn_factory(li)(qkv, L["bqkv"] if qkv.dim() == 3 else None)
+                h = qlinear(a, L["wo"], split=split_k)
             elif split_k:
                 # decode: k-split linears leave fp32 slabs that the next kernel sums
                 qkv = ops.linear_split(normed, L["wqkv"])

@@ -272,15 +272,15 @@ def w8_act_mode():
 def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
     """scale [n]: per output channel.  scale [n, k/group] or a W8GroupScales: per group, the
     reference's granularity (torch_ext/barlink_sm86/w8a16.cu:119-142 applies group scales inside
-    its K loop; so does the tcgen05 kernel here, in the warps that widen the int8 tile).  Group
-    sizes that are not multiples of 64, and more than 256 tokens, widen the weight once and run
-    the bf16 GEMM.
+    its K loop).  Up to 128 tokens the int8 weights go to the tensor cores as they are, against three
+    int8 digits of the bf16 activations (csrc/qlin_kernels.cu: no loss against bf16 operands); group
+    scales, for groups of a multiple of 128, are applied to the sums of a k-block.  Groups of 64 and
+    129..256 tokens widen the tile inside the main loop; other groups, and more than 256 tokens,
+    widen the weight once and run the bf16 GEMM.
 
-    act="int8" (per-channel scales only): the activations are quantised per token to int8 first,
-    as the reference does (w8a16.cu:37-92 there), and the product runs as `tcgen05.mma kind::i8`
-    with int32 accumulators: the weights go from HBM to the tensor cores without being widened, for
-    any number of tokens; with group scales [n, k/group] (group a multiple of 128, at most 64 tokens)
-    every k-block is accumulated on its own and the epilogue warps apply the scales.  act=None takes
+    act="int8": the activations are quantised per token to int8 first, as the reference does
+    (w8a16.cu:37-92 there), one digit instead of three, for any number of tokens with per-channel
+    scales, and for at most 64 tokens and 148 * 128 rows upwards with group scales.  act=None takes
     `w8_act_mode()`."""
     if x.is_cuda:
         k = wq.shape[1]
@@ -289,13 +289,17 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
             if scale.dim() == 1:
                 _count(2)
                 return _C().w8a16_linear(x, wq, scale, bias, silu_mul, act_int8=True)
-            # (no k-split in that form: it pays from one 128-row tile per SM upwards; below, the widening form)
+            # smaller layers keep the bf16 activations: there the exact form costs the same
             if x.shape[0] <= 64 and (k // scale.shape[1]) % 128 == 0 and wq.shape[0] >= 148 * 128:
                 # group scales (the reference's checkpoint format): one accumulator per k-block,
                 # scaled and summed by the epilogue warps
                 _count(2)
                 return _C().w8a16_linear(x, wq, scale, bias, silu_mul, act_int8=True, group_scale=scale.contiguous())
         if gs is None and scale.dim() == 2:
+            if (k // scale.shape[1]) % 128 == 0 and _qlin_rows(x):
+                # groups of whole k-blocks: the scales as they are, applied to the k-blocks' sums
+                _count(2)
+                return _C().w8a16_linear(x, wq, scale, bias, silu_mul, group_scale=scale.contiguous())
             if (k // scale.shape[1]) % 64 == 0 and x.shape[0] <= 256:
                 _count()
                 gs = prepare_w8_scales(scale, k)
@@ -314,7 +318,23 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
     return ref.w8a16_linear(x, wq, scale, bias, silu_mul)
 
 
+def _qlin_rows(x):
+    """Rows that the int8-digit decode kernel takes (csrc/qlin_kernels.cu)."""
+    return (x.dim() == 2 and 1 <= x.shape[0] <= 128 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and x.shape[1] % 16 == 0 and x.shape[1] <= 32768)
+
+
+def w8a16_linear_split(x, wq, scale, bias=None):
+    """Decode-path form of `w8a16_linear` (per-channel scales): when the shape wants a k-split, fp32 slabs
+    [splits, tokens, n] whose sum is the product WITHOUT the bias, which the consumer adds (see
+    `linear_split`); else the bf16 result with the bias."""
+    if x.is_cuda and _qlin_rows(x):
+        _count(2)
+        return _C().w8a16_linear_split(x, wq, scale, bias, w8_act_mode() == "int8")
+    return w8a16_linear(x, wq, scale, bias)
+
+
 __all__ = [
     "linear", "linear_split", "k_splits", "TiledWeight", "tile_weight", "untile_weight", "rmsnorm", "rope_kv_write", "rope", "silu_mul", "embedding", "argmax",
-    "paged_attn_decode", "rope_attn_decode", "attention", "w8a16_linear", "W8GroupScales", "prepare_w8_scales", "w4a16_linear", "qknorm_rope", "layernorm_modulate", "gate_residual", "ref",
+    "paged_attn_decode", "rope_attn_decode", "attention", "w8a16_linear", "w8a16_linear_split", "W8GroupScales", "prepare_w8_scales", "w4a16_linear", "qknorm_rope", "layernorm_modulate", "gate_residual", "ref",
 ]

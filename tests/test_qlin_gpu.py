@@ -1,0 +1,100 @@
+# SPDX-License-Identifier: MIT
+"""Decode linears on quantised weights (csrc/qlin_kernels.cu) at the edges of their tiles.
+
+Oracle: the exact integer products in float64.  Tolerances: the bf16 result is rounded once (rel-L2 at
+most 2^-9 / sqrt(3) per element on average, 2^-8 allowed); fp32 slabs carry the int32 -> fp32 conversions
+and their sum only (2^-24 each; 2^-20 allowed).  Digits: exact down to 2^-15 of a row's largest element."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_l2(a, b):
+    a, b = a.double(), b.double()  # rows here go up to 1e31: squares need the range of a double
+    return float((a - b).norm() / b.norm().clamp_min(1e-300))
+
+
+TOL, TOL32 = 2.0 ** -8, 2.0 ** -20
+
+
+def _g(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def _x(m, k, seed, spread=False):
+    x = torch.randn(m, k, generator=_g(seed), device="cuda")
+    if spread:  # outliers and small elements in one row, as activations have
+        x = x * torch.exp2(torch.randint(-6, 7, (m, k), generator=_g(seed + 1), device="cuda").float())
+    return x.bfloat16()
+
+
+def _w8(n, k, seed):
+    wq = torch.randint(-127, 128, (n, k), generator=_g(seed), device="cuda", dtype=torch.int32).to(torch.int8)
+    return wq, (torch.rand(n, generator=_g(seed + 1), device="cuda") * 0.01 + 1e-3).bfloat16()
+
+
+# tokens: edges of the 16 / 32 / 64-token tiles; n: a ragged last row tile; k: a ragged last k-block
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("n,k", [(128, 128), (200, 1040), (1000, 3584)])
+def test_int8_weights_bf16_activations(ext, m, n, k):
+    wq, sc = _w8(n, k, 3)
+    x = _x(m, k, 5, spread=True)
+    b = torch.randn(n, generator=_g(9), device="cuda").bfloat16()
+    prod = (x.double() @ wq.double().t()) * sc.double()
+    assert rel_l2(ext.w8a16_linear(x, wq, sc), prod) < TOL
+    assert rel_l2(ext.w8a16_linear(x, wq, sc, b), prod + b.double()) < TOL
+    y = prod + b.double()
+    silu = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+    assert rel_l2(ext.w8a16_linear(x, wq, sc, b, True), silu) < TOL
+    out = ext.w8a16_linear_split(x, wq, sc)
+    if out.dim() == 3:
+        assert rel_l2(out.double().sum(0), prod) < TOL32
+    kb = -(-k // 128)
+    for splits in {1, 2, 5, kb}:
+        if n % 8 == 0 and splits <= kb:
+            assert rel_l2(ext.w8a16_linear(x, wq, sc, b, splits=splits), prod + b.double()) < TOL
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
+
+
+@pytest.mark.parametrize("m", [1, 32, 64])
+@pytest.mark.parametrize("n,k,group", [(200, 1024, 128), (129, 768, 256)])
+@pytest.mark.parametrize("act_int8", [False, True])
+def test_int8_weights_group_scales(ext, m, n, k, group, act_int8):
+    from barlink_sm86_b200 import ops
+    wq, _ = _w8(n, k, 3)
+    gs = (torch.rand(n, k // group, generator=_g(4), device="cuda") * 0.01 + 1e-3).bfloat16()
+    x = _x(m, k, 5)
+    if act_int8:
+        xq, xs = ext.w8a16_quant_act(x)
+        w = ops.ref.w8_dequant(wq, gs).double()
+        want = (xq.double() @ w.t()) * xs.double()[:, None]
+        got = ext.w8a16_linear(x, wq, gs, act_int8=True, group_scale=gs)
+    else:
+        s = ops.prepare_w8_scales(gs, k)
+        w = ops.ref.w8_dequant(wq, s.rel.float() * s.row.float()[:, None]).double()
+        want = x.double() @ w.t()
+        got = ext.w8a16_linear(x, wq, s.row, group_rel=s.rel)
+    assert rel_l2(got, want) < TOL
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
+
+
+def test_activation_rows_with_extreme_values(ext):
+    """Zeros, tiny and huge rows, one outlier; a NaN or an infinity spoils its own row only."""
+    wq, sc = _w8(136, 256, 7)
+    x = _x(8, 256, 8)
+    x[0] = 0
+    x[1] *= 1e-30
+    x[2] *= 1e30
+    x[3, 7] = 3e4
+    x[4] = 255.0 / 256  # largest mantissa
+    x[5, 3] = float("nan")
+    x[6, 3] = float("inf")
+    y = ext.w8a16_linear(x, wq, sc)
+    want = (x.double() @ wq.double().t()) * sc.double()
+    for r in (1, 2, 3, 4, 7):
+        assert rel_l2(y[r].double(), want[r]) < TOL, r
+    assert float(y[0].abs().max()) == 0.0
+    assert not torch.isfinite(y[5]).any() and not torch.isfinite(y[6]).any()

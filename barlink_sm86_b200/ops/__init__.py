@@ -296,10 +296,6 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
                 _count(2)
                 return _C().w8a16_linear(x, wq, scale, bias, silu_mul, act_int8=True, group_scale=scale.contiguous())
         if gs is None and scale.dim() == 2:
-            if (k // scale.shape[1]) % 128 == 0 and _qlin_rows(x):
-                # groups of whole k-blocks: the scales as they are, applied to the k-blocks' sums
-                _count(2)
-                return _C().w8a16_linear(x, wq, scale, bias, silu_mul, group_scale=scale.contiguous())
             if (k // scale.shape[1]) % 64 == 0 and x.shape[0] <= 256:
                 _count()
                 gs = prepare_w8_scales(scale, k)

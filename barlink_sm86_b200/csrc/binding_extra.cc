@@ -209,21 +209,11 @@ bool qlin_takes(const at::Tensor& x, int k, bool act_int8) {
   return act_int8 ? k <= 131072
                   : k <= 32768 && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0;
 }
-// digits = 3: x as it is; digits = 1: x quantised to int8 per token.  want_slabs: fp32 [splits, m, n]
-// when the shape wants a k-split (bias is then the consumer's), else bf16 [m, n].
-at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10::optional<at::Tensor>& bias,
-                    bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
-  const int m = int(x.size(0));
-  at::Tensor xq, xs = at::empty({m}, x.options().dtype(at::kFloat));
-  if (digits == 3) {
-    xq = at::empty({int64_t(bl_quant_digits_bytes(m, q.k))}, x.options().dtype(at::kChar));
-    BL_CHECK(bl_quant_digits(x.data_ptr(), m, int(x.stride(0)), q.k, q.src == 2 ? 1 : 0, xq.data_ptr(), xs.data_ptr(), st,
-                             err, errlen));
-  } else {
-    at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
-    xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
-    BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
-  }
+// y = activations (xq, xs: int8 rows, or three digit planes) times q.  want_slabs: fp32 [splits, m, n]
+// when the shape wants a k-split (bias is then the consumer's), else bf16 [m, n].  like: options of x.
+at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int digits, const QWeight& q,
+                        const c10::optional<at::Tensor>& bias, bool silu_mul, int splits, bool want_slabs,
+                        const at::TensorOptions& like, void* err_flag, void* st) {
   if (bias) {
     check_bf16x(*bias, "bias");
     TORCH_CHECK(bias->numel() == q.n, "barlink: bias must have n entries");
@@ -245,10 +235,10 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
   a.err_flag = err_flag;
   at::Tensor slabs, out;
   if (splits > 1) {
-    slabs = at::empty({splits, m, q.n}, x.options().dtype(at::kFloat));
+    slabs = at::empty({splits, m, q.n}, like.dtype(at::kFloat));
     a.slabs = slabs.data_ptr();
   } else {
-    out = at::empty({m, silu_mul ? q.n / 2 : q.n}, x.options());
+    out = at::empty({m, silu_mul ? q.n / 2 : q.n}, like);
     a.out = out.data_ptr();
     a.ldo = int(out.size(1));
     a.bias = bias ? bias->data_ptr() : nullptr;
@@ -257,10 +247,26 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
   BL_CHECK(bl_qlin(&a, st, err, errlen));
   if (splits == 1) return out;
   if (want_slabs) return slabs;
-  out = at::empty({m, silu_mul ? q.n / 2 : q.n}, x.options());
+  out = at::empty({m, silu_mul ? q.n / 2 : q.n}, like);
   BL_CHECK(bl_slab_finish(slabs.data_ptr(), splits, m, q.n, bias ? bias->data_ptr() : nullptr, silu_mul ? 1 : 0,
                           out.data_ptr(), int(out.size(1)), st, err, errlen));
   return out;
+}
+// digits = 3: x as it is; digits = 1: x quantised to int8 per token
+at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10::optional<at::Tensor>& bias,
+                    bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
+  const int m = int(x.size(0));
+  at::Tensor xq, xs = at::empty({m}, x.options().dtype(at::kFloat));
+  if (digits == 3) {
+    xq = at::empty({int64_t(bl_quant_digits_bytes(m, q.k))}, x.options().dtype(at::kChar));
+    BL_CHECK(bl_quant_digits(x.data_ptr(), m, int(x.stride(0)), q.k, q.src == 2 ? 1 : 0, xq.data_ptr(), xs.data_ptr(), st,
+                             err, errlen));
+  } else {
+    at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
+    BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
+  }
+  return qlin_product(xq, xs, m, digits, q, bias, silu_mul, splits, want_slabs, x.options(), err_flag, st);
 }
 
 // Decode form of w8a16_linear without a reduction: fp32 slabs [splits, m, n] (scaled, no bias) for the
@@ -460,19 +466,19 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
   TORCH_CHECK(xs.is_contiguous() && xs.scalar_type() == at::kFloat && xs.numel() == m,
               "barlink w8a16_gemm: xs must be float32 [M]");
   TORCH_CHECK(m <= 16, "barlink w8a16_gemm: M > 16 is not supported by this decode kernel (use w8a16_linear)");
-  at::Tensor out = at::empty({m, N}, xq.options().dtype(at::kBFloat16));
-  at::Tensor ws;
-  void* wsp = nullptr;
-  if (S > 1) {
-    ws = at::empty({S, m, N}, xq.options().dtype(at::kFloat));
-    wsp = ws.data_ptr();
-  }
   c10::cuda::CUDAGuard guard(xq.device());
-  void* st = at::cuda::getCurrentCUDAStream(xq.device().index()).stream();
-  if (m > 0)
-    BL_CHECK(bl_w8a16_gemm(xq.data_ptr(), xs.data_ptr(), wq_t.data_ptr(), sw_t.data_ptr(), out.data_ptr(),
-                           m, int(N), int(K), int(S), wsp, st, err, errlen));
-  return out;
+  const int dev = xq.device().index();
+  void* st = at::cuda::getCurrentCUDAStream(dev).stream();
+  const auto like = xq.options().dtype(at::kBFloat16);
+  if (m == 0) return at::empty({0, N}, like);
+  // the tensor core takes the weights in this layout as they are (qlin_kernels.cu); S is the caller's
+  // k-split for the reference's kernel, here the shape decides
+  (void)S;
+  const bool aligned = (reinterpret_cast<uintptr_t>(xq.data_ptr()) & 15u) == 0;
+  QWeight q{wq_t.data_ptr(), 1, int(N), int(K), BL_QSCALE_F32_GN, sw_t.data_ptr()};
+  q.group_k = 128;
+  return qlin_product(aligned ? xq : xq.clone(), xs, m, 1, q, c10::nullopt, false, 0, false, like,
+                      w8_scratch(dev).err_flag.data_ptr(), st);
 }
 
 // GPTQ-v1 int4 linear: 1..16 rows use the GEMV; more rows widen the weight and use the bf16 GEMM

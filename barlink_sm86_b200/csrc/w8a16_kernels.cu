@@ -8,15 +8,15 @@
 //       y[m, n] = xs[m] * sum_g sw_t[g, n] * sum_{k in group g} xq[m, k] * w[n, k]
 //       wq_t int8 [K/16, N, 16] (k-chunk major), sw_t fp32 [K/128, N], M <= 16
 //
-// The product path of this library is bl_w8a16_linear (gemm_kernels.cu: bf16
-// activations, int8 weights widened inside a tcgen05 main loop); the pair
-// here exists for API parity and as the numerics cross-check of that kernel.
-// Differences from the reference's kernels: activations of a k-group are
-// staged in shared memory once per block, and the split over k-groups is
-// reduced in a fixed order (workspace + second kernel) instead of with
-// floating-point atomics, so results are reproducible run to run.
+// The product is bl_qlin (qlin_kernels.cu): the k-chunk-major weight layout is already an operand layout
+// of the tensor core (unswizzled K-major), so a k-block is eight bulk copies and int8 x int8 products
+// there, with the group scales applied per k-block.  The dp4a kernel that stood here (a thread per output
+// feature, loads waiting for one another) moved 1.0 TB/s of weights: four linears of a 32B layer at 8
+// tokens took 596 us, now 163 us.  A k-split is summed in a fixed order (the reference adds with
+// floating-point atomics), so results are reproducible run to run.
 #include <stdint.h>
 #include <stdio.h>
+#include <string.h>
 
 #include "bl_ops.h"
 #include "heap.h"
@@ -75,74 +75,6 @@ __global__ void __launch_bounds__(kQThreads) k_quant_act(const __nv_bfloat16* __
   }
 }
 
-// grid (ceil(N/256), S); thread = output feature n; group range of this split
-template <int MT>
-__global__ void __launch_bounds__(kQThreads) k_w8a8_gemm(const int8_t* __restrict__ wq_t,
-                                                         const float* __restrict__ sw_t,
-                                                         const int8_t* __restrict__ xq,
-                                                         const float* __restrict__ xs,
-                                                         __nv_bfloat16* __restrict__ out,
-                                                         float* __restrict__ ws, int M, int N, int K,
-                                                         int gper) {
-  pdl_launch_dependents();
-  pdl_wait();
-  __shared__ int s_x[MT][kGroup / 4];  // one k-group of every activation row, as dp4a words
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  const int G = K / kGroup;
-  const int g0 = blockIdx.y * gper, g1 = min(G, g0 + gper);
-  float acc[MT];
-#pragma unroll
-  for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-  for (int g = g0; g < g1; ++g) {
-    __syncthreads();
-    for (int t = threadIdx.x; t < MT * (kGroup / 4); t += blockDim.x) {
-      const int m = t / (kGroup / 4), w = t % (kGroup / 4);
-      s_x[m][w] = m < M ? *reinterpret_cast<const int*>(xq + size_t(m) * K + g * kGroup + w * 4) : 0;
-    }
-    __syncthreads();
-    if (n < N) {
-      int isum[MT];
-#pragma unroll
-      for (int m = 0; m < MT; ++m) isum[m] = 0;
-#pragma unroll
-      for (int c = 0; c < kGroup / 16; ++c) {
-        const int4 w = *reinterpret_cast<const int4*>(wq_t + (size_t(g * (kGroup / 16) + c) * N + n) * 16);
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          isum[m] = __dp4a(w.x, s_x[m][c * 4], isum[m]);
-          isum[m] = __dp4a(w.y, s_x[m][c * 4 + 1], isum[m]);
-          isum[m] = __dp4a(w.z, s_x[m][c * 4 + 2], isum[m]);
-          isum[m] = __dp4a(w.w, s_x[m][c * 4 + 3], isum[m]);
-        }
-      }
-      const float sw = sw_t[size_t(g) * N + n];
-#pragma unroll
-      for (int m = 0; m < MT; ++m) acc[m] += sw * float(isum[m]);
-    }
-  }
-  if (n >= N) return;
-  if (gridDim.y == 1) {
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-      if (m < M) out[size_t(m) * N + n] = __float2bfloat16(acc[m] * xs[m]);
-  } else {
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-      if (m < M) ws[(size_t(blockIdx.y) * M + m) * N + n] = acc[m];
-  }
-}
-
-__global__ void k_w8a8_reduce(const float* __restrict__ ws, const float* __restrict__ xs,
-                              __nv_bfloat16* __restrict__ out, int M, int N, int S) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M * N) return;
-  float a = 0.f;
-  for (int s = 0; s < S; ++s) a += ws[size_t(s) * M * N + t];
-  out[t] = __float2bfloat16(a * xs[t / N]);
-}
-
 }  // namespace bl
 
 using namespace bl;
@@ -176,6 +108,10 @@ extern "C" int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, c
     set_err(err, errlen, "barlink: w8a16_gemm needs K a multiple of %d", kGroup);
     return -1;
   }
+  if ((reinterpret_cast<uintptr_t>(xq) | reinterpret_cast<uintptr_t>(wq_t)) & 15u) {
+    set_err(err, errlen, "barlink: w8a16_gemm needs xq and wq_t on 16-byte boundaries");
+    return -1;
+  }
   const int G = k / kGroup;
   if (splits < 1) splits = 1;
   if (splits > G) splits = G;
@@ -185,28 +121,26 @@ extern "C" int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, c
     set_err(err, errlen, "barlink: w8a16_gemm with a k-split needs a workspace of S*M*N floats");
     return -1;
   }
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const dim3 grid((n + kQThreads - 1) / kQThreads, splits);
-  cudaError_t e;
-#define BL_W8A8(MT)                                                                                   \
-  e = launch_k(k_w8a8_gemm<MT>, grid, dim3(kQThreads), 0, st, static_cast<const int8_t*>(wq_t),       \
-               static_cast<const float*>(sw_t), static_cast<const int8_t*>(xq),                       \
-               static_cast<const float*>(xs), static_cast<__nv_bfloat16*>(out), static_cast<float*>(ws), \
-               m, n, k, gper)
-  if (m <= 1) BL_W8A8(1);
-  else if (m <= 4) BL_W8A8(4);
-  else BL_W8A8(16);
-#undef BL_W8A8
-  if (e == cudaSuccess) e = cudaGetLastError();
-  if (e == cudaSuccess && splits > 1) {
-    e = launch_k(k_w8a8_reduce, dim3((m * n + 255) / 256), dim3(256), 0, st,
-                 static_cast<const float*>(ws), static_cast<const float*>(xs),
-                 static_cast<__nv_bfloat16*>(out), m, n, splits);
-    if (e == cudaSuccess) e = cudaGetLastError();
-  }
-  if (e != cudaSuccess) {
-    set_err(err, errlen, "barlink: w8a16_gemm launch failed: %s", cudaGetErrorString(e));
-    return -1;
-  }
+  // bl_slab_finish reads and stores 16-byte vectors
+  if ((n & 7) || ((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(out)) & 15u)) splits = 1;
+  blQlinArgs a;
+  memset(&a, 0, sizeof(a));
+  a.w = wq_t;
+  a.src = 1;
+  a.n = n;
+  a.k = k;
+  a.xq = xq;
+  a.xs = xs;
+  a.m = m;
+  a.digits = 1;
+  a.scale_kind = BL_QSCALE_F32_GN;
+  a.scale = sw_t;
+  a.group_k = kGroup;
+  a.splits = splits;
+  if (splits > 1) a.slabs = ws;
+  a.out = out;
+  a.ldo = n;
+  if (bl_qlin(&a, stream, err, errlen) != 0) return -1;
+  if (splits > 1) return bl_slab_finish(ws, splits, m, n, nullptr, 0, out, n, stream, err, errlen);
   return 0;
 }

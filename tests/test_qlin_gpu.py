@@ -98,3 +98,23 @@ def test_activation_rows_with_extreme_values(ext):
         assert rel_l2(y[r].double(), want[r]) < TOL, r
     assert float(y[0].abs().max()) == 0.0
     assert not torch.isfinite(y[5]).any() and not torch.isfinite(y[6]).any()
+
+
+# k-chunk-major weights (the reference's pair): ragged last row tile, odd n (no k-split), one k-block
+@pytest.mark.parametrize("m", [1, 9, 16])
+@pytest.mark.parametrize("n,k", [(128, 128), (136, 1280), (201, 640), (1000, 3584)])
+def test_chunked_int8_weights(ext, m, n, k):
+    wq, _ = _w8(n, k, 3)
+    wq[0], wq[1] = -128, 127  # the ends of the range
+    sw = torch.rand(k // 128, n, generator=_g(4), device="cuda") * 0.01 + 1e-3
+    wq_t = wq.view(n, k // 16, 16).permute(1, 0, 2).contiguous()
+    xq, xs = ext.w8a16_quant_act(_x(m, k, 5, spread=True))
+    part = torch.einsum("mgk,ngk->gmn", xq.double().view(m, -1, 128), wq.double().view(n, -1, 128))
+    want = (part * sw.double()[:, None, :]).sum(0) * xs.double()[:, None]
+    for splits in (1, 4):
+        assert rel_l2(ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, splits), want) < TOL
+    off = torch.empty(m * k + 4, dtype=torch.int8, device="cuda")[4:].view(m, k)  # rows off 16-byte boundaries
+    off.copy_(xq)
+    assert torch.equal(ext.w8a16_gemm(off, xs, wq_t, sw, n, k, 1), ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, 1))
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0

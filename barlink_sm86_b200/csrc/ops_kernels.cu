@@ -117,6 +117,83 @@ __global__ void __launch_bounds__(512) k_rmsnorm(const uint4* __restrict__ x,
   }
 }
 
+// The same for many rows (prefill).  A row is read once, so what counts is the bytes in flight: four warps
+// per row, every vector of x and of the residual requested before the first is used, and the row kept in
+// registers as it came (the fp32 copy of the kernel above left two 448-thread blocks on an SM, each
+// waiting for one vector per thread).  8192 x 3584 with residual: 164 us, now 44 us
+// (5.4 TB/s).
+constexpr int kRowThreads = 128;
+__device__ __forceinline__ void unpack8(const uint4& a, float (&f)[8]) {
+  const float2 p0 = unpack_bf16x2(a.x), p1 = unpack_bf16x2(a.y), p2 = unpack_bf16x2(a.z), p3 = unpack_bf16x2(a.w);
+  f[0] = p0.x; f[1] = p0.y; f[2] = p1.x; f[3] = p1.y;
+  f[4] = p2.x; f[5] = p2.y; f[6] = p3.x; f[7] = p3.y;
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+template <int VPT>
+__global__ void __launch_bounds__(kRowThreads) k_rmsnorm_rows(const uint4* __restrict__ x, const uint4* residual,
+                                                              const uint4* __restrict__ gamma,
+                                                              uint4* __restrict__ out, uint4* residual_out, int vpr,
+                                                              float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float s_part[kRowThreads / 32];
+  const size_t base = size_t(blockIdx.x) * vpr;
+  uint4 v[VPT];
+  float ss = 0.f;
+  {
+    uint4 r[VPT];
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = threadIdx.x + k * kRowThreads;
+      v[k] = i < vpr ? x[base + i] : make_uint4(0, 0, 0, 0);
+    }
+    if (residual) {
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int i = threadIdx.x + k * kRowThreads;
+        r[k] = i < vpr ? residual[base + i] : make_uint4(0, 0, 0, 0);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < VPT; ++k) {
+      const int i = threadIdx.x + k * kRowThreads;
+      float f[8];
+      unpack8(v[k], f);
+      if (residual) {
+        float q[8];
+        unpack8(r[k], q);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] += q[j];
+        v[k] = pack8(f);  // the norm sees the stored (rounded) sum
+        if (i < vpr) residual_out[base + i] = v[k];
+        unpack8(v[k], f);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int w = 0; w < kRowThreads / 32; ++w) ss += s_part[w];
+  const float rstd = rsqrtf(ss / float(vpr * 8) + eps);
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int i = threadIdx.x + k * kRowThreads;
+    if (i >= vpr) continue;
+    float f[8], gg[8];
+    unpack8(v[k], f);
+    unpack8(gamma[i], gg);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = __bfloat162float(__float2bfloat16(f[j] * rstd)) * gg[j];
+    out[base + i] = pack8(f);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // RoPE (rotate-half) on q and k of a fused qkv row + paged KV write
 // ---------------------------------------------------------------------------
@@ -189,6 +266,88 @@ __global__ void __launch_bounds__(256) k_rope_kv_write(__nv_bfloat16* __restrict
       __nv_bfloat16* c = v_cache + ((size_t(blk) * nkv + (h - nq - nkv)) * block_size + off) * hd;
       c[i] = v1;
       c[i + half] = v2;
+    }
+  }
+}
+
+// The same on the bf16 buffer of many rows (prefill): one block per row.  A thread owns four rotation pairs
+// (two 8-byte loads) and the same ones in every head it visits, so that their sines and cosines are
+// computed once per row, and kRopeBatch heads are requested at a time.  (One pair per thread with 2-byte
+// accesses and a sincosf for every pair of every head took 189 us for 8192 rows of 36 heads; this takes 56 us.)
+constexpr int kRopeBatch = 5;
+template <bool VEC>
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&f)[4]) {
+  if (VEC) {
+    const uint2 a = *reinterpret_cast<const uint2*>(p);
+    const float2 x = unpack_bf16x2(a.x), y = unpack_bf16x2(a.y);
+    f[0] = x.x; f[1] = x.y; f[2] = y.x; f[3] = y.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) f[j] = __bfloat162float(p[j]);
+  }
+}
+template <bool VEC>
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&f)[4]) {
+  if (VEC) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[j] = __float2bfloat16(f[j]);
+  }
+}
+__global__ void __launch_bounds__(kRowThreads) k_rope_kv_rows(__nv_bfloat16* __restrict__ qkv,
+                                                              const int* __restrict__ positions,
+                                                              const int* __restrict__ slots,
+                                                              __nv_bfloat16* __restrict__ k_cache,
+                                                              __nv_bfloat16* __restrict__ v_cache, int nq, int nkv,
+                                                              int hd, int block_size, float log2_theta) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.x, half = hd >> 1, lph = hd >> 3;  // threads per head
+  const int t = threadIdx.x % lph, h0 = threadIdx.x / lph, hpp = kRowThreads / lph;
+  const int heads = nq + 2 * nkv, i0 = 4 * t;
+  const int slot = slots ? slots[row] : -1;
+  const size_t coff = slot >= 0 ? (size_t(slot / block_size) * nkv * block_size + slot % block_size) * hd : 0;
+  const float pos = float(positions[row]);
+  float sn[4], cs[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float inv = exp2f(-log2_theta * (2.f * float(i0 + j) / float(hd)));
+    sincosf(pos * inv, &sn[j], &cs[j]);
+  }
+  __nv_bfloat16* prow = qkv + size_t(row) * heads * hd;
+  // V heads are only read, and only when there is a cache to write
+  const int last = slot >= 0 ? heads : nq + nkv;
+  for (int hb = h0; hb < last; hb += hpp * kRopeBatch) {
+    float a[kRopeBatch][4], b[kRopeBatch][4];
+#pragma unroll
+    for (int c = 0; c < kRopeBatch; ++c) {
+      const int h = hb + c * hpp;
+      if (h < last) {
+        load4<true>(prow + size_t(h) * hd + i0, a[c]);
+        load4<true>(prow + size_t(h) * hd + i0 + half, b[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kRopeBatch; ++c) {
+      const int h = hb + c * hpp;
+      if (h >= last) break;
+      float o1[4], o2[4];
+      const bool rot = h < nq + nkv;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        o1[j] = rot ? a[c][j] * cs[j] - b[c][j] * sn[j] : a[c][j];
+        o2[j] = rot ? b[c][j] * cs[j] + a[c][j] * sn[j] : b[c][j];
+      }
+      if (rot) {
+        store4<true>(prow + size_t(h) * hd + i0, o1);
+        store4<true>(prow + size_t(h) * hd + i0 + half, o2);
+      }
+      if (h >= nq && slot >= 0) {
+        __nv_bfloat16* cache = (rot ? k_cache : v_cache) + coff + size_t(rot ? h - nq : h - nq - nkv) * block_size * hd;
+        store4<true>(cache + i0, o1);
+        store4<true>(cache + i0 + half, o2);
+      }
     }
   }
 }
@@ -1095,6 +1254,15 @@ extern "C" int bl_rmsnorm(const void* x, const void* residual, const void* gamma
     return -1;
   }
   const int vpr = hidden / 8;
+  // more rows than SMs: rows in flight count, not the latency of one (333 x 3584: 6.8 us with the kernel
+  // below, 4.5 us)
+  if (!partials && rows > 148 && vpr <= 8 * kRowThreads) {
+    launch_k(vpr <= 4 * kRowThreads ? k_rmsnorm_rows<4> : k_rmsnorm_rows<8>, dim3(rows), dim3(kRowThreads), 0,
+             static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<const uint4*>(residual),
+             static_cast<const uint4*>(gamma), static_cast<uint4*>(out), static_cast<uint4*>(residual_out), vpr, eps);
+    OPS_LAUNCH_CHECK("rmsnorm");
+    return 0;
+  }
   int threads = (vpr + 31) / 32 * 32;
   if (threads > 512) threads = 512;
   launch_k(k_rmsnorm, dim3(rows), dim3(threads), 0, static_cast<cudaStream_t>(stream),
@@ -1113,6 +1281,15 @@ extern "C" int bl_rope_kv_write(void* qkv, const void* partials, int nsplit, siz
   if (rows < 1 || hd < 16 || (hd & 15) || hd > 256) {
     set_err(err, errlen, "barlink: rope_kv_write needs head_dim in 16..256, multiple of 16");
     return -1;
+  }
+  // many rows of bf16: heads of a power of two on 8-byte boundaries
+  if (!partials && rows > 148 && (hd & (hd - 1)) == 0 &&
+      ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 7u) == 0) {
+    launch_k(k_rope_kv_rows, dim3(rows), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream),
+             static_cast<__nv_bfloat16*>(qkv), positions, slots, static_cast<__nv_bfloat16*>(k_cache),
+             static_cast<__nv_bfloat16*>(v_cache), nq, nkv, hd, block_size, log2f(theta));
+    OPS_LAUNCH_CHECK("rope_kv_write");
+    return 0;
   }
   const int hpb = kRopeHeads * (hd / 2) <= 256 ? kRopeHeads : 256 / (hd / 2);
   launch_k(k_rope_kv_write, dim3(rows, (nq + 2 * nkv + hpb - 1) / hpb), dim3(hpb * (hd / 2)), 0,
@@ -1376,57 +1553,83 @@ extern "C" int bl_rope_attn_decode(const void* qkv, int q_stride, const void* sl
 // ---------------------------------------------------------------------------
 // Per-head RMSNorm of q and k (weights gq, gk over head_dim = 128) followed by
 // RoPE with 1 or 2 position axes, on a fused qkv row [(3*heads) * 128].
-// One warp per (token, head); lane l owns dims l, l+32, l+64, l+96, which are
-// exactly the rotation partners for both axis layouts.
-__global__ void __launch_bounds__(256) k_qknorm_rope(__nv_bfloat16* __restrict__ qkv,
-                                                     const __nv_bfloat16* __restrict__ gq,
-                                                     const __nv_bfloat16* __restrict__ gk,
-                                                     const int* __restrict__ positions, int heads,
-                                                     int row_stride, float eps, float log2_theta,
-                                                     int axes) {
+// One block per token, 16 threads per head; a thread owns four rotation pairs (two 8-byte accesses),
+// the same ones in every head, so that sines, cosines and norm weights are read once per token.  (A warp
+// per head with 2-byte accesses and its own sincosf took 41 us for 4608 rows of 24 heads; this takes 25.5 us.)
+constexpr int kQkBatch = 6;
+template <bool VEC>
+__global__ void __launch_bounds__(kRowThreads) k_qknorm_rope(__nv_bfloat16* __restrict__ qkv,
+                                                             const __nv_bfloat16* __restrict__ gq,
+                                                             const __nv_bfloat16* __restrict__ gk,
+                                                             const int* __restrict__ positions, int heads,
+                                                             int row_stride, float eps, float log2_theta, int axes) {
   pdl_launch_dependents();
   pdl_wait();
-  const int row = blockIdx.x, lane = threadIdx.x & 31;
-  for (int h = (threadIdx.x >> 5) + blockIdx.y * 8; h < 2 * heads; h += 8 * gridDim.y) {
-    __nv_bfloat16* p = qkv + size_t(row) * row_stride + size_t(h) * 128;  // q heads then k heads
-    const __nv_bfloat16* gm = h < heads ? gq : gk;
-    float x[4];
+  const int row = blockIdx.x, t = threadIdx.x & 15, h0 = threadIdx.x >> 4;
+  constexpr int kHpp = kRowThreads / 16;  // heads per pass
+  // axes = 2: dims [0,64) rotate by axis 0 in pairs (i, i+32), dims [64,128) by axis 1; axes = 1: pairs (i, i+64)
+  const int half = axes == 2 ? 32 : 64;
+  const int i0 = (4 * t) & (half - 1), ax = axes == 2 ? t >> 3 : 0;
+  const int d1 = ax * 64 + i0, d2 = d1 + half;
+  const float pos = float(positions[row * axes + ax]);
+  float sn[4], cs[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) x[j] = __bfloat162float(p[lane + 32 * j]);
-    if (gm) {
-      float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
-      ss = warp_sum(ss);
-      const float rstd = rsqrtf(ss / 128.f + eps);
+  for (int j = 0; j < 4; ++j) {
+    const float inv = exp2f(-log2_theta * (2.f * float(i0 + j) / float(2 * half)));
+    sincosf(pos * inv, &sn[j], &cs[j]);
+  }
+  __nv_bfloat16* prow = qkv + size_t(row) * row_stride;  // q heads then k heads
+  // every thread of a warp makes the same number of passes: the sums go over 16 lanes of it
+  for (int hb = 0; hb < 2 * heads; hb += kHpp * kQkBatch) {
+    float a[kQkBatch][4], b[kQkBatch][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        x[j] = __bfloat162float(__float2bfloat16(x[j] * rstd)) * __bfloat162float(gm[lane + 32 * j]);
-    }
-    if (axes == 2) {
-      // dims [0,64): axis 0, pairs (l, l+32); dims [64,128): axis 1, pairs (l+64, l+96)
-      const float inv = exp2f(-log2_theta * (2.f * float(lane) / 64.f));
+    for (int c = 0; c < kQkBatch; ++c) {
+      const int h = hb + c * kHpp + h0;
+      if (h < 2 * heads) {
+        load4<VEC>(prow + size_t(h) * 128 + d1, a[c]);
+        load4<VEC>(prow + size_t(h) * 128 + d2, b[c]);
+      } else {
 #pragma unroll
-      for (int ax = 0; ax < 2; ++ax) {
-        float sn, cs;
-        sincosf(float(positions[row * 2 + ax]) * inv, &sn, &cs);
-        const float a = x[2 * ax], b = x[2 * ax + 1];
-        x[2 * ax] = a * cs - b * sn;
-        x[2 * ax + 1] = b * cs + a * sn;
-      }
-    } else {
-      // pairs (l, l+64) and (l+32, l+96)
-      const float pos = float(positions[row]);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const float inv = exp2f(-log2_theta * (2.f * float(lane + 32 * j) / 128.f));
-        float sn, cs;
-        sincosf(pos * inv, &sn, &cs);
-        const float a = x[j], b = x[j + 2];
-        x[j] = a * cs - b * sn;
-        x[j + 2] = b * cs + a * sn;
+        for (int j = 0; j < 4; ++j) a[c][j] = b[c][j] = 0.f;
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) p[lane + 32 * j] = __float2bfloat16(x[j]);
+    for (int c = 0; c < kQkBatch; ++c) {
+      const int h = hb + c * kHpp + h0;
+      const __nv_bfloat16* gm = h < heads ? gq : gk;
+      float ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ss += a[c][j] * a[c][j] + b[c][j] * b[c][j];
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (h >= 2 * heads) continue;
+      float x1[4], x2[4];
+      if (gm) {
+        const float rstd = rsqrtf(ss / 128.f + eps);
+        float g1[4], g2[4];
+        load4<VEC>(gm + d1, g1);
+        load4<VEC>(gm + d2, g2);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          x1[j] = __bfloat162float(__float2bfloat16(a[c][j] * rstd)) * g1[j];
+          x2[j] = __bfloat162float(__float2bfloat16(b[c][j] * rstd)) * g2[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          x1[j] = a[c][j];
+          x2[j] = b[c][j];
+        }
+      }
+      float o1[4], o2[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        o1[j] = x1[j] * cs[j] - x2[j] * sn[j];
+        o2[j] = x2[j] * cs[j] + x1[j] * sn[j];
+      }
+      store4<VEC>(prow + size_t(h) * 128 + d1, o1);
+      store4<VEC>(prow + size_t(h) * 128 + d2, o2);
+    }
   }
 }
 
@@ -1500,6 +1703,64 @@ __global__ void __launch_bounds__(512) k_layernorm_modulate(const uint4* __restr
       out[row * vpr + i] = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]),
                                       pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
     }
+  }
+}
+
+// The same for many rows: see k_rmsnorm_rows (4608 x 3072: 17.8 us before, now 10.0 us)
+template <int VPT>
+__global__ void __launch_bounds__(kRowThreads) k_layernorm_rows(const uint4* __restrict__ x,
+                                                                const __nv_bfloat16* __restrict__ shift,
+                                                                const __nv_bfloat16* __restrict__ scale,
+                                                                uint4* __restrict__ out, int vpr, int rows_per_batch,
+                                                                int mod_stride, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float s_a[kRowThreads / 32], s_b[kRowThreads / 32];
+  const size_t base = size_t(blockIdx.x) * vpr;
+  const size_t mod = size_t(int(blockIdx.x) / rows_per_batch) * mod_stride;
+  uint4 v[VPT];
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int i = threadIdx.x + k * kRowThreads;
+    v[k] = i < vpr ? x[base + i] : make_uint4(0, 0, 0, 0);
+  }
+  float sum = 0.f, sq = 0.f;
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    float f[8];
+    unpack8(v[k], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      sum += f[j];
+      sq += f[j] * f[j];
+    }
+  }
+  sum = warp_sum(sum);
+  sq = warp_sum(sq);
+  if ((threadIdx.x & 31) == 0) {
+    s_a[threadIdx.x >> 5] = sum;
+    s_b[threadIdx.x >> 5] = sq;
+  }
+  __syncthreads();
+  sum = sq = 0.f;
+#pragma unroll
+  for (int w = 0; w < kRowThreads / 32; ++w) {
+    sum += s_a[w];
+    sq += s_b[w];
+  }
+  const float n = float(vpr * 8), mean = sum / n;
+  const float rstd = rsqrtf(fmaxf(sq / n - mean * mean, 0.f) + eps);
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const int i = threadIdx.x + k * kRowThreads;
+    if (i >= vpr) continue;
+    float f[8], hs[8], cs[8];
+    unpack8(v[k], f);
+    unpack8(*reinterpret_cast<const uint4*>(shift + mod + i * 8), hs);
+    unpack8(*reinterpret_cast<const uint4*>(scale + mod + i * 8), cs);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = (f[j] - mean) * rstd * (1.f + cs[j]) + hs[j];
+    out[base + i] = pack8(f);
   }
 }
 
@@ -1596,9 +1857,10 @@ extern "C" int bl_qknorm_rope(void* qkv, const void* gq, const void* gk, const i
     set_err(err, errlen, "barlink: qknorm_rope is built for head_dim 128 and 1 or 2 position axes");
     return -1;
   }
-  const int gy = (2 * heads + 7) / 8 < 8 ? (2 * heads + 7) / 8 : 8;
-  launch_k(k_qknorm_rope, dim3(rows, gy), dim3(256), 0, static_cast<cudaStream_t>(stream),
-           static_cast<__nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gq),
+  const bool vec = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(gq) |
+                     reinterpret_cast<uintptr_t>(gk)) & 7u) == 0 && (row_stride & 3) == 0;
+  launch_k(vec ? k_qknorm_rope<true> : k_qknorm_rope<false>, dim3(rows), dim3(kRowThreads), 0,
+           static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gq),
            static_cast<const __nv_bfloat16*>(gk), positions, heads, row_stride, eps, log2f(theta), axes);
   OPS_LAUNCH_CHECK("qknorm_rope");
   return 0;
@@ -1613,6 +1875,13 @@ extern "C" int bl_layernorm_modulate(const void* x, const void* shift, const voi
     return -1;
   }
   const int vpr = hidden / 8;
+  if (rows > 148 && vpr <= 8 * kRowThreads) {  // as in bl_rmsnorm
+    launch_k(vpr <= 4 * kRowThreads ? k_layernorm_rows<4> : k_layernorm_rows<8>, dim3(rows), dim3(kRowThreads), 0,
+             static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<const __nv_bfloat16*>(shift),
+             static_cast<const __nv_bfloat16*>(scale), static_cast<uint4*>(out), vpr, rows_per_batch, mod_stride, eps);
+    OPS_LAUNCH_CHECK("layernorm_modulate");
+    return 0;
+  }
   int threads = (vpr + 31) / 32 * 32;
   if (threads > 512) threads = 512;
   launch_k(k_layernorm_modulate, dim3(rows), dim3(threads), 0, static_cast<cudaStream_t>(stream),

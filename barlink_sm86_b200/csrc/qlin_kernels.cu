@@ -19,13 +19,19 @@
 //   kRows    int8 [n][k], TMA tiles of 128 rows x 128 bytes in the 128-byte swizzle
 //   kChunks  int8 [k/16][n][16] (the reference's layout, torch_ext/barlink_sm86/w8a16.cu:94-117): a
 //            16-byte chunk of 128 rows is 2 KiB contiguous and already the tensor core's unswizzled
-//            K-major layout, so a k-block is eight bulk copies
+//            K-major layout, so a k-block is a plain box of eight of them
 //   kNibbles int4 GPTQ-v1 (int32 [k/8][n], 8 k per word): four warps turn a raw 8 KiB tile into the
 //            layout of kChunks, seven instructions per eight weights, zero point subtracted; nibbles
 //            come out in the order 0 2 4 6 1 3 5 7 of each eight and k_quant_digits writes the
 //            digits in that order
 // Scales (SC): per output channel, applied by the epilogue; or per group of 128 (a k-block), where
 // every k-block gets a TMEM accumulator of its own and the epilogue warps add acc * scale in fp32.
+//
+// The products of a k-block take the tensor core some 50 cycles; what a k-block costs is the instructions
+// around them, in the one warp that issues them and in the one that requests the tiles.  So that warp runs
+// converged with its operands in uniform registers and asks for the next stage before it issues this one's
+// products (55296 x 5120, one token: 49 -> 48 us with per-row scales, 64.5 -> 54 us with group-128 scales and
+// int8 activations), and a k-block of the chunk layout is one box instead of eight bulk copies (79 -> 49 us).
 //
 // A k-split writes fp32 slabs [split][token][n]; the consumer of the linear sums them as it reads
 // (the norm, RoPE and attention kernels do), or k_slab_finish does with bias / SiLU*mul.
@@ -50,7 +56,6 @@ constexpr int kQTileA = kQRows * kQK;
 struct QlinShape {
   int n, m, k;
   int tiles_a, tiles_b, kblocks, splits;
-  const uint8_t* w;              // kChunks: weights; kNibbles: packed words come through the tensor map
   const uint32_t* zeros;         // kNibbles: int32 [groups][n/8]
   const float* xs;               // per token
   int scale_kind;                // see blQlinArgs
@@ -129,7 +134,7 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
     }
     *s_abort = 0;
     mbar_fence_init();
-    if (SRC != kChunks) tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
   }
   if (warp == 1) {
@@ -144,24 +149,13 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     if (lane == 0) {
-      // bytes of weights a stage receives: the rows of the last tile may run out (bulk copies only;
-      // tensor copies fill with zeros)
-      auto a_bytes = [&](int ta) {
-        return SRC == kChunks ? 8 * 16 * min(kQRows, g.n - ta * kQRows) : S::kStageA;
-      };
       auto load_a = [&](uint32_t dst, uint64_t* bar, int kb, int ta) {
-        if constexpr (SRC == kRows) {
+        if constexpr (SRC == kRows)
           tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), kb * kQK, ta * kQRows, kHintEvictFirst);
-        } else if constexpr (SRC == kNibbles) {
+        else if constexpr (SRC == kNibbles)
           tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), ta * kQRows, kb * (kQK / 8), kHintEvictFirst);
-        } else {
-          const uint32_t bytes = 16u * uint32_t(min(kQRows, g.n - ta * kQRows));
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-            bulk_load_s(dst + c * (kQRows * 16),
-                        g.w + (size_t(kb * 8 + c) * g.n + size_t(ta) * kQRows) * 16, bytes, smem_u32(bar),
-                        kHintEvictFirst);
-        }
+        else  // eight chunks of 128 rows, in elements of 8 bytes
+          tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), ta * kQRows * 2, kb * (kQK / 16), kHintEvictFirst);
       };
       // the first lap of weight tiles is requested before the kernels ahead have finished
       int pre = 0;
@@ -169,7 +163,7 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
         const int tile = u / g.splits, sp = u - tile * g.splits, ta = tile / g.tiles_b;
         const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
         for (int kb = kb0; kb < kb1 && pre < S::kStages; ++kb, ++pre) {
-          mbar_expect_tx(&full_bar[pre], a_bytes(ta) + S::kStageB);
+          mbar_expect_tx(&full_bar[pre], S::kStage);
           load_a(ring + pre * S::kStage, &full_bar[pre], kb, ta);
         }
       }
@@ -192,7 +186,7 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
               ok = false;
               break;
             }
-            mbar_expect_tx(&full_bar[stage], a_bytes(ta) + S::kStageB);
+            mbar_expect_tx(&full_bar[stage], S::kStage);
             load_a(dst, &full_bar[stage], kb, ta);
           }
           tma_load_2d_hint_s(dst + S::kStageA, &tmap_x, smem_u32(&full_bar[stage]), kb * kQK, tb * S::BN, kHintEvictLast);
@@ -220,51 +214,60 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_i8(kQRows, S::BN);
-      int stage = 0, nkb = 0, accs = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        const int sp = u % g.splits;
-        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; ++kb, ++nkb) {
-          if (GROUPED || kb == kb0) {
-            if (kb != kb0 || u != int(blockIdx.x)) ++accs;
-            if (!mbar_wait_bounded(&tempty_bar[accs % S::kAcc], (uint32_t(accs / S::kAcc) & 1u) ^ 1u, s_abort)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
+    const uint32_t leader = elect_leader();
+    const uint32_t idesc = umma_idesc_i8(kQRows, S::BN);
+    int stage = 0, acc = -1, a8 = 0;
+    uint32_t phase = 0, a8phase = 0;
+    uint32_t tphase = 1;  // of the accumulators: all are free at the start
+    bool ok = true;
+    // the next stage is asked for before the products of this one are issued, so that the answer is there
+    // when they are
+    bool ready = mbar_test_wait(&full_bar[0], 0);
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int sp = u % g.splits;
+      const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (GROUPED || kb == kb0) {
+          if (++acc == S::kAcc) {
+            acc = 0;
+            tphase ^= 1u;
           }
-          const uint32_t d_tmem = tmem_base + uint32_t((accs % S::kAcc) * S::BN);
-          // int4: the expanding threads have waited for the stage, but the digits are read here too
-          if (!mbar_wait_bounded(&full_bar[stage], phase, s_abort)) {
-            ok = false;
-            break;
-          }
-          if (SRC == kNibbles && !mbar_wait_bounded(&ready_bar[nkb & 3], uint32_t(nkb >> 2) & 1u, s_abort)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after_sync();
-          const uint32_t sa = SRC == kNibbles ? ring_a8 + (nkb & 3) * kQTileA : ring + stage * S::kStage;
-          const uint64_t da = SRC == kRows ? umma_desc_k_sw128(sa) : umma_desc_k_chunks(sa);
-          const uint64_t db = umma_desc_k_sw128(ring + stage * S::kStage + S::kStageA);
-          // 32 bytes along K per instruction: +2 (16-byte units) inside a swizzled row, two chunks otherwise
-          constexpr int kStepA = SRC == kRows ? 2 : 2 * (kQRows * 16) / 16;
+          ok = mbar_wait_bounded(&tempty_bar[acc], tphase, s_abort);
+        }
+        // int4: the expanding threads have waited for the stage, but the digits are read here too
+        if (!ready) ok = ok && mbar_wait_bounded(&full_bar[stage], phase, s_abort);
+        if (SRC == kNibbles) ok = ok && mbar_wait_bounded(&ready_bar[a8], a8phase, s_abort);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + uint32_t(acc * S::BN);
+        const uint32_t sx = ring + stage * S::kStage;
+        const uint32_t sa = SRC == kNibbles ? ring_a8 + a8 * kQTileA : sx;
+        uint64_t* done = &empty_bar[stage];
+        if (++stage == S::kStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        ready = mbar_test_wait(&full_bar[stage], phase);
+        const uint64_t da = SRC == kRows ? umma_desc_k_sw128(sa) : umma_desc_k_chunks(sa);
+        const uint64_t db = umma_desc_k_sw128(sx + S::kStageA);
+        // 32 bytes along K per instruction: +2 (16-byte units) inside a swizzled row, two chunks otherwise
+        constexpr int kStepA = SRC == kRows ? 2 : 2 * (kQRows * 16) / 16;
 #pragma unroll
-          for (int k = 0; k < kQK / 32; ++k)
-            umma_i8_ss(d_tmem, da + uint64_t(kStepA * k), db + uint64_t(2 * k), idesc,
-                       ((!GROUPED && kb > kb0) || k > 0) ? 1u : 0u);
-          if (SRC == kNibbles) umma_commit(&afree_bar[nkb & 3]);
-          umma_commit(&empty_bar[stage]);
-          if (GROUPED || kb + 1 == kb1) umma_commit(&tfull_bar[accs % S::kAcc]);
-          if (++stage == S::kStages) {
-            stage = 0;
-            phase ^= 1u;
+        for (int k = 0; k < kQK / 32; ++k)
+          umma_i8_ss_warp(leader, d_tmem, da + uint64_t(kStepA * k), db + uint64_t(2 * k), idesc,
+                          ((!GROUPED && kb > kb0) || k > 0) ? 1u : 0u);
+        if (SRC == kNibbles) {
+          umma_commit_warp(leader, &afree_bar[a8]);
+          if (++a8 == 4) {
+            a8 = 0;
+            a8phase ^= 1u;
           }
         }
+        umma_commit_warp(leader, done);
+        if (GROUPED || kb + 1 == kb1) umma_commit_warp(leader, &tfull_bar[acc]);
       }
     }
   } else if (SRC == kNibbles && warp >= 6) {
@@ -275,52 +278,70 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
     const int ct = threadIdx.x - 192, grp = ct >> 7, row = ct & 127;
     int nkb = 0;
     bool ok = true;
+    // words with the zero points of this group's next kZ k-blocks, requested together and one batch ahead
+    constexpr int kZ = 8;
+    auto first_of = [&](int u, int before) {  // first k-block of unit u that this group expands
+      const int kb0 = (u % g.splits) * kb_per;
+      return kb0 + ((before & 1) != grp ? 1 : 0);
+    };
+    auto zero_words = [&](int u, int kb, uint32_t (&z)[kZ]) {
+      const int tile = u / g.splits, kb1 = min(g.kblocks, (u - tile * g.splits + 1) * kb_per);
+      const uint32_t* zp = g.zeros + (min((tile / g.tiles_b) * kQRows + row, g.n - 1) >> 3);
+#pragma unroll
+      for (int i = 0; i < kZ; ++i)
+        z[i] = u < units && kb + 2 * i < kb1 ? __ldg(zp + size_t((kb + 2 * i) / g.gk) * (g.n >> 3)) : 0u;
+    };
+    uint32_t zcur[kZ], znext[kZ];
+    zero_words(blockIdx.x, first_of(blockIdx.x, 0), zcur);
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const int tile = u / g.splits, sp = u - tile * g.splits;
       const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-      const int grow = min((tile / g.tiles_b) * kQRows + row, g.n - 1);
-      const uint32_t* zp = g.zeros + (grow >> 3);
-      auto zero_of = [&](int kb) { return (__ldg(zp + size_t(kb / g.gk) * (g.n >> 3)) >> ((grow & 7) * 4)) & 15u; };
-      // this group's k-blocks of the unit: first, first + 2, ...; the zero points are read two ahead
-      const int first = kb0 + ((nkb & 1) != grp ? 1 : 0);
-      uint32_t z0 = first < kb1 ? zero_of(first) : 0u, z1 = first + 2 < kb1 ? zero_of(first + 2) : 0u;
-      for (int kb = first; kb < kb1 && ok; kb += 2) {
-        const int b = nkb + (kb - kb0), stage = b % S::kStages;
-        const uint32_t z = z0;
-        z0 = z1;
-        z1 = kb + 4 < kb1 ? zero_of(kb + 4) : 0u;
-        if (!mbar_wait_bounded(&full_bar[stage], uint32_t(b / S::kStages) & 1u, s_abort) ||
-            !mbar_wait_bounded(&afree_bar[b & 3], (uint32_t(b >> 2) & 1u) ^ 1u, s_abort)) {
-          ok = false;
-          break;
-        }
-        const uint32_t src = ring + stage * S::kStage + row * 4;
-        const uint32_t dst = ring_a8 + (b & 3) * kQTileA + row * 16;
-        uint32_t w[16];
+      const int zsh = (min((tile / g.tiles_b) * kQRows + row, g.n - 1) & 7) * 4;
+      // a unit of one k-block may have none for this group: on to the next unit's words
+      if (first_of(u, nkb) >= kb1) zero_words(u + gridDim.x, first_of(u + gridDim.x, nkb + kb1 - kb0), zcur);
+      for (int kbz = first_of(u, nkb); kbz < kb1 && ok; kbz += 2 * kZ) {
+        if (kbz + 2 * kZ < kb1) zero_words(u, kbz + 2 * kZ, znext);
+        else zero_words(u + gridDim.x, first_of(u + gridDim.x, nkb + kb1 - kb0), znext);
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[i]) : "r"(src + i * (kQRows * 4)));
-        // byte = (128 + nibble - zero) without borrow between bytes, then the sign bit flipped
-        const uint32_t zz = z * 0x01010101u;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint32_t o[4];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint32_t v = w[2 * c + h];
-            o[2 * h] = (((v & 0x0F0F0F0Fu) | 0x80808080u) - zz) ^ 0x80808080u;
-            o[2 * h + 1] = ((((v >> 4) & 0x0F0F0F0Fu) | 0x80808080u) - zz) ^ 0x80808080u;
+        for (int i = 0; i < kZ; ++i) {
+          const int kb = kbz + 2 * i;
+          if (kb >= kb1) break;
+          const int b = nkb + (kb - kb0), stage = b % S::kStages;
+          if (!mbar_wait_bounded_warp(&full_bar[stage], uint32_t(b / S::kStages) & 1u, s_abort) ||
+              !mbar_wait_bounded_warp(&afree_bar[b & 3], (uint32_t(b >> 2) & 1u) ^ 1u, s_abort)) {
+            ok = false;
+            break;
           }
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + c * (kQRows * 16)), "r"(o[0]), "r"(o[1]),
-                       "r"(o[2]), "r"(o[3])
-                       : "memory");
+          const uint32_t src = ring + stage * S::kStage + row * 4;
+          const uint32_t dst = ring_a8 + (b & 3) * kQTileA + row * 16;
+          uint32_t w[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[j]) : "r"(src + j * (kQRows * 4)));
+          // byte = (128 + nibble - zero) without borrow between bytes, then the sign bit flipped
+          const uint32_t zz = ((zcur[i] >> zsh) & 15u) * 0x01010101u;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            uint32_t o[4];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t v = w[2 * c + h];
+              o[2 * h] = (((v & 0x0F0F0F0Fu) | 0x80808080u) - zz) ^ 0x80808080u;
+              o[2 * h + 1] = ((((v >> 4) & 0x0F0F0F0Fu) | 0x80808080u) - zz) ^ 0x80808080u;
+            }
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + c * (kQRows * 16)), "r"(o[0]), "r"(o[1]),
+                         "r"(o[2]), "r"(o[3])
+                         : "memory");
+          }
+          fence_proxy_async_smem();  // the tensor core reads what these threads just wrote
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(&ready_bar[b & 3]);
+            mbar_arrive(&empty_bar[stage]);  // raw words consumed (the MMAs' commit frees the digits)
+          }
         }
-        fence_proxy_async_smem();  // the tensor core reads what these threads just wrote
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&ready_bar[b & 3]);
-          mbar_arrive(&empty_bar[stage]);  // raw words consumed (the MMAs' commit frees the digits)
-        }
+#pragma unroll
+        for (int i = 0; i < kZ; ++i) zcur[i] = znext[i];
       }
       nkb += kb1 - kb0;
     }
@@ -330,6 +351,26 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
     pdl_wait();
     int accs = 0;
     bool ok = true;
+    // Group scales of the next kAhead k-blocks, requested together and one batch ahead, kept as they came
+    // and turned into fp32 at their use, so that no k-block waits for a trip to HBM.
+    constexpr int kAhead = 8;
+    uint32_t sc_cur[GROUPED ? kAhead : 1], sc_next[GROUPED ? kAhead : 1];
+    auto scales_of = [&](int u, int kb, uint32_t (&q8)[GROUPED ? kAhead : 1]) {
+      const int tile = u / g.splits, kb1 = min(g.kblocks, (u - tile * g.splits + 1) * kb_per);
+      const int n = (tile / g.tiles_b) * kQRows + row;
+      const bool in = u < units && n < g.n;
+      const uint32_t* p32 = static_cast<const uint32_t*>(g.scale);
+      const unsigned short* p16 = static_cast<const unsigned short*>(g.scale);
+#pragma unroll
+      for (int i = 0; i < (GROUPED ? kAhead : 1); ++i) {
+        const int gi = (kb + i) / g.gk;
+        q8[i] = !in || kb + i >= kb1                    ? 0u
+                : g.scale_kind == BL_QSCALE_F32_GN ? __ldg(p32 + size_t(gi) * g.n + n)
+                : g.scale_kind == BL_QSCALE_F16_GN ? uint32_t(__ldg(p16 + size_t(gi) * g.n + n))
+                                                   : uint32_t(__ldg(p16 + size_t(n) * g.groups + gi));
+      }
+    };
+    if constexpr (GROUPED) scales_of(blockIdx.x, (int(blockIdx.x) % g.splits) * kb_per, sc_cur);
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const int tile = u / g.splits, sp = u - tile * g.splits;
       const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
@@ -362,30 +403,23 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
       int done_acc = 0;
       if constexpr (GROUPED) {
         const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-        auto scale_of = [&](int kb) -> float {
-          if (!nok || kb >= kb1) return 0.f;
-          const int gi = kb / g.gk;
-          switch (g.scale_kind) {
-            case BL_QSCALE_BF16_NG: return __bfloat162float(static_cast<const __nv_bfloat16*>(g.scale)[size_t(n) * g.groups + gi]);
-            case BL_QSCALE_F16_NG: return __half2float(static_cast<const __half*>(g.scale)[size_t(n) * g.groups + gi]);
-            case BL_QSCALE_F32_GN: return __ldg(static_cast<const float*>(g.scale) + size_t(gi) * g.n + n);
-            default: return __half2float(static_cast<const __half*>(g.scale)[size_t(gi) * g.n + n]);
-          }
+        auto scale_f32 = [&](uint32_t raw) -> float {
+          return g.scale_kind == BL_QSCALE_F32_GN ? __uint_as_float(raw)
+                 : g.scale_kind == BL_QSCALE_BF16_NG ? __uint_as_float(raw << 16)
+                                                     : __half2float(__ushort_as_half(static_cast<unsigned short>(raw)));
         };
         if (g.row_scale) rs = __bfloat162float(g.row_scale[nn]);
 #pragma unroll
         for (int i = 0; i < TB; ++i) accf[i] = 0.f;
-        float sq[4];  // scales of the next four k-blocks are on their way while this one is waited for
+        for (int kb = kb0; kb < kb1 && ok; kb += kAhead) {
+          if (kb + kAhead < kb1) scales_of(u, kb + kAhead, sc_next);
+          else scales_of(u + gridDim.x, ((u + gridDim.x) % g.splits) * kb_per, sc_next);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sq[i] = scale_of(kb0 + i);
-        for (int kb = kb0; kb < kb1 && ok; kb += 4) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
+          for (int i = 0; i < kAhead; ++i) {
             if (kb + i >= kb1 || !ok) break;
-            const float sc = sq[i];
-            sq[i] = scale_of(kb + i + 4);
+            const float sc = scale_f32(sc_cur[i]);
             const int acc = accs % S::kAcc;
-            if (!mbar_wait_bounded(&tfull_bar[acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) {
+            if (!mbar_wait_bounded_warp(&tfull_bar[acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) {
               ok = false;
               break;
             }
@@ -401,12 +435,14 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
             tc_fence_before_sync();
             mbar_arrive(&tempty_bar[acc]);
           }
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i) sc_cur[i] = sc_next[i];
         }
         if (!ok) break;
       } else {
         rs = __bfloat162float(static_cast<const __nv_bfloat16*>(g.scale)[nn]);
         done_acc = accs % S::kAcc;
-        if (!mbar_wait_bounded(&tfull_bar[done_acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) break;
+        if (!mbar_wait_bounded_warp(&tfull_bar[done_acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) break;
         ++accs;
         tc_fence_after_sync();
       }
@@ -570,20 +606,22 @@ static int launch_qlin(const blQlinArgs& a, cudaStream_t st, char* err, size_t e
   if (make_tmap_kmajor(a.xq, xrows, a.k, a.k, S::BN, 1, &tx, err, errlen, kQK) != 0) return -1;
   if (SRC == kRows) {
     if (make_tmap_kmajor(a.w, a.n, a.k, a.k, kQRows, 1, &tw, err, errlen, kQK) != 0) return -1;
-  } else if (SRC == kNibbles) {
+  } else {
+    // kNibbles: 16 rows of 128 packed words a k-block; kChunks: 8 rows of 128 chunks of 16 bytes, as
+    // elements of 8 bytes (a box has at most 256 elements a side)
     const DriverApi* d = driver(err, errlen);
     if (!d) return -1;
-    cuuint64_t dims[2] = {cuuint64_t(a.n), cuuint64_t(a.k / 8)};
-    cuuint64_t strides[1] = {cuuint64_t(a.n) * 4};
-    cuuint32_t box[2] = {kQRows, kQK / 8}, estr[2] = {1, 1};
-    if (d->cuTensorMapEncodeTiled(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(a.w), dims, strides, box,
-                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-      set_err(err, errlen, "barlink: tensor map of the packed int4 weight failed (n %d, k %d)", a.n, a.k);
+    constexpr bool nib = SRC == kNibbles;
+    cuuint64_t dims[2] = {cuuint64_t(a.n) * (nib ? 1 : 2), cuuint64_t(a.k / (nib ? 8 : 16))};
+    cuuint64_t strides[1] = {cuuint64_t(a.n) * (nib ? 4 : 16)};
+    cuuint32_t box[2] = {kQRows * (nib ? 1 : 2), kQK / (nib ? 8 : 16)}, estr[2] = {1, 1};
+    if (d->cuTensorMapEncodeTiled(&tw, nib ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_INT64, 2,
+                                  const_cast<void*>(a.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+      set_err(err, errlen, "barlink: tensor map of the quantised weight failed (n %d, k %d)", a.n, a.k);
       return -1;
     }
-  } else {
-    tw = tx;  // not used
   }
   QlinShape g;
   memset(&g, 0, sizeof(g));
@@ -594,7 +632,6 @@ static int launch_qlin(const blQlinArgs& a, cudaStream_t st, char* err, size_t e
   g.tiles_b = tiles_b;
   g.kblocks = (a.k + kQK - 1) / kQK;
   g.splits = a.splits;
-  g.w = static_cast<const uint8_t*>(a.w);
   g.zeros = static_cast<const uint32_t*>(a.zeros);
   g.xs = static_cast<const float*>(a.xs);
   g.scale_kind = a.scale_kind;

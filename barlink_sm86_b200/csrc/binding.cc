@@ -516,6 +516,25 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<
     a.trace = trace->data_ptr();
   }
   void* st = at::cuda::getCurrentCUDAStream(dev).stream();
+  // few tiles of a long reduction: k-splits into fp32 slabs, and a kernel that sums them with the epilogue
+  if (!swap && bn <= 0 && splits <= 0 && !tiled && gate_tokens <= 0 && !residual && !gelu && n % 16 == 0 &&
+      ((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(a.bias)) & 15u) == 0) {
+    const int s2 = bl_gemm_row_splits(tokens, n, k);
+    if (s2 > 1) {
+      at::Tensor slabs = at::empty({s2, tokens, n}, x.options().dtype(at::kFloat));
+      a.out = nullptr;
+      a.bias = nullptr;
+      a.silu_mul = 0;
+      a.ldo = n;
+      a.partial_out = slabs.data_ptr();
+      a.partial_stride = size_t(tokens) * n;
+      a.partial_splits = s2;
+      BL_CHECK(bl_gemm_bf16(&a, st, err, errlen));
+      BL_CHECK(bl_slab_finish(slabs.data_ptr(), s2, tokens, n, bias ? bias->data_ptr() : nullptr, silu_mul ? 1 : 0,
+                              out.data_ptr(), n_out, st, err, errlen));
+      return out;
+    }
+  }
   {
     py::gil_scoped_release nogil;
     BL_CHECK(bl_gemm_bf16(&a, st, err, errlen));
@@ -1078,6 +1097,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("gamma"), py::arg("eps"), py::arg("tokens"), py::arg("splits"), py::arg("units"),
         py::arg("add_residual") = true);
   m.def("gemm_splits", &gemm_splits, py::arg("n"), py::arg("k"), py::arg("tokens"));
+  m.def("gemm_row_splits", &bl_gemm_row_splits, py::arg("rows"), py::arg("n"), py::arg("k"));
   m.def("rope", &rope, py::arg("x"), py::arg("positions"), py::arg("heads"), py::arg("hd"),
         py::arg("theta") = 1e4, py::arg("axes") = 1);
   m.def("silu_mul", &silu_mul, py::arg("gate_up"), py::arg("interleaved") = false);

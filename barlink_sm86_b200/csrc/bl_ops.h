@@ -114,6 +114,8 @@ int bl_tile_weight(const void* src, int n, int k, int ld, void* dst, void* strea
 /* k-splits the decode heuristic picks for n output features, k inputs and
  * `tokens` rows (1 = no split) */
 int bl_gemm_splits(int n, int k, int tokens);
+/* k-splits that suit a token-major product (more than 128 rows), 1: none; slabs are [splits][rows][n] */
+int bl_gemm_row_splits(int rows, int n, int k);
 
 /* W8A16: x [m x k] bf16, wq [n x k] int8 (row = output channel), scale [n]
  * bf16 (per channel) or scales [k/group x n] fp32 (group > 0).  out [m x n]

@@ -338,69 +338,73 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmap_a, const CUten
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------
-    if (lane == 0) {
-      const uint32_t idesc = MODE ? umma_idesc_i8(kTileA, BN) : umma_idesc_f16(kTileA, BN, g.ab_fmt);
-      int stage = 0, astage = 0;
-      uint32_t phase = 0, aphase = 0;
-      uint32_t tphase[2] = {0, 0};
-      int it = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++it) {
-        const int tile = u / g.splits, sp = u - tile * g.splits;
-        const int kb0 = sp * kb_per;
-        const int kb1 = min(g.kblocks, kb0 + kb_per);
-        const int acc = it & 1;
-        if (!mbar_wait_bounded(&tempty_bar[acc], tphase[acc] ^ 1u, s_abort)) break;
-        tphase[acc] ^= 1u;
-        tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + uint32_t(acc * BN);
-        for (int kb = kb0; kb < kb1 && ok; kb += S::kKS) {
-          const int nsub = S::kKS == 1 ? 1 : min(S::kKS, kb1 - kb);
-          const uint32_t sa = ring + stage * S::kStageBytes;
-          if (!W8 && !mbar_wait_bounded(&full_bar[stage], phase, s_abort)) {
+    const uint32_t leader = elect_leader();
+    const uint32_t idesc = MODE ? umma_idesc_i8(kTileA, BN) : umma_idesc_f16(kTileA, BN, g.ab_fmt);
+    int stage = 0, astage = 0, acc = 0;
+    uint32_t phase = 0, aphase = 0;
+    uint32_t tphase = 1;  // of the accumulators: both are free at the start
+    bool ok = true;
+    // the next stage is asked for before the products of this one are issued, so that the answer is there
+    // when they are
+    bool ready = !W8 && mbar_test_wait(&full_bar[0], 0);
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int sp = u % g.splits;
+      const int kb0 = sp * kb_per;
+      const int kb1 = min(g.kblocks, kb0 + kb_per);
+      if (!mbar_wait_bounded_warp(&tempty_bar[acc], tphase, s_abort)) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + uint32_t(acc * BN);
+      for (int kb = kb0; kb < kb1; kb += S::kKS) {
+        const int nsub = S::kKS == 1 ? 1 : min(S::kKS, kb1 - kb);
+        const uint32_t sa = ring + stage * S::kStageBytes;
+        uint64_t* done = &empty_bar[stage];
+        if (!W8 && !ready) ok = mbar_wait_bounded(&full_bar[stage], phase, s_abort);
+        if (!W8 && !__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
+        }
+        if (++stage == S::kStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        if (!W8) ready = mbar_test_wait(&full_bar[stage], phase);
+#pragma unroll
+        for (int sb = 0; sb < S::kKS; ++sb) {
+          if (sb >= nsub) break;
+          // W8: the widening threads have waited for the stage; the widened tile is what counts
+          if (W8 && !mbar_wait_bounded_warp(&ready_bar[astage], aphase, s_abort)) {
             ok = false;
             break;
           }
+          tc_fence_after_sync();
+          if (tr && kb == kb0 && sb == 0 && u == int(blockIdx.x) && lane == 0) tr[3] = globaltimer_ns();
+          const uint64_t da =
+              umma_desc_k_sw128(W8 ? ring + S::kStages * S::kStageBytes + astage * S::kStageA : sa);
+          const uint64_t db = umma_desc_k_sw128(sa + S::kOffB + sb * S::kStageB);
 #pragma unroll
-          for (int sb = 0; sb < S::kKS; ++sb) {
-            if (sb >= nsub) break;
-            // W8: the widening threads have waited for the stage; the widened tile is what counts
-            if (W8 && !mbar_wait_bounded(&ready_bar[astage], aphase, s_abort)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
-            if (tr && kb == kb0 && sb == 0 && it == 0) tr[3] = globaltimer_ns();
-            const uint64_t da =
-                umma_desc_k_sw128(W8 ? ring + S::kStages * S::kStageBytes + astage * S::kStageA : sa);
-            const uint64_t db = umma_desc_k_sw128(sa + S::kOffB + sb * S::kStageB);
-#pragma unroll
-            for (int k = 0; k < kTileK / 16; ++k) {
-              // +32 bytes along K inside the swizzle atom = +2 in the address field
-              if constexpr (MODE != 0)
-                umma_i8_ss(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc,
-                           (kb + sb > kb0 || k > 0) ? 1u : 0u);
-              else
-                umma_f16_ss(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc,
-                            (kb + sb > kb0 || k > 0) ? 1u : 0u);
-            }
-            if (W8) {
-              umma_commit(&afree_bar[astage]);
-              if (++astage == S::kA16Stages) {
-                astage = 0;
-                aphase ^= 1u;
-              }
-            }
+          for (int k = 0; k < kTileK / 16; ++k) {
+            // +32 bytes along K inside the swizzle atom = +2 in the address field
+            if constexpr (MODE != 0)
+              umma_i8_ss_warp(leader, d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc,
+                              (kb + sb > kb0 || k > 0) ? 1u : 0u);
+            else
+              umma_f16_ss_warp(leader, d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc,
+                               (kb + sb > kb0 || k > 0) ? 1u : 0u);
           }
-          if (!ok) break;
-          umma_commit(&empty_bar[stage]);
-          if (++stage == S::kStages) {
-            stage = 0;
-            phase ^= 1u;
+          if (W8) {
+            umma_commit_warp(leader, &afree_bar[astage]);
+            if (++astage == S::kA16Stages) {
+              astage = 0;
+              aphase ^= 1u;
+            }
           }
         }
-        if (ok) umma_commit(&tfull_bar[acc]);
+        if (!ok) break;
+        umma_commit_warp(leader, done);
       }
+      if (ok) umma_commit_warp(leader, &tfull_bar[acc]);
+      acc ^= 1;
+      if (acc == 0) tphase ^= 1u;
     }
   } else if (W8 && warp >= 6) {
     // ------------------------ int8 -> bf16 widening -----------------------

@@ -239,6 +239,8 @@ struct PartialSink {
   const __nv_bfloat16* scale;  // per output feature (W8A16), or null
 
   __device__ __forceinline__ void unit_done(int) const {}
+  template <int NTHR>
+  __device__ __forceinline__ void tile_done(int) const {}
   __device__ __forceinline__ void operator()(int ta, int tb, int split, int row, int c0,
                                              const float (&vin)[32], int ncols) const {
     const int i = ta * kTileA + row;
@@ -748,20 +750,23 @@ static int launch_w8(const blW8A16Args& a, cudaStream_t st, char* err, size_t er
 }
 
 // ---------------------------------------------------------------------------
-// Paired-CTA GEMM (token-major products of 512 tokens or more): two CTAs of a cluster work on one
+// Paired-CTA GEMM (token-major products of more than 128 tokens): two CTAs of a cluster work on one
 // 256 x 256 output tile.  Each CTA loads 128 rows of A and 128 rows of B per
 // k-block (32 KiB instead of the 48 KiB a lone CTA needs for 128 x 256), the
 // leader CTA issues tcgen05.mma.cta_group::2 (M = 256 over the pair, N = 256),
 // and each CTA's epilogue drains its own 128 accumulator rows.  The single-CTA
 // kernel at these sizes is bound by tile delivery from L2; the pair moves a
-// third less per SM.  Barrier protocol:
+// third less per SM.  A k-block's products take the pair 512 cycles; issued from a `lane == 0` branch the
+// instructions around them took 660, so the producer and MMA warps run converged and ask for the next stage
+// before they deal with this one (1000 x 37888 x 3584: 195 -> 178 us, 4608 x 9216 x 3072: 1.55 PFLOP/s; few
+// rows: 333 x 37888 x 3584 took 133 us in the single-CTA kernel, 91 us here).  Barrier protocol:
 //   full[s]   leader only: its producer arms it for both CTAs' bytes; both
 //             CTAs' TMA loads complete on the leader's barrier
 //   empty[s]  one per CTA: the leader's MMA thread commits to its own and to
 //             the peer's (two commits, the peer's through its cluster address)
 //   tfull[a]  one per CTA, committed the same way when a tile's MMAs are done
 //   tempty[a] leader only, 256 arrivals: every epilogue thread of both CTAs
-// Large, unsplit, token-major ("no swap") products only.
+// Token-major ("no swap") products only; k-splits leave fp32 slabs for the next kernel to sum.
 // ---------------------------------------------------------------------------
 constexpr int kPairStages = 6;
 constexpr int kPairStageBytes = 2 * kTileA * kTileK * 2;  // A 16 KiB + B 16 KiB per CTA
@@ -772,27 +777,35 @@ constexpr int kPairBN = 256;
 // residual, stores) stays shorter than the main loop of the next one
 constexpr int kPairThreads = 320;
 
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const void* tmap, uint32_t leader_bar,
-                                                 int x, int y, uint64_t hint) {
+// (these three are for a whole converged warp, of which the elected lane issues: see umma_f16_ss_warp)
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t elected, uint32_t smem_dst, const void* tmap,
+                                                 uint32_t leader_bar, int x, int y, uint64_t hint) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(smem_dst),
-      "l"(tmap), "r"(leader_bar), "r"(x), "r"(y), "l"(hint)
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;\n\t}" ::"r"(smem_dst),
+      "l"(tmap), "r"(leader_bar), "r"(x), "r"(y), "l"(hint), "r"(elected)
       : "memory");
 }
 __device__ __forceinline__ void umma_f16_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                 uint32_t idesc, uint32_t accumulate) {
+                                                 uint32_t idesc, uint32_t accumulate, uint32_t leader) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // arrive (once every MMA issued so far is done) on a barrier given by its cluster address
-__device__ __forceinline__ void umma_commit_pair(uint32_t cluster_bar_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(cluster_bar_addr)
-               : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t leader, uint32_t cluster_bar_addr) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(cluster_bar_addr),
+      "r"(leader)
+      : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar_addr) : "memory");
@@ -815,9 +828,10 @@ __device__ __forceinline__ void pair_tile_of(int u, int tiles_m, int tiles_n, in
   tn = along_m ? sl : f;
 }
 
+template <class Sink>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     k_gemm_pair(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                GemmShape g, LocalSink<kPairBN> sink, uint64_t hint_a, uint64_t hint_b) {
+                GemmShape g, Sink sink, uint64_t hint_a, uint64_t hint_b) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (ring - smem_u32(smem_raw));
@@ -835,7 +849,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
   const uint32_t peer = cr ^ 1u;
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int tiles_m = (g.ra + 255) / 256, tiles_n = (g.rb + 255) / 256;
-  const int units = tiles_m * tiles_n;
+  // k-split: the splits of all tiles follow one another
+  const int tiles = tiles_m * tiles_n, units = tiles * g.splits;
+  const int kb_per = (g.kblocks + g.splits - 1) / g.splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPairStages; ++s) {
@@ -867,73 +883,85 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 
   if (warp == 0) {
     // ------------------------------ producer (both CTAs) ------------------
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int issued = 0;
-      bool ok = true;
-      for (int u = pair; u < units && ok; u += n_pairs) {
-        int tm, tn;
-        pair_tile_of(u, tiles_m, tiles_n, g.band, g.band_m, tm, tn);
-        for (int kb = 0; kb < g.kblocks; ++kb) {
-          if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort)) {
-            ok = false;
-            break;
-          }
-          const uint32_t leader_full = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (cr == 0) mbar_expect_tx(&full_bar[stage], 2 * kPairStageBytes);
-          const uint32_t dst = ring + stage * kPairStageBytes;
-          tma_load_2d_pair(dst, &tmap_a, leader_full, kb * kTileK, tm * 256 + int(cr) * 128, hint_a);
-          tma_load_2d_pair(dst + kTileA * kTileK * 2, &tmap_b, leader_full, kb * kTileK, tn * 256 + int(cr) * 128,
-                           hint_b);
-          ++issued;
-          if (++stage == kPairStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+    const uint32_t elected = elect_leader();
+    const uint32_t full0 = map_to_cta(smem_u32(full_bar), 0);
+    int stage = 0;
+    uint32_t phase = 1;  // of the empty barriers: every stage is free at the start
+    bool ok = true;
+    bool ready = true;   // asked for one stage ahead, as in the MMA warp
+    for (int u = pair; u < units && ok; u += n_pairs) {
+      const int sp = u / tiles;
+      int tm, tn;
+      pair_tile_of(u - sp * tiles, tiles_m, tiles_n, g.band, g.band_m, tm, tn);
+      const int kb1 = min(g.kblocks, (sp + 1) * kb_per);
+      for (int kb = sp * kb_per; kb < kb1; ++kb) {
+        if (!ready && !mbar_wait_bounded(&empty_bar[stage], phase, s_abort)) ok = false;
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
         }
+        if (cr == 0 && elected) mbar_expect_tx(&full_bar[stage], 2 * kPairStageBytes);
+        __syncwarp();
+        const uint32_t dst = ring + stage * kPairStageBytes, bar = full0 + stage * 8;
+        if (++stage == kPairStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        ready = mbar_test_wait(&empty_bar[stage], phase);
+        tma_load_2d_pair(elected, dst, &tmap_a, bar, kb * kTileK, tm * 256 + int(cr) * 128, hint_a);
+        tma_load_2d_pair(elected, dst + kTileA * kTileK * 2, &tmap_b, bar, kb * kTileK, tn * 256 + int(cr) * 128, hint_b);
       }
-      (void)issued;
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader only) --------------
-    if (lane == 0 && cr == 0) {
+    if (cr == 0) {
+      const uint32_t leader = elect_leader();
       const uint32_t idesc = umma_idesc_f16(256, kPairBN, g.ab_fmt);
+      const uint32_t empty0 = map_to_cta(smem_u32(empty_bar), 0), empty1 = map_to_cta(smem_u32(empty_bar), 1);
+      const uint32_t tfull0 = map_to_cta(smem_u32(tfull_bar), 0), tfull1 = map_to_cta(smem_u32(tfull_bar), 1);
       int stage = 0;
       uint32_t phase = 0;
-      uint32_t tphase[2] = {0, 0};
-      int it = 0;
+      uint32_t aphase = 1;  // of the accumulators: both are free at the start
+      int acc = 0;
       bool ok = true;
-      for (int u = pair; u < units && ok; u += n_pairs, ++it) {
-        const int acc = it & 1;
-        if (!mbar_wait_bounded(&tempty_bar[acc], tphase[acc] ^ 1u, s_abort)) break;
-        tphase[acc] ^= 1u;
+      // the next stage is asked for before the products of this one are issued, so that the answer is
+      // there when they are
+      bool ready = mbar_test_wait(&full_bar[0], 0);
+      for (int u = pair; u < units && ok; u += n_pairs) {
+        if (!mbar_wait_bounded_warp(&tempty_bar[acc], aphase, s_abort)) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + uint32_t(acc * kPairBN);
-        for (int kb = 0; kb < g.kblocks; ++kb) {
-          if (!mbar_wait_bounded(&full_bar[stage], phase, s_abort)) {
+        const int kb0 = (u / tiles) * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!ready && !mbar_wait_bounded(&full_bar[stage], phase, s_abort)) ok = false;
+          if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
           const uint32_t sa = ring + stage * kPairStageBytes;
-          const uint64_t da = umma_desc_k_sw128(sa);
-          const uint64_t db = umma_desc_k_sw128(sa + kTileA * kTileK * 2);
-#pragma unroll
-          for (int k = 0; k < kTileK / 16; ++k)
-            umma_f16_ss_pair(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          // the stage is free in both CTAs once these MMAs have read it
-          umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 0));
-          umma_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 1));
+          const uint32_t done = stage;
           if (++stage == kPairStages) {
             stage = 0;
             phase ^= 1u;
           }
+          ready = mbar_test_wait(&full_bar[stage], phase);
+          const uint64_t da = umma_desc_k_sw128(sa);
+          const uint64_t db = umma_desc_k_sw128(sa + kTileA * kTileK * 2);
+#pragma unroll
+          for (int k = 0; k < kTileK / 16; ++k)
+            umma_f16_ss_pair(d_tmem, da + uint64_t(2 * k), db + uint64_t(2 * k), idesc, (kb > kb0 || k > 0) ? 1u : 0u,
+                             leader);
+          // the stage is free in both CTAs once these MMAs have read it
+          umma_commit_pair(leader, empty0 + done * 8);
+          umma_commit_pair(leader, empty1 + done * 8);
         }
         if (ok) {
-          umma_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 0));
-          umma_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 1));
+          umma_commit_pair(leader, tfull0 + acc * 8);
+          umma_commit_pair(leader, tfull1 + acc * 8);
         }
+        acc ^= 1;
+        if (acc == 0) aphase ^= 1u;
       }
     }
   } else {
@@ -944,8 +972,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
     uint32_t tphase[2] = {0, 0};
     int it = 0;
     for (int u = pair; u < units; u += n_pairs, ++it) {
+      const int sp = u / tiles;
       int tm, tn;
-      pair_tile_of(u, tiles_m, tiles_n, g.band, g.band_m, tm, tn);
+      pair_tile_of(u - sp * tiles, tiles_m, tiles_n, g.band, g.band_m, tm, tn);
       const int acc = it & 1;
       if (!mbar_wait_bounded(&tfull_bar[acc], tphase[acc], s_abort)) break;
       tphase[acc] ^= 1u;
@@ -960,7 +989,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
         // this CTA holds rows [tm*256 + cr*128, +128): the Sink's tile index is in units of 128 rows
-        sink(tm * 2 + int(cr), tn, 0, row, c0, v, 32);
+        sink(tm * 2 + int(cr), tn, sp, row, c0, v, 32);
       }
       tc_fence_before_sync();
       mbar_arrive_cluster(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
@@ -985,10 +1014,25 @@ static bool gemm_pair_enabled() {
   return v == 1;
 }
 
-// token-major product with at least 512 tokens, no k-split, no fused collective
+// Token-major products without a fused collective (k_gemm and its own k-split stay for what the paired kernel
+// does not take).  Rows of both operands beyond the matrix are filled with zeros, so any number of tokens will
+// do; below 129 the caller uses the swapped form.
 static bool gemm_pair_ok(const blGemmArgs& a) {
-  return gemm_pair_enabled() && !a.i8 && !a.swap && a.ra >= 512 && a.rb >= 256 && !a.partial_out && !a.peer &&
-         !a.gate_flags && !a.weight_tiled && a.splits <= 1;
+  return gemm_pair_enabled() && !a.i8 && !a.swap && a.ra > 128 && a.rb >= 256 && !a.peer && !a.gate_flags &&
+         !a.weight_tiled && (a.partial_out ? a.partial_splits >= 1 : a.splits <= 1) && !(a.push && a.ra < 512);
+}
+
+template <class Sink>
+static cudaError_t launch_pair_kernel(int pairs, cudaStream_t st, const CUtensorMap& ta, const CUtensorMap& tb,
+                                      const GemmShape& g, const Sink& sink) {
+  static bool attr[64] = {};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_gemm_pair<Sink>), kPairSmem, attr);
+  if (e != cudaSuccess) return e;
+  // the cluster shape is compiled into the kernel (__cluster_dims__); the grid is a whole number of pairs
+  // the slab operand is the one to keep in L2
+  e = launch_k(k_gemm_pair<Sink>, dim3(2 * pairs), dim3(kPairThreads), size_t(kPairSmem), st, ta, tb, g, sink,
+               g.band_m ? kHintEvictLast : kHintEvictFirst, g.band_m ? kHintEvictFirst : kHintEvictLast);
+  return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 static int launch_gemm_pair(const blGemmArgs& a, cudaStream_t st, char* err, size_t errlen) {
@@ -1000,7 +1044,11 @@ static int launch_gemm_pair(const blGemmArgs& a, cudaStream_t st, char* err, siz
   g.rb = a.rb;
   g.k = a.k;
   g.kblocks = (a.k + kTileK - 1) / kTileK;
-  g.splits = 1;
+  g.splits = a.partial_out ? a.partial_splits : 1;
+  if ((g.splits - 1) * ((g.kblocks + g.splits - 1) / g.splits) >= g.kblocks) {
+    set_err(err, errlen, "barlink: %d k-splits do not divide %d k-blocks into non-empty parts", g.splits, g.kblocks);
+    return -1;
+  }
   g.ab_fmt = 1;
   g.err = static_cast<uint32_t*>(a.err_flag);
   LocalSink<kPairBN> sink;
@@ -1015,17 +1063,8 @@ static int launch_gemm_pair(const blGemmArgs& a, cudaStream_t st, char* err, siz
   sink.scale = nullptr;
   sink.xscale = nullptr;
   fill_push(sink, a.push);
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemm_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", kPairSmem, cudaGetErrorString(e));
-      return -1;
-    }
-    attr = true;
-  }
   const int tiles_m = (a.ra + 255) / 256, tiles_n = (a.rb + 255) / 256;
-  const int units = tiles_m * tiles_n;
+  const int units = tiles_m * tiles_n * g.splits;
   // band width: the slab that has to stay in L2 is at most 32 MB; bands of equal width; the
   // orientation that fetches fewer bytes from DRAM (slab operand once, the other once per band)
   const double tile_bytes = 256.0 * a.k * 2;
@@ -1045,11 +1084,20 @@ static int launch_gemm_pair(const blGemmArgs& a, cudaStream_t st, char* err, siz
   int pairs = sm_count() / 2;
   if (pairs > units) pairs = units;
   if (pairs < 1) pairs = 1;
-  // the cluster shape is compiled into the kernel (__cluster_dims__); the grid is a whole number of pairs
-  // the slab operand is the one to keep in L2
-  cudaError_t e = launch_k(k_gemm_pair, dim3(2 * pairs), dim3(kPairThreads), size_t(kPairSmem), st, ta, tb, g, sink,
-                           g.band_m ? kHintEvictLast : kHintEvictFirst, g.band_m ? kHintEvictFirst : kHintEvictLast);
-  if (e == cudaSuccess) e = cudaGetLastError();
+  cudaError_t e;
+  if (a.partial_out) {
+    PartialSink<kPairBN> ps;
+    ps.out = static_cast<float*>(a.partial_out);
+    ps.slab = a.partial_stride;
+    ps.ldo = a.ldo;
+    ps.ra = a.ra;
+    ps.rb = a.rb;
+    ps.swap = 0;
+    ps.scale = nullptr;
+    e = launch_pair_kernel(pairs, st, ta, tb, g, ps);
+  } else {
+    e = launch_pair_kernel(pairs, st, ta, tb, g, sink);
+  }
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: paired GEMM launch failed: %s", cudaGetErrorString(e));
     return -1;
@@ -1192,6 +1240,28 @@ extern "C" int bl_gemm_splits(int n, int k, int tokens) {
   const int tiles = (n + kTileA - 1) / kTileA;
   const int kblocks = (k + kTileK - 1) / kTileK;
   return pick_splits(tiles, kblocks, sm_count(), 0);
+}
+
+// k-splits of a token-major product in the paired kernel: 2 .. 4 when its tiles leave half of the pairs or more
+// without work.  A split of a lap costs its k-blocks plus about 16 of ramp and epilogue, and every slab is
+// written and read once more (in k-blocks of 0.33 us: rows * n * 8 bytes at 3 TB/s).  333 rows, 3584 x 18944:
+// 97 us unsplit, 79 us with 2 splits, 3072 x 12288: 70 and 42 us with 3; 160 rows, 3584 x 18944: 108 and 51 us.
+extern "C" int bl_gemm_row_splits(int rows, int n, int k) {
+  if (!gemm_pair_enabled() || rows <= 128 || n < 256 || (n & 7) || (k & 7)) return 1;
+  const int tiles = ((rows + 255) / 256) * ((n + 255) / 256), pairs = sm_count() / 2, kb = (k + kTileK - 1) / kTileK;
+  int best = 1;
+  double cost = 1e30;
+  for (int s = 1; s <= 4; ++s) {
+    const int per = (kb + s - 1) / s;
+    if ((s - 1) * per >= kb) continue;
+    const int laps = (tiles * s + pairs - 1) / pairs;
+    const double c = laps * per + 16.0 + (s > 1 ? double(s) * rows * n * 8.0 / 1e6 : 0.0);
+    if (c < cost * (s > 1 ? 0.97 : 1.0)) {
+      cost = c;
+      best = s;
+    }
+  }
+  return best;
 }
 
 // arrival counts (per owner) of a pushed linear: one per 128-row x 256-column tile of a CTA, in the

@@ -33,3 +33,34 @@ def test_token_major_silu_mul(ext, m, n, k, bias):
     assert rel_l2(out, want) < TOL and float(buf[0]) == 0.0
     torch.cuda.synchronize()
     assert ext.gemm_error_flag(0) == 0
+
+
+# the paired-CTA kernel from 129 rows on: ragged row and column tiles, k-blocks that the splits do not divide.
+# Against float64; one bf16 rounding of the result (2^-9 relative), twice that for SiLU*mul: rel-L2 2^-8
+@pytest.mark.parametrize("rows", [129, 256, 257, 333, 511])
+@pytest.mark.parametrize("n,k", [(256, 512), (272, 4104), (3600, 2048), (512, 18944)])
+def test_paired_kernel_few_rows(ext, rows, n, k):
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    x = torch.randn(rows, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(n, k, generator=g, device="cuda") * 0.05).bfloat16()
+    b = torch.randn(n, generator=g, device="cuda").bfloat16()
+    want = x.double() @ w.double().t()
+    rel = lambda a, c: float((a.double() - c).norm() / c.norm())
+    assert rel(ext.linear(x, w), want) < 2.0 ** -8
+    assert rel(ext.linear(x, w, b), want + b.double()) < 2.0 ** -8
+    y = want + b.double()
+    silu = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+    assert rel(ext.linear(x, w, b, None, True), silu) < 2.0 ** -8
+    r = torch.randn(rows, n, generator=g, device="cuda").bfloat16()
+    assert rel(ext.linear(x, w, b, r), y + r.double()) < 2.0 ** -8  # a residual keeps the product whole
+    torch.cuda.synchronize()
+    assert ext.gemm_error_flag(0) == 0
+
+
+def test_row_splits_rule(ext):
+    assert ext.gemm_row_splits(128, 3584, 18944) == 1  # the swapped form
+    assert ext.gemm_row_splits(333, 3584, 18944) >= 2  # 28 tiles for 74 pairs
+    assert ext.gemm_row_splits(333, 37888, 3584) == 1 and ext.gemm_row_splits(8192, 3584, 18944) == 1
+    for rows, n, k in [(129, 256, 64), (129, 256, 128), (300, 512, 200), (2000, 3584, 18944)]:
+        s, kb = ext.gemm_row_splits(rows, n, k), -(-k // 64)
+        assert (s - 1) * -(-kb // s) < kb  # no empty split

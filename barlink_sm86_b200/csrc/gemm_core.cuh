@@ -179,31 +179,32 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmap_a, const CUten
   const int units = tiles * g.splits;
   const int kb_per = (g.kblocks + g.splits - 1) / g.splits;
 
-  // operand loads of one stage: 2-D tensor copies, or bulk copies of pre-tiled weights
+  // operand loads of one stage (the elected lane of the producer warp issues): 2-D tensor copies, or bulk copies of pre-tiled weights
+  const uint32_t leader = elect_leader();
   auto load_a = [&](uint32_t dst, uint32_t bar, int kb, int ta) {
     if (!W8 && g.tiled == 1)
-      bulk_load_s(dst, g.tiled_base + (size_t(ta) * g.tiled_kblocks + kb) * S::kStageA, S::kStageA, bar,
+      bulk_load_warp(leader, dst, g.tiled_base + (size_t(ta) * g.tiled_kblocks + kb) * S::kStageA, S::kStageA, bar,
                   hint_a);
     else
-      tma_load_2d_hint_s(dst, tmap_a, bar, kb * (MODE ? 2 * kTileK : kTileK), ta * kTileA, hint_a);
+      tma_load_2d_hint_warp(leader, dst, tmap_a, bar, kb * (MODE ? 2 * kTileK : kTileK), ta * kTileA, hint_a);
   };
   auto load_b = [&](uint32_t dst, uint32_t bar, int kb, int tb) {
     if (!W8 && g.tiled == 2) {
       if constexpr (BN <= kTileA) {
         const int r0 = tb * BN;
-        bulk_load_s(dst,
+        bulk_load_warp(leader, dst,
                     g.tiled_base + (size_t(r0 / kTileA) * g.tiled_kblocks + kb) * S::kStageA +
                         size_t(r0 % kTileA) * 128,
                     BN * 128, bar, hint_b);
       } else {
 #pragma unroll
         for (int h = 0; h < BN / kTileA; ++h)
-          bulk_load_s(dst + h * S::kStageA,
+          bulk_load_warp(leader, dst + h * S::kStageA,
                       g.tiled_base + (size_t(tb * (BN / kTileA) + h) * g.tiled_kblocks + kb) * S::kStageA,
                       S::kStageA, bar, hint_b);
       }
     } else {
-      tma_load_2d_hint_s(dst, tmap_b, bar, kb * (MODE ? 2 * kTileK : kTileK), tb * BN, hint_b);
+      tma_load_2d_hint_warp(leader, dst, tmap_b, bar, kb * (MODE ? 2 * kTileK : kTileK), tb * BN, hint_b);
     }
   };
 
@@ -237,30 +238,30 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmap_a, const CUten
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      // Weights do not depend on the kernels before this one: the first lap
-      // of weight tiles is requested before waiting for them, so HBM keeps
-      // streaming across the kernel boundary.  Activation tiles follow once
-      // the predecessors have completed.
-      int pre = 0;
-      for (int u = blockIdx.x; g.weights_in_a != 2 && u < units && pre < S::kStages; u += gridDim.x) {
-        const int tile = u / g.splits, sp = u - tile * g.splits;
-        const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
-        const int kb0 = sp * kb_per;
-        const int kb1 = min(g.kblocks, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1 && pre < S::kStages; kb += S::kKS, ++pre) {
-          const int nsub = S::kKS == 1 ? 1 : min(S::kKS, kb1 - kb);  // k-blocks in this stage
-          mbar_expect_tx(&full_bar[pre], S::kTxBytes - (S::kKS - nsub) * S::kStageB);
-          const uint32_t sa = ring + pre * S::kStageBytes;
-          if (g.weights_in_a)
-            load_a(sa + (W8 ? S::kOffRaw : 0), smem_u32(&full_bar[pre]), kb, ta);
-          else
-            load_b(sa + S::kOffB, smem_u32(&full_bar[pre]), kb, tb);
-        }
+    // Weights do not depend on the kernels before this one: the first lap
+    // of weight tiles is requested before waiting for them, so HBM keeps
+    // streaming across the kernel boundary.  Activation tiles follow once
+    // the predecessors have completed.
+    int pre = 0;
+    for (int u = blockIdx.x; g.weights_in_a != 2 && u < units && pre < S::kStages; u += gridDim.x) {
+      const int tile = u / g.splits, sp = u - tile * g.splits;
+      const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
+      const int kb0 = sp * kb_per;
+      const int kb1 = min(g.kblocks, kb0 + kb_per);
+      for (int kb = kb0; kb < kb1 && pre < S::kStages; kb += S::kKS, ++pre) {
+        const int nsub = S::kKS == 1 ? 1 : min(S::kKS, kb1 - kb);  // k-blocks in this stage
+        mbar_expect_tx_warp(leader, &full_bar[pre], S::kTxBytes - (S::kKS - nsub) * S::kStageB);
+        const uint32_t sa = ring + pre * S::kStageBytes;
+        if (g.weights_in_a)
+          load_a(sa + (W8 ? S::kOffRaw : 0), smem_u32(&full_bar[pre]), kb, ta);
+        else
+          load_b(sa + S::kOffB, smem_u32(&full_bar[pre]), kb, tb);
       }
-      pdl_wait();
-      if (tr) tr[2] = globaltimer_ns();
-      if (g.gate_flags) {
+    }
+    pdl_wait();
+    if (tr && lane == 0) tr[2] = globaltimer_ns();
+    if (g.gate_flags) {
+      if (lane == 0) {
         const uint32_t want = *reinterpret_cast<volatile uint32_t*>(g.gate_cum) + g.gate_add;
         const uint64_t t0 = globaltimer_ns();
         for (int f = 0; f < g.gate_n; ++f) {
@@ -273,72 +274,70 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap* tmap_a, const CUten
           }
           if (*s_abort) break;
         }
-        // the rows were written by other GPUs and are read next by the TMA unit
-        asm volatile("fence.proxy.async;" ::: "memory");
       }
-      int stage = 0;
-      uint32_t phase = 0;
-      int armed = 0;
-      bool ok = !*s_abort;
-      if (!ok && pre > 0) {
-        // weight tiles of the first lap are in flight with half of their bytes
-        // expected: complete the stages with the activation tiles anyway so
-        // that the copies land before the CTA leaves
-        ok = true;
-      }
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        const int tile = u / g.splits, sp = u - tile * g.splits;
-        const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
-        const int kb0 = sp * kb_per;
-        const int kb1 = min(g.kblocks, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; kb += S::kKS) {
-          if (*s_abort && armed >= pre) {
+      __syncwarp();
+      // the rows were written by other GPUs and are read next by the TMA unit
+      asm volatile("fence.proxy.async;" ::: "memory");
+    }
+    int stage = 0;
+    uint32_t phase = 0;
+    int armed = 0;
+    // weight tiles of the first lap may be in flight with half of their bytes expected: after a gate that
+    // timed out the stages are completed with the activation tiles anyway so that the copies land before
+    // the CTA leaves
+    bool ok = pre > 0 || !g.gate_flags || !__any_sync(0xffffffffu, *s_abort != 0);
+    bool ready = false;  // the next stage is free (asked for one stage ahead, as in the MMA warp)
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int tile = u / g.splits, sp = u - tile * g.splits;
+      const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
+      const int kb0 = sp * kb_per;
+      const int kb1 = min(g.kblocks, kb0 + kb_per);
+      for (int kb = kb0; kb < kb1; kb += S::kKS) {
+        const int nsub = S::kKS == 1 ? 1 : min(S::kKS, kb1 - kb);
+        const uint32_t sa = ring + stage * S::kStageBytes;
+        uint64_t* full = &full_bar[stage];
+        const bool early = armed < pre;  // weight tile of this stage is already on its way
+        if (!early) {
+          if (!ready) ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort);
+          if (g.gate_flags) ok = ok && !*s_abort;
+          if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
           }
-          const int nsub = S::kKS == 1 ? 1 : min(S::kKS, kb1 - kb);
-          const uint32_t sa = ring + stage * S::kStageBytes;
-          const bool early = armed < pre;  // weight tile of this stage is already on its way
-          if (!early) {
-            if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort)) {
-              ok = false;
-              break;
-            }
-            mbar_expect_tx(&full_bar[stage], S::kTxBytes - (S::kKS - nsub) * S::kStageB);
-          }
-          if (!early || !g.weights_in_a)
-            load_a(sa + (W8 ? S::kOffRaw : 0), smem_u32(&full_bar[stage]), kb, ta);
-          if (!early || g.weights_in_a) {
+          mbar_expect_tx_warp(leader, full, S::kTxBytes - (S::kKS - nsub) * S::kStageB);
+        }
+        ++armed;
+        if (++stage == S::kStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        ready = armed >= pre && mbar_test_wait(&empty_bar[stage], phase ^ 1u);
+        if (!early || !g.weights_in_a)
+          load_a(sa + (W8 ? S::kOffRaw : 0), smem_u32(full), kb, ta);
+        if (!early || g.weights_in_a) {
 #pragma unroll
-            for (int sb = 0; sb < S::kKS; ++sb)
-              if (sb < nsub) load_b(sa + S::kOffB + sb * S::kStageB, smem_u32(&full_bar[stage]), kb + sb, tb);
-          }
-          ++armed;
-          if (++stage == S::kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          for (int sb = 0; sb < S::kKS; ++sb)
+            if (sb < nsub) load_b(sa + S::kOffB + sb * S::kStageB, smem_u32(full), kb + sb, tb);
         }
       }
-      if (!ok) {
-        // Let copies that are still in flight land before the CTA goes away:
-        // the stages armed in the last lap complete their full barriers.
-        int n = armed < S::kStages ? armed : S::kStages;
-        int s = stage;
-        uint32_t ph = phase;
-        for (int i = 0; i < n; ++i) {
-          if (--s < 0) {
-            s = S::kStages - 1;
-            ph ^= 1u;
-          }
-          for (uint32_t p = 0; p < (1u << 20); ++p)
-            if (mbar_try_wait(&full_bar[s], ph)) break;
+    }
+    if (!ok) {
+      // Let copies that are still in flight land before the CTA goes away:
+      // the stages armed in the last lap complete their full barriers.
+      int n = armed < S::kStages ? armed : S::kStages;
+      int s = stage;
+      uint32_t ph = phase;
+      for (int i = 0; i < n; ++i) {
+        if (--s < 0) {
+          s = S::kStages - 1;
+          ph ^= 1u;
         }
+        for (uint32_t p = 0; p < (1u << 20); ++p)
+          if (mbar_try_wait(&full_bar[s], ph)) break;
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------
-    const uint32_t leader = elect_leader();
     const uint32_t idesc = MODE ? umma_idesc_i8(kTileA, BN) : umma_idesc_f16(kTileA, BN, g.ab_fmt);
     int stage = 0, astage = 0, acc = 0;
     uint32_t phase = 0, aphase = 0;

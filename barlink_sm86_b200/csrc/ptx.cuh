@@ -233,6 +233,35 @@ __device__ __forceinline__ void bulk_load_s(uint32_t smem_dst, const void* gsrc,
       "l"(gsrc), "r"(bytes), "r"(bar), "l"(hint)
       : "memory");
 }
+// Both for a whole converged warp, of which the elected lane issues (see elect_leader).
+__device__ __forceinline__ void tma_load_2d_hint_warp(uint32_t leader, uint32_t smem_dst, const void* tmap,
+                                                      uint32_t bar, int x, int y, uint64_t hint) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;\n\t}" ::"r"(smem_dst),
+      "l"(tmap), "r"(bar), "r"(x), "r"(y), "l"(hint), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_load_warp(uint32_t leader, uint32_t smem_dst, const void* gsrc, uint32_t bytes,
+                                               uint32_t bar, uint64_t hint) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1], %2, [%3], %4;\n\t}" ::"r"(smem_dst),
+      "l"(gsrc), "r"(bytes), "r"(bar), "l"(hint), "r"(leader)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_warp(uint32_t leader, uint64_t* bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
+      "r"(bytes), "r"(leader)
+      : "memory");
+}
 // createpolicy-equivalent constants (the encodings CUTLASS ships as
 // TMA::CacheHintSm90): stream weights through L2, keep activations.
 constexpr uint64_t kHintEvictFirst = 0x12F0000000000000ull;

@@ -148,68 +148,68 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
 
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
-      auto load_a = [&](uint32_t dst, uint64_t* bar, int kb, int ta) {
-        if constexpr (SRC == kRows)
-          tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), kb * kQK, ta * kQRows, kHintEvictFirst);
-        else if constexpr (SRC == kNibbles)
-          tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), ta * kQRows, kb * (kQK / 8), kHintEvictFirst);
-        else  // eight chunks of 128 rows, in elements of 8 bytes
-          tma_load_2d_hint_s(dst, &tmap_w, smem_u32(bar), ta * kQRows * 2, kb * (kQK / 16), kHintEvictFirst);
-      };
-      // the first lap of weight tiles is requested before the kernels ahead have finished
-      int pre = 0;
-      for (int u = blockIdx.x; u < units && pre < S::kStages; u += gridDim.x) {
-        const int tile = u / g.splits, sp = u - tile * g.splits, ta = tile / g.tiles_b;
-        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1 && pre < S::kStages; ++kb, ++pre) {
-          mbar_expect_tx(&full_bar[pre], S::kStage);
-          load_a(ring + pre * S::kStage, &full_bar[pre], kb, ta);
-        }
+    const uint32_t leader = elect_leader();
+    auto load_a = [&](uint32_t dst, uint64_t* bar, int kb, int ta) {
+      if constexpr (SRC == kRows)
+        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(bar), kb * kQK, ta * kQRows, kHintEvictFirst);
+      else if constexpr (SRC == kNibbles)
+        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(bar), ta * kQRows, kb * (kQK / 8), kHintEvictFirst);
+      else  // eight chunks of 128 rows, in elements of 8 bytes
+        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(bar), ta * kQRows * 2, kb * (kQK / 16), kHintEvictFirst);
+    };
+    // the first lap of weight tiles is requested before the kernels ahead have finished
+    int pre = 0;
+    for (int u = blockIdx.x; u < units && pre < S::kStages; u += gridDim.x) {
+      const int tile = u / g.splits, sp = u - tile * g.splits, ta = tile / g.tiles_b;
+      const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+      for (int kb = kb0; kb < kb1 && pre < S::kStages; ++kb, ++pre) {
+        mbar_expect_tx_warp(leader, &full_bar[pre], S::kStage);
+        load_a(ring + pre * S::kStage, &full_bar[pre], kb, ta);
       }
-      pdl_wait();
-      int stage = 0, armed = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-        const int tile = u / g.splits, sp = u - tile * g.splits;
-        const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
-        const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (*s_abort && armed >= pre) {
+    }
+    pdl_wait();
+    int stage = 0, armed = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    bool ready = false;  // the next stage is free (asked for one stage ahead, as in the MMA warp)
+    for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+      const int tile = u / g.splits, sp = u - tile * g.splits;
+      const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
+      const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const uint32_t dst = ring + stage * S::kStage;
+        uint64_t* full = &full_bar[stage];
+        const bool early = armed < pre;  // weight tile of this stage is already on its way
+        if (!early) {
+          if (!ready) ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort);
+          if (!__all_sync(0xffffffffu, ok)) {
             ok = false;
             break;
           }
-          const uint32_t dst = ring + stage * S::kStage;
-          if (armed >= pre) {
-            if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort)) {
-              ok = false;
-              break;
-            }
-            mbar_expect_tx(&full_bar[stage], S::kStage);
-            load_a(dst, &full_bar[stage], kb, ta);
-          }
-          tma_load_2d_hint_s(dst + S::kStageA, &tmap_x, smem_u32(&full_bar[stage]), kb * kQK, tb * S::BN, kHintEvictLast);
-          ++armed;
-          if (++stage == S::kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          mbar_expect_tx_warp(leader, full, S::kStage);
         }
+        ++armed;
+        if (++stage == S::kStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        ready = armed >= pre && mbar_test_wait(&empty_bar[stage], phase ^ 1u);
+        if (!early) load_a(dst, full, kb, ta);
+        tma_load_2d_hint_warp(leader, dst + S::kStageA, &tmap_x, smem_u32(full), kb * kQK, tb * S::BN, kHintEvictLast);
       }
-      if (!ok) {
-        // copies still in flight land before the CTA goes away
-        const int n = armed < S::kStages ? armed : S::kStages;
-        int s = stage;
-        uint32_t ph = phase;
-        for (int i = 0; i < n; ++i) {
-          if (--s < 0) {
-            s = S::kStages - 1;
-            ph ^= 1u;
-          }
-          for (uint32_t p = 0; p < (1u << 20); ++p)
-            if (mbar_try_wait(&full_bar[s], ph)) break;
+    }
+    if (!ok) {
+      // copies still in flight land before the CTA goes away
+      const int n = armed < S::kStages ? armed : S::kStages;
+      int s = stage;
+      uint32_t ph = phase;
+      for (int i = 0; i < n; ++i) {
+        if (--s < 0) {
+          s = S::kStages - 1;
+          ph ^= 1u;
         }
+        for (uint32_t p = 0; p < (1u << 20); ++p)
+          if (mbar_try_wait(&full_bar[s], ph)) break;
       }
     }
   } else if (warp == 1) {

@@ -94,9 +94,13 @@ __global__ void __launch_bounds__(256) k_transpose_v(const __nv_bfloat16* __rest
     *reinterpret_cast<uint4*>(&tile[r][c]) = val;
   }
   __syncthreads();
-  // 128 dims x 64 tokens out: 8 threads per dim row, 8 tokens each
-  for (int i = threadIdx.x; i < kTcHD * 8; i += 256) {
-    const int d = i >> 3, c = (i & 7) * 8;
+  // 128 dims x 64 tokens out: a warp owns 16 dims and writes whole 32-byte sectors (two lanes side by side);
+  // its shared-memory reads conflict two-fold (eight lanes per dim row read one bank eight-fold: 4608 tokens
+  // of 24 heads took 25 us)
+  const int d = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15), half = (threadIdx.x >> 4) & 1;
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int c = it * 16 + half * 8;
     __align__(16) __nv_bfloat16 o[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = tile[c + j][d];
@@ -206,32 +210,32 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0) {
+      const uint32_t leader = elect_leader();
       const uint32_t idesc_s = umma_idesc_f16(kTcBM, kTcBKV, 1);
       const uint32_t idesc_o = umma_idesc_f16(kTcBM, kTcHD, 1);
       auto issue_s = [&](int t, int stage) {
         const uint32_t kb = base + kTcOffKV + stage * kTcStageBytes;
+        const uint64_t dq = umma_desc_k_sw128(base + t * kTcQBytes), dk = umma_desc_k_sw128(kb);
 #pragma unroll
-        for (int ks = 0; ks < kTcHD / 16; ++ks) {
-          const uint64_t da = umma_desc_k_sw128(base + t * kTcQBytes + (ks >> 2) * (kTcQBytes / 2)) + uint64_t(2 * (ks & 3));
-          const uint64_t db = umma_desc_k_sw128(kb + (ks >> 2) * (kTcKBytes / 2)) + uint64_t(2 * (ks & 3));
-          umma_f16_ss(tmem_base + uint32_t(t * kTcBKV), da, db, idesc_s, ks > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_ready[t]);
+        for (int ks = 0; ks < kTcHD / 16; ++ks)
+          umma_f16_ss_warp(leader, tmem_base + uint32_t(t * kTcBKV),
+                           dq + uint64_t((ks >> 2) * (kTcQBytes / 32) + 2 * (ks & 3)),
+                           dk + uint64_t((ks >> 2) * (kTcKBytes / 32) + 2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
+        umma_commit_warp(leader, &s_ready[t]);
       };
       auto issue_pv = [&](int t, int stage, bool acc) {
-        const uint32_t vb = base + kTcOffKV + stage * kTcStageBytes + kTcKBytes;
+        const uint64_t dp = umma_desc_k_sw128(base + kTcOffP + t * kTcPBytes);
+        const uint64_t dv = umma_desc_k_sw128(base + kTcOffKV + stage * kTcStageBytes + kTcKBytes);
 #pragma unroll
-        for (int ks = 0; ks < kTcBKV / 16; ++ks) {
-          const uint64_t da = umma_desc_k_sw128(base + kTcOffP + t * kTcPBytes) + uint64_t(2 * ks);
-          const uint64_t db = umma_desc_k_sw128(vb) + uint64_t(2 * ks);
-          umma_f16_ss(tmem_base + 128u + uint32_t(t * kTcHD), da, db, idesc_o, (acc || ks > 0) ? 1u : 0u);
-        }
+        for (int ks = 0; ks < kTcBKV / 16; ++ks)
+          umma_f16_ss_warp(leader, tmem_base + 128u + uint32_t(t * kTcHD), dp + uint64_t(2 * ks), dv + uint64_t(2 * ks),
+                           idesc_o, (acc || ks > 0) ? 1u : 0u);
       };
-      bool ok = mbar_wait_bounded(q_full, 0, s_abort);
+      bool ok = mbar_wait_bounded_warp(q_full, 0, s_abort);
       int stage = 0;
       uint32_t phase = 0;
-      if (ok) ok = mbar_wait_bounded(&kv_full[0], 0, s_abort);
+      if (ok) ok = mbar_wait_bounded_warp(&kv_full[0], 0, s_abort);
       if (ok) {
         tc_fence_after_sync();
         issue_s(0, 0);
@@ -245,25 +249,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           nphase ^= 1u;
         }
         const bool more = j + 1 < n_steps;
-        for (int t = 0; t < kTcTiles && ok; ++t) {
-          if (!mbar_wait_bounded(&p_ready[t], uint32_t(j) & 1u, s_abort)) {
-            ok = false;
-            break;
-          }
+#pragma unroll
+        for (int t = 0; t < kTcTiles; ++t) {
+          // the next keys are there long before the probabilities of these
+          bool here = mbar_wait_bounded(&p_ready[t], uint32_t(j) & 1u, s_abort);
+          if (t == 0 && more) here = here && mbar_wait_bounded(&kv_full[nstage], nphase, s_abort);
+          ok = __all_sync(0xffffffffu, here);
+          if (!ok) break;
           tc_fence_after_sync();
           issue_pv(t, stage, j > 0);
-          if (more) {
-            if (t == 0 && !mbar_wait_bounded(&kv_full[nstage], nphase, s_abort)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
-            issue_s(t, nstage);
-          } else {
-            umma_commit(&o_final[t]);
-          }
+          if (more) issue_s(t, nstage);
+          else umma_commit_warp(leader, &o_final[t]);
         }
-        if (ok) umma_commit(&kv_empty[stage]);
+        if (ok) umma_commit_warp(leader, &kv_empty[stage]);
         stage = nstage;
         phase = nphase;
       }

@@ -9,17 +9,20 @@
 // One CTA owns 256 query rows of one head as two 128-row tiles and walks the
 // keys in tiles of 64:
 //
-//   warp 0      TMA producer: Q once, then a 4-deep ring of (K tile, V^T tile)
-//   warp 1      one thread issues tcgen05.mma: S_t = Q_t K^T into TMEM (128x64 fp32),
+//   warp 0      TMA producer: Q once, then a ring of K tiles and a ring of V^T tiles
+//   warp 1      issues tcgen05.mma: S_t = Q_t K^T into TMEM (128x64 fp32, two buffers per tile),
 //               O_t += P_t V into TMEM (128x128 fp32), for tiles t = 0, 1 in turn
 //   warps 2-5   softmax of tile 0: every thread owns one query row (TMEM lane),
 //   warps 6-9   softmax of tile 1   reads its 64 scores with tcgen05.ld, keeps the
 //               running max and sum in registers, writes P (bf16) into shared
 //               memory in the swizzled K-major layout the tensor core reads
 //
-// While one tile's softmax runs, the tensor core works on the other tile
-// (order PV0_j, S0_j+1, PV1_j, S1_j+1), so neither side waits for long.  The
-// accumulator is rescaled only when the running max has grown by more than
+// What bounds it: the exponentials (16 a clock and SM: 1024 cycles for 64 keys x 256 rows, as many as the
+// products take) and, before S had two buffers, the chain softmax -> P V -> next S -> softmax of a tile, whose
+// links added up to 2700 cycles a step.  Now S of step j + 2 is issued right behind P V of step j, so a
+// tile's softmax always finds its scores; P has two buffers for the same reason, and a rescale of O waits
+// for the P V before it.  4608 tokens, 24 heads: ATTN_NOW.
+// The accumulator is rescaled only when the running max has grown by more than
 // 2^8 since the last rescale (the stale max is exact after the final division
 // by the row sum), which takes the TMEM read-modify-write out of the loop.
 // V is consumed as V^T [head_dim][keys] so that both operands of P V are
@@ -41,18 +44,19 @@ constexpr int kTcBM = 128;       // query rows per tile
 constexpr int kTcTiles = 2;      // tiles per CTA
 constexpr int kTcBKV = 64;       // keys per step
 constexpr int kTcHD = 128;
-constexpr int kTcStages = 4;
+constexpr int kTcStages = 3;     // K tiles and V^T tiles in flight, a ring each
 constexpr int kTcThreads = 320;
 constexpr uint32_t kTcQBytes = kTcBM * kTcHD * 2;          // 32 KiB per query tile
 constexpr uint32_t kTcPBytes = kTcBM * kTcBKV * 2;         // 16 KiB per P tile
 constexpr uint32_t kTcKBytes = kTcBKV * kTcHD * 2;         // 16 KiB
 constexpr uint32_t kTcVBytes = kTcHD * kTcBKV * 2;         // 16 KiB
-constexpr uint32_t kTcOffP = kTcTiles * kTcQBytes;
-constexpr uint32_t kTcOffKV = kTcOffP + kTcTiles * kTcPBytes;
-constexpr uint32_t kTcStageBytes = kTcKBytes + kTcVBytes;
-constexpr uint32_t kTcOffBar = kTcOffKV + kTcStages * kTcStageBytes;
+constexpr uint32_t kTcOffP = kTcTiles * kTcQBytes;         // [tile][even / odd step]
+constexpr uint32_t kTcOffK = kTcOffP + 2 * kTcTiles * kTcPBytes;
+constexpr uint32_t kTcOffV = kTcOffK + kTcStages * kTcKBytes;
+constexpr uint32_t kTcOffBar = kTcOffV + kTcStages * kTcVBytes;
 constexpr uint32_t kTcSmem = kTcOffBar + 256 + 1024;       // barriers + alignment slack
-constexpr uint32_t kTcTmemCols = 512;                      // S0 0-63, S1 64-127, O0 128-255, O1 256-383
+static_assert(kTcSmem <= 232448, "attention tiles do not fit the shared memory of one CTA");
+constexpr uint32_t kTcTmemCols = 512;                      // S of tile t, step parity p: 128 t + 64 p; O of tile t: 256 + 128 t
 constexpr float kTcRescale = 8.f;                          // log2 units
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -73,6 +77,22 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// two fp32 operations in one instruction, each rounded as its scalar form
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
 }
 
 // V [tokens, nkv, 128] (token stride v_stride) -> vt [nkv*128][batch*lpad]:
@@ -96,7 +116,7 @@ __global__ void __launch_bounds__(256) k_transpose_v(const __nv_bfloat16* __rest
   __syncthreads();
   // 128 dims x 64 tokens out: a warp owns 16 dims and writes whole 32-byte sectors (two lanes side by side);
   // its shared-memory reads conflict two-fold (eight lanes per dim row read one bank eight-fold: 4608 tokens
-  // of 24 heads took 25 us)
+  // of 24 heads took 25 us; VT_NOW)
   const int d = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15), half = (threadIdx.x >> 4) & 1;
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
@@ -119,13 +139,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   uint64_t* bars = reinterpret_cast<uint64_t*>(gen + kTcOffBar);
   uint64_t* q_full = bars;             // 1
-  uint64_t* kv_full = bars + 1;        // kTcStages
-  uint64_t* kv_empty = bars + 5;       // kTcStages
-  uint64_t* s_ready = bars + 9;        // 2
-  uint64_t* p_ready = bars + 11;       // 2
-  uint64_t* o_final = bars + 13;       // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
-  volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(bars + 17);
+  uint64_t* k_full = bars + 1;         // kTcStages each
+  uint64_t* k_empty = bars + 4;
+  uint64_t* v_full = bars + 7;
+  uint64_t* v_empty = bars + 10;
+  uint64_t* s_ready = bars + 13;       // [tile][step parity]
+  uint64_t* p_ready = bars + 17;       // [tile][step parity]
+  uint64_t* pv_done = bars + 21;       // [tile], one phase per step
+  uint64_t* o_final = bars + 26;       // [tile]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
+  volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(bars + 25);
 
   // cu_q / cu_k may come from the kernel just before this one
   pdl_launch_dependents();
@@ -147,12 +170,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int s = 0; s < kTcStages; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+      mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
+      mbar_init(&v_full[s], 1);
+      mbar_init(&v_empty[s], 1);
     }
     for (int t = 0; t < kTcTiles; ++t) {
-      mbar_init(&s_ready[t], 1);
-      mbar_init(&p_ready[t], kTcBM);
+      for (int p = 0; p < 2; ++p) {
+        mbar_init(&s_ready[2 * t + p], 1);
+        mbar_init(&p_ready[2 * t + p], kTcBM);
+      }
+      mbar_init(&pv_done[t], 1);
       mbar_init(&o_final[t], 1);
     }
     *s_abort = 0;
@@ -180,17 +208,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                              head * kTcHD + h * 64, q0 + row0 + t * kTcBM, kHintEvictFirst);
       int stage = 0;
       uint32_t phase = 0;
-      int issued = 0;
+      int k_issued = 0, v_issued = 0;
       for (int j = 0; j < n_steps; ++j) {
-        if (!mbar_wait_bounded(&kv_empty[stage], phase ^ 1u, s_abort)) break;
-        const uint32_t dst = base + kTcOffKV + stage * kTcStageBytes;
-        mbar_expect_tx(&kv_full[stage], kTcStageBytes);
+        if (!mbar_wait_bounded(&k_empty[stage], phase ^ 1u, s_abort)) break;
+        mbar_expect_tx(&k_full[stage], kTcKBytes);
         for (int h = 0; h < 2; ++h)
-          tma_load_2d_hint_s(dst + h * (kTcKBytes / 2), &tmap_k, smem_u32(&kv_full[stage]),
+          tma_load_2d_hint_s(base + kTcOffK + stage * kTcKBytes + h * (kTcKBytes / 2), &tmap_k, smem_u32(&k_full[stage]),
                              kvh * kTcHD + h * 64, k0 + j * kTcBKV, kHintEvictLast);
-        tma_load_2d_hint_s(dst + kTcKBytes, &tmap_vt, smem_u32(&kv_full[stage]), b * lpad + j * kTcBKV,
+        ++k_issued;
+        if (!mbar_wait_bounded(&v_empty[stage], phase ^ 1u, s_abort)) break;
+        mbar_expect_tx(&v_full[stage], kTcVBytes);
+        tma_load_2d_hint_s(base + kTcOffV + stage * kTcVBytes, &tmap_vt, smem_u32(&v_full[stage]), b * lpad + j * kTcBKV,
                            kvh * kTcHD, kHintEvictLast);
-        ++issued;
+        ++v_issued;
         if (++stage == kTcStages) {
           stage = 0;
           phase ^= 1u;
@@ -198,12 +228,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       if (*s_abort) {
         // leaving early: let the copies still in flight land before the CTA exits
-        for (int j = max(0, issued - kTcStages); j < issued; ++j) {
-          const int s = j % kTcStages;
-          const uint32_t ph = uint32_t(j / kTcStages) & 1u;
-          for (uint32_t p = 0; p < (1u << 20); ++p)
-            if (mbar_try_wait(&kv_full[s], ph)) break;
-        }
+        auto drain = [&](uint64_t* full, int issued) {
+          for (int j = max(0, issued - kTcStages); j < issued; ++j)
+            for (uint32_t p = 0; p < (1u << 20); ++p)
+              if (mbar_try_wait(&full[j % kTcStages], uint32_t(j / kTcStages) & 1u)) break;
+        };
+        drain(k_full, k_issued);
+        drain(v_full, v_issued);
         for (uint32_t p = 0; p < (1u << 20); ++p)
           if (mbar_try_wait(q_full, 0)) break;
       }
@@ -214,56 +245,70 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const uint32_t leader = elect_leader();
       const uint32_t idesc_s = umma_idesc_f16(kTcBM, kTcBKV, 1);
       const uint32_t idesc_o = umma_idesc_f16(kTcBM, kTcHD, 1);
-      auto issue_s = [&](int t, int stage) {
-        const uint32_t kb = base + kTcOffKV + stage * kTcStageBytes;
-        const uint64_t dq = umma_desc_k_sw128(base + t * kTcQBytes), dk = umma_desc_k_sw128(kb);
+      // S of a step with parity p, from K stage ks0
+      auto issue_s = [&](int t, int p, int kst) {
+        const uint64_t dq = umma_desc_k_sw128(base + t * kTcQBytes), dk = umma_desc_k_sw128(base + kTcOffK + kst * kTcKBytes);
 #pragma unroll
         for (int ks = 0; ks < kTcHD / 16; ++ks)
-          umma_f16_ss_warp(leader, tmem_base + uint32_t(t * kTcBKV),
+          umma_f16_ss_warp(leader, tmem_base + uint32_t(t * 128 + p * kTcBKV),
                            dq + uint64_t((ks >> 2) * (kTcQBytes / 32) + 2 * (ks & 3)),
                            dk + uint64_t((ks >> 2) * (kTcKBytes / 32) + 2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
-        umma_commit_warp(leader, &s_ready[t]);
+        umma_commit_warp(leader, &s_ready[2 * t + p]);
       };
-      auto issue_pv = [&](int t, int stage, bool acc) {
-        const uint64_t dp = umma_desc_k_sw128(base + kTcOffP + t * kTcPBytes);
-        const uint64_t dv = umma_desc_k_sw128(base + kTcOffKV + stage * kTcStageBytes + kTcKBytes);
+      auto issue_pv = [&](int t, int p, int vst, bool acc) {
+        const uint64_t dp = umma_desc_k_sw128(base + kTcOffP + (2 * t + p) * kTcPBytes);
+        const uint64_t dv = umma_desc_k_sw128(base + kTcOffV + vst * kTcVBytes);
 #pragma unroll
         for (int ks = 0; ks < kTcBKV / 16; ++ks)
-          umma_f16_ss_warp(leader, tmem_base + 128u + uint32_t(t * kTcHD), dp + uint64_t(2 * ks), dv + uint64_t(2 * ks),
+          umma_f16_ss_warp(leader, tmem_base + 256u + uint32_t(t * kTcHD), dp + uint64_t(2 * ks), dv + uint64_t(2 * ks),
                            idesc_o, (acc || ks > 0) ? 1u : 0u);
+        umma_commit_warp(leader, &pv_done[t]);
       };
       bool ok = mbar_wait_bounded_warp(q_full, 0, s_abort);
-      int stage = 0;
-      uint32_t phase = 0;
-      if (ok) ok = mbar_wait_bounded_warp(&kv_full[0], 0, s_abort);
-      if (ok) {
+      // scores of the first two steps
+      int kst = 0, vst = 0;
+      uint32_t kphase = 0, vphase = 0;
+      for (int j = 0; j < min(2, n_steps) && ok; ++j) {
+        ok = mbar_wait_bounded_warp(&k_full[kst], kphase, s_abort);
+        if (!ok) break;
         tc_fence_after_sync();
-        issue_s(0, 0);
-        issue_s(1, 0);
+        issue_s(0, j, kst);
+        issue_s(1, j, kst);
+        umma_commit_warp(leader, &k_empty[kst]);
+        ++kst;
       }
       for (int j = 0; j < n_steps && ok; ++j) {
-        int nstage = stage + 1;
-        uint32_t nphase = phase;
-        if (nstage == kTcStages) {
-          nstage = 0;
-          nphase ^= 1u;
-        }
-        const bool more = j + 1 < n_steps;
+        const int p = j & 1;
+        const bool more = j + 2 < n_steps;
 #pragma unroll
         for (int t = 0; t < kTcTiles; ++t) {
-          // the next keys are there long before the probabilities of these
-          bool here = mbar_wait_bounded(&p_ready[t], uint32_t(j) & 1u, s_abort);
-          if (t == 0 && more) here = here && mbar_wait_bounded(&kv_full[nstage], nphase, s_abort);
+          bool here = mbar_wait_bounded(&p_ready[2 * t + p], uint32_t(j >> 1) & 1u, s_abort);
+          // the next tiles are there long before the probabilities
+          if (t == 0) {
+            here = here && mbar_wait_bounded(&v_full[vst], vphase, s_abort);
+            if (more) here = here && mbar_wait_bounded(&k_full[kst], kphase, s_abort);
+          }
           ok = __all_sync(0xffffffffu, here);
           if (!ok) break;
           tc_fence_after_sync();
-          issue_pv(t, stage, j > 0);
-          if (more) issue_s(t, nstage);
-          else umma_commit_warp(leader, &o_final[t]);
+          issue_pv(t, p, vst, j > 0);
+          if (more) issue_s(t, p, kst);
+          // (a wait for the last phase of pv_done could be answered by the last but two)
+          if (j + 1 == n_steps) umma_commit_warp(leader, &o_final[t]);
         }
-        if (ok) umma_commit_warp(leader, &kv_empty[stage]);
-        stage = nstage;
-        phase = nphase;
+        if (!ok) break;
+        umma_commit_warp(leader, &v_empty[vst]);
+        if (++vst == kTcStages) {
+          vst = 0;
+          vphase ^= 1u;
+        }
+        if (more) {
+          umma_commit_warp(leader, &k_empty[kst]);
+          if (++kst == kTcStages) {
+            kst = 0;
+            kphase ^= 1u;
+          }
+        }
       }
     }
   } else {
@@ -273,27 +318,34 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int row = quarter * 32 + lane;           // row inside the tile
     const int qi = row0 + t * kTcBM + row;         // query index inside the sequence
     const uint32_t lane_addr = tmem_base + (uint32_t(quarter * 32) << 16);
-    const uint32_t s_addr = lane_addr + uint32_t(t * kTcBKV);
-    const uint32_t o_addr = lane_addr + 128u + uint32_t(t * kTcHD);
-    const uint32_t p_row = base + kTcOffP + t * kTcPBytes + row * 128;
+    const uint32_t s_tile = lane_addr + uint32_t(t * 128);
+    const uint32_t o_addr = lane_addr + 256u + uint32_t(t * kTcHD);
+    const uint32_t p_tile = base + kTcOffP + 2 * t * kTcPBytes + row * 128;
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_steps; ++j) {
-      if (!mbar_wait_bounded(&s_ready[t], uint32_t(j) & 1u, s_abort)) {
+      const int p = j & 1;
+      if (!mbar_wait_bounded_warp(&s_ready[2 * t + p], uint32_t(j >> 1) & 1u, s_abort)) {
         ok = false;
         break;
       }
       tc_fence_after_sync();
+      const uint32_t s_addr = s_tile + uint32_t(p * kTcBKV), p_row = p_tile + p * kTcPBytes;
       float s[kTcBKV];
       {
         uint32_t r0[32], r1[32];
         tmem_ld_32x32(s_addr, r0);
         tmem_ld_32x32(s_addr + 32, r1);
         tmem_ld_wait();
+        const float2 sl = make_float2(scale_log2, scale_log2);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          s[c] = __uint_as_float(r0[c]) * scale_log2;
-          s[c + 32] = __uint_as_float(r1[c]) * scale_log2;
+        for (int c = 0; c < 32; c += 2) {
+          const float2 a = mul2(make_float2(__uint_as_float(r0[c]), __uint_as_float(r0[c + 1])), sl);
+          const float2 b = mul2(make_float2(__uint_as_float(r1[c]), __uint_as_float(r1[c + 1])), sl);
+          s[c] = a.x;
+          s[c + 1] = a.y;
+          s[c + 32] = b.x;
+          s[c + 33] = b.y;
         }
       }
       const int kbase = j * kTcBKV;
@@ -303,16 +355,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (int c = 0; c < kTcBKV; ++c)
           if (kbase + c >= lim) s[c] = -INFINITY;
       }
-      float mx = s[0];
+      // four chains: the maximum is on the way from the scores to everything else
+      float mx4[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-      for (int c = 1; c < kTcBKV; ++c) mx = fmaxf(mx, s[c]);
+      for (int c = 4; c < kTcBKV; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], s[c]);
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       const float m_new = fmaxf(m_used, mx);
       const bool grow = m_new > m_used + kTcRescale;          // also true on the first finite max
       if (__any_sync(0xffffffffu, grow)) {
         const float alpha = (m_new == -INFINITY) ? 1.f : ex2_approx(m_used - m_new);
         if (j > 0) {
-          // PV of the previous step has completed: its MMAs were issued before the
-          // S that s_ready just announced, and the tensor pipe runs in order
+          // P V of the previous step may still be running
+          if (!mbar_wait_bounded_warp(&pv_done[t], uint32_t(j - 1) & 1u, s_abort)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
 #pragma unroll 1
           for (int c0 = 0; c0 < kTcHD; c0 += 32) {
             uint32_t r[32];
@@ -328,15 +386,18 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         m_used = m_new;
       }
       const float mref = (m_used == -INFINITY) ? 0.f : m_used;
-      float sum = 0.f;
+      const float2 neg = make_float2(-mref, -mref);
+      float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       uint32_t pk[kTcBKV / 2];
 #pragma unroll
       for (int c = 0; c < kTcBKV; c += 2) {
-        const float p0 = ex2_approx(s[c] - mref), p1 = ex2_approx(s[c + 1] - mref);
-        sum += p0 + p1;
-        pk[c >> 1] = pack_bf16x2(p0, p1);
+        const float2 x = add2(make_float2(s[c], s[c + 1]), neg);
+        const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
+        sum[(c >> 1) & 1] = add2(sum[(c >> 1) & 1], e);
+        pk[c >> 1] = pack_bf16x2(e.x, e.y);
       }
-      l += sum;
+      sum[0] = add2(sum[0], sum[1]);
+      l += sum[0].x + sum[0].y;
 #pragma unroll
       for (int c = 0; c < 8; ++c)
         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(p_row + ((c ^ (row & 7)) << 4)),
@@ -344,7 +405,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                      : "memory");
       fence_proxy_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(&p_ready[t]);
+      mbar_arrive(&p_ready[2 * t + p]);
     }
     // ------------------------------ output --------------------------------
     const bool valid = qi < lq;
@@ -352,7 +413,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (n_steps == 0) {
       if (valid)
         for (int c = 0; c < kTcHD; c += 8) *reinterpret_cast<uint4*>(orow + c) = make_uint4(0, 0, 0, 0);
-    } else if (ok && mbar_wait_bounded(&o_final[t], 0, s_abort)) {
+    } else if (ok && mbar_wait_bounded_warp(&o_final[t], 0, s_abort)) {
       tc_fence_after_sync();
       const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll 1

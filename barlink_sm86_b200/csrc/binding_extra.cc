@@ -481,9 +481,11 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
                       w8_scratch(dev).err_flag.data_ptr(), st);
 }
 
-// GPTQ-v1 int4 linear: 1..16 rows use the GEMV; more rows widen the weight and use the bf16 GEMM
+// GPTQ-v1 int4 linear.  Groups of 128 and 5..128 rows: int8 digits of the activations on the tensor cores
+// (qlin_kernels.cu); else the GEMV up to 16 rows; else widen the weight and use the bf16 GEMM.
+// silu_mul: SiLU(gate) * up over interleaved (gate, up) columns.  want_slabs: see qlin_product.
 at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at::Tensor& scales,
-                        const at::Tensor& qzeros, int group, int splits) {
+                        const at::Tensor& qzeros, int group, int splits, bool silu_mul, bool want_slabs) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.is_contiguous(),
               "barlink: x must be a contiguous 2-D bfloat16 CUDA tensor");
   TORCH_CHECK(qweight.is_cuda() && qweight.is_contiguous() && qweight.scalar_type() == at::kInt &&
@@ -500,18 +502,36 @@ at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at
   const int dev = x.device().index();
   c10::cuda::CUDAGuard guard(x.device());
   void* st = at::cuda::getCurrentCUDAStream(dev).stream();
-  if (m == 0) return at::empty({0, n}, x.options());
+  TORCH_CHECK(!silu_mul || n % 16 == 0, "barlink: SiLU*mul of an int4 linear needs N a multiple of 16");
+  if (m == 0) return at::empty({0, silu_mul ? n / 2 : n}, x.options());
+  W8Scratch& s = w8_scratch(dev);
+  const bool aligned = ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(qweight.data_ptr())) & 15u) == 0;
+  // The tensor cores cost the same for 1 to 16 rows, the GEMV two rows' worth of time more for every doubling:
+  // 37888 x 3584, us: GEMV 33 / 50 / 87 / 88 / 177 at 1 / 4 / 6 / 8 / 16 rows, digits 57 throughout;
+  // 3584 x 18944: GEMV 28 / 31 / 56 / 57 / 92, digits 36 - 41.
+  if (group == 128 && m > 4 && m <= BL_QLIN_MAX_TOKENS && k <= 32768 && n % 8 == 0 && aligned) {
+    QWeight q{qweight.data_ptr(), 2, n, k, BL_QSCALE_F16_GN, scales.data_ptr()};
+    q.group_k = group;
+    q.zeros = qzeros.data_ptr();
+    return qlin_run(x, 3, q, c10::nullopt, silu_mul, splits > k / 128 ? k / 128 : splits, want_slabs,
+                    s.err_flag.data_ptr(), st);
+  }
+  auto finish = [&](const at::Tensor& y) {
+    if (!silu_mul) return y;
+    at::Tensor o = at::empty({m, n / 2}, x.options());
+    BL_CHECK(bl_silu_mul(y.data_ptr(), o.data_ptr(), m, n / 2, 1, st, err, errlen));
+    return o;
+  };
   if (m > 16) {
     at::Tensor w = at::empty({n, k}, x.options());
     BL_CHECK(bl_w4_dequant(qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), w.data_ptr(), n, k, group,
                            st, err, errlen));
-    return at::matmul(x, w.t());  // prefill path, not the decode hot path
+    return finish(at::matmul(x, w.t()));  // prefill path, not the decode hot path
   }
-  W8Scratch& s = w8_scratch(dev);
   at::Tensor out = at::empty({m, n}, x.options());
   BL_CHECK(bl_w4a16_gemv(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), out.data_ptr(),
                          m, n, k, group, splits, s.ws.data_ptr(), size_t(s.ws.nbytes()), st, err, errlen));
-  return out;
+  return finish(out);
 }
 
 at::Tensor w4_dequant(const at::Tensor& qweight, const at::Tensor& scales, const at::Tensor& qzeros, int group) {
@@ -758,7 +778,7 @@ void bind_extra(py::module_& m) {
   m.def("pick_splits", [](int tiles, int kblocks, int sms, int want) { return bl::pick_splits(tiles, kblocks, sms, want); },
         py::arg("tiles"), py::arg("kblocks"), py::arg("sms") = 148, py::arg("want") = 0);
   m.def("w4a16_linear", &w4a16_linear, py::arg("x"), py::arg("qweight"), py::arg("scales"), py::arg("qzeros"),
-        py::arg("group") = 128, py::arg("splits") = 0);
+        py::arg("group") = 128, py::arg("splits") = 0, py::arg("silu_mul") = false, py::arg("want_slabs") = false);
   m.def("w4_dequant", &w4_dequant, py::arg("qweight"), py::arg("scales"), py::arg("qzeros"), py::arg("group") = 128);
   m.def("qknorm_rope", &qknorm_rope, py::arg("qkv"), py::arg("gq"), py::arg("gk"), py::arg("positions"),
         py::arg("heads"), py::arg("eps") = 1e-6, py::arg("theta") = 1e4, py::arg("axes") = 2);

@@ -40,7 +40,9 @@ __global__ void __launch_bounds__(kW4Threads) k_w4a16_gemv(const __nv_bfloat16* 
                                                            __nv_bfloat16* __restrict__ out,
                                                            float* __restrict__ ws, int M, int N, int K,
                                                            int group, int gper) {
-  pdl_launch_dependents();
+  // the kernels behind this one start when it ends: resident early they only took its slots (7B shape, one
+  // sequence, MLP in int4: 3.22 ms a step with an early start of this kernel's dependents,
+  // 2.79 ms without)
   pdl_wait();
   __shared__ float s_x[MT][kW4MaxGroup];
   const int n = (blockIdx.x * kW4Threads + threadIdx.x) * 4;
@@ -115,7 +117,6 @@ __global__ void __launch_bounds__(kW4Threads) k_w4a16_gemv(const __nv_bfloat16* 
 }
 
 __global__ void k_w4_reduce(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int MN, int S) {
-  pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= MN) return;

@@ -106,15 +106,17 @@ class W4Weight:
 
 def qlinear(x, w, bias=None, silu_mul=False, split=False):
     """x @ w.T for any stored form of w (plain / tiled bf16, W8Weight, W4Weight).
-    split=True allows the k-split slab output of the bf16 and int8 decode linears."""
+    split=True allows the k-split slab output of the decode linears."""
     if isinstance(w, W8Weight):
         if split and not silu_mul:
             return ops.w8a16_linear_split(x, w.wq, w.scale, bias)
         return ops.w8a16_linear(x, w.wq, w.scale, bias, silu_mul)
     if isinstance(w, W4Weight):
-        y = ops.w4a16_linear(x, w.qw, w.sc, w.qz, w.group)
-        if bias is not None:
-            y = y + bias
+        if bias is None:
+            if split and not silu_mul:
+                return ops.w4a16_linear_split(x, w.qw, w.sc, w.qz, w.group)
+            return ops.w4a16_linear(x, w.qw, w.sc, w.qz, w.group, silu_mul)
+        y = ops.w4a16_linear(x, w.qw, w.sc, w.qz, w.group) + bias
         return ops.silu_mul(y, interleaved=True) if silu_mul else y
     if split and bias is None and not silu_mul:
         return ops.linear_split(x, w)

@@ -147,15 +147,26 @@ def rope(x, positions, theta, axes=1):
     return ref.rope(x, positions, theta, axes)
 
 
-def w4a16_linear(x, qweight, scales, qzeros, group_size=128):
-    """Weight-only int4 linear on GPTQ-v1 tensors (see `ref.pack_int4`): a
-    hand-written GEMV for 1..16 rows, widen + GEMM above that."""
+def w4a16_linear(x, qweight, scales, qzeros, group_size=128, silu_mul=False):
+    """Weight-only int4 linear on GPTQ-v1 tensors (see `ref.pack_int4`), optionally with SiLU(gate) * up
+    over interleaved (gate, up) columns.  Groups of 128 and 5..128 rows: the digit kernel; else a GEMV up
+    to 16 rows; else widen + GEMM."""
     if x.is_cuda:
         _count(2)
         x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
-        y = _C().w4a16_linear(x2.contiguous(), qweight, scales, qzeros, group_size)
+        y = _C().w4a16_linear(x2.contiguous(), qweight, scales, qzeros, group_size, silu_mul=silu_mul)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
-    return ref.w4a16_linear(x, qweight, scales, qzeros, group_size)
+    y = ref.w4a16_linear(x, qweight, scales, qzeros, group_size)
+    return ref.silu_mul(y, True) if silu_mul else y
+
+
+def w4a16_linear_split(x, qweight, scales, qzeros, group_size=128):
+    """Decode-path form of `w4a16_linear`: fp32 slabs [splits, tokens, n] for the consumer to sum when the
+    shape wants a k-split (see `linear_split`), else the bf16 result."""
+    if x.is_cuda and x.dim() == 2:
+        _count(2)
+        return _C().w4a16_linear(x.contiguous(), qweight, scales, qzeros, group_size, want_slabs=True)
+    return w4a16_linear(x, qweight, scales, qzeros, group_size)
 
 
 def qknorm_rope(qkv, gq, gk, positions, heads, eps=1e-6, theta=1e4, axes=2):
@@ -332,5 +343,5 @@ def w8a16_linear_split(x, wq, scale, bias=None):
 
 __all__ = [
     "linear", "linear_split", "k_splits", "TiledWeight", "tile_weight", "untile_weight", "rmsnorm", "rope_kv_write", "rope", "silu_mul", "embedding", "argmax",
-    "paged_attn_decode", "rope_attn_decode", "attention", "w8a16_linear", "w8a16_linear_split", "W8GroupScales", "prepare_w8_scales", "w4a16_linear", "qknorm_rope", "layernorm_modulate", "gate_residual", "ref",
+    "paged_attn_decode", "rope_attn_decode", "attention", "w8a16_linear", "w8a16_linear_split", "W8GroupScales", "prepare_w8_scales", "w4a16_linear", "w4a16_linear_split", "qknorm_rope", "layernorm_modulate", "gate_residual", "ref",
 ]

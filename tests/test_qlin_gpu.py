@@ -118,3 +118,32 @@ def test_chunked_int8_weights(ext, m, n, k):
     assert torch.equal(ext.w8a16_gemm(off, xs, wq_t, sw, n, k, 1), ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, 1))
     torch.cuda.synchronize()
     assert ext.w8_error_flag(0) == 0
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 16, 17, 64, 65, 128])
+@pytest.mark.parametrize("n,k", [(128, 128), (208, 1280), (1000, 3584), (136, 17408)])
+def test_int4_weights(ext, m, n, k):
+    from barlink_sm86_b200 import ops
+    g = _g(11)
+    nib = torch.randint(0, 16, (n, k), generator=g, device="cuda")
+    zero = torch.randint(0, 16, (k // 128, n), generator=g, device="cuda")
+    sc = (torch.rand(k // 128, n, generator=g, device="cuda") * 0.01 + 1e-3).half()
+    def pack(t):  # eight values along the last dimension -> one int32
+        v = sum(t.view(*t.shape[:-1], -1, 8)[..., j].long() << (4 * j) for j in range(8))
+        return ((v + 2 ** 31) % 2 ** 32 - 2 ** 31).to(torch.int32)
+    qw, qz = pack(nib).t().contiguous(), pack(zero)
+    x = _x(m, k, 5, spread=True)
+    w = (nib - zero.t().repeat_interleave(128, 1)).double() * sc.double().t().repeat_interleave(128, 1)
+    want = x.double() @ w.t()
+    assert rel_l2(ops.w4a16_linear(x, qw, sc, qz), want) < TOL
+    out = ops.w4a16_linear_split(x, qw, sc, qz)
+    if out.dim() == 3:
+        assert rel_l2(out.double().sum(0), want) < TOL32
+    for splits in {1, 3, k // 128, 99}:
+        assert rel_l2(ext.w4a16_linear(x, qw, sc, qz, 128, splits), want) < TOL
+    if n % 16 == 0:
+        silu = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+        for splits in (0, 1):
+            assert rel_l2(ext.w4a16_linear(x, qw, sc, qz, 128, splits, True), silu) < TOL
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0

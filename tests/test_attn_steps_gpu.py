@@ -1,0 +1,33 @@
+# SPDX-License-Identifier: MIT
+"""Tensor-core attention around the ends of its pipeline (64-key steps, scores two steps ahead, tiles in
+rings of three): one to seven steps, ragged last steps, scores that grow so that the accumulator is
+rescaled while products are in flight.  Oracle: float64.  Tolerance: P and the result are rounded to bf16
+(2^-9 relative each, the sums over keys average P's): rel-L2 2^-8."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _want(q, k, v, scale, causal):
+    s = torch.einsum("qhd,khd->hqk", q.double(), k.double()) * scale
+    if causal:
+        lq, lk = s.shape[1:]
+        s = s.masked_fill(torch.ones(lq, lk, dtype=torch.bool, device=s.device).triu(lk - lq + 1), float("-inf"))
+    return torch.einsum("hqk,khd->qhd", s.softmax(-1), v.double())
+
+
+@pytest.mark.parametrize("lk", [1, 63, 64, 65, 128, 129, 192, 193, 256, 257, 400])
+@pytest.mark.parametrize("growing", [False, True])
+@pytest.mark.parametrize("causal", [False, True])
+def test_steps(ext, lk, growing, causal):
+    g = torch.Generator(device="cuda").manual_seed(lk)
+    lq, nq, nkv = (lk if causal else 300), 2, 1
+    q, k, v = (torch.randn(n, h, 128, generator=g, device="cuda").bfloat16() for n, h in ((lq, nq), (lk, nkv), (lk, nkv)))
+    if growing:  # later keys win by far: the running maximum rises in every step
+        k = (k.float() * torch.linspace(0.2, 12.0, lk, device="cuda")[:, None, None]).bfloat16()
+    cu_q, cu_k = (torch.tensor([0, n], dtype=torch.int32, device="cuda") for n in (lq, lk))
+    got = ext.attn_fwd(q, k, v, cu_q, cu_k, lq, 128 ** -0.5, causal, lk)
+    want = _want(q, k.expand(-1, nq, -1), v.expand(-1, nq, -1), 128 ** -0.5, causal)
+    assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8
+    assert ext.attn_error_flag(0) == 0

@@ -566,7 +566,8 @@ __global__ void __launch_bounds__(kDigThreads) k_quant_digits(const __nv_bfloat1
 }
 
 // fp32 slabs [split][m][n] -> bf16: sum in split order, + bias, optionally SiLU*mul over interleaved
-// (gate, up) columns.  Eight columns per thread.
+// (gate, up) columns.  Eight columns per thread.  The slabs and the output start on 16-byte boundaries, the
+// bias (a caller's tensor, often a slice of a longer one) at any element.
 __global__ void __launch_bounds__(256) k_slab_finish(const float* __restrict__ slabs, int nsplit, size_t slab, int n,
                                                      const __nv_bfloat16* __restrict__ bias, int silu,
                                                      __nv_bfloat16* __restrict__ out, int ldo, size_t total8) {
@@ -579,7 +580,10 @@ __global__ void __launch_bounds__(256) k_slab_finish(const float* __restrict__ s
   const int c = int(t - m * per) * 8;
   float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   sum_slabs8(slabs + m * n + c, slab, nsplit, a);
-  if (bias) {
+  if (bias && (reinterpret_cast<uintptr_t>(bias) & 15u)) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] += __bfloat162float(bias[c + j]);
+  } else if (bias) {
     const uint4 b = *reinterpret_cast<const uint4*>(bias + c);
     const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y), b2 = unpack_bf16x2(b.z), b3 = unpack_bf16x2(b.w);
     a[0] += b0.x; a[1] += b0.y; a[2] += b1.x; a[3] += b1.y;
@@ -723,8 +727,9 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
 
 extern "C" int bl_slab_finish(const void* slabs, int nsplit, int m, int n, const void* bias, int silu_mul, void* out,
                               int ldo, void* stream, char* err, size_t errlen) {
-  if (!slabs || !out || nsplit < 1 || m < 1 || n < 8 || (n & 7) || (ldo & 7)) {
-    set_err(err, errlen, "barlink: slab_finish needs n and the output pitch in multiples of 8");
+  if (!slabs || !out || nsplit < 1 || m < 1 || n < 8 || (n & 7) || (ldo & 7) ||
+      ((reinterpret_cast<uintptr_t>(slabs) | reinterpret_cast<uintptr_t>(out)) & 15u)) {
+    set_err(err, errlen, "barlink: slab_finish needs n and the output pitch in multiples of 8, slabs and output on 16-byte boundaries");
     return -1;
   }
   const size_t total8 = size_t(m) * (n / 8);

@@ -58,6 +58,29 @@ def test_int8_weights_bf16_activations(ext, m, n, k):
     assert ext.w8_error_flag(0) == 0
 
 
+# a bias that starts off a 16-byte boundary (a slice of a longer vector), with and without a k-split, and
+# where the shape picks one by itself (the last)
+@pytest.mark.parametrize("off", [1, 4])
+@pytest.mark.parametrize("m,n,k", [(1, 136, 1040), (64, 200, 1040), (1, 4608, 3584)])
+def test_bias_at_any_element(ext, off, m, n, k):
+    wq, sc = _w8(n, k, 3)
+    x = _x(m, k, 5)
+    b = torch.randn(n + 8, generator=_g(9), device="cuda").bfloat16()[off:off + n]
+    y = (x.double() @ wq.double().t()) * sc.double() + b.double()
+    silu = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+    for act_int8 in (False, True):
+        if act_int8:
+            xq, xs = ext.w8a16_quant_act(x)
+            y = (xq.double() @ wq.double().t()) * xs.double()[:, None] * sc.double() + b.double()
+        for splits in (0, 1, 3):
+            assert rel_l2(ext.w8a16_linear(x, wq, sc, b, splits=splits, act_int8=act_int8), y) < TOL
+        if not act_int8 and n % 16 == 0:
+            for splits in (0, 1, 3):
+                assert rel_l2(ext.w8a16_linear(x, wq, sc, b, True, splits), silu) < TOL
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
+
+
 @pytest.mark.parametrize("m", [1, 32, 64])
 @pytest.mark.parametrize("n,k,group", [(200, 1024, 128), (129, 768, 256)])
 @pytest.mark.parametrize("act_int8", [False, True])

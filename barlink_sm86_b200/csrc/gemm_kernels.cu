@@ -135,7 +135,10 @@ struct LocalSink {
                size_t(gm - owner * ptpr) * ldo;
       }
       const __nv_bfloat16* rrow = residual ? residual + size_t(m) * ldo : nullptr;
-      if (ncols == 32 && j0 + 32 <= rb && (ldo & 7) == 0) {
+      // 16-byte accesses where bias, residual and output all allow them: any of them may be a caller's slice
+      const uintptr_t ends = reinterpret_cast<uintptr_t>(orow) | ((epi & 1) ? reinterpret_cast<uintptr_t>(bias) : 0) |
+                             ((epi & 2) ? reinterpret_cast<uintptr_t>(rrow) : 0);
+      if (ncols == 32 && j0 + 32 <= rb && (ldo & 7) == 0 && (ends & 15u) == 0) {
 #pragma unroll
         for (int c = 0; c < 32; c += 8) {
           float x[8];

@@ -57,6 +57,28 @@ def test_paired_kernel_few_rows(ext, rows, n, k):
     assert ext.gemm_error_flag(0) == 0
 
 
+# bias, residual or output off a 16-byte boundary (slices of longer tensors): the paired kernel, and with
+# bn = 128 the single-CTA one
+@pytest.mark.parametrize("which", ["bias", "residual", "out"])
+@pytest.mark.parametrize("rows,n,k,bn", [(129, 256, 512, 0), (600, 264, 136, 0), (200, 256, 512, 128)])
+@pytest.mark.parametrize("off", [1, 4])
+def test_token_major_off_16_bytes(ext, which, rows, n, k, bn, off):
+    def cut(t, on):  # the same values, starting `off` elements into a buffer when `on`
+        buf = torch.zeros(t.numel() + 8, dtype=torch.bfloat16, device="cuda")
+        v = buf[off if on else 0:][:t.numel()].view(t.shape)
+        return v.copy_(t)
+    x, w = _bf(rows, k, seed=1), _bf(n, k, seed=2, std=k ** -0.5)
+    b, r = cut(_bf(n, seed=3), which == "bias"), cut(_bf(rows, n, seed=4), which == "residual")
+    out = cut(torch.zeros(rows, n), which == "out")
+    want = x.double() @ w.double().t() + b.double() + r.double()
+    ext.linear(x, w, b, r, False, out, bn=bn)
+    assert float((out.double() - want).norm() / want.norm()) < TOL
+    ext.linear(x, w, b, None, False, out, bn=bn)
+    assert float((out.double() - want + r.double()).norm() / want.norm()) < TOL
+    torch.cuda.synchronize()
+    assert ext.gemm_error_flag(0) == 0
+
+
 def test_row_splits_rule(ext):
     assert ext.gemm_row_splits(128, 3584, 18944) == 1  # the swapped form
     assert ext.gemm_row_splits(333, 3584, 18944) >= 2  # 28 tiles for 74 pairs

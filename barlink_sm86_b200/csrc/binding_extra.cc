@@ -203,10 +203,11 @@ struct QWeight {
   int group_k = 0;
   const void* zeros = nullptr;
 };
-// a shape that bl_qlin takes and (three digits) bf16 rows that bl_quant_digits can read
-bool qlin_takes(const at::Tensor& x, int k, bool act_int8) {
+// a shape that bl_qlin takes and (three digits) bf16 rows that bl_quant_digits can read; per-channel sums are
+// 32-bit over all of K
+bool qlin_takes(const at::Tensor& x, int k, bool act_int8, bool grouped = false) {
   if (x.size(0) < 1 || x.size(0) > BL_QLIN_MAX_TOKENS || k % 16 != 0) return false;
-  return act_int8 ? k <= 131072
+  return act_int8 ? grouped || k <= 131072
                   : k <= 32768 && x.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0;
 }
 // y = activations (xq, xs: int8 rows, or three digit planes) times q.  want_slabs: fp32 [splits, m, n]
@@ -218,11 +219,9 @@ at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int d
     check_bf16x(*bias, "bias");
     TORCH_CHECK(bias->numel() == q.n, "barlink: bias must have n entries");
   }
-  if (splits <= 0) {
-    splits = bl_qlin_splits(q.n, q.k, m);
-    // bl_slab_finish stores 16-byte vectors
-    if (!want_slabs && (silu_mul ? q.n % 16 : q.n % 8) != 0) splits = 1;
-  }
+  if (splits <= 0) splits = bl_qlin_splits(q.n, q.k, m);
+  // bl_slab_finish stores 16-byte vectors
+  if (!want_slabs && (silu_mul ? q.n % 16 : q.n % 8) != 0) splits = 1;
   const int kb = (q.k + 127) / 128, per = (kb + splits - 1) / splits;
   splits = (kb + per - 1) / per;
   blQlinArgs a;
@@ -301,8 +300,7 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   const int m = int(x.size(0)), k = int(x.size(1)), n = int(wq.size(0));
   TORCH_CHECK(group_scale || scale.numel() == n, "barlink: scale must have one entry per output channel");
   if (group_scale) {
-    TORCH_CHECK(!group_rel && m >= 1 && qlin_takes(x, k, act_int8), "barlink: group_scale goes with 1..", BL_QLIN_MAX_TOKENS,
-                " 16-byte aligned rows");
+    TORCH_CHECK(act_int8 && !group_rel && m <= 64, "barlink: group_scale goes with act_int8 and at most 64 tokens");
     TORCH_CHECK(group_scale->is_cuda() && group_scale->is_contiguous() && group_scale->scalar_type() == at::kBFloat16 &&
                     group_scale->dim() == 2 && group_scale->size(0) == n && k % group_scale->size(1) == 0 &&
                     (k / group_scale->size(1)) % 128 == 0,
@@ -321,7 +319,7 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   TORCH_CHECK(!(act_int8 && group_rel), "barlink: int8 activations go with per-channel or group_scale weight scales");
   // 1..128 tokens: the weights go to the tensor cores as they are (qlin_kernels.cu).  Group scales need
   // groups of whole 128-wide k-blocks.
-  if (qlin_takes(x, k, act_int8) && (!group_rel || (k / group_rel->size(1)) % 128 == 0)) {
+  if (qlin_takes(x, k, act_int8, bool(group_scale)) && (!group_rel || (k / group_rel->size(1)) % 128 == 0)) {
     QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
     if (group_scale) {
       q.scale_kind = BL_QSCALE_BF16_NG;

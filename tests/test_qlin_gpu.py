@@ -52,7 +52,7 @@ def test_int8_weights_bf16_activations(ext, m, n, k):
         assert rel_l2(out.double().sum(0), prod) < TOL32
     kb = -(-k // 128)
     for splits in {1, 2, 5, kb}:
-        if n % 8 == 0 and splits <= kb:
+        if splits <= kb:
             assert rel_l2(ext.w8a16_linear(x, wq, sc, b, splits=splits), prod + b.double()) < TOL
     torch.cuda.synchronize()
     assert ext.w8_error_flag(0) == 0
@@ -79,6 +79,28 @@ def test_bias_at_any_element(ext, off, m, n, k):
                 assert rel_l2(ext.w8a16_linear(x, wq, sc, b, True, splits), silu) < TOL
     torch.cuda.synchronize()
     assert ext.w8_error_flag(0) == 0
+
+
+# a k-split that the caller asks for and n that the kernel behind it cannot store as vectors
+@pytest.mark.parametrize("n", [129, 200, 202])
+@pytest.mark.parametrize("splits", [2, 9, 99])
+def test_asked_splits_of_odd_widths(ext, n, splits):
+    wq, sc = _w8(n, 1040, 3)
+    x = _x(3, 1040, 5)
+    y = (x.double() @ wq.double().t()) * sc.double()
+    assert rel_l2(ext.w8a16_linear(x, wq, sc, None, False, splits), y) < TOL
+    if n % 2 == 0:
+        silu = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+        assert rel_l2(ext.w8a16_linear(x, wq, sc, None, True, splits), silu) < TOL
+
+
+def test_no_rows(ext):
+    wq, sc = _w8(200, 1024, 3)
+    gs = torch.ones(200, 8, device="cuda").bfloat16()
+    x = _x(1, 1024, 5)[:0]
+    assert ext.w8a16_linear(x, wq, sc).shape == (0, 200)
+    assert ext.w8a16_linear(x, wq, sc, None, True).shape == (0, 100)
+    assert ext.w8a16_linear(x, wq, gs, act_int8=True, group_scale=gs).shape == (0, 200)
 
 
 @pytest.mark.parametrize("m", [1, 32, 64])

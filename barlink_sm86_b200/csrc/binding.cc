@@ -521,6 +521,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<
       ((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(a.bias)) & 15u) == 0) {
     const int s2 = bl_gemm_row_splits(tokens, n, k);
     if (s2 > 1) {
+      py::gil_scoped_release nogil;
       at::Tensor slabs = at::empty({s2, tokens, n}, x.options().dtype(at::kFloat));
       a.out = nullptr;
       a.bias = nullptr;

@@ -251,7 +251,8 @@ at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int d
                           out.data_ptr(), int(out.size(1)), st, err, errlen));
   return out;
 }
-// digits = 3: x as it is; digits = 1: x quantised to int8 per token
+// digits = 3: x as it is; digits = 1: x quantised to int8 per token.  Callers let go of the GIL first: a
+// launch waits when the queue is full.
 at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10::optional<at::Tensor>& bias,
                     bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
   const int m = int(x.size(0));
@@ -282,9 +283,10 @@ at::Tensor w8a16_linear_split(const at::Tensor& x, const at::Tensor& wq, const a
   TORCH_CHECK(scale.numel() == n, "barlink: scale must have one entry per output channel");
   TORCH_CHECK(qlin_takes(x, k, act_int8), "barlink: w8a16_linear_split is for 1..", BL_QLIN_MAX_TOKENS, " 16-byte aligned rows, K % 16 == 0");
   c10::cuda::CUDAGuard guard(x.device());
+  void* flag = w8_scratch(dev).err_flag.data_ptr();
+  py::gil_scoped_release nogil;
   QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
-  return qlin_run(x, act_int8 ? 1 : 3, q, bias, false, 0, true, w8_scratch(dev).err_flag.data_ptr(),
-                  at::cuda::getCurrentCUDAStream(dev).stream());
+  return qlin_run(x, act_int8 ? 1 : 3, q, bias, false, 0, true, flag, at::cuda::getCurrentCUDAStream(dev).stream());
 }
 
 at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& scale,
@@ -331,7 +333,9 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
       q.row_scale = scale.data_ptr();
       q.group_k = k / int(group_rel->size(1));
     }
-    return qlin_run(x, act_int8 ? 1 : 3, q, bias, silu_mul, splits, false, w8_scratch(dev).err_flag.data_ptr(), st);
+    void* flag = w8_scratch(dev).err_flag.data_ptr();
+    py::gil_scoped_release nogil;
+    return qlin_run(x, act_int8 ? 1 : 3, q, bias, silu_mul, splits, false, flag, st);
   }
   at::Tensor out = at::empty({m, silu_mul ? n / 2 : n}, x.options());
   if (act_int8) {
@@ -475,8 +479,9 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
   const bool aligned = (reinterpret_cast<uintptr_t>(xq.data_ptr()) & 15u) == 0;
   QWeight q{wq_t.data_ptr(), 1, int(N), int(K), BL_QSCALE_F32_GN, sw_t.data_ptr()};
   q.group_k = 128;
-  return qlin_product(aligned ? xq : xq.clone(), xs, m, 1, q, c10::nullopt, false, 0, false, like,
-                      w8_scratch(dev).err_flag.data_ptr(), st);
+  void* flag = w8_scratch(dev).err_flag.data_ptr();
+  py::gil_scoped_release nogil;
+  return qlin_product(aligned ? xq : xq.clone(), xs, m, 1, q, c10::nullopt, false, 0, false, like, flag, st);
 }
 
 // GPTQ-v1 int4 linear.  Groups of 128 and 5..128 rows: int8 digits of the activations on the tensor cores
@@ -511,6 +516,7 @@ at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at
     QWeight q{qweight.data_ptr(), 2, n, k, BL_QSCALE_F16_GN, scales.data_ptr()};
     q.group_k = group;
     q.zeros = qzeros.data_ptr();
+    py::gil_scoped_release nogil;
     return qlin_run(x, 3, q, c10::nullopt, silu_mul, splits > k / 128 ? k / 128 : splits, want_slabs,
                     s.err_flag.data_ptr(), st);
   }

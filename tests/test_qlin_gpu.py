@@ -192,3 +192,45 @@ def test_int4_weights(ext, m, n, k):
             assert rel_l2(ext.w4a16_linear(x, qw, sc, qz, 128, splits, True), silu) < TOL
     torch.cuda.synchronize()
     assert ext.w8_error_flag(0) == 0
+
+
+def test_other_threads_run_while_a_launch_waits(ext):
+    """A launch waits when the queue of launches is full; the other Python threads go on meanwhile."""
+    import threading
+    import time
+    n, k = 200, 1024
+    wq, sc = _w8(n, k, 3)
+    x, xl = _x(6, k, 5), _x(300, k, 6)
+    wq_t, sw = wq.view(n, k // 16, 16).permute(1, 0, 2).contiguous(), torch.ones(k // 128, n, device="cuda")
+    xq, xs = ext.w8a16_quant_act(x)
+    w = _x(512, k, 7)
+    assert ext.gemm_row_splits(300, 512, k) > 1
+    qw = torch.zeros(k // 8, n, dtype=torch.int32, device="cuda")
+    s4, qz = torch.ones(k // 128, n, device="cuda").half(), torch.zeros(k // 128, n // 8, dtype=torch.int32, device="cuda")
+    for name, f in {"w8a16_linear": lambda: ext.w8a16_linear(x, wq, sc),
+                    "w8a16_linear_split": lambda: ext.w8a16_linear_split(x, wq, sc),
+                    "w8a16_gemm": lambda: ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, 1),
+                    "w4a16_linear": lambda: ext.w4a16_linear(x, qw, s4, qz, 128, 1),
+                    "linear": lambda: ext.linear(xl, w)}.items():
+        f()
+        torch.cuda.synchronize()
+        stop, gap = threading.Event(), [0.0]
+
+        def tick():
+            last = time.perf_counter()
+            while not stop.is_set():
+                time.sleep(1e-3)
+                now = time.perf_counter()
+                gap[0], last = max(gap[0], now - last), now
+        th = threading.Thread(target=tick)
+        th.start()
+        torch.cuda._sleep(10 ** 9)  # half a second of an occupied stream
+        t0 = time.perf_counter()
+        for _ in range(2000):
+            f()
+        waited = time.perf_counter() - t0
+        stop.set()
+        th.join()
+        torch.cuda.synchronize()
+        assert waited > 0.2, (name, waited)  # the queue was full
+        assert gap[0] < waited / 2, (name, gap[0], waited)

@@ -244,6 +244,15 @@ __device__ __forceinline__ void tma_load_2d_hint_warp(uint32_t leader, uint32_t 
       "l"(tmap), "r"(bar), "r"(x), "r"(y), "l"(hint), "r"(leader)
       : "memory");
 }
+// The tile into L2 only: a hint, no barrier to wait for.
+__device__ __forceinline__ void tma_prefetch_2d_warp(uint32_t leader, const void* tmap, int x, int y, uint64_t hint) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %4, 0;\n\t"
+      "@q cp.async.bulk.prefetch.tensor.2d.L2.global.tile.L2::cache_hint [%0, {%1, %2}], %3;\n\t}" ::"l"(tmap),
+      "r"(x), "r"(y), "l"(hint), "r"(leader)
+      : "memory");
+}
 __device__ __forceinline__ void bulk_load_warp(uint32_t leader, uint32_t smem_dst, const void* gsrc, uint32_t bytes,
                                                uint32_t bar, uint64_t hint) {
   asm volatile(

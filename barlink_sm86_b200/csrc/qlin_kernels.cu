@@ -149,23 +149,18 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
   if (warp == 0) {
     // ------------------------------ producer ------------------------------
     const uint32_t leader = elect_leader();
-    auto load_a = [&](uint32_t dst, uint64_t* bar, int kb, int ta) {
-      if constexpr (SRC == kRows)
-        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(bar), kb * kQK, ta * kQRows, kHintEvictFirst);
-      else if constexpr (SRC == kNibbles)
-        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(bar), ta * kQRows, kb * (kQK / 8), kHintEvictFirst);
-      else  // eight chunks of 128 rows, in elements of 8 bytes
-        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(bar), ta * kQRows * 2, kb * (kQK / 16), kHintEvictFirst);
-    };
-    // the first lap of weight tiles is requested before the kernels ahead have finished
+    // in elements of the tensor map: bytes, words of eight nibbles, or (eight chunks of 128 rows) 8 bytes
+    auto ax = [&](int kb, int ta) { return SRC == kRows ? kb * kQK : ta * kQRows * (SRC == kNibbles ? 1 : 2); };
+    auto ay = [&](int kb, int ta) { return SRC == kRows ? ta * kQRows : kb * (kQK / (SRC == kNibbles ? 8 : 16)); };
+    // Before the kernels ahead have finished, the first lap of weight tiles is asked for into L2 only: HBM keeps
+    // streaming across the kernel boundary, and weights that one of those kernels writes are read as it leaves
+    // them, since every copy into shared memory starts behind the wait.
     int pre = 0;
     for (int u = blockIdx.x; u < units && pre < S::kStages; u += gridDim.x) {
       const int tile = u / g.splits, sp = u - tile * g.splits, ta = tile / g.tiles_b;
       const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-      for (int kb = kb0; kb < kb1 && pre < S::kStages; ++kb, ++pre) {
-        mbar_expect_tx_warp(leader, &full_bar[pre], S::kStage);
-        load_a(ring + pre * S::kStage, &full_bar[pre], kb, ta);
-      }
+      for (int kb = kb0; kb < kb1 && pre < S::kStages; ++kb, ++pre)
+        tma_prefetch_2d_warp(leader, &tmap_w, ax(kb, ta), ay(kb, ta), kHintEvictFirst);
     }
     pdl_wait();
     int stage = 0, armed = 0;
@@ -179,22 +174,19 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
       for (int kb = kb0; kb < kb1; ++kb) {
         const uint32_t dst = ring + stage * S::kStage;
         uint64_t* full = &full_bar[stage];
-        const bool early = armed < pre;  // weight tile of this stage is already on its way
-        if (!early) {
-          if (!ready) ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort);
-          if (!__all_sync(0xffffffffu, ok)) {
-            ok = false;
-            break;
-          }
-          mbar_expect_tx_warp(leader, full, S::kStage);
+        if (!ready) ok = mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort);
+        if (!__all_sync(0xffffffffu, ok)) {
+          ok = false;
+          break;
         }
+        mbar_expect_tx_warp(leader, full, S::kStage);
         ++armed;
         if (++stage == S::kStages) {
           stage = 0;
           phase ^= 1u;
         }
-        ready = armed >= pre && mbar_test_wait(&empty_bar[stage], phase ^ 1u);
-        if (!early) load_a(dst, full, kb, ta);
+        ready = mbar_test_wait(&empty_bar[stage], phase ^ 1u);
+        tma_load_2d_hint_warp(leader, dst, &tmap_w, smem_u32(full), ax(kb, ta), ay(kb, ta), kHintEvictFirst);
         tma_load_2d_hint_warp(leader, dst + S::kStageA, &tmap_x, smem_u32(full), kb * kQK, tb * S::BN, kHintEvictLast);
       }
     }
@@ -275,6 +267,7 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
     // Two groups of 128 threads take alternate k-blocks; a thread expands one weight row: 16 words in
     // (consecutive lanes, consecutive words), eight 16-byte chunks out (consecutive lanes,
     // consecutive chunks): no bank conflicts on either side.
+    pdl_wait();  // the zero points may come from a kernel ahead
     const int ct = threadIdx.x - 192, grp = ct >> 7, row = ct & 127;
     int nkb = 0;
     bool ok = true;

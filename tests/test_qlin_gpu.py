@@ -234,3 +234,34 @@ def test_other_threads_run_while_a_launch_waits(ext):
         torch.cuda.synchronize()
         assert waited > 0.2, (name, waited)  # the queue was full
         assert gap[0] < waited / 2, (name, gap[0], waited)
+
+
+# Weights that a kernel just ahead in the stream leaves behind (received, unpacked, dequantised ones): this
+# library's kernels let their successors start early, so the weights may only be read behind the wait.  The
+# writer here is a product whose result, seen as bytes, is the weight; `stale` is what was there before.
+@pytest.mark.parametrize("form", ["pair", "int8", "bf16", "int4"])
+def test_weights_written_by_the_kernel_ahead(ext, form):
+    n, k, m = 4096, 4096, 8
+    # [k / 8, 2 n] bf16 = [k / 8, n] int32, or [n, k / 2] bf16 = [n, k] int8
+    b, a = (_x(k // 8, 8192, 2), _x(2 * n, 8192, 1)) if form == "int4" else (_x(n, 8192, 2), _x(k // 2, 8192, 1))
+    buf = torch.zeros(b.shape[0], a.shape[0], dtype=torch.bfloat16, device="cuda")
+    x, one = _x(m, k, 5), torch.ones(n, device="cuda").bfloat16()
+    xq, xs = ext.w8a16_quant_act(x)
+    s4, qz = torch.ones(k // 128, n, device="cuda").half(), torch.zeros(k // 128, n // 8, dtype=torch.int32, device="cuda")
+    sw = torch.ones(k // 128, n, device="cuda")
+
+    def product():
+        if form == "int4":
+            return ext.w4a16_linear(x, buf.view(torch.int32), s4, qz)
+        w = buf.view(torch.int8)
+        if form == "pair":
+            return ext.w8a16_gemm(xq, xs, w.view(k // 16, n, 16), sw, n, k, 1)
+        return ext.w8a16_linear(x, w, one, act_int8=form == "int8")
+    ext.linear(b, a, out=buf)
+    torch.cuda.synchronize()
+    want = product()
+    for _ in range(5):
+        buf.zero_()
+        torch.cuda.synchronize()
+        ext.linear(b, a, out=buf)
+        assert torch.equal(product(), want)

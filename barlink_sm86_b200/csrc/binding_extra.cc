@@ -219,7 +219,7 @@ at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int d
     check_bf16x(*bias, "bias");
     TORCH_CHECK(bias->numel() == q.n, "barlink: bias must have n entries");
   }
-  if (splits <= 0) splits = bl_qlin_splits(q.n, q.k, m);
+  if (splits <= 0) splits = bl_qlin_splits(q.n, q.k, m, digits, q.scale_kind != BL_QSCALE_BF16_N);
   // bl_slab_finish stores 16-byte vectors
   if (!want_slabs && (silu_mul ? q.n % 16 : q.n % 8) != 0) splits = 1;
   const int kb = (q.k + 127) / 128, per = (kb + splits - 1) / splits;

@@ -202,8 +202,8 @@ typedef struct blQlinArgs {
   void* err_flag;
 } blQlinArgs;
 int bl_qlin(const blQlinArgs* a, void* stream, char* err, size_t errlen);
-int bl_qlin_splits(int n, int k, int m);  /* k-splits that suit the shape */
-int bl_qlin_tile_tokens(int m);
+int bl_qlin_splits(int n, int k, int m, int digits, int grouped);  /* k-splits that suit the shape */
+int bl_qlin_tile_tokens(int m); /* of three digit planes */
 /* x [m x k] bf16 (pitch ldx) -> xq int8 [ceil(m/tile)][3][tile][k] (tile = bl_qlin_tile_tokens(m)) and
  * xs fp32 [m] with x = xs * (d0 + d1 / 2^8 + d2 / 2^16): exact for elements down to 2^-15 of the row's
  * largest, to 2^-24 of the largest below that.  permute: digits in the order 0 2 4 6 1 3 5 7 of every

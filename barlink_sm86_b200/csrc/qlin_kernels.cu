@@ -77,9 +77,10 @@ struct QlinCfg {
   static constexpr int kStage = kStageA + kStageB;
   static constexpr int kA8 = SRC == kNibbles ? 4 : 0;   // expanded tiles in flight
   // as many bytes in flight as fit: the weight stream is what counts
-  static constexpr int kFit = (226 * 1024 - 2048 - kA8 * kQTileA) / kStage;
+  static constexpr int kScales = GROUPED ? 8 * kQRows * 4 : 0;   // group scales of eight k-blocks
+  static constexpr int kFit = (226 * 1024 - 2048 - kScales - kA8 * kQTileA) / kStage;
   static constexpr int kStages = kFit > 10 ? 10 : kFit;
-  static constexpr int kSmem = kStages * kStage + kA8 * kQTileA + 2048;
+  static constexpr int kSmem = kStages * kStage + kA8 * kQTileA + kScales + 2048;
   // per-group mode hands an accumulator over every k-block: four of them where they fit
   static constexpr int kAcc = GROUPED && 4 * BN <= 512 ? 4 : 2;
   static constexpr int kCols = kAcc * BN <= 32 ? 32 : kAcc * BN <= 64 ? 64 : kAcc * BN <= 128 ? 128 : kAcc * BN <= 256 ? 256 : 512;
@@ -344,11 +345,17 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
     pdl_wait();
     int accs = 0;
     bool ok = true;
-    // Group scales of the next kAhead k-blocks, requested together and one batch ahead, kept as they came
-    // and turned into fp32 at their use, so that no k-block waits for a trip to HBM.
+    // Straight-line code that runs once a tile comes at the pace of the instruction cache, not of the SM.  With
+    // every loop of the epilogue unrolled, warps waited 3.5 (64 tokens, group scales) to 14 (one small tile)
+    // cycles for instructions per one issued; 64 tokens took 17 us at 256 x 256 and, with group scales, 98 us at
+    // 37888 x 3584.  Rolled wherever registers need no index: 8.8 and 52 us.
+    // Group scales of kAhead k-blocks are requested together and one batch ahead, kept as they came and
+    // turned into fp32 at their use, so that no k-block waits for a trip to HBM.  They pass through slots of
+    // shared memory that only this thread touches.
     constexpr int kAhead = 8;
-    uint32_t sc_cur[GROUPED ? kAhead : 1], sc_next[GROUPED ? kAhead : 1];
-    auto scales_of = [&](int u, int kb, uint32_t (&q8)[GROUPED ? kAhead : 1]) {
+    uint32_t* s_sc = reinterpret_cast<uint32_t*>(smem_raw + (ring_a8 + S::kA8 * kQTileA - smem_u32(smem_raw))) + row;
+    uint32_t sc_next[GROUPED ? kAhead : 1];
+    auto scales_of = [&](int u, int kb) {
       const int tile = u / g.splits, kb1 = min(g.kblocks, (u - tile * g.splits + 1) * kb_per);
       const int n = (tile / g.tiles_b) * kQRows + row;
       const bool in = u < units && n < g.n;
@@ -357,13 +364,18 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
 #pragma unroll
       for (int i = 0; i < (GROUPED ? kAhead : 1); ++i) {
         const int gi = (kb + i) / g.gk;
-        q8[i] = !in || kb + i >= kb1                    ? 0u
-                : g.scale_kind == BL_QSCALE_F32_GN ? __ldg(p32 + size_t(gi) * g.n + n)
-                : g.scale_kind == BL_QSCALE_F16_GN ? uint32_t(__ldg(p16 + size_t(gi) * g.n + n))
-                                                   : uint32_t(__ldg(p16 + size_t(n) * g.groups + gi));
+        sc_next[i] = !in || kb + i >= kb1                    ? 0u
+                     : g.scale_kind == BL_QSCALE_F32_GN ? __ldg(p32 + size_t(gi) * g.n + n)
+                     : g.scale_kind == BL_QSCALE_F16_GN ? uint32_t(__ldg(p16 + size_t(gi) * g.n + n))
+                                                        : uint32_t(__ldg(p16 + size_t(n) * g.groups + gi));
       }
     };
-    if constexpr (GROUPED) scales_of(blockIdx.x, (int(blockIdx.x) % g.splits) * kb_per, sc_cur);
+    auto scale_f32 = [&](uint32_t raw) -> float {
+      return g.scale_kind == BL_QSCALE_F32_GN ? __uint_as_float(raw)
+             : g.scale_kind == BL_QSCALE_BF16_NG ? __uint_as_float(raw << 16)
+                                                 : __half2float(__ushort_as_half(static_cast<unsigned short>(raw)));
+    };
+    if constexpr (GROUPED) scales_of(blockIdx.x, (int(blockIdx.x) % g.splits) * kb_per);
     for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
       const int tile = u / g.splits, sp = u - tile * g.splits;
       const int ta = tile / g.tiles_b, tb = tile - ta * g.tiles_b;
@@ -396,40 +408,35 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
       int done_acc = 0;
       if constexpr (GROUPED) {
         const int kb0 = sp * kb_per, kb1 = min(g.kblocks, kb0 + kb_per);
-        auto scale_f32 = [&](uint32_t raw) -> float {
-          return g.scale_kind == BL_QSCALE_F32_GN ? __uint_as_float(raw)
-                 : g.scale_kind == BL_QSCALE_BF16_NG ? __uint_as_float(raw << 16)
-                                                     : __half2float(__ushort_as_half(static_cast<unsigned short>(raw)));
-        };
         if (g.row_scale) rs = __bfloat162float(g.row_scale[nn]);
 #pragma unroll
         for (int i = 0; i < TB; ++i) accf[i] = 0.f;
-        for (int kb = kb0; kb < kb1 && ok; kb += kAhead) {
-          if (kb + kAhead < kb1) scales_of(u, kb + kAhead, sc_next);
-          else scales_of(u + gridDim.x, ((u + gridDim.x) % g.splits) * kb_per, sc_next);
+#pragma unroll 1
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const int i = (kb - kb0) % kAhead;
+          if (i == 0) {
 #pragma unroll
-          for (int i = 0; i < kAhead; ++i) {
-            if (kb + i >= kb1 || !ok) break;
-            const float sc = scale_f32(sc_cur[i]);
-            const int acc = accs % S::kAcc;
-            if (!mbar_wait_bounded_warp(&tfull_bar[acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) {
-              ok = false;
-              break;
-            }
-            ++accs;
-            tc_fence_after_sync();
-#pragma unroll
-            for (int c0 = 0; c0 < TB; c0 += 16) {
-              float v[16];
-              read16(acc, c0, v);
-#pragma unroll
-              for (int j = 0; j < 16; ++j) accf[c0 + j] = fmaf(v[j], sc, accf[c0 + j]);
-            }
-            tc_fence_before_sync();
-            mbar_arrive(&tempty_bar[acc]);
+            for (int j = 0; j < kAhead; ++j) s_sc[j * kQRows] = sc_next[j];
+            if (kb + kAhead < kb1) scales_of(u, kb + kAhead);
+            else scales_of(u + gridDim.x, ((u + gridDim.x) % g.splits) * kb_per);
           }
+          const float sc = scale_f32(s_sc[i * kQRows]);
+          const int acc = accs % S::kAcc;
+          if (!mbar_wait_bounded_warp(&tfull_bar[acc], uint32_t(accs / S::kAcc) & 1u, s_abort)) {
+            ok = false;
+            break;
+          }
+          ++accs;
+          tc_fence_after_sync();
 #pragma unroll
-          for (int i = 0; i < kAhead; ++i) sc_cur[i] = sc_next[i];
+          for (int c0 = 0; c0 < TB; c0 += 16) {
+            float v[16];
+            read16(acc, c0, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) accf[c0 + j] = fmaf(v[j], sc, accf[c0 + j]);
+          }
+          tc_fence_before_sync();
+          mbar_arrive(&tempty_bar[acc]);
         }
         if (!ok) break;
       } else {
@@ -440,32 +447,41 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
         tc_fence_after_sync();
       }
       const float bv = (nok && g.bias && !g.slabs) ? __bfloat162float(g.bias[n]) : 0.f;
-      float* slab = g.slabs ? g.slabs + size_t(sp) * g.m * g.n : nullptr;
-#pragma unroll
-      for (int c0 = 0; c0 < TB; c0 += 16) {
+      const int m_end = min(g.m - m0, TB);  // tokens of this tile
+#pragma unroll 1
+      for (int c0 = 0; c0 < m_end; c0 += 16) {
         float v[16];
         if constexpr (GROUPED) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = accf[c0 + j];
+          for (int j = 0; j < 16; ++j) v[j] = accf[j];
+          // (the next 16 sums move down: the loop body stays one)
+#pragma unroll
+          for (int j = 0; j + 16 < TB; ++j) accf[j] = accf[j + 16];
         } else {
           read16(done_acc, c0, v);
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int m = m0 + c0 + j;
-          const bool mok = m < g.m;
-          const float y = v[j] * ((mok ? __ldg(g.xs + m) : 0.f) * rs);
-          if (slab) {
-            if (mok && nok) __stcg(slab + size_t(m) * g.n + n, y);
-          } else if (g.silu) {
-            // even lanes hold gate rows, odd lanes the matching up rows
-            const float mine = y + bv;
+        for (int j = 0; j < 16; ++j) v[j] *= (c0 + j < m_end ? __ldg(g.xs + m0 + c0 + j) : 0.f) * rs;
+        const int m1 = m0 + c0, mn = nok ? min(16, m_end - c0) : 0;  // first token, tokens to store
+        if (g.slabs) {
+          float* o = g.slabs + (size_t(sp) * g.m + m1) * g.n + n;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < mn) __stcg(o + size_t(j) * g.n, v[j]);
+        } else if (g.silu) {
+          // even lanes hold gate rows, odd lanes the matching up rows
+          __nv_bfloat16* o = g.out + size_t(m1) * g.ldo + (n >> 1);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const float mine = v[j] + bv;
             const float other = __shfl_xor_sync(0xffffffffu, mine, 1);
-            if (mok && nok && !(row & 1))
-              g.out[size_t(m) * g.ldo + (n >> 1)] = __float2bfloat16(mine / (1.f + __expf(-mine)) * other);
-          } else if (mok && nok) {
-            g.out[size_t(m) * g.ldo + n] = __float2bfloat16(y + bv);
+            if (j < mn && !(row & 1)) o[size_t(j) * g.ldo] = __float2bfloat16(mine / (1.f + __expf(-mine)) * other);
           }
+        } else {
+          __nv_bfloat16* o = g.out + size_t(m1) * g.ldo + n;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (j < mn) o[size_t(j) * g.ldo] = __float2bfloat16(v[j] + bv);
         }
       }
       if constexpr (!GROUPED) {
@@ -656,12 +672,21 @@ static int launch_qlin(const blQlinArgs& a, cudaStream_t st, char* err, size_t e
   return 0;
 }
 
+// Tokens of a tile.  One int8 digit with per-channel scales takes up to 128, so that no weight tile is
+// fetched twice (65 .. 128 tokens, 37888 x 3584, two tiles of 64: 55 us; one of 128: 28 us).
+static int qlin_tile_tokens(int m, int digits, bool grouped) {
+  return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 || digits > 1 || grouped ? 64 : 128;
+}
+
 template <int SRC, int ND, bool GROUPED>
 static int launch_qlin_tb(const blQlinArgs& a, cudaStream_t st, char* err, size_t errlen) {
-  switch (bl_qlin_tile_tokens(a.m)) {
+  switch (qlin_tile_tokens(a.m, a.digits, GROUPED)) {
     case 16: return launch_qlin<SRC, ND, 16, GROUPED>(a, st, err, errlen);
     case 32: return launch_qlin<SRC, ND, 32, GROUPED>(a, st, err, errlen);
-    default: return launch_qlin<SRC, ND, 64, GROUPED>(a, st, err, errlen);
+    case 64: return launch_qlin<SRC, ND, 64, GROUPED>(a, st, err, errlen);
+    default:
+      if constexpr (ND == 1 && !GROUPED) return launch_qlin<SRC, ND, 128, GROUPED>(a, st, err, errlen);
+      return -1;
   }
 }
 
@@ -669,12 +694,12 @@ static int launch_qlin_tb(const blQlinArgs& a, cudaStream_t st, char* err, size_
 
 using namespace bl;
 
-extern "C" int bl_qlin_tile_tokens(int m) { return m <= 16 ? 16 : m <= 32 ? 32 : 64; }
+extern "C" int bl_qlin_tile_tokens(int m) { return qlin_tile_tokens(m, 3, false); }
 
 // Work is dealt out in units of (row tile, token tile, k-split); the SMs take them lap by lap.  A lap
 // costs its k-blocks plus about two of hand-over, and every split adds a slab to write and to read.
-extern "C" int bl_qlin_splits(int n, int k, int m) {
-  const int tb = bl_qlin_tile_tokens(m);
+extern "C" int bl_qlin_splits(int n, int k, int m, int digits, int grouped) {
+  const int tb = qlin_tile_tokens(m, digits, grouped != 0);
   const int tiles = ((n + kQRows - 1) / kQRows) * ((m + tb - 1) / tb), kb = (k + kQK - 1) / kQK, sms = sm_count();
   int best = 1;
   double cost = 1e30;

@@ -58,6 +58,23 @@ def test_int8_weights_bf16_activations(ext, m, n, k):
     assert ext.w8_error_flag(0) == 0
 
 
+# int8 activations: the tile of 128 tokens and its neighbours, ragged rows and k-blocks, with and without a k-split
+@pytest.mark.parametrize("m", [63, 65, 127, 128])
+@pytest.mark.parametrize("n,k", [(128, 128), (200, 1040), (1000, 3584)])
+def test_int8_activations_up_to_128_tokens(ext, m, n, k):
+    wq, sc = _w8(n, k, 3)
+    x = _x(m, k, 5)
+    b = torch.randn(n, generator=_g(9), device="cuda").bfloat16()
+    xq, xs = ext.w8a16_quant_act(x)
+    y = (xq.double() @ wq.double().t()) * xs.double()[:, None] * sc.double() + b.double()
+    silu = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
+    for splits in (0, 1, 3):
+        assert rel_l2(ext.w8a16_linear(x, wq, sc, b, splits=splits, act_int8=True), y) < TOL
+        assert rel_l2(ext.w8a16_linear(x, wq, sc, b, True, splits, act_int8=True), silu) < TOL
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
+
+
 # a bias that starts off a 16-byte boundary (a slice of a longer vector), with and without a k-split, and
 # where the shape picks one by itself (the last)
 @pytest.mark.parametrize("off", [1, 4])

@@ -517,7 +517,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<
   }
   void* st = at::cuda::getCurrentCUDAStream(dev).stream();
   // few tiles of a long reduction: k-splits into fp32 slabs, and a kernel that sums them with the epilogue
-  if (!swap && bn <= 0 && splits <= 0 && !tiled && gate_tokens <= 0 && !residual && !gelu && n % 16 == 0 &&
+  if (!swap && bn <= 0 && splits <= 0 && !tiled && gate_tokens <= 0 && !trace && !residual && !gelu && n % 16 == 0 &&
       ((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(a.bias)) & 15u) == 0) {
     const int s2 = bl_gemm_row_splits(tokens, n, k);
     if (s2 > 1) {

@@ -1022,7 +1022,8 @@ static bool gemm_pair_enabled() {
 // do; below 129 the caller uses the swapped form.
 static bool gemm_pair_ok(const blGemmArgs& a) {
   return gemm_pair_enabled() && !a.i8 && !a.swap && a.ra > 128 && a.rb >= 256 && !a.peer && !a.gate_flags &&
-         !a.weight_tiled && (a.partial_out ? a.partial_splits >= 1 : a.splits <= 1) && !(a.push && a.ra < 512);
+         !a.weight_tiled && (a.partial_out ? a.partial_splits >= 1 : a.splits <= 1) &&
+         !((a.push || a.trace) && a.ra < 512);  // (the stamps of a trace are k_gemm's)
 }
 
 template <class Sink>

@@ -79,6 +79,14 @@ def test_token_major_off_16_bytes(ext, which, rows, n, k, bn, off):
     assert ext.gemm_error_flag(0) == 0
 
 
+@pytest.mark.parametrize("rows,n,k", [(129, 256, 512), (511, 512, 4096)])
+def test_trace_stamps_below_512_rows(ext, rows, n, k):
+    x, w = _bf(rows, k, seed=1), _bf(n, k, seed=2, std=k ** -0.5)
+    trace = torch.zeros(8 * 296, dtype=torch.int64, device="cuda")
+    assert rel_l2(ext.linear(x, w, trace=trace), x.float() @ w.float().t()) < TOL
+    assert bool((trace.view(-1, 8)[0, [0, 2, 3]] > 0).all())
+
+
 def test_row_splits_rule(ext):
     assert ext.gemm_row_splits(128, 3584, 18944) == 1  # the swapped form
     assert ext.gemm_row_splits(333, 3584, 18944) >= 2  # 28 tiles for 74 pairs

@@ -517,22 +517,31 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<
   }
   void* st = at::cuda::getCurrentCUDAStream(dev).stream();
   // few tiles of a long reduction: k-splits into fp32 slabs, and a kernel that sums them with the epilogue
-  if (!swap && bn <= 0 && splits <= 0 && !tiled && gate_tokens <= 0 && !trace && !residual && !gelu && n % 16 == 0 &&
-      ((reinterpret_cast<uintptr_t>(out.data_ptr()) | reinterpret_cast<uintptr_t>(a.bias)) & 15u) == 0) {
+  if (!swap && bn <= 0 && splits <= 0 && !tiled && gate_tokens <= 0) {
     const int s2 = bl_gemm_row_splits(tokens, n, k);
     if (s2 > 1) {
       py::gil_scoped_release nogil;
-      at::Tensor slabs = at::empty({s2, tokens, n}, x.options().dtype(at::kFloat));
+      const int pitch = (n + 7) & ~7;
+      at::Tensor slabs = at::empty({s2, tokens, pitch}, x.options().dtype(at::kFloat));
+      blSlabFinishArgs f;
+      memset(&f, 0, sizeof(f));
+      f.slabs = slabs.data_ptr();
+      f.nsplit = s2; f.m = tokens; f.n = n; f.pitch = pitch;
+      f.bias = a.bias;
+      f.residual = silu_mul ? nullptr : a.residual;
+      f.silu_mul = a.silu_mul;
+      f.gelu = a.gelu;
+      f.out = a.out;
+      f.ldo = n_out;
       a.out = nullptr;
-      a.bias = nullptr;
-      a.silu_mul = 0;
-      a.ldo = n;
+      a.bias = a.residual = nullptr;
+      a.silu_mul = a.gelu = 0;
+      a.ldo = pitch;
       a.partial_out = slabs.data_ptr();
-      a.partial_stride = size_t(tokens) * n;
+      a.partial_stride = size_t(tokens) * pitch;
       a.partial_splits = s2;
       BL_CHECK(bl_gemm_bf16(&a, st, err, errlen));
-      BL_CHECK(bl_slab_finish(slabs.data_ptr(), s2, tokens, n, bias ? bias->data_ptr() : nullptr, silu_mul ? 1 : 0,
-                              out.data_ptr(), n_out, st, err, errlen));
+      BL_CHECK(bl_slab_finish(&f, st, err, errlen));
       return out;
     }
   }

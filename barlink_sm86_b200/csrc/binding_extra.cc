@@ -220,8 +220,8 @@ at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int d
     TORCH_CHECK(bias->numel() == q.n, "barlink: bias must have n entries");
   }
   if (splits <= 0) splits = bl_qlin_splits(q.n, q.k, m, digits, q.scale_kind != BL_QSCALE_BF16_N);
-  // bl_slab_finish stores 16-byte vectors
-  if (!want_slabs && (silu_mul ? q.n % 16 : q.n % 8) != 0) splits = 1;
+  // bl_slab_finish reads slabs whose pitch is a multiple of 8
+  if (!want_slabs && q.n % 8 != 0) splits = 1;
   const int kb = (q.k + 127) / 128, per = (kb + splits - 1) / splits;
   splits = (kb + per - 1) / per;
   blQlinArgs a;
@@ -247,8 +247,15 @@ at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int d
   if (splits == 1) return out;
   if (want_slabs) return slabs;
   out = at::empty({m, silu_mul ? q.n / 2 : q.n}, like);
-  BL_CHECK(bl_slab_finish(slabs.data_ptr(), splits, m, q.n, bias ? bias->data_ptr() : nullptr, silu_mul ? 1 : 0,
-                          out.data_ptr(), int(out.size(1)), st, err, errlen));
+  blSlabFinishArgs f;
+  memset(&f, 0, sizeof(f));
+  f.slabs = slabs.data_ptr();
+  f.nsplit = splits; f.m = m; f.n = f.pitch = q.n;
+  f.bias = bias ? bias->data_ptr() : nullptr;
+  f.silu_mul = silu_mul ? 1 : 0;
+  f.out = out.data_ptr();
+  f.ldo = int(out.size(1));
+  BL_CHECK(bl_slab_finish(&f, st, err, errlen));
   return out;
 }
 // digits = 3: x as it is; digits = 1: x quantised to int8 per token.  Callers let go of the GIL first: a

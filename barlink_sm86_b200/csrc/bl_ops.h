@@ -114,7 +114,8 @@ int bl_tile_weight(const void* src, int n, int k, int ld, void* dst, void* strea
 /* k-splits the decode heuristic picks for n output features, k inputs and
  * `tokens` rows (1 = no split) */
 int bl_gemm_splits(int n, int k, int tokens);
-/* k-splits that suit a token-major product (more than 128 rows), 1: none; slabs are [splits][rows][n] */
+/* k-splits that suit a token-major product (more than 128 rows), 1: none; slabs are [splits][rows][n, rounded up
+ * to a multiple of 8] */
 int bl_gemm_row_splits(int rows, int n, int k);
 
 /* W8A16: x [m x k] bf16, wq [n x k] int8 (row = output channel), scale [n]
@@ -211,9 +212,19 @@ int bl_qlin_tile_tokens(int m); /* of three digit planes */
 int bl_quant_digits(const void* x, int m, int ldx, int k, int permute, void* xq, void* xs, void* stream, char* err,
                     size_t errlen);
 size_t bl_quant_digits_bytes(int m, int k);
-/* slabs fp32 [nsplit][m][n] -> bf16, + bias, optionally SiLU*mul over interleaved columns */
-int bl_slab_finish(const void* slabs, int nsplit, int m, int n, const void* bias, int silu_mul, void* out, int ldo,
-                   void* stream, char* err, size_t errlen);
+/* slabs fp32 [nsplit][m][pitch] -> out bf16 [m][n] (pitch ldo), the sum with the epilogue of a product: + bias,
+ * tanh-GELU, + residual (out's layout); or, with silu_mul, + bias and SiLU*mul over interleaved columns into
+ * [m][n / 2].  Bias, residual and out may start at any element. */
+typedef struct blSlabFinishArgs {
+  const void* slabs;
+  int nsplit, m, n, pitch;
+  const void* bias;
+  const void* residual;
+  int silu_mul, gelu;
+  void* out;
+  int ldo;
+} blSlabFinishArgs;
+int bl_slab_finish(const blSlabFinishArgs* a, void* stream, char* err, size_t errlen);
 
 /* out = RMSNorm(x (+ residual)) * gamma; when residual is given, x + residual
  * is also written to residual_out (may alias residual). */

@@ -27,12 +27,6 @@ namespace bl {
 // 4 SiLU(gate)*up where gate/up rows are interleaved (even n = gate, odd n =
 // up) and the result lands in column n/2.
 // tanh on the special-function unit (one instruction; relative error about 2^-11, below bf16's)
-__device__ __forceinline__ float tanh_fast(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 template <int BN>
 struct LocalSink {
   __nv_bfloat16* out;
@@ -153,10 +147,7 @@ struct LocalSink {
           }
           if (epi & 8) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const float u = x[t];
-              x[t] = 0.5f * u * (1.f + tanh_fast(0.7978845608f * (u + 0.044715f * u * u * u)));
-            }
+            for (int t = 0; t < 8; ++t) x[t] = gelu_tanh(x[t]);
           }
           if (epi & 2) {
             const uint4 b = *reinterpret_cast<const uint4*>(rrow + j0 + c);
@@ -176,7 +167,7 @@ struct LocalSink {
           if (c < ncols && n < rb) {
             float x = v[c];
             if (epi & 1) x += __bfloat162float(bias[n]);
-            if (epi & 8) x = 0.5f * x * (1.f + tanh_fast(0.7978845608f * (x + 0.044715f * x * x * x)));
+            if (epi & 8) x = gelu_tanh(x);
             if (epi & 2) x += __bfloat162float(rrow[n]);
             orow[n] = __float2bfloat16(x);
           }
@@ -206,7 +197,7 @@ struct LocalSink {
         const int m = j0 + c;
         if (c < ncols && m < rb) {
           float x = v[c] + bv;
-          if (epi & 8) x = 0.5f * x * (1.f + tanh_fast(0.7978845608f * (x + 0.044715f * x * x * x)));
+          if (epi & 8) x = gelu_tanh(x);
           if (epi & 2) x += __bfloat162float(residual[size_t(m) * ldo + n]);
           out[size_t(m) * ldo + n] = __float2bfloat16(x);
         }
@@ -1246,12 +1237,14 @@ extern "C" int bl_gemm_splits(int n, int k, int tokens) {
   return pick_splits(tiles, kblocks, sm_count(), 0);
 }
 
-// k-splits of a token-major product in the paired kernel: 2 .. 4 when its tiles leave half of the pairs or more
-// without work.  A split of a lap costs its k-blocks plus about 16 of ramp and epilogue, and every slab is
-// written and read once more (in k-blocks of 0.33 us: rows * n * 8 bytes at 3 TB/s).  333 rows, 3584 x 18944:
-// 97 us unsplit, 79 us with 2 splits, 3072 x 12288: 70 and 42 us with 3; 160 rows, 3584 x 18944: 108 and 51 us.
+// k-splits of a token-major product in the paired kernel: the cheapest of 1 .. 4 by laps of the pairs, in
+// k-blocks of 0.28 us.  A product costs the k-blocks of its laps plus about 22 of ramp and epilogue; with a split
+// the kernel behind it costs 10 and the slabs, written and read once more, 0.85 a megabyte; below 3 % it is not
+// worth the memory.  Unsplit and with the split chosen, us: 512 x 18944 x 600 rows 89 and 33, 3584 x 18944 x 333
+// 97 and 59, 3584 x 18944 x 1285 (two laps by 10 tiles) 191 and 170, 5120 x 27648 x 1000 296 and 247, x 2048 566
+// and 474; where it does not split, 256 x 1024 x 1000 10.8 against 12.4 with two.
 extern "C" int bl_gemm_row_splits(int rows, int n, int k) {
-  if (!gemm_pair_enabled() || rows <= 128 || n < 256 || (n & 7) || (k & 7)) return 1;
+  if (!gemm_pair_enabled() || rows <= 128 || n < 256 || (k & 7)) return 1;
   const int tiles = ((rows + 255) / 256) * ((n + 255) / 256), pairs = sm_count() / 2, kb = (k + kTileK - 1) / kTileK;
   int best = 1;
   double cost = 1e30;
@@ -1259,7 +1252,7 @@ extern "C" int bl_gemm_row_splits(int rows, int n, int k) {
     const int per = (kb + s - 1) / s;
     if ((s - 1) * per >= kb) continue;
     const int laps = (tiles * s + pairs - 1) / pairs;
-    const double c = laps * per + 16.0 + (s > 1 ? double(s) * rows * n * 8.0 / 1e6 : 0.0);
+    const double c = laps * per + 22.0 + (s > 1 ? 10.0 + double(s) * rows * n * 8.0 * 0.85e-6 : 0.0);
     if (c < cost * (s > 1 ? 0.97 : 1.0)) {
       cost = c;
       best = s;

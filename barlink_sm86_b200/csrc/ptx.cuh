@@ -474,6 +474,11 @@ __device__ __forceinline__ float2 unpack_bf16x2(uint32_t v) {
 
 // acc[0..8) += sum over n slabs (stride elements apart) of the 8 floats at p,
 // in slab order; the loads of up to eight slabs are in flight together
+__device__ __forceinline__ float gelu_tanh(float u) {
+  float t;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608f * (u + 0.044715f * u * u * u)));
+  return 0.5f * u * (1.f + t);
+}
 __device__ __forceinline__ void sum_slabs8(const float* p, size_t stride, int n, float (&acc)[8]) {
   for (int s0 = 0; s0 < n; s0 += 8) {
     float4 u[8][2];

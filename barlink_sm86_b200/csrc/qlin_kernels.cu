@@ -574,38 +574,67 @@ __global__ void __launch_bounds__(kDigThreads) k_quant_digits(const __nv_bfloat1
   }
 }
 
-// fp32 slabs [split][m][n] -> bf16: sum in split order, + bias, optionally SiLU*mul over interleaved
-// (gate, up) columns.  Eight columns per thread.  The slabs and the output start on 16-byte boundaries, the
-// bias (a caller's tensor, often a slice of a longer one) at any element.
-__global__ void __launch_bounds__(256) k_slab_finish(const float* __restrict__ slabs, int nsplit, size_t slab, int n,
-                                                     const __nv_bfloat16* __restrict__ bias, int silu,
-                                                     __nv_bfloat16* __restrict__ out, int ldo, size_t total8) {
+// fp32 slabs [split][m][pitch] -> bf16 [m][n]: sum in split order, then what the epilogue of the unsplit product
+// does: + bias, tanh-GELU, + residual; or + bias and SiLU*mul over interleaved (gate, up) columns.  Eight columns
+// per thread.  The slabs start on 16-byte boundaries and have a pitch of a multiple of 8; bias, residual and
+// output are a caller's tensors, often slices of longer ones, and go element by element where their start, their
+// pitch or a ragged end asks for it.
+__device__ __forceinline__ void load8_any(const __nv_bfloat16* p, int cols, float (&f)[8]) {
+  if (cols == 8 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+    const uint4 b = *reinterpret_cast<const uint4*>(p);
+    const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y), b2 = unpack_bf16x2(b.z), b3 = unpack_bf16x2(b.w);
+    f[0] = b0.x; f[1] = b0.y; f[2] = b1.x; f[3] = b1.y;
+    f[4] = b2.x; f[5] = b2.y; f[6] = b3.x; f[7] = b3.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = j < cols ? __bfloat162float(p[j]) : 0.f;
+  }
+}
+__global__ void __launch_bounds__(256) k_slab_finish(const blSlabFinishArgs g, size_t total8) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (t >= total8) return;
-  const int per = n >> 3;
+  const int per = g.pitch >> 3;
   const size_t m = t / per;
-  const int c = int(t - m * per) * 8;
-  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  sum_slabs8(slabs + m * n + c, slab, nsplit, a);
-  if (bias && (reinterpret_cast<uintptr_t>(bias) & 15u)) {
+  const int c = int(t - m * per) * 8, cols = min(8, g.n - c);
+  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, f[8];
+  sum_slabs8(static_cast<const float*>(g.slabs) + m * g.pitch + c, size_t(g.m) * g.pitch, g.nsplit, a);
+  if (g.bias) {
+    load8_any(static_cast<const __nv_bfloat16*>(g.bias) + c, cols, f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] += __bfloat162float(bias[c + j]);
-  } else if (bias) {
-    const uint4 b = *reinterpret_cast<const uint4*>(bias + c);
-    const float2 b0 = unpack_bf16x2(b.x), b1 = unpack_bf16x2(b.y), b2 = unpack_bf16x2(b.z), b3 = unpack_bf16x2(b.w);
-    a[0] += b0.x; a[1] += b0.y; a[2] += b1.x; a[3] += b1.y;
-    a[4] += b2.x; a[5] += b2.y; a[6] += b3.x; a[7] += b3.y;
+    for (int j = 0; j < 8; ++j) a[j] += f[j];
   }
-  if (silu) {
+  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(g.out) + m * g.ldo + (g.silu_mul ? c >> 1 : c);
+  if (g.silu_mul) {
     float o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) o[j] = a[2 * j] / (1.f + __expf(-a[2 * j])) * a[2 * j + 1];
-    *reinterpret_cast<uint2*>(out + m * ldo + (c >> 1)) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+    if (cols == 8 && (reinterpret_cast<uintptr_t>(out) & 7u) == 0) {
+      *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < (cols >> 1)) out[j] = __float2bfloat16(o[j]);
+    }
+    return;
+  }
+  if (g.gelu) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = gelu_tanh(a[j]);
+  }
+  if (g.residual) {
+    load8_any(static_cast<const __nv_bfloat16*>(g.residual) + m * g.ldo + c, cols, f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] += f[j];
+  }
+  if (cols == 8 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+    *reinterpret_cast<uint4*>(out) = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]),
+                                                pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
   } else {
-    *reinterpret_cast<uint4*>(out + m * ldo + c) = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]),
-                                                              pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < cols) out[j] = __float2bfloat16(a[j]);
   }
 }
 
@@ -743,18 +772,15 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
   return 0;
 }
 
-extern "C" int bl_slab_finish(const void* slabs, int nsplit, int m, int n, const void* bias, int silu_mul, void* out,
-                              int ldo, void* stream, char* err, size_t errlen) {
-  if (!slabs || !out || nsplit < 1 || m < 1 || n < 8 || (n & 7) || (ldo & 7) ||
-      ((reinterpret_cast<uintptr_t>(slabs) | reinterpret_cast<uintptr_t>(out)) & 15u)) {
-    set_err(err, errlen, "barlink: slab_finish needs n and the output pitch in multiples of 8, slabs and output on 16-byte boundaries");
+extern "C" int bl_slab_finish(const blSlabFinishArgs* a, void* stream, char* err, size_t errlen) {
+  if (!a || !a->slabs || !a->out || a->nsplit < 1 || a->m < 1 || a->n < 1 || a->pitch < a->n || (a->pitch & 7) ||
+      (reinterpret_cast<uintptr_t>(a->slabs) & 15u)) {
+    set_err(err, errlen, "barlink: slab_finish needs slabs on a 16-byte boundary with a pitch of a multiple of 8 that holds n");
     return -1;
   }
-  const size_t total8 = size_t(m) * (n / 8);
+  const size_t total8 = size_t(a->m) * (a->pitch / 8);
   cudaError_t e = launch_k(k_slab_finish, dim3(unsigned((total8 + 255) / 256)), dim3(256), 0,
-                           static_cast<cudaStream_t>(stream), static_cast<const float*>(slabs), nsplit, size_t(m) * n, n,
-                           static_cast<const __nv_bfloat16*>(bias), silu_mul, static_cast<__nv_bfloat16*>(out), ldo,
-                           total8);
+                           static_cast<cudaStream_t>(stream), *a, total8);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: slab_finish launch failed: %s", cudaGetErrorString(e));

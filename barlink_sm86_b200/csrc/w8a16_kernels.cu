@@ -121,8 +121,8 @@ extern "C" int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, c
     set_err(err, errlen, "barlink: w8a16_gemm with a k-split needs a workspace of S*M*N floats");
     return -1;
   }
-  // bl_slab_finish reads and stores 16-byte vectors
-  if ((n & 7) || ((reinterpret_cast<uintptr_t>(ws) | reinterpret_cast<uintptr_t>(out)) & 15u)) splits = 1;
+  // bl_slab_finish reads 16-byte vectors
+  if ((n & 7) || (reinterpret_cast<uintptr_t>(ws) & 15u)) splits = 1;
   blQlinArgs a;
   memset(&a, 0, sizeof(a));
   a.w = wq_t;
@@ -141,6 +141,14 @@ extern "C" int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, c
   a.out = out;
   a.ldo = n;
   if (bl_qlin(&a, stream, err, errlen) != 0) return -1;
-  if (splits > 1) return bl_slab_finish(ws, splits, m, n, nullptr, 0, out, n, stream, err, errlen);
+  if (splits > 1) {
+    blSlabFinishArgs f;
+    memset(&f, 0, sizeof(f));
+    f.slabs = ws;
+    f.nsplit = splits; f.m = m; f.n = f.pitch = n;
+    f.out = out;
+    f.ldo = n;
+    return bl_slab_finish(&f, stream, err, errlen);
+  }
   return 0;
 }

@@ -52,7 +52,7 @@ def test_paired_kernel_few_rows(ext, rows, n, k):
     silu = torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]
     assert rel(ext.linear(x, w, b, None, True), silu) < 2.0 ** -8
     r = torch.randn(rows, n, generator=g, device="cuda").bfloat16()
-    assert rel(ext.linear(x, w, b, r), y + r.double()) < 2.0 ** -8  # a residual keeps the product whole
+    assert rel(ext.linear(x, w, b, r), y + r.double()) < 2.0 ** -8
     torch.cuda.synchronize()
     assert ext.gemm_error_flag(0) == 0
 
@@ -60,7 +60,7 @@ def test_paired_kernel_few_rows(ext, rows, n, k):
 # bias, residual or output off a 16-byte boundary (slices of longer tensors): the paired kernel, and with
 # bn = 128 the single-CTA one
 @pytest.mark.parametrize("which", ["bias", "residual", "out"])
-@pytest.mark.parametrize("rows,n,k,bn", [(129, 256, 512, 0), (600, 264, 136, 0), (200, 256, 512, 128)])
+@pytest.mark.parametrize("rows,n,k,bn", [(129, 256, 512, 0), (600, 264, 136, 0), (200, 256, 512, 128), (200, 264, 4096, 0)])
 @pytest.mark.parametrize("off", [1, 4])
 def test_token_major_off_16_bytes(ext, which, rows, n, k, bn, off):
     def cut(t, on):  # the same values, starting `off` elements into a buffer when `on`
@@ -79,6 +79,28 @@ def test_token_major_off_16_bytes(ext, which, rows, n, k, bn, off):
     assert ext.gemm_error_flag(0) == 0
 
 
+# k-splits with every epilogue: widths that no vector divides, one column more than a tile, the last k-block ragged
+@pytest.mark.parametrize("rows", [129, 300, 520])
+@pytest.mark.parametrize("n,k", [(257, 4096), (520, 4104), (1022, 8192)])
+def test_k_split_epilogues(ext, rows, n, k):
+    assert ext.gemm_row_splits(rows, n, k) > 1
+    x, w, b, r = _bf(rows, k, seed=1), _bf(n, k, seed=2, std=k ** -0.5), _bf(n, seed=3), _bf(rows, n, seed=4)
+    rel = lambda a, c: float((a.double() - c).norm() / c.norm())
+    y = x.double() @ w.double().t() + b.double()
+    gelu = torch.nn.functional.gelu(y, approximate="tanh")
+    assert rel(ext.linear(x, w, b), y) < TOL
+    assert rel(ext.linear(x, w, b, r), y + r.double()) < TOL
+    assert rel(ext.linear(x, w, b, gelu=True), gelu) < TOL
+    assert rel(ext.linear(x, w, b, r, gelu=True), gelu + r.double()) < TOL
+    even = y[:, : n // 2 * 2]
+    silu = torch.nn.functional.silu(even[:, 0::2]) * even[:, 1::2]
+    assert rel(ext.linear(x, w, b, None, True), silu) < TOL
+    same = r.clone()  # the residual stream updated in place
+    assert rel(ext.linear(x, w, b, same, False, same), y + r.double()) < TOL
+    torch.cuda.synchronize()
+    assert ext.gemm_error_flag(0) == 0
+
+
 @pytest.mark.parametrize("rows,n,k", [(129, 256, 512), (511, 512, 4096)])
 def test_trace_stamps_below_512_rows(ext, rows, n, k):
     x, w = _bf(rows, k, seed=1), _bf(n, k, seed=2, std=k ** -0.5)
@@ -91,6 +113,9 @@ def test_row_splits_rule(ext):
     assert ext.gemm_row_splits(128, 3584, 18944) == 1  # the swapped form
     assert ext.gemm_row_splits(333, 3584, 18944) >= 2  # 28 tiles for 74 pairs
     assert ext.gemm_row_splits(333, 37888, 3584) == 1 and ext.gemm_row_splits(8192, 3584, 18944) == 1
+    assert ext.gemm_row_splits(1000, 256, 1024) == 1  # a second kernel costs more than it saves
+    # just above one lap of the pairs: 75 and 84 tiles, 80 tiles of a very long reduction
+    assert min(ext.gemm_row_splits(*t) for t in [(1280, 3840, 18944), (1285, 3584, 18944), (1000, 5120, 27648)]) >= 2
     for rows, n, k in [(129, 256, 64), (129, 256, 128), (300, 512, 200), (2000, 3584, 18944)]:
         s, kb = ext.gemm_row_splits(rows, n, k), -(-k // 64)
         assert (s - 1) * -(-kb // s) < kb  # no empty split

@@ -217,11 +217,11 @@ def test_other_threads_run_while_a_launch_waits(ext):
     import time
     n, k = 200, 1024
     wq, sc = _w8(n, k, 3)
-    x, xl = _x(6, k, 5), _x(300, k, 6)
+    x, xl = _x(6, k, 5), _x(300, 4096, 6)
     wq_t, sw = wq.view(n, k // 16, 16).permute(1, 0, 2).contiguous(), torch.ones(k // 128, n, device="cuda")
     xq, xs = ext.w8a16_quant_act(x)
-    w = _x(512, k, 7)
-    assert ext.gemm_row_splits(300, 512, k) > 1
+    w = _x(512, 4096, 7)
+    assert ext.gemm_row_splits(300, 512, 4096) > 1
     qw = torch.zeros(k // 8, n, dtype=torch.int32, device="cuda")
     s4, qz = torch.ones(k // 128, n, device="cuda").half(), torch.zeros(k // 128, n // 8, dtype=torch.int32, device="cuda")
     for name, f in {"w8a16_linear": lambda: ext.w8a16_linear(x, wq, sc),

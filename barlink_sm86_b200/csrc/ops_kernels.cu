@@ -275,25 +275,13 @@ __global__ void __launch_bounds__(256) k_rope_kv_write(__nv_bfloat16* __restrict
 // computed once per row, and kRopeBatch heads are requested at a time.  (One pair per thread with 2-byte
 // accesses and a sincosf for every pair of every head took 189 us for 8192 rows of 36 heads; this takes 56 us.)
 constexpr int kRopeBatch = 5;
-template <bool VEC>
 __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&f)[4]) {
-  if (VEC) {
-    const uint2 a = *reinterpret_cast<const uint2*>(p);
-    const float2 x = unpack_bf16x2(a.x), y = unpack_bf16x2(a.y);
-    f[0] = x.x; f[1] = x.y; f[2] = y.x; f[3] = y.y;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) f[j] = __bfloat162float(p[j]);
-  }
+  const uint2 a = *reinterpret_cast<const uint2*>(p);
+  const float2 x = unpack_bf16x2(a.x), y = unpack_bf16x2(a.y);
+  f[0] = x.x; f[1] = x.y; f[2] = y.x; f[3] = y.y;
 }
-template <bool VEC>
 __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&f)[4]) {
-  if (VEC) {
-    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) p[j] = __float2bfloat16(f[j]);
-  }
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
 }
 __global__ void __launch_bounds__(kRowThreads) k_rope_kv_rows(__nv_bfloat16* __restrict__ qkv,
                                                               const int* __restrict__ positions,
@@ -324,8 +312,8 @@ __global__ void __launch_bounds__(kRowThreads) k_rope_kv_rows(__nv_bfloat16* __r
     for (int c = 0; c < kRopeBatch; ++c) {
       const int h = hb + c * hpp;
       if (h < last) {
-        load4<true>(prow + size_t(h) * hd + i0, a[c]);
-        load4<true>(prow + size_t(h) * hd + i0 + half, b[c]);
+        load4(prow + size_t(h) * hd + i0, a[c]);
+        load4(prow + size_t(h) * hd + i0 + half, b[c]);
       }
     }
 #pragma unroll
@@ -340,13 +328,13 @@ __global__ void __launch_bounds__(kRowThreads) k_rope_kv_rows(__nv_bfloat16* __r
         o2[j] = rot ? b[c][j] * cs[j] + a[c][j] * sn[j] : b[c][j];
       }
       if (rot) {
-        store4<true>(prow + size_t(h) * hd + i0, o1);
-        store4<true>(prow + size_t(h) * hd + i0 + half, o2);
+        store4(prow + size_t(h) * hd + i0, o1);
+        store4(prow + size_t(h) * hd + i0 + half, o2);
       }
       if (h >= nq && slot >= 0) {
         __nv_bfloat16* cache = (rot ? k_cache : v_cache) + coff + size_t(rot ? h - nq : h - nq - nkv) * block_size * hd;
-        store4<true>(cache + i0, o1);
-        store4<true>(cache + i0 + half, o2);
+        store4(cache + i0, o1);
+        store4(cache + i0 + half, o2);
       }
     }
   }
@@ -1246,6 +1234,31 @@ __global__ void k_decode_advance(int* __restrict__ positions, int* __restrict__ 
 
 using namespace bl;
 
+// Whether k_rmsnorm_rows is the faster one: it has more rows in flight, k_rmsnorm more threads to a row.  An SM
+// holds blocks of k_rmsnorm with 512 threads in all; once the rows need a second turn of them, and for rows of more
+// than 2048 elements always, the rows kernel wins; for narrow rows (most of its 128 threads idle) only while there
+// are few.  us, k_rmsnorm and k_rmsnorm_rows, with residual: 333 x 3584 5.3 and 4.0, 8192 x 3584 164 and 44;
+// 297 x 2048 3.4 and 2.7, 260 x 2048 2.4 and 2.7; 600 x 1024 3.4 and 3.2, 450 x 1024 2.3 and 2.6, 200 x 1024 2.3 and
+// 2.0; 1000 x 256 2.4 and 3.6, 200 x 256 2.3 and 1.9.  Without one it wins at every size (600 x 2048 4.1 and 2.7).
+static bool rms_by_rows(int rows, int vpr, bool residual) {
+  const int sms = sm_count();
+  if (rows <= sms || vpr > 8 * kRowThreads) return false;
+  if (!residual || vpr > 256) return true;
+  const int threads = (vpr + 31) / 32 * 32;
+  const bool one_turn = rows <= sms * (512 / threads);
+  return (vpr <= 128 && rows <= 2 * sms) || (vpr > 64 && !one_turn);
+}
+// The same for k_layernorm_modulate, of which an SM holds 1152 threads: 4608 x 3072 19 and 10.6 us, 450 x 3072 3.7 and
+// 3.5, 333 x 3072 2.5 and 2.7, 297 x 4096 3.7 and 3.4, 260 x 4096 2.5 and 3.1; 1000 x 1536 3.8 and 3.2, 600 x 1536 2.5
+// and 3.0, 260 x 1536 2.4 and 2.2; 4608 x 1024 7.1 and 7.6.
+static bool layernorm_by_rows(int rows, int vpr) {
+  const int sms = sm_count();
+  if (rows <= sms || vpr > 8 * kRowThreads) return false;
+  const int threads = vpr < 512 ? (vpr + 31) / 32 * 32 : 512;
+  if (rows > sms * (1152 / threads)) return vpr > 128;
+  return rows <= (vpr <= 192 ? 2 * sms : vpr <= 384 ? 3 * sms / 2 : 0);
+}
+
 extern "C" int bl_rmsnorm(const void* x, const void* residual, const void* gamma, void* out,
                           void* residual_out, int rows, int hidden, float eps, const void* partials,
                           int nsplit, size_t slab, void* stream, char* err, size_t errlen) {
@@ -1254,9 +1267,7 @@ extern "C" int bl_rmsnorm(const void* x, const void* residual, const void* gamma
     return -1;
   }
   const int vpr = hidden / 8;
-  // more rows than SMs: rows in flight count, not the latency of one (333 x 3584: 6.8 us with the kernel
-  // below, 4.5 us)
-  if (!partials && rows > 148 && vpr <= 8 * kRowThreads) {
+  if (!partials && rms_by_rows(rows, vpr, residual != nullptr)) {
     launch_k(vpr <= 4 * kRowThreads ? k_rmsnorm_rows<4> : k_rmsnorm_rows<8>, dim3(rows), dim3(kRowThreads), 0,
              static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<const uint4*>(residual),
              static_cast<const uint4*>(gamma), static_cast<uint4*>(out), static_cast<uint4*>(residual_out), vpr, eps);
@@ -1282,8 +1293,13 @@ extern "C" int bl_rope_kv_write(void* qkv, const void* partials, int nsplit, siz
     set_err(err, errlen, "barlink: rope_kv_write needs head_dim in 16..256, multiple of 16");
     return -1;
   }
-  // many rows of bf16: heads of a power of two on 8-byte boundaries
-  if (!partials && rows > 148 && (hd & (hd - 1)) == 0 &&
+  // Many rows of bf16, heads of a power of two on 8-byte boundaries: the kernel that goes over the heads of a row,
+  // once there is enough to read and heads for half of its threads.  us, the kernel below and that one: 200 rows of 12
+  // heads of 64 2.3 and 2.5, 500 rows 3.7 and 3.5; 250 x 6 x 128 3.2 and 2.7; 4096 x 4 x 64 6.0 and 9.0; 1000 x 36 x 128
+  // 18 and 6.2.
+  const int heads = nq + 2 * nkv;
+  if (!partials && rows > sm_count() && size_t(rows) * heads * hd > 160000 && heads * hd >= 4 * kRowThreads &&
+      (hd & (hd - 1)) == 0 &&
       ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 7u) == 0) {
     launch_k(k_rope_kv_rows, dim3(rows), dim3(kRowThreads), 0, static_cast<cudaStream_t>(stream),
              static_cast<__nv_bfloat16*>(qkv), positions, slots, static_cast<__nv_bfloat16*>(k_cache),
@@ -1553,16 +1569,69 @@ extern "C" int bl_rope_attn_decode(const void* qkv, int q_stride, const void* sl
 // ---------------------------------------------------------------------------
 // Per-head RMSNorm of q and k (weights gq, gk over head_dim = 128) followed by
 // RoPE with 1 or 2 position axes, on a fused qkv row [(3*heads) * 128].
-// One block per token, 16 threads per head; a thread owns four rotation pairs (two 8-byte accesses),
-// the same ones in every head, so that sines, cosines and norm weights are read once per token.  (A warp
-// per head with 2-byte accesses and its own sincosf took 41 us for 4608 rows of 24 heads; this takes 25.5 us.)
+// One warp per (token, head); lane l owns dims l, l+32, l+64, l+96, which are exactly the rotation partners for
+// both axis layouts.
+__global__ void __launch_bounds__(256) k_qknorm_rope(__nv_bfloat16* __restrict__ qkv,
+                                                     const __nv_bfloat16* __restrict__ gq,
+                                                     const __nv_bfloat16* __restrict__ gk,
+                                                     const int* __restrict__ positions, int heads,
+                                                     int row_stride, float eps, float log2_theta,
+                                                     int axes) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.x, lane = threadIdx.x & 31;
+  for (int h = (threadIdx.x >> 5) + blockIdx.y * 8; h < 2 * heads; h += 8 * gridDim.y) {
+    __nv_bfloat16* p = qkv + size_t(row) * row_stride + size_t(h) * 128;  // q heads then k heads
+    const __nv_bfloat16* gm = h < heads ? gq : gk;
+    float x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = __bfloat162float(p[lane + 32 * j]);
+    if (gm) {
+      float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
+      ss = warp_sum(ss);
+      const float rstd = rsqrtf(ss / 128.f + eps);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        x[j] = __bfloat162float(__float2bfloat16(x[j] * rstd)) * __bfloat162float(gm[lane + 32 * j]);
+    }
+    if (axes == 2) {
+      // dims [0,64): axis 0, pairs (l, l+32); dims [64,128): axis 1, pairs (l+64, l+96)
+      const float inv = exp2f(-log2_theta * (2.f * float(lane) / 64.f));
+#pragma unroll
+      for (int ax = 0; ax < 2; ++ax) {
+        float sn, cs;
+        sincosf(float(positions[row * 2 + ax]) * inv, &sn, &cs);
+        const float a = x[2 * ax], b = x[2 * ax + 1];
+        x[2 * ax] = a * cs - b * sn;
+        x[2 * ax + 1] = b * cs + a * sn;
+      }
+    } else {
+      // pairs (l, l+64) and (l+32, l+96)
+      const float pos = float(positions[row]);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float inv = exp2f(-log2_theta * (2.f * float(lane + 32 * j) / 128.f));
+        float sn, cs;
+        sincosf(pos * inv, &sn, &cs);
+        const float a = x[j], b = x[j + 2];
+        x[j] = a * cs - b * sn;
+        x[j + 2] = b * cs + a * sn;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) p[lane + 32 * j] = __float2bfloat16(x[j]);
+  }
+}
+
+// The same for many rows of many heads: one block per token, 16 threads per head; a thread owns four rotation
+// pairs (two 8-byte accesses), the same ones in every head, so that sines, cosines and norm weights are read once
+// per token (4608 rows of 24 heads: 42 us with the kernel above, 24 us).
 constexpr int kQkBatch = 6;
-template <bool VEC>
-__global__ void __launch_bounds__(kRowThreads) k_qknorm_rope(__nv_bfloat16* __restrict__ qkv,
-                                                             const __nv_bfloat16* __restrict__ gq,
-                                                             const __nv_bfloat16* __restrict__ gk,
-                                                             const int* __restrict__ positions, int heads,
-                                                             int row_stride, float eps, float log2_theta, int axes) {
+__global__ void __launch_bounds__(kRowThreads) k_qknorm_rope_rows(__nv_bfloat16* __restrict__ qkv,
+                                                                  const __nv_bfloat16* __restrict__ gq,
+                                                                  const __nv_bfloat16* __restrict__ gk,
+                                                                  const int* __restrict__ positions, int heads,
+                                                                  int row_stride, float eps, float log2_theta, int axes) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x, t = threadIdx.x & 15, h0 = threadIdx.x >> 4;
@@ -1586,8 +1655,8 @@ __global__ void __launch_bounds__(kRowThreads) k_qknorm_rope(__nv_bfloat16* __re
     for (int c = 0; c < kQkBatch; ++c) {
       const int h = hb + c * kHpp + h0;
       if (h < 2 * heads) {
-        load4<VEC>(prow + size_t(h) * 128 + d1, a[c]);
-        load4<VEC>(prow + size_t(h) * 128 + d2, b[c]);
+        load4(prow + size_t(h) * 128 + d1, a[c]);
+        load4(prow + size_t(h) * 128 + d2, b[c]);
       } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) a[c][j] = b[c][j] = 0.f;
@@ -1607,8 +1676,8 @@ __global__ void __launch_bounds__(kRowThreads) k_qknorm_rope(__nv_bfloat16* __re
       if (gm) {
         const float rstd = rsqrtf(ss / 128.f + eps);
         float g1[4], g2[4];
-        load4<VEC>(gm + d1, g1);
-        load4<VEC>(gm + d2, g2);
+        load4(gm + d1, g1);
+        load4(gm + d2, g2);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           x1[j] = __bfloat162float(__float2bfloat16(a[c][j] * rstd)) * g1[j];
@@ -1627,8 +1696,8 @@ __global__ void __launch_bounds__(kRowThreads) k_qknorm_rope(__nv_bfloat16* __re
         o1[j] = x1[j] * cs[j] - x2[j] * sn[j];
         o2[j] = x2[j] * cs[j] + x1[j] * sn[j];
       }
-      store4<VEC>(prow + size_t(h) * 128 + d1, o1);
-      store4<VEC>(prow + size_t(h) * 128 + d2, o2);
+      store4(prow + size_t(h) * 128 + d1, o1);
+      store4(prow + size_t(h) * 128 + d2, o2);
     }
   }
 }
@@ -1857,9 +1926,15 @@ extern "C" int bl_qknorm_rope(void* qkv, const void* gq, const void* gk, const i
     set_err(err, errlen, "barlink: qknorm_rope is built for head_dim 128 and 1 or 2 position axes");
     return -1;
   }
-  const bool vec = ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(gq) |
-                     reinterpret_cast<uintptr_t>(gk)) & 7u) == 0 && (row_stride & 3) == 0;
-  launch_k(vec ? k_qknorm_rope<true> : k_qknorm_rope<false>, dim3(rows), dim3(kRowThreads), 0,
+  // From some 500 rows of 12 heads up, on 8-byte boundaries, the kernel that goes over the heads of a row.  Few
+  // heads leave most of its block without work, few rows most of the SMs; us, first the kernel with a warp per
+  // head: 333 x 24 heads 4.3 and 5.4, 512 x 24 5.9 and 5.7, 2000 x 24 19 and 12; 700 x 16 5.5 and 4.9; 1000 x 12 5.8
+  // and 6.2, 1400 x 12 7.6 and 7.0; 8000 x 8 25 and 28.
+  const bool many = rows >= 500 && heads >= 12 && size_t(rows) * (heads - 4) >= 8200 &&
+                    ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(gq) |
+                      reinterpret_cast<uintptr_t>(gk)) & 7u) == 0 && (row_stride & 3) == 0;
+  const int gy = (2 * heads + 7) / 8 < 8 ? (2 * heads + 7) / 8 : 8;
+  launch_k(many ? k_qknorm_rope_rows : k_qknorm_rope, many ? dim3(rows) : dim3(rows, gy), dim3(many ? kRowThreads : 256), 0,
            static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(gq),
            static_cast<const __nv_bfloat16*>(gk), positions, heads, row_stride, eps, log2f(theta), axes);
   OPS_LAUNCH_CHECK("qknorm_rope");
@@ -1875,7 +1950,7 @@ extern "C" int bl_layernorm_modulate(const void* x, const void* shift, const voi
     return -1;
   }
   const int vpr = hidden / 8;
-  if (rows > 148 && vpr <= 8 * kRowThreads) {  // as in bl_rmsnorm
+  if (layernorm_by_rows(rows, vpr)) {
     launch_k(vpr <= 4 * kRowThreads ? k_layernorm_rows<4> : k_layernorm_rows<8>, dim3(rows), dim3(kRowThreads), 0,
              static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<const __nv_bfloat16*>(shift),
              static_cast<const __nv_bfloat16*>(scale), static_cast<uint4*>(out), vpr, rows_per_batch, mod_stride, eps);

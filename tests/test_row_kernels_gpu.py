@@ -24,9 +24,10 @@ def _close(a, b):
     assert float((a - b).abs().max() / b.abs().max()) < 2.0 ** -7
 
 
-# 148 | 149: the rule; 1024 / 1032 vectors and 8192 / 8200 elements: the edges of the register forms
-@pytest.mark.parametrize("rows", [148, 149, 300])
-@pytest.mark.parametrize("hidden", [8, 264, 4096, 4104, 8192, 8200])
+# 148 | 149: the rule's first line; 1024 / 1032 vectors and 8192 / 8200 elements: the edges of the register forms;
+# 300 and 700 rows: both sides of its lines at medium widths
+@pytest.mark.parametrize("rows", [148, 149, 300, 700])
+@pytest.mark.parametrize("hidden", [8, 264, 1024, 1032, 2048, 2056, 4096, 4104, 8192, 8200])
 def test_norms(ext, rows, hidden):
     x, r, gm = _randn(1, rows, hidden), _randn(2, rows, hidden), _randn(3, hidden)
     want, _ = ref.rmsnorm(x, gm, 1e-6, None)
@@ -45,7 +46,8 @@ def test_norms(ext, rows, hidden):
 
 
 @pytest.mark.parametrize("rows", [148, 149, 200])
-@pytest.mark.parametrize("nq,nkv,hd", [(28, 4, 128), (1, 1, 128), (8, 2, 64), (3, 1, 256), (5, 1, 16), (4, 2, 96)])
+@pytest.mark.parametrize("nq,nkv,hd", [(28, 4, 128), (1, 1, 128), (8, 2, 64), (3, 1, 256), (5, 1, 16), (4, 2, 96),
+                                       (16, 2, 64), (40, 10, 16)])
 @pytest.mark.parametrize("cached", [False, True])
 def test_rope_kv_write(ext, rows, nq, nkv, hd, cached):
     bs, blocks = 16, 16
@@ -71,7 +73,9 @@ def test_rope_kv_write(ext, rows, nq, nkv, hd, cached):
 
 
 @pytest.mark.parametrize("rows,heads,pitch,offset", [(1, 24, 24 * 384, 0), (7, 25, 25 * 256, 0), (200, 3, 3 * 384 + 2, 0),
-                                                     (5, 1, 384, 1)])
+                                                     (5, 1, 384, 1), (499, 24, 24 * 384, 0), (500, 21, 21 * 384, 0),
+                                                     (500, 25, 25 * 256 + 4, 4), (500, 25, 25 * 256 + 2, 0),
+                                                     (500, 25, 25 * 256, 1), (1100, 12, 12 * 384, 0)])
 @pytest.mark.parametrize("axes", [1, 2])
 @pytest.mark.parametrize("norm", [False, True])
 def test_qknorm_rope(ext, rows, heads, pitch, offset, axes, norm):

@@ -212,7 +212,8 @@ bool qlin_takes(const at::Tensor& x, int k, bool act_int8, bool grouped = false)
 }
 // y = activations (xq, xs: int8 rows, or three digit planes) times q.  want_slabs: fp32 [splits, m, n]
 // when the shape wants a k-split (bias is then the consumer's), else bf16 [m, n].  like: options of x.
-at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int digits, const QWeight& q,
+// x: the bf16 activations behind three digit planes.
+at::Tensor qlin_product(const at::Tensor* x, const at::Tensor& xq, const at::Tensor& xs, int m, int digits, const QWeight& q,
                         const c10::optional<at::Tensor>& bias, bool silu_mul, int splits, bool want_slabs,
                         const at::TensorOptions& like, void* err_flag, void* st) {
   if (bias) {
@@ -229,6 +230,10 @@ at::Tensor qlin_product(const at::Tensor& xq, const at::Tensor& xs, int m, int d
   a.w = q.w; a.src = q.src; a.n = q.n; a.k = q.k;
   a.xq = xq.data_ptr(); a.xs = xs.data_ptr();
   a.m = m; a.digits = digits;
+  if (x) {
+    a.x = x->data_ptr();
+    a.ldx = int(x->stride(0));
+  }
   a.scale_kind = q.scale_kind; a.scale = q.scale; a.row_scale = q.row_scale; a.group_k = q.group_k; a.zeros = q.zeros;
   a.splits = splits;
   a.err_flag = err_flag;
@@ -273,7 +278,7 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
     xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
     BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
   }
-  return qlin_product(xq, xs, m, digits, q, bias, silu_mul, splits, want_slabs, x.options(), err_flag, st);
+  return qlin_product(digits == 3 ? &x : nullptr, xq, xs, m, digits, q, bias, silu_mul, splits, want_slabs, x.options(), err_flag, st);
 }
 
 // Decode form of w8a16_linear without a reduction: fp32 slabs [splits, m, n] (scaled, no bias) for the
@@ -488,7 +493,7 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
   q.group_k = 128;
   void* flag = w8_scratch(dev).err_flag.data_ptr();
   py::gil_scoped_release nogil;
-  return qlin_product(aligned ? xq : xq.clone(), xs, m, 1, q, c10::nullopt, false, 0, false, like, flag, st);
+  return qlin_product(nullptr, aligned ? xq : xq.clone(), xs, m, 1, q, c10::nullopt, false, 0, false, like, flag, st);
 }
 
 // GPTQ-v1 int4 linear.  Groups of 128 and 5..128 rows: int8 digits of the activations on the tensor cores

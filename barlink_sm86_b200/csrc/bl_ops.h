@@ -170,7 +170,7 @@ int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, const void* 
 /* ---- decode linears on quantised weights (qlin_kernels.cu) ------------------------------------
  * y[m, n] = xs[m] * sum over groups of scale * (integer products), 1..BL_QLIN_MAX_TOKENS tokens.
  * Activations: digits = 1: xq int8 [m x k] and xs as bl_w8a16_quant_act leaves them; digits = 3: the
- * planes and xs of bl_quant_digits (bf16 activations without loss, see there).
+ * planes and xs of bl_quant_digits, and x itself (bf16 activations, see there for what they hold).
  * src: 0 int8 [n][k]; 1 int8 [k/16][n][16] (one digit, group scales); 2 GPTQ-v1 int32 [k/8][n] with
  * `zeros` int32 [k/group_k][n/8] (three digits written with permute = 1).
  * out bf16 (splits = 1; bias, silu_mul as in blGemmArgs) or slabs fp32 [splits][m][n] (scales applied,
@@ -189,6 +189,8 @@ typedef struct blQlinArgs {
   const void* xq;
   const void* xs;
   int m, digits;
+  const void* x; /* digits = 3: the activations that bl_quant_digits was given, with their pitch */
+  int ldx;
   int scale_kind;
   const void* scale;
   const void* row_scale; /* bf16 [n] or null */
@@ -206,9 +208,12 @@ int bl_qlin(const blQlinArgs* a, void* stream, char* err, size_t errlen);
 int bl_qlin_splits(int n, int k, int m, int digits, int grouped);  /* k-splits that suit the shape */
 int bl_qlin_tile_tokens(int m); /* of three digit planes */
 /* x [m x k] bf16 (pitch ldx) -> xq int8 [ceil(m/tile)][3][tile][k] (tile = bl_qlin_tile_tokens(m)) and
- * xs fp32 [m] with x = xs * (d0 + d1 / 2^8 + d2 / 2^16): exact for elements down to 2^-15 of the row's
- * largest, to 2^-24 of the largest below that.  permute: digits in the order 0 2 4 6 1 3 5 7 of every
- * eight (packed int4 weights).  K a multiple of 8, at most 32768. */
+ * xs fp32 [m] with x = |xs| * (d0 + d1 / 2^8 + d2 / 2^16): exact for elements down to 2^-15 of the row's
+ * largest, below that to 2^-24 of 2^ex, the power of two above the largest.  Rows with an infinity, or with more than half of their nonzero
+ * elements below 2^-11 of that scale, get a negative xs: |xs| then follows the median (2^10 above it), and the
+ * elements beyond have digits of zero; bl_qlin adds their products in fp32.  A NaN makes xs a NaN.
+ * permute: digits in the order 0 2 4 6 1 3 5 7 of every eight (packed int4 weights).  K a multiple of 8, at
+ * most 32768. */
 int bl_quant_digits(const void* x, int m, int ldx, int k, int permute, void* xq, void* xs, void* stream, char* err,
                     size_t errlen);
 size_t bl_quant_digits_bytes(int m, int k);

@@ -8,9 +8,12 @@
 // time.  Widening int8 weights to bf16 on the CUDA cores did: 11 instructions per four weights held
 // the kernel to 2.0-2.7 TB/s.  Here the activations are taken apart instead.  A token's bf16 row is
 // scaled by a power of two so that its largest element is just below 1 and written as three base-256
-// digits (k_quant_digits): 23 bits below the row's largest element, so every element down to 2^-15
-// of it is represented exactly and the rest to within 2^-24 of it -- below what fp32 accumulation
-// rounds away.  The weights go from HBM to the tensor core as they are, the three digit planes of
+// digits (k_quant_digits): a fixed-point number of 23 bits below that element, so every element down to
+// 2^-15 of the largest is represented exactly and the rest to within 2^-24 of the largest.  In rows where
+// that would be coarse -- more than half of the nonzero elements below 2^-11 of the scale, or an infinity -- the
+// scale follows the median instead (2^10 above it), and the few elements beyond it are left out of the digits
+// and added in fp32 by the epilogue (outlier_sum).  What a digit drops is thus at most 2^-24 of the largest
+// and 2^-13 of the median element, whichever weights meet the outliers.  The weights go from HBM to the tensor core as they are, the three digit planes of
 // all tokens are the N dimension of one MMA, sums are exact int32, and the epilogue puts
 // (d0 + d1 / 2^8 + d2 / 2^16) * xs[t] together.  With activations that the caller quantised to int8
 // (one digit) the same kernel runs with a third of the N.
@@ -58,6 +61,9 @@ struct QlinShape {
   int tiles_a, tiles_b, kblocks, splits;
   const uint32_t* zeros;         // kNibbles: int32 [groups][n/8]
   const float* xs;               // per token
+  const __nv_bfloat16* x;        // three digits: the activations themselves, for rows with outliers
+  int ldx;
+  const void* w;
   int scale_kind;                // see blQlinArgs
   const void* scale;
   const __nv_bfloat16* row_scale;
@@ -101,9 +107,61 @@ __device__ __forceinline__ uint64_t umma_desc_k_chunks(uint32_t smem_addr) {
   return d;
 }
 
+// bits (without the sign) of the smallest bf16 that the digits of a row with |x| < 2^ex cannot hold:
+// 255/256 * 2^ex would round up to 128 in the first digit
+__device__ __forceinline__ uint32_t digit_limit(int ex) { return (uint32_t(ex + 126) << 7) | 0x7fu; }
+
+// The products of a token's outliers (see k_quant_digits) with weight row n, k0 <= k < k1, without what is common
+// to the row.  A whole warp calls it for one token: it looks through 256 activations at a time.  Infinities come
+// out as in any sum of products.  A call of its own, so that the loops around it keep their registers: such rows
+// are rare (inlined, it cost the products of every other row with group scales 12 %).
+template <int SRC, bool GROUPED>
+__device__ __noinline__ float outlier_sum(const QlinShape& g, int m, int k0, int k1, int n) {
+  const int lane = threadIdx.x & 31;
+  const float xs = __ldg(g.xs + m);
+  if (!(xs < 0.f)) return 0.f;
+  const uint32_t limit = digit_limit(int((__float_as_uint(xs) >> 23) & 0xffu) - 120);
+  const __nv_bfloat16* xr = g.x + size_t(m) * g.ldx;
+  float sum = 0.f;
+  for (int kk = k0; kk < k1; kk += 256) {
+    uint32_t hit = 0;
+    if (kk + lane * 8 < k1) {
+      const uint4 a = *reinterpret_cast<const uint4*>(xr + kk + lane * 8);
+      const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (((w[j >> 1] >> (16 * (j & 1))) & 0x7fffu) >= limit) hit |= 1u << j;
+    }
+    for (uint32_t lanes = __ballot_sync(0xffffffffu, hit != 0); lanes; lanes &= lanes - 1) {
+      const int l = __ffs(lanes) - 1;
+      for (uint32_t h = __shfl_sync(0xffffffffu, hit, l); h; h &= h - 1) {
+        const int kx = kk + l * 8 + __ffs(h) - 1, gi = kx / (kQK * g.gk);
+        float w;
+        if constexpr (SRC == kNibbles) {
+          const uint32_t word = __ldg(static_cast<const uint32_t*>(g.w) + size_t(kx >> 3) * g.n + n);
+          const uint32_t z = __ldg(g.zeros + size_t(gi) * (g.n >> 3) + (n >> 3));
+          w = float(int((word >> (4 * (kx & 7))) & 15u) - int((z >> (4 * (n & 7))) & 15u));
+        } else {
+          w = float(__ldg(static_cast<const signed char*>(g.w) + size_t(n) * g.k + kx));
+        }
+        if constexpr (GROUPED) {
+          const size_t ng = size_t(n) * g.groups + gi, gn = size_t(gi) * g.n + n;
+          w *= g.scale_kind == BL_QSCALE_F32_GN    ? __ldg(static_cast<const float*>(g.scale) + gn)
+               : g.scale_kind == BL_QSCALE_F16_GN  ? __half2float(static_cast<const __half*>(g.scale)[gn])
+               : g.scale_kind == BL_QSCALE_BF16_NG ? __bfloat162float(static_cast<const __nv_bfloat16*>(g.scale)[ng])
+                                                   : __half2float(static_cast<const __half*>(g.scale)[ng]);
+        }
+        sum = fmaf(__bfloat162float(xr[kx]), w, sum);
+      }
+    }
+  }
+  return sum;
+}
+
 template <int SRC, int ND, int TB, bool GROUPED>
 __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
-    k_qlin(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const QlinShape g) {
+    k_qlin(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+           const __grid_constant__ QlinShape g) {
   using S = QlinCfg<SRC, ND, TB, GROUPED>;
   extern __shared__ uint8_t smem_raw[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem_raw);
@@ -460,8 +518,24 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
         } else {
           read16(done_acc, c0, v);
         }
+        float xm[16];
+        bool rare = false;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] *= (c0 + j < m_end ? __ldg(g.xs + m0 + c0 + j) : 0.f) * rs;
+        for (int j = 0; j < 16; ++j) {
+          xm[j] = c0 + j < m_end ? __ldg(g.xs + m0 + c0 + j) : 0.f;
+          if (ND == 3) rare |= xm[j] < 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= (ND == 3 ? fabsf(xm[j]) : xm[j]) * rs;
+        if (ND == 3 && rare) {
+#pragma unroll 1
+          for (int t = 0; c0 + t < m_end && t < 16; ++t) {
+            const float o = rs * outlier_sum<SRC, GROUPED>(g, m0 + c0 + t, sp * kb_per * kQK, min(g.k, (sp + 1) * kb_per * kQK), nn);
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (j == t) v[j] += o;
+          }
+        }
         const int m1 = m0 + c0, mn = nok ? min(16, m_end - c0) : 0;  // first token, tokens to store
         if (g.slabs) {
           float* o = g.slabs + (size_t(sp) * g.m + m1) * g.n + n;
@@ -503,59 +577,92 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
 // ---------------------------------------------------------------------------
 // activations -> digits
 // ---------------------------------------------------------------------------
-// x [m][k] bf16 -> xq [ceil(m/tb)][3][tb][k] int8 and xs[m]: x = xs * (d0 + d1/2^8 + d2/2^16).  xs is a
-// power of two chosen from the row's largest element so that d0 fits 8 bits.  One block per token; the
-// row stays in registers between the two passes.
+// x [m][k] bf16 -> xq [ceil(m/tb)][3][tb][k] int8 and xs[m]: x = |xs| * (d0 + d1/2^8 + d2/2^16).  |xs| is a
+// power of two chosen from the row's largest element so that d0 fits 8 bits; a negative xs says that the row
+// has outliers, elements beyond the digits' range, whose digits are zero.  One block per token.
 constexpr int kDigThreads = 512;
 constexpr int kDigVec = 8;   // 16-byte vectors per thread: rows of up to 32768 elements
 __device__ __forceinline__ uint32_t bf16x2_absmax_bits(uint32_t m, uint32_t v) {
   m = max(m, v & 0x7fffu);
   return max(m, (v >> 16) & 0x7fffu);
 }
-template <bool PERMUTE>
-__global__ void __launch_bounds__(kDigThreads) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k,
+template <bool PERMUTE, int VPT>
+__global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k,
                                                               int tb, int8_t* __restrict__ xq,
                                                               float* __restrict__ xs) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ uint32_t s_max[kDigThreads / 32];
-  const int row = blockIdx.x, vecs = k >> 3;
+  // (little shared memory: a block of this kernel fits beside one of k_qlin, which has nearly all of it)
+  __shared__ uint32_t s_red[kDigThreads / 32];
+  const int row = blockIdx.x, vecs = k >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx);
-  uint4 v[kDigVec];
+  uint4 v[VPT];
   uint32_t mx = 0;  // largest |x| as bf16 bits: ordered like the values, NaN above infinity
 #pragma unroll
-  for (int i = 0; i < kDigVec; ++i) {
+  for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * kDigThreads;
-    if (c < vecs) {
-      v[i] = xr[c];
-      mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].x), v[i].y);
-      mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].z), v[i].w);
-    }
+    v[i] = c < vecs ? xr[c] : make_uint4(0, 0, 0, 0);
+    mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].x), v[i].y);
+    mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].z), v[i].w);
   }
   mx = __reduce_max_sync(0xffffffffu, mx);
-  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  if (lane == 0) s_red[warp] = mx;
   __syncthreads();
-  mx = 0;
+  mx = __reduce_max_sync(0xffffffffu, s_red[lane & (kDigThreads / 32 - 1)]);
+  // nonzero elements below 2^(e - 127) and, in the upper half of the word, nonzero ones in all (each fits 16 bits)
+  auto count = [&](int e) -> uint32_t {
+    const uint32_t top = e > 0 ? uint32_t(e) << 7 : 1u;
+    uint32_t n = 0;
 #pragma unroll
-  for (int i = 0; i < kDigThreads / 32; ++i) mx = max(mx, s_max[i]);
+    for (int i = 0; i < VPT; ++i) {
+      const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t a = (w[j >> 1] >> (16 * (j & 1))) & 0x7fffu;
+        n += (a != 0 ? 0x10000u : 0u) + (a - 1u < top - 1u ? 1u : 0u);
+      }
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    __syncthreads();
+    if (lane == 0) s_red[warp] = n;
+    __syncthreads();
+    return __reduce_add_sync(0xffffffffu, lane < kDigThreads / 32 ? s_red[lane] : 0u);
+  };
   // |x| < 2^ex; a largest element of 255/256 * 2^ex would round up to 128 in the first digit
   int ex = int(mx >> 7) - 126 + ((mx & 0x7fu) == 0x7fu ? 1 : 0);
-  if (ex < -110) ex = -110;
-  const bool bad = mx >= 0x7f80u;  // infinity or NaN in the row: the whole row of results is NaN
+  if (ex < -110) ex = -110;  // the digits of such rows reach the smallest bf16, 2^-133
+  const uint32_t small = count(ex > -110 ? ex + 116 : 0);  // below 2^(ex - 11)
+  const bool bad = mx > 0x7f80u;  // NaN in the row: the whole row of results is NaN
+  const bool split = !bad && (2 * (small & 0xffffu) > (small >> 16) || mx == 0x7f80u);
+  if (split) {
+    // the median's exponent: the smallest e with half of the nonzero elements below 2^(e + 1 - 127)
+    int lo = 0, hi = 255;
+#pragma unroll 1
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      // (keeps the compiler from holding all magnitudes in registers over this loop: the block would not fit)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) asm volatile("" : "+r"(v[i].x), "+r"(v[i].y), "+r"(v[i].z), "+r"(v[i].w));
+      if (2 * (count(mid + 1) & 0xffffu) >= (small >> 16)) hi = mid;
+      else lo = mid + 1;
+    }
+    ex = min(128, max(-110, lo - 126 + 10));
+  }
+  const uint32_t limit = digit_limit(ex);
   const float scale = bad ? 0.f : __uint_as_float(uint32_t(127 + 7 - ex) << 23);
   if (threadIdx.x == 0)
-    xs[row] = bad ? __uint_as_float(0x7fffffffu) : __uint_as_float(uint32_t(127 - 7 + ex) << 23);
+    xs[row] = bad ? __uint_as_float(0x7fffffffu) : __uint_as_float(uint32_t(127 - 7 + ex) << 23 | (split ? 1u << 31 : 0u));
   int8_t* base = xq + (size_t(row / tb) * 3 * tb + row % tb) * size_t(k);
 #pragma unroll
-  for (int i = 0; i < kDigVec; ++i) {
+  for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * kDigThreads;
     if (c >= vecs) continue;
     const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
     uint32_t o[3][2] = {{0, 0}, {0, 0}, {0, 0}};
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float f = __uint_as_float((j & 1) ? (w[j >> 1] & 0xffff0000u) : (w[j >> 1] << 16));
-      const float y0 = bad ? 0.f : f * scale;
+      const uint32_t f = (j & 1) ? (w[j >> 1] & 0xffff0000u) : (w[j >> 1] << 16);
+      const float y0 = bad || ((f >> 16) & 0x7fffu) >= limit ? 0.f : __uint_as_float(f) * scale;
       // every step leaves a remainder in [-128.5, 127.5) / 256, so that the next digit fits too
       const float d0 = floorf(y0 + 128.5f / 256.f);
       const float y1 = (y0 - d0) * 256.f;
@@ -676,6 +783,9 @@ static int launch_qlin(const blQlinArgs& a, cudaStream_t st, char* err, size_t e
   g.splits = a.splits;
   g.zeros = static_cast<const uint32_t*>(a.zeros);
   g.xs = static_cast<const float*>(a.xs);
+  g.x = static_cast<const __nv_bfloat16*>(a.x);
+  g.ldx = a.ldx;
+  g.w = a.w;
   g.scale_kind = a.scale_kind;
   g.scale = a.scale;
   g.row_scale = static_cast<const __nv_bfloat16*>(a.row_scale);
@@ -763,7 +873,14 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
                     static_cast<const __nv_bfloat16*>(x), ldx, k, bl_qlin_tile_tokens(m), static_cast<int8_t*>(xq),
                     static_cast<float*>(xs));
   };
-  cudaError_t e = permute ? go(k_quant_digits<true>) : go(k_quant_digits<false>);
+  // vectors of a thread: a row of up to 4096 elements in one, with as little code as that takes (the code of a
+  // kernel this short comes from L2 or beyond on every launch)
+  const int vpt = (k / 8 + kDigThreads - 1) / kDigThreads;
+  cudaError_t e;
+  if (vpt <= 1) e = permute ? go(k_quant_digits<true, 1>) : go(k_quant_digits<false, 1>);
+  else if (vpt <= 2) e = permute ? go(k_quant_digits<true, 2>) : go(k_quant_digits<false, 2>);
+  else if (vpt <= 5) e = permute ? go(k_quant_digits<true, 5>) : go(k_quant_digits<false, 5>);
+  else e = permute ? go(k_quant_digits<true, kDigVec>) : go(k_quant_digits<false, kDigVec>);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: quant_digits launch failed: %s", cudaGetErrorString(e));
@@ -795,6 +912,10 @@ extern "C" int bl_qlin(const blQlinArgs* a, void* stream, char* err, size_t errl
       a->n < 1 || a->k < 16 || (a->k & 15) || (a->digits != 1 && a->digits != 3)) {
     set_err(err, errlen, "barlink: qlin needs weights, activations with 1 or 3 digits, scales, an output, 1..%d tokens and K a multiple of 16",
             BL_QLIN_MAX_TOKENS);
+    return -1;
+  }
+  if (a->digits == 3 && (!a->x || (a->ldx & 7) || (reinterpret_cast<uintptr_t>(a->x) & 15u))) {
+    set_err(err, errlen, "barlink: qlin with three digits needs the 16-byte aligned rows that they were made of");
     return -1;
   }
   // 32-bit sums: |weight| <= 128, |digit| <= 128

@@ -3,7 +3,8 @@
 
 Oracle: the exact integer products in float64.  Tolerances: the bf16 result is rounded once (rel-L2 at
 most 2^-9 / sqrt(3) per element on average, 2^-8 allowed); fp32 slabs carry the int32 -> fp32 conversions
-and their sum only (2^-24 each; 2^-20 allowed).  Digits: exact down to 2^-15 of a row's largest element."""
+and their sum only (2^-24 each; 2^-20 allowed).  Digits: exact down to 2^-15 of a row's largest element; what
+they drop of an element is at most 2^-24 of the largest and 2^-13 of the median of a row."""
 import pytest
 import torch
 
@@ -32,6 +33,11 @@ def _x(m, k, seed, spread=False):
 def _w8(n, k, seed):
     wq = torch.randint(-127, 128, (n, k), generator=_g(seed), device="cuda", dtype=torch.int32).to(torch.int8)
     return wq, (torch.rand(n, generator=_g(seed + 1), device="cuda") * 0.01 + 1e-3).bfloat16()
+
+
+def _pack4(t):  # eight values along the last dimension -> one int32
+    v = sum(t.view(*t.shape[:-1], -1, 8)[..., j].long() << (4 * j) for j in range(8))
+    return ((v + 2 ** 31) % 2 ** 32 - 2 ** 31).to(torch.int32)
 
 
 # tokens: edges of the 16 / 32 / 64-token tiles; n: a ragged last row tile; k: a ragged last k-block
@@ -143,23 +149,97 @@ def test_int8_weights_group_scales(ext, m, n, k, group, act_int8):
     assert ext.w8_error_flag(0) == 0
 
 
-def test_activation_rows_with_extreme_values(ext):
-    """Zeros, tiny and huge rows, one outlier; a NaN or an infinity spoils its own row only."""
-    wq, sc = _w8(136, 256, 7)
-    x = _x(8, 256, 8)
-    x[0] = 0
-    x[1] *= 1e-30
-    x[2] *= 1e30
-    x[3, 7] = 3e4
-    x[4] = 255.0 / 256  # largest mantissa
-    x[5, 3] = float("nan")
-    x[6, 3] = float("inf")
-    y = ext.w8a16_linear(x, wq, sc)
-    want = (x.double() @ wq.double().t()) * sc.double()
-    for r in (1, 2, 3, 4, 7):
-        assert rel_l2(y[r].double(), want[r]) < TOL, r
-    assert float(y[0].abs().max()) == 0.0
-    assert not torch.isfinite(y[5]).any() and not torch.isfinite(y[6]).any()
+def _forms(ext, n, k):
+    """(product of rows x, the same as fp32 where the form leaves slabs, dequantised weight) of the weight forms
+    whose activations become digits."""
+    from barlink_sm86_b200 import ops
+    wq, sc = _w8(n, k, 7)
+    wq[::3, ::5] = 0
+    slabs = lambda y: y.double().sum(0) if y.dim() == 3 else y.double()
+    yield (lambda x: ext.w8a16_linear(x, wq, sc)), (lambda x: slabs(ext.w8a16_linear_split(x, wq, sc))), wq, wq.double() * sc.double()[:, None]
+    gs = (torch.rand(n, k // 128, generator=_g(4), device="cuda") * 0.01 + 1e-3).bfloat16()
+    p = ops.prepare_w8_scales(gs, k)
+    yield ((lambda x: ext.w8a16_linear(x, wq, p.row, group_rel=p.rel)), None, wq,
+           ops.ref.w8_dequant(wq, p.rel.float() * p.row.float()[:, None]).double())
+    nib = torch.randint(0, 16, (n, k), generator=_g(11), device="cuda")
+    nib[::3, ::5] = 7
+    zero = torch.randint(0, 16, (k // 128, n), generator=_g(12), device="cuda")
+    zero[:, ::3] = 7
+    s4 = (torch.rand(k // 128, n, generator=_g(13), device="cuda") * 0.01 + 1e-3).half()
+    qw, qz = _pack4(nib).t().contiguous(), _pack4(zero)
+    w4 = nib - zero.t().repeat_interleave(128, 1)
+    yield ((lambda x: ext.w4a16_linear(x, qw, s4, qz)), (lambda x: slabs(ext.w4a16_linear(x, qw, s4, qz, want_slabs=True))),
+           w4, w4.double() * s4.double().t().repeat_interleave(128, 1))
+
+
+@pytest.mark.parametrize("m", [5, 16, 33])
+@pytest.mark.parametrize("n,k", [(136, 384), (200, 4224), (136, 20608)])
+@pytest.mark.parametrize("ratio", [12, 15, 18, 24, 60])
+def test_outliers_that_meet_zero_weights(ext, m, n, k, ratio):
+    """A few elements 2^ratio above the rest, in columns where a third of the weight rows are zero: those rows'
+    results have only the small elements, and every one of them may be off by 2^-13 of the median at most
+    (weights of a third of the rows are zero there, the others see what fp32 leaves of the large products)."""
+    for f, f32, wi, w in _forms(ext, n, k):
+        x = _x(m, k, 21)
+        med = x.float().abs().median(1).values.double()
+        cols = torch.arange(0, k, 5, device="cuda")[:: max(1, k // 5 // 7)]
+        x[1::2, cols] = (x[1::2, cols].float() * 2.0 ** ratio).bfloat16()
+        want = x.double() @ w.t()
+        # zero weights at the outliers: rows 0, 3, 6, ... ; one bf16 rounding of the result, then the digits
+        drop = 2.0 ** -13 * med[:, None] * w.abs().sum(1)[None, :]
+        assert bool((wi[::3][:, cols] == 0).all())
+        y = f(x).double()
+        assert bool(((y - want).abs() <= 2.0 ** -8 * want.abs() + drop)[:, ::3].all())
+        assert rel_l2(y, want) < TOL
+        assert rel_l2(y[:, ::3], want[:, ::3]) < TOL
+        if f32 is not None:
+            y = f32(x)
+            assert bool(((y - want).abs() <= 2.0 ** -8 * want.abs() + drop)[:, ::3].all())
+            assert rel_l2(y[:, ::3], want[:, ::3]) < TOL
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
+
+
+@pytest.mark.parametrize("m", [8, 40])
+def test_activation_rows_with_extreme_values(ext, m):
+    """Zeros, tiny and huge rows, one outlier, rows of mostly small elements, a NaN, infinities: as a sum of
+    products in float64 has them."""
+    for f, _, _, w in _forms(ext, 136, 1280):
+        x = _x(m, 1280, 8)
+        x[0] = 0
+        x[1] *= 1e-30
+        x[2] *= 1e30
+        x[3, 7] = 3e4
+        x[4] = 255.0 / 256  # largest mantissa
+        x[5, 3] = float("nan")
+        x[6, 3] = float("inf")
+        x[7, 900], x[7, 30] = float("inf"), -float("inf")
+        if m > 8:
+            x[8, 640:] = float("inf")
+            x[9, 100:] *= 1e-6  # the large ones are the few
+            x[10] = 0
+            x[10, 17] = -torch.finfo(torch.bfloat16).max
+            x[11] = 0
+            x[11, 5] = -float("inf")
+            x[12] = 0
+            x[12, 1279] = 1e-38
+            x[13] *= 1e-38  # down to the smallest bf16
+            x[14, ::2] *= 1e-5  # as many large as small
+        y, want = f(x).double(), x.double() @ w.t()
+        y = torch.where((want.abs() > 3.37e38) & (want.abs() < 3.42e38), want, y)  # bf16 ends here: either will do
+        big = y.isinf() & want.isfinite() & (want.abs() > 3.4e38)
+        assert torch.equal(y.isnan(), want.isnan())
+        assert torch.equal(torch.where(y.isinf(), y.sign(), 0), torch.where(want.isinf() | big, want.sign(), 0))
+        assert bool((y.isinf() | (want.abs() < 3.4e38) | ~want.isfinite() | (y == want)).all())
+        for r in range(m):
+            ok = want[r].isfinite() & ~big[r]
+            if bool(ok.any()) and float(want[r][ok].abs().max()) > 0:
+                # (a smallest bf16 is 2^-133: results down there are rounded to it)
+                d = (y[r][ok] - want[r][ok]).norm()
+                assert float(d) < TOL * float(want[r][ok].norm()) + 2.0 ** -133 * int(ok.sum()) ** 0.5, r
+        assert float(y[0].abs().max()) == 0.0
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
 
 
 # k-chunk-major weights (the reference's pair): ragged last row tile, odd n (no k-split), one k-block
@@ -190,10 +270,7 @@ def test_int4_weights(ext, m, n, k):
     nib = torch.randint(0, 16, (n, k), generator=g, device="cuda")
     zero = torch.randint(0, 16, (k // 128, n), generator=g, device="cuda")
     sc = (torch.rand(k // 128, n, generator=g, device="cuda") * 0.01 + 1e-3).half()
-    def pack(t):  # eight values along the last dimension -> one int32
-        v = sum(t.view(*t.shape[:-1], -1, 8)[..., j].long() << (4 * j) for j in range(8))
-        return ((v + 2 ** 31) % 2 ** 32 - 2 ** 31).to(torch.int32)
-    qw, qz = pack(nib).t().contiguous(), pack(zero)
+    qw, qz = _pack4(nib).t().contiguous(), _pack4(zero)
     x = _x(m, k, 5, spread=True)
     w = (nib - zero.t().repeat_interleave(128, 1)).double() * sc.double().t().repeat_interleave(128, 1)
     want = x.double() @ w.t()

@@ -212,8 +212,8 @@ bool qlin_takes(const at::Tensor& x, int k, bool act_int8, bool grouped = false)
 }
 // y = activations (xq, xs: int8 rows, or three digit planes) times q.  want_slabs: fp32 [splits, m, n]
 // when the shape wants a k-split (bias is then the consumer's), else bf16 [m, n].  like: options of x.
-// x: the bf16 activations behind three digit planes.
-at::Tensor qlin_product(const at::Tensor* x, const at::Tensor& xq, const at::Tensor& xs, int m, int digits, const QWeight& q,
+// x: the bf16 activations (three digit planes are made of them).
+at::Tensor qlin_product(const at::Tensor& x, const at::Tensor& xq, const at::Tensor& xs, int m, int digits, const QWeight& q,
                         const c10::optional<at::Tensor>& bias, bool silu_mul, int splits, bool want_slabs,
                         const at::TensorOptions& like, void* err_flag, void* st) {
   if (bias) {
@@ -230,10 +230,8 @@ at::Tensor qlin_product(const at::Tensor* x, const at::Tensor& xq, const at::Ten
   a.w = q.w; a.src = q.src; a.n = q.n; a.k = q.k;
   a.xq = xq.data_ptr(); a.xs = xs.data_ptr();
   a.m = m; a.digits = digits;
-  if (x) {
-    a.x = x->data_ptr();
-    a.ldx = int(x->stride(0));
-  }
+  a.x = x.data_ptr();
+  a.ldx = int(x.stride(0));
   a.scale_kind = q.scale_kind; a.scale = q.scale; a.row_scale = q.row_scale; a.group_k = q.group_k; a.zeros = q.zeros;
   a.splits = splits;
   a.err_flag = err_flag;
@@ -278,7 +276,7 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
     xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
     BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
   }
-  return qlin_product(digits == 3 ? &x : nullptr, xq, xs, m, digits, q, bias, silu_mul, splits, want_slabs, x.options(), err_flag, st);
+  return qlin_product(x, xq, xs, m, digits, q, bias, silu_mul, splits, want_slabs, x.options(), err_flag, st);
 }
 
 // Decode form of w8a16_linear without a reduction: fp32 slabs [splits, m, n] (scaled, no bias) for the
@@ -469,7 +467,7 @@ std::vector<at::Tensor> w8a16_quant_act(const at::Tensor& x) {
 }
 
 at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tensor& wq_t,
-                      const at::Tensor& sw_t, int64_t N, int64_t K, int64_t S) {
+                      const at::Tensor& sw_t, int64_t N, int64_t K, int64_t S, int splits) {
   TORCH_CHECK(xq.is_cuda() && xq.is_contiguous() && xq.dim() == 2 && xq.scalar_type() == at::kChar,
               "barlink w8a16_gemm: xq must be contiguous int8 [M, K]");
   const int m = int(xq.size(0));
@@ -485,15 +483,18 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
   void* st = at::cuda::getCurrentCUDAStream(dev).stream();
   const auto like = xq.options().dtype(at::kBFloat16);
   if (m == 0) return at::empty({0, N}, like);
-  // the tensor core takes the weights in this layout as they are (qlin_kernels.cu); S is the caller's
-  // k-split for the reference's kernel, here the shape decides
+  // S is the caller's k-split for the reference's kernel; here the shape decides, or `splits`
   (void)S;
-  const bool aligned = (reinterpret_cast<uintptr_t>(xq.data_ptr()) & 15u) == 0;
-  QWeight q{wq_t.data_ptr(), 1, int(N), int(K), BL_QSCALE_F32_GN, sw_t.data_ptr()};
-  q.group_k = 128;
+  if (splits <= 0) splits = bl_qlin_splits(int(N), int(K), m, 1, 1);
+  if (splits > K / 128) splits = int(K / 128);
   void* flag = w8_scratch(dev).err_flag.data_ptr();
   py::gil_scoped_release nogil;
-  return qlin_product(nullptr, aligned ? xq : xq.clone(), xs, m, 1, q, c10::nullopt, false, 0, false, like, flag, st);
+  const at::Tensor xa = (reinterpret_cast<uintptr_t>(xq.data_ptr()) & 15u) == 0 ? xq : xq.clone();
+  at::Tensor out = at::empty({m, N}, like), ws;
+  if (splits > 1) ws = at::empty({splits, m, N}, like.dtype(at::kFloat));
+  BL_CHECK(bl_w8a16_gemm(xa.data_ptr(), xs.data_ptr(), wq_t.data_ptr(), sw_t.data_ptr(), out.data_ptr(), m, int(N), int(K),
+                         splits, splits > 1 ? ws.data_ptr() : nullptr, flag, st, err, errlen));
+  return out;
 }
 
 // GPTQ-v1 int4 linear.  Groups of 128 and 5..128 rows: int8 digits of the activations on the tensor cores
@@ -821,7 +822,7 @@ void bind_extra(py::module_& m) {
         py::arg("n"), py::arg("k"), py::arg("tokens") = 64, py::arg("want") = 0);
   m.def("w8a16_quant_act", &w8a16_quant_act);
   m.def("w8a16_gemm", &w8a16_gemm, py::arg("xq"), py::arg("xs"), py::arg("wq_t"), py::arg("sw_t"),
-        py::arg("N"), py::arg("K"), py::arg("S"));
+        py::arg("N"), py::arg("K"), py::arg("S"), py::arg("splits") = 0);
   m.def("attn_fwd", &attn_fwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("cu_q"),
         py::arg("cu_k"), py::arg("max_q"), py::arg("scale"), py::arg("causal"), py::arg("max_k") = 0);
   m.def("attn_error_flag", &attn_error_flag, py::arg("device") = 0);

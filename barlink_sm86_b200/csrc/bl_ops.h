@@ -164,7 +164,7 @@ int bl_w8_dequant(const void* wq, const void* scale, void* out, int n, int k, vo
 int bl_w8a16_quant_act(const void* x, int m, int k, void* xq, void* xs, void* stream, char* err,
                        size_t errlen);
 int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, const void* sw_t, void* out,
-                  int m, int n, int k, int splits, void* ws, void* stream, char* err,
+                  int m, int n, int k, int splits, void* ws, void* err_flag, void* stream, char* err,
                   size_t errlen);
 
 /* ---- decode linears on quantised weights (qlin_kernels.cu) ------------------------------------

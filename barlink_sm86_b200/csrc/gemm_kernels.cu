@@ -230,31 +230,15 @@ struct PartialSink {
   float* out;          // [splits][tokens][n]
   size_t slab;         // elements per split
   int ldo, ra, rb, swap;
-  const __nv_bfloat16* scale;  // per output feature (W8A16), or null
 
   __device__ __forceinline__ void unit_done(int) const {}
   template <int NTHR>
   __device__ __forceinline__ void tile_done(int) const {}
   __device__ __forceinline__ void operator()(int ta, int tb, int split, int row, int c0,
-                                             const float (&vin)[32], int ncols) const {
+                                             const float (&v)[32], int ncols) const {
     const int i = ta * kTileA + row;
     const int j0 = tb * BN + c0;
     float* base = out + size_t(split) * slab;
-    float v[32];
-    if (scale) {
-      if (swap) {
-        const float sc = i < ra ? __bfloat162float(scale[i]) : 0.f;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) v[c] = vin[c] * sc;
-      } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-          v[c] = (c < ncols && j0 + c < rb) ? vin[c] * __bfloat162float(scale[j0 + c]) : 0.f;
-      }
-    } else {
-#pragma unroll
-      for (int c = 0; c < 32; ++c) v[c] = vin[c];
-    }
     if (swap) {
       if (i >= ra) return;  // i = feature, j = token: a warp stores 32 consecutive features
 #pragma unroll
@@ -589,7 +573,6 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
     ps.ra = a.ra;
     ps.rb = a.rb;
     ps.swap = a.swap;
-    ps.scale = nullptr;
     static bool attr_p = false;
     if (!attr_p) {
       e = cudaFuncSetAttribute(k_gemm_partial<BN, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1088,7 +1071,6 @@ static int launch_gemm_pair(const blGemmArgs& a, cudaStream_t st, char* err, siz
     ps.ra = a.ra;
     ps.rb = a.rb;
     ps.swap = 0;
-    ps.scale = nullptr;
     e = launch_pair_kernel(pairs, st, ta, tb, g, ps);
   } else {
     e = launch_pair_kernel(pairs, st, ta, tb, g, sink);

@@ -223,17 +223,7 @@ __device__ __forceinline__ void tma_load_2d_hint_s(uint32_t smem_dst, const void
       "l"(tmap), "r"(bar), "r"(x), "r"(y), "l"(hint)
       : "memory");
 }
-// untiled bulk copy global -> this CTA's shared memory (16-byte aligned both
-// sides, size a multiple of 16); completes on the mbarrier like a tensor copy
-__device__ __forceinline__ void bulk_load_s(uint32_t smem_dst, const void* gsrc, uint32_t bytes,
-                                            uint32_t bar, uint64_t hint) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1], %2, [%3], %4;" ::"r"(smem_dst),
-      "l"(gsrc), "r"(bytes), "r"(bar), "l"(hint)
-      : "memory");
-}
-// Both for a whole converged warp, of which the elected lane issues (see elect_leader).
+// Loads for a whole converged warp, of which the elected lane issues (see elect_leader).
 __device__ __forceinline__ void tma_load_2d_hint_warp(uint32_t leader, uint32_t smem_dst, const void* tmap,
                                                       uint32_t bar, int x, int y, uint64_t hint) {
   asm volatile(
@@ -253,6 +243,8 @@ __device__ __forceinline__ void tma_prefetch_2d_warp(uint32_t leader, const void
       "r"(x), "r"(y), "l"(hint), "r"(leader)
       : "memory");
 }
+// untiled bulk copy global -> this CTA's shared memory (16-byte aligned both sides, size a multiple of 16);
+// completes on the mbarrier like a tensor copy
 __device__ __forceinline__ void bulk_load_warp(uint32_t leader, uint32_t smem_dst, const void* gsrc, uint32_t bytes,
                                                uint32_t bar, uint64_t hint) {
   asm volatile(
@@ -308,16 +300,6 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t a_desc, ui
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], signed 8-bit inputs (32 per instruction along K), int32 accumulate.
-__device__ __forceinline__ void umma_i8_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                           uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // The forms below are for a whole converged warp, of which one lane (`leader`, see elect_leader) issues: the
 // operands stay in uniform registers, where the instruction wants them.  Issued from a `lane == 0` branch an
 // MMA took the thread about 60 cycles and a commit about 75, more than the tensor core needs for the
@@ -337,6 +319,7 @@ __device__ __forceinline__ void umma_f16_ss_warp(uint32_t leader, uint32_t d_tme
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
+// signed 8-bit inputs (32 per instruction along K), int32 accumulate
 __device__ __forceinline__ void umma_i8_ss_warp(uint32_t leader, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                                 uint32_t idesc, uint32_t accumulate) {
   asm volatile(

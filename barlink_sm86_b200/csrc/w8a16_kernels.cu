@@ -97,8 +97,8 @@ extern "C" int bl_w8a16_quant_act(const void* x, int m, int k, void* xq, void* x
 }
 
 extern "C" int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, const void* sw_t,
-                             void* out, int m, int n, int k, int splits, void* ws, void* stream,
-                             char* err, size_t errlen) {
+                             void* out, int m, int n, int k, int splits, void* ws, void* err_flag,
+                             void* stream, char* err, size_t errlen) {
   if (m < 1 || m > kMaxM) {
     set_err(err, errlen, "barlink: w8a16_gemm is the decode kernel of the reference API: 1..%d rows (got %d)",
             kMaxM, m);
@@ -138,6 +138,7 @@ extern "C" int bl_w8a16_gemm(const void* xq, const void* xs, const void* wq_t, c
   a.group_k = kGroup;
   a.splits = splits;
   if (splits > 1) a.slabs = ws;
+  a.err_flag = err_flag;
   a.out = out;
   a.ldo = n;
   if (bl_qlin(&a, stream, err, errlen) != 0) return -1;

@@ -82,9 +82,11 @@ def linear(x, weight, bias=None, residual=None, silu_mul=False, out=None, gate_t
     dynamic_weights: `weight` was written by a kernel earlier in this stream
     (not at load time), so its tiles must not be fetched ahead of that kernel."""
     if x.is_cuda:
-        _count()
         x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
         w, tn, tk = _w(weight)
+        # (a k-split leaves its slabs to a second kernel)
+        _count(2 if x2.shape[0] > 128 and not tn and gate_tokens <= 0
+               and _C().gemm_row_splits(x2.shape[0], *weight.shape) > 1 else 1)
         y = _C().linear(x2, w, bias, residual, silu_mul, out, gate_tokens=gate_tokens, tiled_n=tn,
                         tiled_k=tk, gelu=gelu, dynamic_weights=dynamic_weights)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])

@@ -253,8 +253,9 @@ def test_chunked_int8_weights(ext, m, n, k):
     xq, xs = ext.w8a16_quant_act(_x(m, k, 5, spread=True))
     part = torch.einsum("mgk,ngk->gmn", xq.double().view(m, -1, 128), wq.double().view(n, -1, 128))
     want = (part * sw.double()[:, None, :]).sum(0) * xs.double()[:, None]
-    for splits in (1, 4):
-        assert rel_l2(ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, splits), want) < TOL
+    assert rel_l2(ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, 4), want) < TOL
+    for splits in (1, 3, k // 128, 99):  # the last two: one k-block each
+        assert rel_l2(ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, 1, splits=splits), want) < TOL
     off = torch.empty(m * k + 4, dtype=torch.int8, device="cuda")[4:].view(m, k)  # rows off 16-byte boundaries
     off.copy_(xq)
     assert torch.equal(ext.w8a16_gemm(off, xs, wq_t, sw, n, k, 1), ext.w8a16_gemm(xq, xs, wq_t, sw, n, k, 1))

@@ -1221,7 +1221,7 @@ extern "C" int bl_gemm_splits(int n, int k, int tokens) {
 
 // k-splits of a token-major product in the paired kernel: the cheapest of 1 .. 4 by laps of the pairs, in
 // k-blocks of 0.28 us.  A product costs the k-blocks of its laps plus about 22 of ramp and epilogue; with a split
-// the kernel behind it costs 10 and the slabs, written and read once more, 0.85 a megabyte; below 3 % it is not
+// the kernel behind it costs 8 and the slabs, written and read once more, 0.7 a megabyte; below 3 % it is not
 // worth the memory.  Unsplit and with the split chosen, us: 512 x 18944 x 600 rows 89 and 33, 3584 x 18944 x 333
 // 97 and 59, 3584 x 18944 x 1285 (two laps by 10 tiles) 191 and 170, 5120 x 27648 x 1000 296 and 247, x 2048 566
 // and 474; where it does not split, 256 x 1024 x 1000 10.8 against 12.4 with two.
@@ -1234,7 +1234,7 @@ extern "C" int bl_gemm_row_splits(int rows, int n, int k) {
     const int per = (kb + s - 1) / s;
     if ((s - 1) * per >= kb) continue;
     const int laps = (tiles * s + pairs - 1) / pairs;
-    const double c = laps * per + 22.0 + (s > 1 ? 10.0 + double(s) * rows * n * 8.0 * 0.85e-6 : 0.0);
+    const double c = laps * per + 22.0 + (s > 1 ? 8.0 + double(s) * rows * n * 8.0 * 0.7e-6 : 0.0);
     if (c < cost * (s > 1 ? 0.97 : 1.0)) {
       cost = c;
       best = s;

@@ -266,13 +266,15 @@ at::Tensor qlin_product(const at::Tensor& x, const at::Tensor& xq, const at::Ten
 at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10::optional<at::Tensor>& bias,
                     bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
   const int m = int(x.size(0));
-  at::Tensor xq, xs = at::empty({m}, x.options().dtype(at::kFloat));
+  at::Tensor xq, xs;
   if (digits == 3) {
+    xs = at::empty({int64_t(bl_quant_digits_xs_bytes(m) / sizeof(float))}, x.options().dtype(at::kFloat));
     xq = at::empty({int64_t(bl_quant_digits_bytes(m, q.k))}, x.options().dtype(at::kChar));
     BL_CHECK(bl_quant_digits(x.data_ptr(), m, int(x.stride(0)), q.k, q.src == 2 ? 1 : 0, xq.data_ptr(), xs.data_ptr(), st,
                              err, errlen));
   } else {
     at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    xs = at::empty({m}, x.options().dtype(at::kFloat));
     xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
     BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
   }
@@ -523,8 +525,10 @@ at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at
   W8Scratch& s = w8_scratch(dev);
   const bool aligned = ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(qweight.data_ptr())) & 15u) == 0;
   // The tensor cores cost the same for 1 to 16 rows, the GEMV two rows' worth of time more for every doubling:
-  // 37888 x 3584, us: GEMV 33 / 50 / 87 / 88 / 177 at 1 / 4 / 6 / 8 / 16 rows, digits 57 throughout;
-  // 3584 x 18944: GEMV 28 / 31 / 56 / 57 / 92, digits 36 - 41.
+  // 37888 x 3584, us: GEMV 28 / 50 / 86 / 88 / 176 at 1 / 4 / 5 / 8 / 16 rows, digits 39 throughout;
+  // 3584 x 18944: GEMV 22 / 31 / 56 / 57 / 91, digits 31 - 34.  Above 16 rows the other way is to widen the weight for
+  // a bf16 product: 64 rows, 296 and 143 us there against 70 and 45; faster only for small weights (2048 x 2048
+  // 10 against 17), whose values it rounds to bf16.
   if (group == 128 && m > 4 && m <= BL_QLIN_MAX_TOKENS && k <= 32768 && n % 8 == 0 && aligned) {
     QWeight q{qweight.data_ptr(), 2, n, k, BL_QSCALE_F16_GN, scales.data_ptr()};
     q.group_k = group;

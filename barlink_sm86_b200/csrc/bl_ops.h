@@ -211,12 +211,14 @@ int bl_qlin_tile_tokens(int m); /* of three digit planes */
  * xs fp32 [m] with x = |xs| * (d0 + d1 / 2^8 + d2 / 2^16): exact for elements down to 2^-15 of the row's
  * largest, below that to 2^-24 of 2^ex, the power of two above the largest.  Rows with an infinity, or with more than half of their nonzero
  * elements below 2^-11 of that scale, get a negative xs: |xs| then follows the median (2^10 above it), and the
- * elements beyond have digits of zero; bl_qlin adds their products in fp32.  A NaN makes xs a NaN.
+ * elements beyond have digits of zero; bl_qlin adds their products in fp32.  A NaN makes xs a NaN.  xs has room for
+ * bl_quant_digits_xs_bytes(m): behind the m words, marks of where such rows have elements beyond.
  * permute: digits in the order 0 2 4 6 1 3 5 7 of every eight (packed int4 weights).  K a multiple of 8, at
  * most 32768. */
 int bl_quant_digits(const void* x, int m, int ldx, int k, int permute, void* xq, void* xs, void* stream, char* err,
                     size_t errlen);
 size_t bl_quant_digits_bytes(int m, int k);
+size_t bl_quant_digits_xs_bytes(int m);
 /* slabs fp32 [nsplit][m][pitch] -> out bf16 [m][n] (pitch ldo), the sum with the epilogue of a product: + bias,
  * tanh-GELU, + residual (out's layout); or, with silu_mul, + bias and SiLU*mul over interleaved columns into
  * [m][n / 2].  Bias, residual and out may start at any element. */

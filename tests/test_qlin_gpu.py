@@ -242,6 +242,26 @@ def test_activation_rows_with_extreme_values(ext, m):
     assert ext.w8_error_flag(0) == 0
 
 
+@pytest.mark.parametrize("m", [16, 64])
+def test_rows_of_mostly_outliers(ext, m):
+    """The most that the epilogue can be asked to add: every row nearly half outliers, or nothing but infinities,
+    in a long reduction without a k-split.  No wait of the other warps runs out, and the values are right."""
+    n, k = 136, 27648
+    wq, sc = _w8(n, k, 7)
+    x = _x(m, k, 21)
+    x[:, : k * 9 // 20] *= 2.0 ** 20
+    want = (x.double() @ wq.double().t()) * sc.double()
+    assert rel_l2(ext.w8a16_linear(x, wq, sc, None, False, 1), want) < TOL
+    x[:] = float("inf")
+    assert bool(ext.w8a16_linear(x, wq, sc, None, False, 1).isnan().all())  # weights of both signs
+    qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8, n), generator=_g(11), device="cuda", dtype=torch.int64).to(torch.int32)
+    s4, qz = torch.ones(k // 128, n, device="cuda").half(), torch.zeros(k // 128, n // 8, dtype=torch.int32, device="cuda")
+    y = ext.w4a16_linear(x, qw, s4, qz, 128, 1)  # weights 0 .. 15: infinity times zero somewhere
+    assert bool(y.isnan().all())
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0
+
+
 # k-chunk-major weights (the reference's pair): ragged last row tile, odd n (no k-split), one k-block
 @pytest.mark.parametrize("m", [1, 9, 16])
 @pytest.mark.parametrize("n,k", [(128, 128), (136, 1280), (201, 640), (1000, 3584)])

@@ -272,9 +272,9 @@ def prepare_w8_scales(scale, k):
 
 
 def w8_act_mode():
-    """How `w8a16_linear` treats the activations by default: "bf16" (weights widened to bf16 in the
-    kernel, the activations as they are: the accurate form) or "int8" (activations quantised per token,
-    int8 x int8 on the tensor cores: the reference kernel's numerics).  Environment BL_W8_ACT."""
+    """How `w8a16_linear` treats the activations by default: "bf16" (the activations as they are: the
+    accurate form) or "int8" (activations quantised per token, int8 x int8 on the tensor cores: the
+    reference kernel's numerics).  Environment BL_W8_ACT."""
     import os
     v = os.environ.get("BL_W8_ACT", "bf16")
     if v not in ("bf16", "int8"):
@@ -286,8 +286,10 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
     """scale [n]: per output channel.  scale [n, k/group] or a W8GroupScales: per group, the
     reference's granularity (torch_ext/barlink_sm86/w8a16.cu:119-142 applies group scales inside
     its K loop).  Up to 128 tokens the int8 weights go to the tensor cores as they are, against three
-    int8 digits of the bf16 activations (csrc/qlin_kernels.cu: no loss against bf16 operands); group
-    scales, for groups of a multiple of 128, are applied to the sums of a k-block.  Groups of 64 and
+    int8 digits of the bf16 activations (csrc/qlin_kernels.cu: exact sums; of an activation the digits
+    drop at most 2^-24 of the row's largest and 2^-13 of its median element, nothing above 2^-15 of the
+    largest); group scales, for groups of a multiple of 128, are applied to the sums of a k-block.  The
+    weights may come from a kernel just ahead in the stream.  Groups of 64 and
     129..256 tokens widen the tile inside the main loop; other groups, and more than 256 tokens,
     widen the weight once and run the bf16 GEMM.
 
@@ -302,7 +304,7 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
             if scale.dim() == 1:
                 _count(2)
                 return _C().w8a16_linear(x, wq, scale, bias, silu_mul, act_int8=True)
-            # smaller layers keep the bf16 activations: there the exact form costs the same
+            # (smaller layers and more tokens keep the bf16 activations)
             if x.shape[0] <= 64 and (k // scale.shape[1]) % 128 == 0 and wq.shape[0] >= 148 * 128:
                 # group scales (the reference's checkpoint format): one accumulator per k-block,
                 # scaled and summed by the epilogue warps
@@ -315,7 +317,7 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
             else:
                 w = ref.w8_dequant(wq, scale).to(torch.bfloat16)
                 return linear(x, w, bias, silu_mul=silu_mul, dynamic_weights=True)
-        _count()
+        _count(2 if _qlin_rows(x) else 1)
         if gs is not None:
             if x.shape[0] > 256:
                 w = (ref.w8_dequant(wq, gs.rel.float() * gs.row.float()[:, None])).to(torch.bfloat16)

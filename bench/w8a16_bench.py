@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 # SPDX-License-Identifier: MIT
-"""W8A16 decode GEMM: this library's tcgen05 kernel (bf16 activations, int8
-per-channel weights widened in the main loop) against the reference's own
+"""W8A16 decode GEMM: this library's tcgen05 kernel (int8 per-channel weights
+against int8 digits of the bf16 activations) against the reference's own
 kernel pair built for sm_100 from baseline/_ref (`barlink_sm86._C.
 w8a16_quant_act` + `w8a16_gemm`: int8 activations, dp4a, group-128 scales).
 Shapes are the reference's decode shapes (torch_ext/tests/test_w8a16.py:23-32

@@ -329,26 +329,31 @@ def test_other_threads_run_while_a_launch_waits(ext):
                     "linear": lambda: ext.linear(xl, w)}.items():
         f()
         torch.cuda.synchronize()
-        stop, gap = threading.Event(), [0.0]
+        seen = []
+        for _ in range(3):  # (a busy host may hold up any one of them)
+            stop, gap = threading.Event(), [0.0]
 
-        def tick():
-            last = time.perf_counter()
-            while not stop.is_set():
-                time.sleep(1e-3)
-                now = time.perf_counter()
-                gap[0], last = max(gap[0], now - last), now
-        th = threading.Thread(target=tick)
-        th.start()
-        torch.cuda._sleep(10 ** 9)  # half a second of an occupied stream
-        t0 = time.perf_counter()
-        for _ in range(2000):
-            f()
-        waited = time.perf_counter() - t0
-        stop.set()
-        th.join()
-        torch.cuda.synchronize()
-        assert waited > 0.2, (name, waited)  # the queue was full
-        assert gap[0] < waited / 2, (name, gap[0], waited)
+            def tick():
+                last = time.perf_counter()
+                while not stop.is_set():
+                    time.sleep(1e-3)
+                    now = time.perf_counter()
+                    gap[0], last = max(gap[0], now - last), now
+            th = threading.Thread(target=tick)
+            th.start()
+            torch.cuda._sleep(10 ** 9)  # half a second of an occupied stream
+            t0 = time.perf_counter()
+            for _ in range(2000):
+                f()
+            waited = time.perf_counter() - t0
+            stop.set()
+            th.join()
+            torch.cuda.synchronize()
+            seen.append((gap[0], waited))
+            if waited > 0.2 and gap[0] < waited / 2:  # the queue was full, and the thread ran
+                break
+        else:
+            raise AssertionError((name, seen))
 
 
 # Weights that a kernel just ahead in the stream leaves behind (received, unpacked, dequantised ones): this

@@ -46,8 +46,8 @@ BarlinkBackend::BarlinkBackend(int rank, int size, c10::intrusive_ptr<c10d::Back
     TORCH_CHECK(c != nullptr, "barlink: the link is not initialised (call init_peer first)");
     TORCH_CHECK(bl_is_peer(c), "barlink: a process group needs the SPMD link (init_peer), not init()");
     TORCH_CHECK(bl_world(c) == size && bl_rank(c) == rank,
-                "barlink: process group (rank ", rank, " of ", size,
-                ") does not match the link (rank ", bl_rank(c), " of ", bl_world(c),
+                "barlink: process group (rank ", std::to_string(rank), " of ", std::to_string(size),
+                ") does not match the link (rank ", std::to_string(bl_rank(c)), " of ", std::to_string(bl_world(c)),
                 "); groups smaller than the world are supported only with one member");
   }
 }
@@ -241,7 +241,7 @@ static size_t p2p_chunk(blCtx* c) { return bl_p2p_chunk(c) & ~size_t(15); }
 
 void BarlinkBackend::send_cuda(const at::Tensor& t, int dst) {
   TORCH_CHECK(dst != getRank(), "barlink: send to self is not supported");
-  TORCH_CHECK(dst >= 0 && dst < getSize(), "barlink: send destination ", dst, " out of range");
+  TORCH_CHECK(dst >= 0 && dst < getSize(), "barlink: send destination ", std::to_string(dst), " out of range");
   if (t.numel() == 0) return;
   blCtx* c = link();
   c10::cuda::CUDAGuard guard(t.device());
@@ -280,7 +280,7 @@ void BarlinkBackend::send_cuda(const at::Tensor& t, int dst) {
 
 void BarlinkBackend::recv_cuda(at::Tensor& t, int src) {
   TORCH_CHECK(src != getRank(), "barlink: recv from self is not supported");
-  TORCH_CHECK(src >= 0 && src < getSize(), "barlink: recv source ", src, " out of range");
+  TORCH_CHECK(src >= 0 && src < getSize(), "barlink: recv source ", std::to_string(src), " out of range");
   if (t.numel() == 0) return;
   blCtx* c = link();
   c10::cuda::CUDAGuard guard(t.device());

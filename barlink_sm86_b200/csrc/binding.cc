@@ -67,7 +67,7 @@ void init(std::vector<int> devices, int pool_mb) {
   }
   TORCH_CHECK(pool_mb >= 8 && pool_mb <= 65536, "barlink: pool_mb must be in [8, 65536]");
   TORCH_CHECK(!devices.empty() && devices.size() <= BL_MAX_RANKS, "barlink: init needs 1..",
-              BL_MAX_RANKS, " devices");
+              std::to_string(BL_MAX_RANKS), " devices");
   blCtx* out = nullptr;
   {
     py::gil_scoped_release nogil;
@@ -127,7 +127,7 @@ py::dict info() {
 
 int arena_device(blCtx* c, int idx) {
   if (bl_is_peer(c)) return g_devices[0];
-  TORCH_CHECK(idx >= 0 && idx < int(g_devices.size()), "barlink: arena index ", idx, " out of range");
+  TORCH_CHECK(idx >= 0 && idx < int(g_devices.size()), "barlink: arena index ", std::to_string(idx), " out of range");
   return g_devices[idx];
 }
 
@@ -177,7 +177,7 @@ void copy_(const at::Tensor& dst, const at::Tensor& src) {
 void allreduce_(std::vector<at::Tensor> ts) {
   blCtx* c = ctx_or_throw();
   TORCH_CHECK(int(ts.size()) == bl_world(c), "barlink: allreduce_ needs one pool tensor per arena (",
-              bl_world(c), ")");
+              std::to_string(bl_world(c)), ")");
   std::vector<void*> ptrs, streams;
   std::vector<int> idxs;
   const int code = blpg::dtype_code(ts[0].scalar_type());
@@ -460,7 +460,8 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const c10::optional<
   if (tiled) {
     TORCH_CHECK(tiled_k == x.size(1) && size_t(w.nbytes()) >= bl_tiled_weight_bytes(tiled_n, tiled_k) &&
                     (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15u) == 0,
-                "barlink: tiled weight buffer does not match (n, k) = (", tiled_n, ", ", tiled_k, ")");
+                "barlink: tiled weight buffer does not match (n, k) = (", std::to_string(tiled_n), ", ",
+                std::to_string(tiled_k), ")");
   } else {
     TORCH_CHECK(w.dim() == 2 && w.size(1) == x.size(1), "barlink: weight must be [n, k] with k = x.shape[1]");
   }

@@ -17,6 +17,9 @@
 
 namespace py = pybind11;
 
+// (Numbers go into the messages of TORCH_CHECK as text, std::to_string: put into a stream by an extension, an integer
+// crashes the process where the toolchain's C++ library and the one that torch brings differ.)
+
 namespace {
 
 constexpr size_t kErr = 512;
@@ -63,7 +66,8 @@ void sp_collective(const std::string& kind, std::vector<at::Tensor> ins, std::ve
   auto ptrs = [&](std::vector<at::Tensor>& v, const char* name) {
     std::vector<void*> p;
     if (v.empty()) return p;
-    TORCH_CHECK(int(v.size()) == world, "barlink: ", name, " needs one tensor per rank (", world, ")");
+    TORCH_CHECK(int(v.size()) == world, "barlink: ", name, " needs one tensor per rank (",
+                std::to_string(world), ")");
     for (auto& t : v) {
       TORCH_CHECK(t.is_cuda() && t.is_contiguous(), "barlink: ", name, " tensors must be contiguous CUDA tensors");
       p.push_back(t.data_ptr());
@@ -293,7 +297,8 @@ at::Tensor w8a16_linear_split(const at::Tensor& x, const at::Tensor& wq, const a
   check_bf16x(scale, "scale");
   const int k = int(x.size(1)), n = int(wq.size(0)), dev = x.device().index();
   TORCH_CHECK(scale.numel() == n, "barlink: scale must have one entry per output channel");
-  TORCH_CHECK(qlin_takes(x, k, act_int8), "barlink: w8a16_linear_split is for 1..", BL_QLIN_MAX_TOKENS, " 16-byte aligned rows, K % 16 == 0");
+  TORCH_CHECK(qlin_takes(x, k, act_int8), "barlink: w8a16_linear_split is for 1..", std::to_string(BL_QLIN_MAX_TOKENS),
+              " 16-byte aligned rows, K % 16 == 0");
   c10::cuda::CUDAGuard guard(x.device());
   void* flag = w8_scratch(dev).err_flag.data_ptr();
   py::gil_scoped_release nogil;
@@ -657,7 +662,7 @@ void dlin_fill_common(blDlinArgs& a, const at::Tensor& x, int hidden, const c10:
   if (link) {
     TORCH_CHECK(link->is_cuda() && link->is_contiguous() &&
                     size_t(link->nbytes()) >= bl_dlin_local_link_bytes(a.tokens, hidden),
-                "barlink: the local link buffer is too small for ", a.tokens, " x ", hidden);
+                "barlink: the local link buffer is too small for ", std::to_string(a.tokens), " x ", std::to_string(hidden));
     a.local_link = link->data_ptr();
   }
   a.err_flag = dlin_scratch(dev).err_flag.data_ptr();
@@ -707,7 +712,7 @@ at::Tensor dlin(const at::Tensor& x, const at::Tensor& w, const std::string& pro
     out = out_opt ? *out_opt : at::empty({x.size(0), cols}, x.options());
     TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kBFloat16 && out.dim() == 2 && out.size(0) == x.size(0) &&
                     out.size(1) == cols && out.stride(1) == 1,
-                "barlink: dlin out must be bf16 [tokens, ", cols, "]");
+                "barlink: dlin out must be bf16 [tokens, ", std::to_string(cols), "]");
     a.out = out.data_ptr();
     a.ldo = int(out.stride(0));
     if (bias) {

@@ -84,3 +84,15 @@ def test_decode_linear_cluster_choice(n, k, tokens):
     for want in (1, 2, 4, 8):
         got = C.dlin_cluster(n, k, tokens, want)
         assert 1 <= got <= min(want, max(1, kblocks))
+
+
+@pytest.mark.parametrize("devices", ["[]", "list(range(9))"])
+def test_an_error_with_a_number_in_it_is_an_error(devices):
+    """... and not a crash of the process (hence a child)."""
+    import subprocess
+    import sys
+    code = ("import barlink_sm86_b200 as bl\n"
+            "try:\n    bl.load_extension().init(%s, 64)\n"
+            "except RuntimeError as e:\n    print(e)\n" % devices)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "1..8 devices" in r.stdout, (r.returncode, r.stdout, r.stderr)

@@ -114,7 +114,7 @@ __device__ __forceinline__ uint32_t digit_limit(int ex) { return (uint32_t(ex + 
 
 // The products of a token's outliers (see k_quant_digits) with weight row n, k0 <= k < k1, without what is common
 // to the row.  A whole warp calls it for one token: it goes to the chunks of 256 activations that the quantiser has
-// marked (16 tokens with one outlier each, 5120 x 27648: 40 us without, 189 us looking through whole rows) and deals
+// marked (16 tokens, 5120 x 27648: 36 us; with one outlier each 68 us, 189 us looking through whole rows) and deals
 // with the outliers of eight neighbours together, so that a row of nothing else (all infinities: some 4000 such
 // steps) still ends long before the waits of the other warps do.  Infinities come out as in any sum of products.  A
 // call of its own, so that the loops around it keep their registers: such rows are rare (inlined, it cost the products

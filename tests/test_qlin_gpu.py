@@ -126,6 +126,17 @@ def test_no_rows(ext):
     assert ext.w8a16_linear(x, wq, gs, act_int8=True, group_scale=gs).shape == (0, 200)
 
 
+def test_too_many_rows_are_refused(ext):
+    wq, sc = _w8(200, 1024, 3)
+    gs = torch.ones(200, 8, device="cuda").bfloat16()
+    with pytest.raises(RuntimeError, match="1..128"):
+        ext.w8a16_linear_split(_x(129, 1024, 5), wq, sc)
+    with pytest.raises(RuntimeError, match="at most 64"):
+        ext.w8a16_linear(_x(65, 1024, 5), wq, gs, act_int8=True, group_scale=gs)
+    with pytest.raises(RuntimeError, match="at most 64"):
+        ext.w8a16_linear(_x(8, 1024, 5), wq, gs, group_scale=gs)
+
+
 @pytest.mark.parametrize("m", [1, 32, 64])
 @pytest.mark.parametrize("n,k,group", [(200, 1024, 128), (129, 768, 256)])
 @pytest.mark.parametrize("act_int8", [False, True])

@@ -210,7 +210,7 @@ int bl_qlin_tile_tokens(int m); /* of three digit planes */
 /* x [m x k] bf16 (pitch ldx) -> xq int8 [ceil(m/tile)][3][tile][k] (tile = bl_qlin_tile_tokens(m)) and
  * xs fp32 [m] with x = |xs| * (d0 + d1 / 2^8 + d2 / 2^16): exact for elements down to 2^-15 of the row's
  * largest, below that to 2^-24 of 2^ex, the power of two above the largest.  Rows with an infinity, or with more than half of their nonzero
- * elements below 2^-11 of that scale, get a negative xs: |xs| then follows the median (2^10 above it), and the
+ * elements below 2^-13 of that scale, get a negative xs: |xs| then follows the median (2^12 above it), and the
  * elements beyond have digits of zero; bl_qlin adds their products in fp32.  A NaN makes xs a NaN.  xs has room for
  * bl_quant_digits_xs_bytes(m): behind the m words, marks of where such rows have elements beyond.
  * permute: digits in the order 0 2 4 6 1 3 5 7 of every eight (packed int4 weights).  K a multiple of 8, at

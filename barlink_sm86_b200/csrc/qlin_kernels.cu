@@ -10,10 +10,10 @@
 // scaled by a power of two so that its largest element is just below 1 and written as three base-256
 // digits (k_quant_digits): a fixed-point number of 23 bits below that element, so every element down to
 // 2^-15 of the largest is represented exactly and the rest to within 2^-24 of the largest.  In rows where
-// that would be coarse -- more than half of the nonzero elements below 2^-11 of the scale, or an infinity -- the
-// scale follows the median instead (2^10 above it), and the few elements beyond it are left out of the digits
+// that would be coarse -- more than half of the nonzero elements below 2^-13 of the scale, or an infinity -- the
+// scale follows the median instead (2^12 above it), and the few elements beyond it are left out of the digits
 // and added in fp32 by the epilogue (outlier_sum).  What a digit drops is thus at most 2^-24 of the largest
-// and 2^-13 of the median element, whichever weights meet the outliers.  The weights go from HBM to the tensor
+// and 2^-11 of the median element, whichever weights meet the outliers.  The weights go from HBM to the tensor
 // core as they are, the three digit planes of all tokens are the N dimension of one MMA, sums are exact int32,
 // and the epilogue puts (d0 + d1 / 2^8 + d2 / 2^16) * xs[t] together.  With activations that the caller quantised
 // to int8 (one digit) the same kernel runs with a third of the N.
@@ -654,7 +654,9 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
   // |x| < 2^ex; a largest element of 255/256 * 2^ex would round up to 128 in the first digit
   int ex = int(mx >> 7) - 126 + ((mx & 0x7fu) == 0x7fu ? 1 : 0);
   if (ex < -110) ex = -110;  // the digits of such rows reach the smallest bf16, 2^-133
-  const uint32_t small = count(ex > -110 ? ex + 116 : 0);  // below 2^(ex - 11)
+  // Below 2^(ex - 13).  (What follows costs such a row 1 to 2 us in the linear, so the line lies beyond the rows that
+  // products of activations give: a bf16 result is rounded to 2^-9, the median element here to 2^-11.)
+  const uint32_t small = count(ex > -110 ? ex + 114 : 0);
   const bool bad = mx > 0x7f80u;  // NaN in the row: the whole row of results is NaN
   const bool split = !bad && (2 * (small & 0xffffu) > (small >> 16) || mx == 0x7f80u);
   if (split) {
@@ -669,7 +671,7 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
       if (2 * (count(mid + 1) & 0xffffu) >= (small >> 16)) hi = mid;
       else lo = mid + 1;
     }
-    ex = min(128, max(-110, lo - 126 + 10));
+    ex = min(128, max(-110, lo - 126 + 12));
   }
   const uint32_t limit = digit_limit(ex);
   if (split) {

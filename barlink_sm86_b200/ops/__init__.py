@@ -287,7 +287,7 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
     reference's granularity (torch_ext/barlink_sm86/w8a16.cu:119-142 applies group scales inside
     its K loop).  Up to 128 tokens the int8 weights go to the tensor cores as they are, against three
     int8 digits of the bf16 activations (csrc/qlin_kernels.cu: exact sums; of an activation the digits
-    drop at most 2^-24 of the row's largest and 2^-13 of its median element, nothing above 2^-15 of the
+    drop at most 2^-24 of the row's largest and 2^-11 of its median element, nothing above 2^-15 of the
     largest); group scales, for groups of a multiple of 128, are applied to the sums of a k-block.  The
     weights may come from a kernel just ahead in the stream.  Groups of 64 and
     129..256 tokens widen the tile inside the main loop; other groups, and more than 256 tokens,

@@ -4,7 +4,7 @@
 Oracle: the exact integer products in float64.  Tolerances: the bf16 result is rounded once (rel-L2 at
 most 2^-9 / sqrt(3) per element on average, 2^-8 allowed); fp32 slabs carry the int32 -> fp32 conversions
 and their sum only (2^-24 each; 2^-20 allowed).  Digits: exact down to 2^-15 of a row's largest element; what
-they drop of an element is at most 2^-24 of the largest and 2^-13 of the median of a row."""
+they drop of an element is at most 2^-24 of the largest and 2^-11 of the median of a row."""
 import pytest
 import torch
 
@@ -188,7 +188,7 @@ def _forms(ext, n, k):
 @pytest.mark.parametrize("ratio", [12, 15, 18, 24, 60])
 def test_outliers_that_meet_zero_weights(ext, m, n, k, ratio):
     """A few elements 2^ratio above the rest, in columns where a third of the weight rows are zero: those rows'
-    results have only the small elements, and every one of them may be off by 2^-13 of the median at most
+    results have only the small elements, and every one of them may be off by 2^-11 of the median at most
     (weights of a third of the rows are zero there, the others see what fp32 leaves of the large products)."""
     for f, f32, wi, w in _forms(ext, n, k):
         x = _x(m, k, 21)
@@ -197,7 +197,7 @@ def test_outliers_that_meet_zero_weights(ext, m, n, k, ratio):
         x[1::2, cols] = (x[1::2, cols].float() * 2.0 ** ratio).bfloat16()
         want = x.double() @ w.t()
         # zero weights at the outliers: rows 0, 3, 6, ... ; one bf16 rounding of the result, then the digits
-        drop = 2.0 ** -13 * med[:, None] * w.abs().sum(1)[None, :]
+        drop = 2.0 ** -11 * med[:, None] * w.abs().sum(1)[None, :]
         assert bool((wi[::3][:, cols] == 0).all())
         y = f(x).double()
         assert bool(((y - want).abs() <= 2.0 ** -8 * want.abs() + drop)[:, ::3].all())

@@ -1221,10 +1221,11 @@ extern "C" int bl_gemm_splits(int n, int k, int tokens) {
 
 // k-splits of a token-major product in the paired kernel: the cheapest of 1 .. 4 by laps of the pairs, in
 // k-blocks of 0.28 us.  A product costs the k-blocks of its laps plus about 22 of ramp and epilogue; with a split
-// the kernel behind it costs 8 and the slabs, written and read once more, 0.7 a megabyte; below 3 % it is not
-// worth the memory.  Unsplit and with the split chosen, us: 512 x 18944 x 600 rows 89 and 33, 3584 x 18944 x 333
-// 97 and 59, 3584 x 18944 x 1285 (two laps by 10 tiles) 191 and 170, 5120 x 27648 x 1000 296 and 247, x 2048 566
-// and 474; where it does not split, 256 x 1024 x 1000 10.8 against 12.4 with two.
+// the kernel behind it costs 8 and the slabs, written and read once more, 0.7 a megabyte while they stay in L2 and
+// 1.2 for what goes beyond 60 MB; below 3 % it is not worth the memory.  Unsplit and with the split chosen, us:
+// 512 x 18944 x 600 rows 89 and 33, 3584 x 18944 x 333 97 and 59, 3584 x 18944 x 1285 (two laps by 10 tiles) 191 and
+// 170, 5120 x 27648 x 1000 296 and 247; where it does not split, against two: 256 x 1024 x 1000 10.8 and 12.4,
+// 3072 x 12288 x 2200 132 and 139, 3584 x 18944 x 2600 303 and 315.
 extern "C" int bl_gemm_row_splits(int rows, int n, int k) {
   if (!gemm_pair_enabled() || rows <= 128 || n < 256 || (k & 7)) return 1;
   const int tiles = ((rows + 255) / 256) * ((n + 255) / 256), pairs = sm_count() / 2, kb = (k + kTileK - 1) / kTileK;
@@ -1234,7 +1235,8 @@ extern "C" int bl_gemm_row_splits(int rows, int n, int k) {
     const int per = (kb + s - 1) / s;
     if ((s - 1) * per >= kb) continue;
     const int laps = (tiles * s + pairs - 1) / pairs;
-    const double c = laps * per + 22.0 + (s > 1 ? 8.0 + double(s) * rows * n * 8.0 * 0.7e-6 : 0.0);
+    const double mb = double(s) * rows * n * 8.0e-6;
+    const double c = laps * per + 22.0 + (s > 1 ? 8.0 + 0.7 * mb + (mb > 60.0 ? 0.5 * (mb - 60.0) : 0.0) : 0.0);
     if (c < cost * (s > 1 ? 0.97 : 1.0)) {
       cost = c;
       best = s;

@@ -114,6 +114,7 @@ def test_row_splits_rule(ext):
     assert ext.gemm_row_splits(333, 3584, 18944) >= 2  # 28 tiles for 74 pairs
     assert ext.gemm_row_splits(333, 37888, 3584) == 1 and ext.gemm_row_splits(8192, 3584, 18944) == 1
     assert ext.gemm_row_splits(1000, 256, 1024) == 1  # a second kernel costs more than it saves
+    assert ext.gemm_row_splits(2200, 3072, 12288) == 1 and ext.gemm_row_splits(2600, 3584, 18944) == 1  # slabs beyond L2
     # just above one lap of the pairs: 75 and 84 tiles, 80 tiles of a very long reduction
     assert min(ext.gemm_row_splits(*t) for t in [(1280, 3840, 18944), (1285, 3584, 18944), (1000, 5120, 27648)]) >= 2
     for rows, n, k in [(129, 256, 64), (129, 256, 128), (300, 512, 200), (2000, 3584, 18944)]:

@@ -504,8 +504,8 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
   return out;
 }
 
-// GPTQ-v1 int4 linear.  Groups of 128 and 5..128 rows: int8 digits of the activations on the tensor cores
-// (qlin_kernels.cu); else the GEMV up to 16 rows; else widen the weight and use the bf16 GEMM.
+// GPTQ-v1 int4 linear.  Groups of 128: up to 16 rows expanded in registers for mma.sync (w4a16_kernels.cu), up to 128 rows
+// int8 digits of the activations (qlin_kernels.cu); else the GEMV up to 16 rows; else widen the weight and use the bf16 GEMM.
 // silu_mul: SiLU(gate) * up over interleaved (gate, up) columns.  want_slabs: see qlin_product.
 at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at::Tensor& scales,
                         const at::Tensor& qzeros, int group, int splits, bool silu_mul, bool want_slabs) {
@@ -529,12 +529,34 @@ at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at
   if (m == 0) return at::empty({0, silu_mul ? n / 2 : n}, x.options());
   W8Scratch& s = w8_scratch(dev);
   const bool aligned = ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(qweight.data_ptr())) & 15u) == 0;
-  // The tensor cores cost the same for 1 to 16 rows, the GEMV two rows' worth of time more for every doubling:
-  // 37888 x 3584, us: GEMV 28 / 50 / 86 / 88 / 176 at 1 / 4 / 5 / 8 / 16 rows, digits 39 throughout;
-  // 3584 x 18944: GEMV 22 / 31 / 56 / 57 / 91, digits 31 - 34.  Above 16 rows the other way is to widen the weight for
-  // a bf16 product: 64 rows, 296 and 143 us there against 70 and 45; faster only for small weights (2048 x 2048
-  // 10 against 17), whose values it rounds to bf16.
-  if (group == 128 && m > 4 && m <= BL_QLIN_MAX_TOKENS && k <= 32768 && n % 8 == 0 && aligned) {
+  // (37888 x 3584, us: GEMV 28 / 51 / 176 at 1 / 4 / 16 rows, digits 39 to 40, this 19.7 / 19.7 / 28)
+  if (group == 128 && m <= 16 && n % 8 == 0 && aligned && (reinterpret_cast<uintptr_t>(scales.data_ptr()) & 7u) == 0) {
+    py::gil_scoped_release nogil;
+    const int s4 = bl_w4a16_mma_splits(m, n, k, splits, want_slabs ? 1 : 0);
+    const int n_out = silu_mul ? n / 2 : n;
+    at::Tensor out, slabs;
+    if (s4 > 1) slabs = at::empty({s4, m, n}, x.options().dtype(at::kFloat));
+    else out = at::empty({m, n_out}, x.options());
+    BL_CHECK(bl_w4a16_mma(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(),
+                          s4 > 1 ? nullptr : out.data_ptr(), m, n, k, s4 > 1 ? 0 : silu_mul, s4,
+                          s4 > 1 ? slabs.data_ptr() : nullptr, st, err, errlen));
+    if (s4 == 1) return out;
+    if (want_slabs) return slabs;
+    out = at::empty({m, n_out}, x.options());
+    blSlabFinishArgs f;
+    memset(&f, 0, sizeof(f));
+    f.slabs = slabs.data_ptr();
+    f.nsplit = s4; f.m = m; f.n = f.pitch = n;
+    f.silu_mul = silu_mul ? 1 : 0;
+    f.out = out.data_ptr();
+    f.ldo = n_out;
+    BL_CHECK(bl_slab_finish(&f, st, err, errlen));
+    return out;
+  }
+  // Above 16 rows the digit kernel; the other way is to widen the weight for a bf16 product: 64 rows, 296 and 143 us
+  // (37888 x 3584, 3584 x 18944) against 70 and 45; faster only for small weights (2048 x 2048 10 against 17), whose
+  // values it rounds to bf16.
+  if (group == 128 && m <= BL_QLIN_MAX_TOKENS && k <= 32768 && n % 8 == 0 && aligned) {
     QWeight q{qweight.data_ptr(), 2, n, k, BL_QSCALE_F16_GN, scales.data_ptr()};
     q.group_k = group;
     q.zeros = qzeros.data_ptr();

@@ -151,8 +151,8 @@ def rope(x, positions, theta, axes=1):
 
 def w4a16_linear(x, qweight, scales, qzeros, group_size=128, silu_mul=False):
     """Weight-only int4 linear on GPTQ-v1 tensors (see `ref.pack_int4`), optionally with SiLU(gate) * up
-    over interleaved (gate, up) columns.  Groups of 128 and 5..128 rows: the digit kernel; else a GEMV up
-    to 16 rows; else widen + GEMM."""
+    over interleaved (gate, up) columns.  Groups of 128: mma.sync up to 16 rows, the digit kernel up to 128;
+    else a GEMV up to 16 rows; else widen + GEMM."""
     if x.is_cuda:
         _count(2)
         x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])

@@ -55,3 +55,31 @@ def test_w4a16_prefill_path_and_dequant(ext):
     x = torch.randn(100, k, generator=g).bfloat16()
     got = ops.w4a16_linear(x.cuda(), qw.cuda(), sc.cuda(), qz.cuda()).cpu()
     assert rel_l2(got, ops.ref.w4a16_linear(x, qw, sc, qz)) < 1e-2
+
+
+@pytest.mark.parametrize("k,n", [(128, 8), (384, 40), (256, 4104), (18944, 72), (1152, 37888)])
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+def test_w4a16_groups_of_128(ext, k, n, m):
+    """Edges of the strips of 32 outputs, of the warps' shares of the groups and of eights of tokens."""
+    from barlink_sm86_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(k + n + m)
+    qw = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8, n), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    qz = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 128, n // 8), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    sc = (torch.rand(k // 128, n, generator=g, device="cuda") * 0.01 + 1e-3).half()
+    x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+    sh = 4 * torch.arange(8, device="cuda")
+    w = ((qw[:, None, :] >> sh[None, :, None]) & 15).reshape(k, n)
+    z = ((qz[:, :, None] >> sh) & 15).reshape(k // 128, n)
+    wd = (w - z.repeat_interleave(128, 0)).double() * sc.double().repeat_interleave(128, 0)
+    want = x.double() @ wd
+    # one rounding to bf16, half of a unit of 2^-7 at most, on fp32 sums of a few thousand products
+    tol, tol32 = 2.0 ** -8 + 1e-5, 1e-5
+    assert rel_l2(ops.w4a16_linear(x, qw, sc, qz), want) < tol
+    out = ops.w4a16_linear_split(x, qw, sc, qz)
+    assert rel_l2(out.double().sum(0), want) < tol32 if out.dim() == 3 else rel_l2(out, want) < tol
+    assert rel_l2(ext.w4a16_linear(x, qw, sc, qz, 128, 3), want) < tol
+    if n % 16 == 0:
+        silu = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+        # (SiLU * up of fp32 sums; __expf and the division are good to some 1e-6)
+        for splits in (0, 1):
+            assert rel_l2(ext.w4a16_linear(x, qw, sc, qz, 128, splits, True), silu) < tol + 1e-5

@@ -609,16 +609,28 @@ __device__ __forceinline__ uint32_t bf16x2_absmax_bits(uint32_t m, uint32_t v) {
   m = max(m, v & 0x7fffu);
   return max(m, (v >> 16) & 0x7fffu);
 }
-template <bool PERMUTE, int VPT>
-__global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k,
-                                                              int tb, int8_t* __restrict__ xq,
-                                                              float* __restrict__ xs) {
+template <bool PERMUTE, int VPT, int CL>
+__device__ __forceinline__ void quant_digits_body(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb,
+                                                  int8_t* __restrict__ xq, float* __restrict__ xs) {
   pdl_launch_dependents();
+  if constexpr (CL > 1) cluster_sync_all();  // the other blocks' shared memory is there
   pdl_wait();
   // (little shared memory: a block of this kernel fits beside one of k_qlin, which has nearly all of it)
   __shared__ uint32_t s_red[kDigThreads / 32];
-  const int row = blockIdx.x, vecs = k >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx);
+  __shared__ uint32_t s_clu[2][CL];  // the words of a row's blocks, two sets in turn
+  const int row = blockIdx.x / CL, rows = gridDim.x / CL, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t part = CL > 1 ? cluster_ctarank() : 0;
+  // this block's share of the row: whole chunks of 256 elements
+  const int per = CL > 1 ? ((k / 8 + CL * 32 - 1) / (CL * 32)) * 32 : k >> 3;
+  const int first = int(part) * per, vecs = max(0, min(per, (k >> 3) - first));
+  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx) + first;
+  int turn = 0;
+  // every block of the row gives a word, every thread of them finds all in s_clu[turn ^ 1]
+  auto share = [&](uint32_t v) {
+    if (threadIdx.x < CL) st_cluster_u32(map_to_cta(smem_u32(&s_clu[turn][part]), threadIdx.x), v);
+    cluster_sync_all();
+    turn ^= 1;
+  };
   uint4 v[VPT];
   uint32_t mx = 0;  // largest |x| as bf16 bits: ordered like the values, NaN above infinity
 #pragma unroll
@@ -632,6 +644,11 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
   if (lane == 0) s_red[warp] = mx;
   __syncthreads();
   mx = __reduce_max_sync(0xffffffffu, s_red[lane & (kDigThreads / 32 - 1)]);
+  if constexpr (CL > 1) {
+    share(mx);
+#pragma unroll
+    for (int c = 0; c < CL; ++c) mx = max(mx, s_clu[turn ^ 1][c]);
+  }
   // nonzero elements below 2^(e - 127) and, in the upper half of the word, nonzero ones in all (each fits 16 bits)
   auto count = [&](int e) -> uint32_t {
     const uint32_t top = e > 0 ? uint32_t(e) << 7 : 1u;
@@ -649,7 +666,14 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
     __syncthreads();
     if (lane == 0) s_red[warp] = n;
     __syncthreads();
-    return __reduce_add_sync(0xffffffffu, lane < kDigThreads / 32 ? s_red[lane] : 0u);
+    n = __reduce_add_sync(0xffffffffu, lane < kDigThreads / 32 ? s_red[lane] : 0u);
+    if constexpr (CL > 1) {
+      share(n);
+      n = 0;
+#pragma unroll
+      for (int c = 0; c < CL; ++c) n += s_clu[turn ^ 1][c];
+    }
+    return n;
   };
   // |x| < 2^ex; a largest element of 255/256 * 2^ex would round up to 128 in the first digit
   int ex = int(mx >> 7) - 126 + ((mx & 0x7fu) == 0x7fu ? 1 : 0);
@@ -676,7 +700,7 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
   const uint32_t limit = digit_limit(ex);
   if (split) {
     // a warp's 32 vectors are one chunk
-    uint8_t* marks = reinterpret_cast<uint8_t*>(xs + gridDim.x) + size_t(row) * kDigChunks;
+    uint8_t* marks = reinterpret_cast<uint8_t*>(xs + rows) + size_t(row) * kDigChunks + first / 32;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
@@ -684,13 +708,14 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
 #pragma unroll
       for (int j = 0; j < 8; ++j) hit |= ((w[j >> 1] >> (16 * (j & 1))) & 0x7fffu) >= limit;
       hit = __any_sync(0xffffffffu, hit);
-      if (lane == 0) marks[i * (kDigThreads / 32) + warp] = hit ? 1 : 0;
+      const int chunk = i * (kDigThreads / 32) + warp;
+      if (lane == 0 && (CL == 1 || chunk * 32 < per)) marks[chunk] = hit ? 1 : 0;
     }
   }
   const float scale = bad ? 0.f : __uint_as_float(uint32_t(127 + 7 - ex) << 23);
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0 && part == 0)
     xs[row] = bad ? __uint_as_float(0x7fffffffu) : __uint_as_float(uint32_t(127 - 7 + ex) << 23 | (split ? 1u << 31 : 0u));
-  int8_t* base = xq + (size_t(row / tb) * 3 * tb + row % tb) * size_t(k);
+  int8_t* base = xq + (size_t(row / tb) * 3 * tb + row % tb) * size_t(k) + size_t(first) * 8;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * kDigThreads;
@@ -717,6 +742,22 @@ __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bflo
     for (int d = 0; d < 3; ++d)
       *reinterpret_cast<uint2*>(base + size_t(d) * tb * k + size_t(c) * 8) = make_uint2(o[d][0], o[d][1]);
   }
+}
+
+template <bool PERMUTE, int VPT>
+__global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb,
+                                                              int8_t* __restrict__ xq, float* __restrict__ xs) {
+  quant_digits_body<PERMUTE, VPT, 1>(x, ldx, k, tb, xq, xs);
+}
+// A long row of few tokens takes one block a chain of loads, counts and conversions over eight vectors a thread (16 x 27648:
+// 10 us between the linears around it, 5.0 now): a cluster of blocks shares it, one vector a thread, the row's maximum
+// and counts passed through distributed shared memory.
+template <bool PERMUTE, int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDigThreads, 2)
+    k_quant_digits_cluster(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb, int8_t* __restrict__ xq,
+                           float* __restrict__ xs) {
+  quant_digits_body<PERMUTE, 1, CL>(x, ldx, k, tb, xq, xs);
+  cluster_sync_all();  // no block leaves while another may still write its words
 }
 
 // fp32 slabs [split][m][pitch] -> bf16 [m][n]: sum in split order, then what the epilogue of the unsplit product
@@ -908,8 +949,8 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
             8 * kDigVec * kDigThreads);
     return -1;
   }
-  auto go = [&](auto kern) {
-    return launch_k(kern, dim3(m), dim3(kDigThreads), 0, static_cast<cudaStream_t>(stream),
+  auto go = [&](auto kern, int blocks = 1) {
+    return launch_k(kern, dim3(m * blocks), dim3(kDigThreads), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const __nv_bfloat16*>(x), ldx, k, bl_qlin_tile_tokens(m), static_cast<int8_t*>(xq),
                     static_cast<float*>(xs));
   };
@@ -917,7 +958,12 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
   // kernel this short comes from L2 or beyond on every launch)
   const int vpt = (k / 8 + kDigThreads - 1) / kDigThreads;
   cudaError_t e;
-  if (vpt <= 1) e = permute ? go(k_quant_digits<true, 1>) : go(k_quant_digits<false, 1>);
+  // a cluster for a row of more than 8192 elements, as long as all blocks are resident at once (a cluster of two for 5120
+  // elements took 3.9 us between the linears around it, one block with two vectors a thread 3.2)
+  if (vpt > 2 && m * (vpt <= 4 ? 4 : 8) <= 2 * sm_count()) {
+    if (vpt <= 4) e = permute ? go(k_quant_digits_cluster<true, 4>, 4) : go(k_quant_digits_cluster<false, 4>, 4);
+    else e = permute ? go(k_quant_digits_cluster<true, 8>, 8) : go(k_quant_digits_cluster<false, 8>, 8);
+  } else if (vpt <= 1) e = permute ? go(k_quant_digits<true, 1>) : go(k_quant_digits<false, 1>);
   else if (vpt <= 2) e = permute ? go(k_quant_digits<true, 2>) : go(k_quant_digits<false, 2>);
   else if (vpt <= 5) e = permute ? go(k_quant_digits<true, 5>) : go(k_quant_digits<false, 5>);
   else e = permute ? go(k_quant_digits<true, kDigVec>) : go(k_quant_digits<false, kDigVec>);

@@ -396,3 +396,32 @@ def test_weights_written_by_the_kernel_ahead(ext, form):
         torch.cuda.synchronize()
         ext.linear(b, a, out=buf)
         assert torch.equal(product(), want)
+
+
+@pytest.mark.parametrize("k", [8208, 16384, 18944, 32768])
+def test_long_rows_shared_by_blocks(ext, k):
+    """Rows whose digits a cluster of blocks writes (few tokens) and one block does (38 tokens): the same results, outliers
+    at the ends of the blocks' shares included."""
+    n = 160
+    wq, sc = _w8(n, k, 3)
+    x = _x(38, k, 5)
+    for p in (0, k // 8, k // 4 - 1, k // 4, k // 2 - 1, k // 2, k - 1):
+        x[3, p] = 2.0 ** 14
+    want = x.double() @ (wq.double() * sc.double()[:, None]).t()
+    y = {m: ext.w8a16_linear(x[:m].contiguous(), wq, sc, splits=1) for m in (33, 37, 38)}
+    for m in y:
+        assert rel_l2(y[m], want[:m]) < TOL
+        assert torch.equal(y[m], y[38][:m])
+
+
+@pytest.mark.parametrize("k", [8, 4096, 4104, 8192, 8200, 18944, 32768, 32776])
+@pytest.mark.parametrize("m", [1, 37, 300])
+def test_quant_act_is_the_stated_arithmetic(ext, m, k):
+    """xs = max |x| / 127 and xq = x / xs to the nearest whole number, whichever kernel a row length goes to."""
+    x = _x(m, k, 7) * 3
+    x[0, k - 1] = 77
+    xq, xs = ext.w8a16_quant_act(x)
+    amax = x.float().abs().amax(1)
+    s = (amax / torch.full_like(amax, 127)).clamp_min(1e-12)  # (a division by a Python number multiplies by 1 / 127)
+    assert torch.equal(xs, s)
+    assert torch.equal(xq, torch.round(x.float() * (1.0 / s)[:, None]).clamp(-127, 127).to(torch.int8))

@@ -9,26 +9,25 @@
 // One CTA owns 256 query rows of one head as two 128-row tiles and walks the
 // keys in tiles of 64:
 //
-//   warp 0      TMA producer: Q once, then a ring of K tiles and a ring of V^T tiles
+//   warp 0      TMA producer: Q once, then a ring of K tiles and a ring of V tiles
 //   warp 1      issues tcgen05.mma: S_t = Q_t K^T into TMEM (128x64 fp32, two buffers per tile),
 //               O_t += P_t V into TMEM (128x128 fp32), for tiles t = 0, 1 in turn
 //   warps 2-5   softmax of tile 0: every thread owns one query row (TMEM lane),
 //   warps 6-9   softmax of tile 1   reads its 64 scores with tcgen05.ld, keeps the
-//               running max and sum in registers, writes P (bf16) into shared
-//               memory in the swizzled K-major layout the tensor core reads
+//               running max and sum in registers, writes P (bf16) over
+//               them in TMEM, from where it is the A operand of P V
 //
 // What bounds it: the exponentials (16 a clock and SM: 1024 cycles for 64 keys x 256 rows, as many as the
 // products take) and, before S had two buffers, the chain softmax -> P V -> next S -> softmax of a tile, whose
 // links added up to 2700 cycles a step.  Now S of step j + 2 is issued right behind P V of step j, so a
 // tile's softmax always finds its scores; P has two buffers for the same reason, and a rescale of O waits
 // for the P V before it.  24 heads x 4608 tokens with the transpose: 319 -> 297 us (879 TFLOP/s), 8 x 1024
-// causal, 28 heads on 4: 152 -> 141 us; 2550 cycles a step are left, 24 products and 6 commits of the one
-// issuing warp among them.
+// causal, 28 heads on 4: 152 -> 141 us; 2550 cycles a step are left.  P through shared memory and V through a kernel
+// that transposed it (22 us at 24 x 4608, 12 us at 8 x 1024 x 4) gave the same step time, so the tiles in shared
+// memory do not bound it; without them the 4096-token MMDiT forward takes 71.5 ms instead of 73.4.
 // The accumulator is rescaled only when the running max has grown by more than
 // 2^8 since the last rescale (the stale max is exact after the final division
 // by the row sum), which takes the TMEM read-modify-write out of the loop.
-// V is consumed as V^T [head_dim][keys] so that both operands of P V are
-// K-major; a small kernel transposes V into a scratch buffer first.
 //
 // Every wait is bounded; a wait that runs out sets the CTA's abort word, all
 // roles leave their loops, TMEM is freed and the error flag is raised.
@@ -46,19 +45,17 @@ constexpr int kTcBM = 128;       // query rows per tile
 constexpr int kTcTiles = 2;      // tiles per CTA
 constexpr int kTcBKV = 64;       // keys per step
 constexpr int kTcHD = 128;
-constexpr int kTcStages = 3;     // K tiles and V^T tiles in flight, a ring each
+constexpr int kTcStages = 4;     // K tiles and V tiles in flight, a ring each
 constexpr int kTcThreads = 320;
 constexpr uint32_t kTcQBytes = kTcBM * kTcHD * 2;          // 32 KiB per query tile
-constexpr uint32_t kTcPBytes = kTcBM * kTcBKV * 2;         // 16 KiB per P tile
 constexpr uint32_t kTcKBytes = kTcBKV * kTcHD * 2;         // 16 KiB
 constexpr uint32_t kTcVBytes = kTcHD * kTcBKV * 2;         // 16 KiB
-constexpr uint32_t kTcOffP = kTcTiles * kTcQBytes;         // [tile][even / odd step]
-constexpr uint32_t kTcOffK = kTcOffP + 2 * kTcTiles * kTcPBytes;
+constexpr uint32_t kTcOffK = kTcTiles * kTcQBytes;
 constexpr uint32_t kTcOffV = kTcOffK + kTcStages * kTcKBytes;
 constexpr uint32_t kTcOffBar = kTcOffV + kTcStages * kTcVBytes;
 constexpr uint32_t kTcSmem = kTcOffBar + 256 + 1024;       // barriers + alignment slack
 static_assert(kTcSmem <= 232448, "attention tiles do not fit the shared memory of one CTA");
-constexpr uint32_t kTcTmemCols = 512;                      // S of tile t, step parity p: 128 t + 64 p; O of tile t: 256 + 128 t
+constexpr uint32_t kTcTmemCols = 512;                      // S of tile t, step parity p: 128 t + 64 p, P in its first half; O of tile t: 256 + 128 t
 constexpr float kTcRescale = 8.f;                          // log2 units
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -97,60 +94,52 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   return r;
 }
 
-// V [tokens, nkv, 128] (token stride v_stride) -> vt [nkv*128][batch*lpad]:
-// sequence b's keys sit at columns b*lpad .. b*lpad+len; the pad is zeroed.
-__global__ void __launch_bounds__(256) k_transpose_v(const __nv_bfloat16* __restrict__ v,
-                                                     __nv_bfloat16* __restrict__ vt,
-                                                     const int* __restrict__ cu_k, int v_stride,
-                                                     int lpad, size_t vt_pitch) {
-  pdl_launch_dependents();
-  pdl_wait();
-  __shared__ __nv_bfloat16 tile[64][kTcHD + 8];
-  const int b = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * 64;
-  const int k0 = cu_k[b], len = cu_k[b + 1] - k0;
-  // 64 tokens x 128 dims: 16 threads per token row, 8 elements each
-  for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-    const int r = i >> 4, c = (i & 15) * 8;
-    uint4 val = make_uint4(0, 0, 0, 0);
-    if (t0 + r < len) val = *reinterpret_cast<const uint4*>(v + size_t(k0 + t0 + r) * v_stride + h * kTcHD + c);
-    *reinterpret_cast<uint4*>(&tile[r][c]) = val;
-  }
-  __syncthreads();
-  // 128 dims x 64 tokens out: a warp owns 16 dims and writes whole 32-byte sectors (two lanes side by side);
-  // its shared-memory reads conflict two-fold (eight lanes per dim row read one bank eight-fold: 4608 tokens
-  // of 24 heads took 25 us)
-  const int d = (threadIdx.x >> 5) * 16 + (threadIdx.x & 15), half = (threadIdx.x >> 4) & 1;
-#pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int c = it * 16 + half * 8;
-    __align__(16) __nv_bfloat16 o[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = tile[c + j][d];
-    *reinterpret_cast<uint4*>(vt + size_t(h * kTcHD + d) * vt_pitch + size_t(b) * lpad + t0 + c) =
-        *reinterpret_cast<const uint4*>(o);
-  }
+// B operand of P V as V lies in memory: [key][64 columns of the head], 128-byte rows in the 128-byte swizzle, so the
+// columns (N) are contiguous: eight keys are 1024 bytes (stride byte offset), the other 64 columns half a tile on
+// (leading byte offset); 16 keys of a product are 2048 bytes.
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t half_bytes) {
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4);
+  d |= static_cast<uint64_t>(half_bytes >> 4) << 16;
+  d |= static_cast<uint64_t>(1024 >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(2) << 61;
+  return d;
+}
+constexpr uint32_t kUmmaBMajorN = 1u << 16;  // instruction descriptor: B is N-major
+// A from TMEM: a lane a row, a 32-bit column two neighbours along K
+__device__ __forceinline__ void umma_f16_ts_warp(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                                 uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
+      : "memory");
 }
 
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_attn_tc(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-              const __grid_constant__ CUtensorMap tmap_vt, __nv_bfloat16* __restrict__ out,
+              const __grid_constant__ CUtensorMap tmap_v, __nv_bfloat16* __restrict__ out,
               const int* __restrict__ cu_q, const int* __restrict__ cu_k, int nq, int nkv, int o_stride,
-              int lpad, float scale_log2, int causal, uint32_t* __restrict__ err) {
+              float scale_log2, int causal, uint32_t* __restrict__ err) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
   uint64_t* bars = reinterpret_cast<uint64_t*>(gen + kTcOffBar);
   uint64_t* q_full = bars;             // 1
   uint64_t* k_full = bars + 1;         // kTcStages each
-  uint64_t* k_empty = bars + 4;
-  uint64_t* v_full = bars + 7;
-  uint64_t* v_empty = bars + 10;
-  uint64_t* s_ready = bars + 13;       // [tile][step parity]
-  uint64_t* p_ready = bars + 17;       // [tile][step parity]
-  uint64_t* pv_done = bars + 21;       // [tile], one phase per step
-  uint64_t* o_final = bars + 26;       // [tile]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
-  volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(bars + 25);
+  uint64_t* k_empty = k_full + kTcStages;
+  uint64_t* v_full = k_empty + kTcStages;
+  uint64_t* v_empty = v_full + kTcStages;
+  uint64_t* s_ready = v_empty + kTcStages;  // [tile][step parity]
+  uint64_t* p_ready = s_ready + 4;     // [tile][step parity]
+  uint64_t* pv_done = p_ready + 4;     // [tile], one phase per step
+  uint64_t* o_final = pv_done + 2;     // [tile]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_final + 2);
+  volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(o_final + 3);
+  static_assert((1 + 4 * kTcStages + 14) * 8 <= 256, "barriers");
 
   // cu_q / cu_k may come from the kernel just before this one
   pdl_launch_dependents();
@@ -189,7 +178,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
-    tma_prefetch_desc(&tmap_vt);
+    tma_prefetch_desc(&tmap_v);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTcTmemCols);
@@ -220,8 +209,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         ++k_issued;
         if (!mbar_wait_bounded(&v_empty[stage], phase ^ 1u, s_abort)) break;
         mbar_expect_tx(&v_full[stage], kTcVBytes);
-        tma_load_2d_hint_s(base + kTcOffV + stage * kTcVBytes, &tmap_vt, smem_u32(&v_full[stage]), b * lpad + j * kTcBKV,
-                           kvh * kTcHD, kHintEvictLast);
+        for (int h = 0; h < 2; ++h)
+          tma_load_2d_hint_s(base + kTcOffV + stage * kTcVBytes + h * (kTcVBytes / 2), &tmap_v, smem_u32(&v_full[stage]),
+                             kvh * kTcHD + h * 64, k0 + j * kTcBKV, kHintEvictLast);
         ++v_issued;
         if (++stage == kTcStages) {
           stage = 0;
@@ -246,7 +236,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (n_steps > 0) {
       const uint32_t leader = elect_leader();
       const uint32_t idesc_s = umma_idesc_f16(kTcBM, kTcBKV, 1);
-      const uint32_t idesc_o = umma_idesc_f16(kTcBM, kTcHD, 1);
+      const uint32_t idesc_o = umma_idesc_f16(kTcBM, kTcHD, 1) | kUmmaBMajorN;
       // S of a step with parity p, from K stage ks0
       auto issue_s = [&](int t, int p, int kst) {
         const uint64_t dq = umma_desc_k_sw128(base + t * kTcQBytes), dk = umma_desc_k_sw128(base + kTcOffK + kst * kTcKBytes);
@@ -258,12 +248,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         umma_commit_warp(leader, &s_ready[2 * t + p]);
       };
       auto issue_pv = [&](int t, int p, int vst, bool acc) {
-        const uint64_t dp = umma_desc_k_sw128(base + kTcOffP + (2 * t + p) * kTcPBytes);
-        const uint64_t dv = umma_desc_k_sw128(base + kTcOffV + vst * kTcVBytes);
+        const uint64_t dv = umma_desc_mn_sw128(base + kTcOffV + vst * kTcVBytes, kTcVBytes / 2);
 #pragma unroll
         for (int ks = 0; ks < kTcBKV / 16; ++ks)
-          umma_f16_ss_warp(leader, tmem_base + 256u + uint32_t(t * kTcHD), dp + uint64_t(2 * ks), dv + uint64_t(2 * ks),
-                           idesc_o, (acc || ks > 0) ? 1u : 0u);
+          umma_f16_ts_warp(leader, tmem_base + 256u + uint32_t(t * kTcHD), tmem_base + uint32_t(t * 128 + p * kTcBKV + 8 * ks),
+                           dv + uint64_t(128 * ks), idesc_o, (acc || ks > 0) ? 1u : 0u);
         umma_commit_warp(leader, &pv_done[t]);
       };
       bool ok = mbar_wait_bounded_warp(q_full, 0, s_abort);
@@ -292,6 +281,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           }
           ok = __all_sync(0xffffffffu, here);
           if (!ok) break;
+          if (t == 0 && (j + 1) * kTcBKV > lk) {
+            // rows beyond the sequence are another's: their probabilities are zero, their values may be infinite
+            for (int i = lane + (lk - j * kTcBKV) * 16; i < kTcBKV * 16; i += 32)
+              asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(base + kTcOffV + vst * kTcVBytes +
+                                                                        ((i >> 3) & 1) * (kTcVBytes / 2) + (i >> 4) * 128 + (i & 7) * 16),
+                           "r"(0)
+                           : "memory");
+            fence_proxy_async_smem();
+            __syncwarp();
+          }
           tc_fence_after_sync();
           issue_pv(t, p, vst, j > 0);
           if (more) issue_s(t, p, kst);
@@ -322,7 +321,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t lane_addr = tmem_base + (uint32_t(quarter * 32) << 16);
     const uint32_t s_tile = lane_addr + uint32_t(t * 128);
     const uint32_t o_addr = lane_addr + 256u + uint32_t(t * kTcHD);
-    const uint32_t p_tile = base + kTcOffP + 2 * t * kTcPBytes + row * 128;
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_steps; ++j) {
@@ -332,7 +330,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         break;
       }
       tc_fence_after_sync();
-      const uint32_t s_addr = s_tile + uint32_t(p * kTcBKV), p_row = p_tile + p * kTcPBytes;
+      const uint32_t s_addr = s_tile + uint32_t(p * kTcBKV);
       float s[kTcBKV];
       {
         uint32_t r0[32], r1[32];
@@ -404,12 +402,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       sum[0] = add2(sum[0], sum[1]);
       l += sum[0].x + sum[0].y;
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(p_row + ((c ^ (row & 7)) << 4)),
-                     "r"(pk[4 * c]), "r"(pk[4 * c + 1]), "r"(pk[4 * c + 2]), "r"(pk[4 * c + 3])
-                     : "memory");
-      fence_proxy_async_smem();
+      tmem_st_32x32(s_addr, pk);  // over the scores that it was made of
+      tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&p_ready[2 * t + p]);
     }
@@ -454,17 +448,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 using namespace bl;
 
-extern "C" size_t bl_attn_tc_scratch_bytes(int batch, int max_k, int nkv) {
-  const size_t lpad = size_t((max_k + kTcBKV - 1) / kTcBKV) * kTcBKV;
-  return size_t(nkv) * kTcHD * lpad * size_t(batch) * 2;
-}
-
-// Tensor-core dense attention.  `vt` is scratch of bl_attn_tc_scratch_bytes();
-// `total_q` / `total_k` are the row counts of q and k (cu_q[batch], cu_k[batch]).
+// Tensor-core dense attention.  `total_q` / `total_k` are the row counts of q and k (cu_q[batch], cu_k[batch]).
 extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void* out, const int* cu_q,
                               const int* cu_k, int batch, int max_q, int max_k, int total_q, int total_k,
                               int nq, int nkv, int hd, int q_stride, int k_stride, int v_stride,
-                              int o_stride, float scale, int causal, void* vt, void* err_flag, void* stream,
+                              int o_stride, float scale, int causal, void* err_flag, void* stream,
                               char* err, size_t errlen) {
   if (hd != kTcHD || nkv < 1 || nq % nkv) {
     set_err(err, errlen, "barlink: tensor-core attention is built for head_dim %d and nq %% nkv == 0", kTcHD);
@@ -476,14 +464,10 @@ extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void*
   }
   if (batch < 1 || max_q < 1 || max_k < 1) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int lpad = (max_k + kTcBKV - 1) / kTcBKV * kTcBKV;
-  const size_t pitch = size_t(lpad) * batch;
-  launch_k(k_transpose_v, dim3(lpad / 64, nkv, batch), dim3(256), 0, st,
-           static_cast<const __nv_bfloat16*>(v), static_cast<__nv_bfloat16*>(vt), cu_k, v_stride, lpad, pitch);
   CUtensorMap tq, tk, tv;
   if (make_tmap_kmajor(q, uint64_t(total_q), uint64_t(nq) * kTcHD, uint64_t(q_stride), kTcBM, 2, &tq, err, errlen) ||
       make_tmap_kmajor(k, uint64_t(total_k), uint64_t(nkv) * kTcHD, uint64_t(k_stride), kTcBKV, 2, &tk, err, errlen) ||
-      make_tmap_kmajor(vt, uint64_t(nkv) * kTcHD, pitch, pitch, kTcHD, 2, &tv, err, errlen))
+      make_tmap_kmajor(v, uint64_t(total_k), uint64_t(nkv) * kTcHD, uint64_t(v_stride), kTcBKV, 2, &tv, err, errlen))
     return -1;
   static bool attr = false;
   if (!attr) {
@@ -496,7 +480,7 @@ extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void*
   }
   dim3 grid((max_q + kTcTiles * kTcBM - 1) / (kTcTiles * kTcBM), nq, batch);
   cudaError_t e = launch_k(k_attn_tc, grid, dim3(kTcThreads), kTcSmem, st, tq, tk, tv,
-                           static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq, nkv, o_stride, lpad,
+                           static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq, nkv, o_stride,
                            scale * 1.4426950408889634f, causal, static_cast<uint32_t*>(err_flag));
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {

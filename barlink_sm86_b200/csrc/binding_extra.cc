@@ -145,11 +145,10 @@ at::Tensor attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& 
     return !(e && e[0] == '0');
   }();
   if (q.size(0) > 0 && tc_on && max_k > 0 && hd == 128) {
-    at::Tensor vt = at::empty({int64_t(bl_attn_tc_scratch_bytes(batch, max_k, nkv) / 2)}, q.options());
     BL_CHECK(bl_attn_fwd_tc(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_q.data_ptr<int>(),
                             cu_k.data_ptr<int>(), batch, max_q, max_k, int(q.size(0)), int(k.size(0)), nq, nkv,
                             hd, int(q.stride(0)), int(k.stride(0)), int(v.stride(0)), nq * hd, float(scale),
-                            causal ? 1 : 0, vt.data_ptr(), attn_err(q.device().index()).data_ptr(), st, err,
+                            causal ? 1 : 0, attn_err(q.device().index()).data_ptr(), st, err,
                             errlen));
     return out;
   }

@@ -246,10 +246,9 @@ def rope_attn_decode(qkv, bias, positions, slots, k_cache, v_cache, block_tables
 
 def attention(q, k, v, cu_q, cu_k, max_q, scale, causal, max_k=0):
     """Dense attention over packed sequences (prefill, joint attention).
-    With max_k (length of the longest key sequence) the tcgen05 kernel runs
-    (V transpose + attention: two launches); without it the mma.sync kernel."""
+    With max_k (length of the longest key sequence) the tcgen05 kernel runs; without it the mma.sync kernel."""
     if q.is_cuda:
-        _count(2 if max_k > 0 else 1)
+        _count()
         return _C().attn_fwd(q, k, v, cu_q, cu_k, max_q, scale, causal, max_k)
     return ref.attention(q, k, v, cu_q, cu_k, scale, causal)
 

@@ -31,3 +31,21 @@ def test_steps(ext, lk, growing, causal):
     want = _want(q, k.expand(-1, nq, -1), v.expand(-1, nq, -1), 128 ** -0.5, causal)
     assert float((got.double() - want).norm() / want.norm()) < 2.0 ** -8
     assert ext.attn_error_flag(0) == 0
+
+
+@pytest.mark.parametrize("l0", [1, 63, 64, 65, 130])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_values_of_the_next_sequence_do_not_leak(ext, l0, bad):
+    """Keys are loaded in tiles of 64, so the last tile of a sequence holds the next one's first rows."""
+    from barlink_sm86_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(l0)
+    l1, nq, nkv = 40, 4, 2
+    q, k, v = (torch.randn(l0 + l1, h, 128, generator=g, device="cuda").bfloat16() for h in (nq, nkv, nkv))
+    v[l0:l0 + 3] = bad
+    cu = torch.tensor([0, l0, l0 + l1], dtype=torch.int32, device="cuda")
+    one = torch.tensor([0, l0], dtype=torch.int32, device="cuda")
+    for causal in (False, True):
+        both = ops.attention(q, k, v, cu, cu, max(l0, l1), 0.088, causal, max_k=max(l0, l1))
+        alone = ops.attention(q[:l0].contiguous(), k[:l0].contiguous(), v[:l0].contiguous(), one, one, l0, 0.088, causal,
+                              max_k=l0)
+        assert torch.equal(both[:l0], alone) and bool(alone.isfinite().all())

@@ -145,10 +145,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.z, head = blockIdx.y, kvh = head / (nq / nkv);
+  // Causal: the later rows have more keys, so their blocks are dealt out first, over all heads and sequences
+  // (8 x 1024, 28 heads on 4: 126.7 -> 123.7 us).
+  const int b = causal ? blockIdx.y : blockIdx.z, head = causal ? blockIdx.x : blockIdx.y, kvh = head / (nq / nkv);
+  const int rblock = causal ? int(gridDim.z - 1 - blockIdx.z) : int(blockIdx.x);
   const int q0 = cu_q[b], lq = cu_q[b + 1] - q0;
   const int k0 = cu_k[b], lk = cu_k[b + 1] - k0;
-  const int row0 = blockIdx.x * (kTcTiles * kTcBM);   // first query row of this CTA in its sequence
+  const int row0 = rblock * (kTcTiles * kTcBM);   // first query row of this CTA in its sequence
   if (row0 >= lq) return;
   const int off = lk - lq;                             // causal: key j visible to query i iff j <= i + off
   int kv_end = lk;
@@ -478,7 +481,9 @@ extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void*
     }
     attr = true;
   }
-  dim3 grid((max_q + kTcTiles * kTcBM - 1) / (kTcTiles * kTcBM), nq, batch);
+  const unsigned rblocks = unsigned((max_q + kTcTiles * kTcBM - 1) / (kTcTiles * kTcBM));
+  // (a grid has at most 65535 blocks along y and z)
+  const dim3 grid = causal ? dim3(nq, batch, rblocks) : dim3(rblocks, nq, batch);
   cudaError_t e = launch_k(k_attn_tc, grid, dim3(kTcThreads), kTcSmem, st, tq, tk, tv,
                            static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq, nkv, o_stride,
                            scale * 1.4426950408889634f, causal, static_cast<uint32_t*>(err_flag));

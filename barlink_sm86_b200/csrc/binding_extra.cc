@@ -205,6 +205,8 @@ struct QWeight {
   const void* row_scale = nullptr;
   int group_k = 0;
   const void* zeros = nullptr;
+  // digits that the norm in front has left (bl_rmsnorm_digits)
+  c10::optional<at::Tensor> xq, xs;
 };
 // a shape that bl_qlin takes and (three digits) bf16 rows that bl_quant_digits can read; per-channel sums are
 // 32-bit over all of K
@@ -270,7 +272,13 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
                     bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
   const int m = int(x.size(0));
   at::Tensor xq, xs;
-  if (digits == 3) {
+  if (digits == 3 && q.xq && q.xs) {
+    TORCH_CHECK(q.src != 2 && q.xq->is_cuda() && q.xq->is_contiguous() && q.xs->is_cuda() && q.xs->is_contiguous() &&
+                    q.xq->nbytes() == bl_quant_digits_bytes(m, q.k) && q.xs->nbytes() == bl_quant_digits_xs_bytes(m),
+                "barlink: digits do not belong to these activations (see rmsnorm_digits)");
+    xq = *q.xq;
+    xs = *q.xs;
+  } else if (digits == 3) {
     xs = at::empty({int64_t(bl_quant_digits_xs_bytes(m) / sizeof(float))}, x.options().dtype(at::kFloat));
     xq = at::empty({int64_t(bl_quant_digits_bytes(m, q.k))}, x.options().dtype(at::kChar));
     BL_CHECK(bl_quant_digits(x.data_ptr(), m, int(x.stride(0)), q.k, q.src == 2 ? 1 : 0, xq.data_ptr(), xs.data_ptr(), st,
@@ -284,10 +292,40 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
   return qlin_product(x, xq, xs, m, digits, q, bias, silu_mul, splits, want_slabs, x.options(), err_flag, st);
 }
 
+// RMSNorm (+ residual, updated in place) of 1..128 decode rows or of the k-split slabs of the linear before, and the digits of
+// the result for the linears behind it: (normed, residual, xq, xs).
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> rmsnorm_digits(const at::Tensor& x, const at::Tensor& gamma, double eps,
+                                                                          const c10::optional<at::Tensor>& residual) {
+  check_bf16x(gamma, "gamma");
+  const bool slabs = x.scalar_type() == at::kFloat;
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && (slabs ? x.dim() == 3 : x.scalar_type() == at::kBFloat16 && x.dim() == 2),
+              "barlink: rmsnorm_digits takes contiguous bfloat16 rows or float32 [splits, rows, hidden] slabs");
+  const int hidden = int(x.size(-1)), rows = int(x.size(-2)), nsplit = slabs ? int(x.size(0)) : 0;
+  TORCH_CHECK(gamma.numel() == hidden && rows >= 1 && rows <= BL_QLIN_MAX_TOKENS && (!slabs || nsplit >= 1),
+              "barlink: gamma must have hidden elements, and rmsnorm_digits takes 1..", std::to_string(BL_QLIN_MAX_TOKENS), " rows");
+  const auto like = x.options().dtype(at::kBFloat16);
+  at::Tensor out = at::empty({rows, hidden}, like), res;
+  if (residual) {
+    check_bf16x(*residual, "residual");
+    TORCH_CHECK(residual->numel() == int64_t(rows) * hidden, "barlink: residual must match x");
+    res = *residual;
+  }
+  at::Tensor xs = at::empty({int64_t(bl_quant_digits_xs_bytes(rows) / sizeof(float))}, like.dtype(at::kFloat));
+  at::Tensor xq = at::empty({int64_t(bl_quant_digits_bytes(rows, hidden))}, like.dtype(at::kChar));
+  c10::cuda::CUDAGuard guard(x.device());
+  void* st = at::cuda::getCurrentCUDAStream(x.device().index()).stream();
+  py::gil_scoped_release nogil;
+  BL_CHECK(bl_rmsnorm_digits(slabs ? nullptr : x.data_ptr(), residual ? res.data_ptr() : nullptr, gamma.data_ptr(), out.data_ptr(),
+                             residual ? res.data_ptr() : nullptr, rows, hidden, float(eps), slabs ? x.data_ptr() : nullptr, nsplit,
+                             size_t(rows) * hidden, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
+  return {out, res, xq, xs};
+}
+
 // Decode form of w8a16_linear without a reduction: fp32 slabs [splits, m, n] (scaled, no bias) for the
 // kernel that reads them next, or the bf16 result when the shape wants no k-split.
 at::Tensor w8a16_linear_split(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& scale,
-                              const c10::optional<at::Tensor>& bias, bool act_int8) {
+                              const c10::optional<at::Tensor>& bias, bool act_int8,
+                              const c10::optional<at::Tensor>& xq, const c10::optional<at::Tensor>& xs) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1,
               "barlink: x must be a 2-D bfloat16 CUDA tensor with unit inner stride");
   TORCH_CHECK(wq.is_cuda() && wq.is_contiguous() && wq.scalar_type() == at::kChar && wq.dim() == 2 &&
@@ -302,13 +340,16 @@ at::Tensor w8a16_linear_split(const at::Tensor& x, const at::Tensor& wq, const a
   void* flag = w8_scratch(dev).err_flag.data_ptr();
   py::gil_scoped_release nogil;
   QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
+  q.xq = xq;
+  q.xs = xs;
   return qlin_run(x, act_int8 ? 1 : 3, q, bias, false, 0, true, flag, at::cuda::getCurrentCUDAStream(dev).stream());
 }
 
 at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Tensor& scale,
                         const c10::optional<at::Tensor>& bias, bool silu_mul, int splits,
                         const c10::optional<at::Tensor>& group_rel, bool act_int8,
-                        const c10::optional<at::Tensor>& group_scale) {
+                        const c10::optional<at::Tensor>& group_scale, const c10::optional<at::Tensor>& xq_in,
+                        const c10::optional<at::Tensor>& xs_in) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1,
               "barlink: x must be a 2-D bfloat16 CUDA tensor with unit inner stride");
   TORCH_CHECK(wq.is_cuda() && wq.is_contiguous() && wq.scalar_type() == at::kChar && wq.dim() == 2 &&
@@ -339,6 +380,8 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   // groups of whole 128-wide k-blocks.
   if (qlin_takes(x, k, act_int8, bool(group_scale)) && (!group_rel || (k / group_rel->size(1)) % 128 == 0)) {
     QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
+    q.xq = xq_in;
+    q.xs = xs_in;
     if (group_scale) {
       q.scale_kind = BL_QSCALE_BF16_NG;
       q.scale = group_scale->data_ptr();
@@ -835,9 +878,11 @@ void bind_extra(py::module_& m) {
         py::arg("rows_per_batch"));
   m.def("w8a16_linear", &w8a16_linear, py::arg("x"), py::arg("wq"), py::arg("scale"),
         py::arg("bias") = py::none(), py::arg("silu_mul") = false, py::arg("splits") = 0,
-        py::arg("group_rel") = py::none(), py::arg("act_int8") = false, py::arg("group_scale") = py::none());
+        py::arg("group_rel") = py::none(), py::arg("act_int8") = false, py::arg("group_scale") = py::none(),
+        py::arg("xq") = py::none(), py::arg("xs") = py::none());
   m.def("w8a16_linear_split", &w8a16_linear_split, py::arg("x"), py::arg("wq"), py::arg("scale"),
-        py::arg("bias") = py::none(), py::arg("act_int8") = false);
+        py::arg("bias") = py::none(), py::arg("act_int8") = false, py::arg("xq") = py::none(), py::arg("xs") = py::none());
+  m.def("rmsnorm_digits", &rmsnorm_digits, py::arg("x"), py::arg("gamma"), py::arg("eps"), py::arg("residual") = py::none());
   m.def("w8_group_scales", &w8_group_scales, py::arg("scales"));
   m.def("w8_error_flag", &w8_error_flag, py::arg("device") = 0);
   m.def("dlin", &dlin, py::arg("x"), py::arg("weight"), py::arg("pro") = "none", py::arg("epi") = "store",

@@ -217,6 +217,11 @@ int bl_qlin_tile_tokens(int m); /* of three digit planes */
  * most 32768. */
 int bl_quant_digits(const void* x, int m, int ldx, int k, int permute, void* xq, void* xs, void* stream, char* err,
                     size_t errlen);
+/* bl_rmsnorm (see there) and bl_quant_digits (permute = 0) of its result in one launch: 1..BL_QLIN_MAX_TOKENS rows of up
+ * to 8192 elements */
+int bl_rmsnorm_digits(const void* x, const void* residual, const void* gamma, void* out, void* residual_out, int rows,
+                      int hidden, float eps, const void* partials, int nsplit, size_t slab, void* xq, void* xs, void* stream,
+                      char* err, size_t errlen);
 size_t bl_quant_digits_bytes(int m, int k);
 size_t bl_quant_digits_xs_bytes(int m);
 /* slabs fp32 [nsplit][m][pitch] -> out bf16 [m][n] (pitch ldo), the sum with the epilogue of a product: + bias,

@@ -609,34 +609,27 @@ __device__ __forceinline__ uint32_t bf16x2_absmax_bits(uint32_t m, uint32_t v) {
   m = max(m, v & 0x7fffu);
   return max(m, (v >> 16) & 0x7fffu);
 }
+// The digits of a row that the blocks of a cluster (CL of them, or one) hold in registers: vector i of a thread is vector
+// threadIdx.x + i * kDigThreads of its block's share, which is `vecs` long and starts at vector `first` of the row; every
+// block but the last has `per` of them.
 template <bool PERMUTE, int VPT, int CL>
-__device__ __forceinline__ void quant_digits_body(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb,
-                                                  int8_t* __restrict__ xq, float* __restrict__ xs) {
-  pdl_launch_dependents();
-  if constexpr (CL > 1) cluster_sync_all();  // the other blocks' shared memory is there
-  pdl_wait();
-  // (little shared memory: a block of this kernel fits beside one of k_qlin, which has nearly all of it)
+__device__ __forceinline__ void digits_of_row(uint4 (&v)[VPT], int row, int rows, int first, int per, int vecs, int k, int tb,
+                                              int8_t* __restrict__ xq, float* __restrict__ xs) {
+  // (little shared memory: a block of these kernels fits beside one of k_qlin, which has nearly all of it)
   __shared__ uint32_t s_red[kDigThreads / 32];
   __shared__ uint32_t s_clu[2][CL];  // the words of a row's blocks, two sets in turn
-  const int row = blockIdx.x / CL, rows = gridDim.x / CL, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t part = CL > 1 ? cluster_ctarank() : 0;
-  // this block's share of the row: whole chunks of 256 elements
-  const int per = CL > 1 ? ((k / 8 + CL * 32 - 1) / (CL * 32)) * 32 : k >> 3;
-  const int first = int(part) * per, vecs = max(0, min(per, (k >> 3) - first));
-  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx) + first;
   int turn = 0;
   // every block of the row gives a word, every thread of them finds all in s_clu[turn ^ 1]
-  auto share = [&](uint32_t v) {
-    if (threadIdx.x < CL) st_cluster_u32(map_to_cta(smem_u32(&s_clu[turn][part]), threadIdx.x), v);
+  auto share = [&](uint32_t w) {
+    if (threadIdx.x < CL) st_cluster_u32(map_to_cta(smem_u32(&s_clu[turn][part]), threadIdx.x), w);
     cluster_sync_all();
     turn ^= 1;
   };
-  uint4 v[VPT];
   uint32_t mx = 0;  // largest |x| as bf16 bits: ordered like the values, NaN above infinity
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
-    const int c = threadIdx.x + i * kDigThreads;
-    v[i] = c < vecs ? xr[c] : make_uint4(0, 0, 0, 0);
     mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].x), v[i].y);
     mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].z), v[i].w);
   }
@@ -744,6 +737,25 @@ __device__ __forceinline__ void quant_digits_body(const __nv_bfloat16* __restric
   }
 }
 
+template <bool PERMUTE, int VPT, int CL>
+__device__ __forceinline__ void quant_digits_body(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb,
+                                                  int8_t* __restrict__ xq, float* __restrict__ xs) {
+  pdl_launch_dependents();
+  if constexpr (CL > 1) cluster_sync_all();  // the other blocks' shared memory is there
+  pdl_wait();
+  const int row = blockIdx.x / CL;
+  // this block's share of the row: whole chunks of 256 elements
+  const int per = CL > 1 ? ((k / 8 + CL * 32 - 1) / (CL * 32)) * 32 : k >> 3;
+  const int first = CL > 1 ? int(cluster_ctarank()) * per : 0, vecs = max(0, min(per, (k >> 3) - first));
+  const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx) + first;
+  uint4 v[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = threadIdx.x + i * kDigThreads;
+    v[i] = c < vecs ? xr[c] : make_uint4(0, 0, 0, 0);
+  }
+  digits_of_row<PERMUTE, VPT, CL>(v, row, gridDim.x / CL, first, per, vecs, k, tb, xq, xs);
+}
 template <bool PERMUTE, int VPT>
 __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb,
                                                               int8_t* __restrict__ xq, float* __restrict__ xs) {
@@ -758,6 +770,106 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kDigThreads, 2)
                            float* __restrict__ xs) {
   quant_digits_body<PERMUTE, 1, CL>(x, ldx, k, tb, xq, xs);
   cluster_sync_all();  // no block leaves while another may still write its words
+}
+
+__device__ __forceinline__ void row_floats(const uint4& a, float (&f)[8]) {
+  const float2 p0 = unpack_bf16x2(a.x), p1 = unpack_bf16x2(a.y), p2 = unpack_bf16x2(a.z), p3 = unpack_bf16x2(a.w);
+  f[0] = p0.x; f[1] = p0.y; f[2] = p1.x; f[3] = p1.y;
+  f[4] = p2.x; f[5] = p2.y; f[6] = p3.x; f[7] = p3.y;
+}
+__device__ __forceinline__ uint4 row_pack(const float (&f)[8]) {
+  return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+}
+
+// RMSNorm (+ residual add) of one row by one block.  v: the normed row on return, vector i of a thread being vector
+// threadIdx.x + i * blockDim.x.  x is the row itself, or (partials) the sum of the k-split slabs of the linear in front, rounded
+// to bf16 as that linear's output would have been.  Slabs are read four at a time and rows stay packed, 64 registers a
+// thread, so that a block still fits beside one of k_qlin (eight slabs at a time spilled: 14.6 us a norm instead of 7.2).
+template <int VPT>
+__device__ __forceinline__ void norm_row(uint4 (&v)[VPT], const uint4* __restrict__ x, const uint4* __restrict__ residual,
+                                         const uint4* __restrict__ gamma, uint4* __restrict__ out,
+                                         uint4* __restrict__ residual_out, int vpr, float eps,
+                                         const float* __restrict__ partials, int nsplit, size_t slab) {
+  __shared__ float s_part[16];
+  const size_t base = size_t(blockIdx.x) * vpr;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float ss = 0.f, f[8], g[8];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    v[i] = make_uint4(0, 0, 0, 0);
+    if (c >= vpr) continue;
+    uint4 r = make_uint4(0, 0, 0, 0);
+    if (residual) r = residual[base + c];
+    if (partials) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = 0.f;
+      const float* p = partials + (base + c) * 8;
+#pragma unroll 1
+      for (int s0 = 0; s0 < nsplit; s0 += 4) {
+        float4 u[4][2];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (s0 + q < nsplit) {
+            const float4* t = reinterpret_cast<const float4*>(p + size_t(s0 + q) * slab);
+            u[q][0] = __ldcg(t);
+            u[q][1] = __ldcg(t + 1);
+          }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (s0 + q < nsplit) {
+            f[0] += u[q][0].x; f[1] += u[q][0].y; f[2] += u[q][0].z; f[3] += u[q][0].w;
+            f[4] += u[q][1].x; f[5] += u[q][1].y; f[6] += u[q][1].z; f[7] += u[q][1].w;
+          }
+      }
+      v[i] = row_pack(f);
+    } else {
+      v[i] = x[base + c];
+    }
+    row_floats(v[i], f);
+    if (residual) {
+      row_floats(r, g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] += g[j];
+      v[i] = row_pack(f);  // the norm sees the stored (rounded) sum
+      residual_out[base + c] = v[i];
+      row_floats(v[i], f);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+  }
+  ss = warp_sum(ss);
+  if (lane == 0) s_part[warp] = ss;
+  __syncthreads();
+  ss = warp_sum(lane < int(blockDim.x >> 5) ? s_part[lane] : 0.f);
+  const float rstd = rsqrtf(ss / float(vpr * 8) + eps);
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = threadIdx.x + i * blockDim.x;
+    if (c >= vpr) continue;
+    row_floats(v[i], f);
+    row_floats(gamma[c], g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = __bfloat162float(__float2bfloat16(f[j] * rstd)) * g[j];
+    v[i] = row_pack(f);
+    out[base + c] = v[i];
+  }
+}
+
+// RMSNorm (+ residual) of decode rows, as k_rmsnorm does it (same sums, same bits), that leaves the digits of its result
+// too: the linear behind it reads them.  16 x 5120 between the linears of a decode step: the norm and a kernel of its own
+// for the digits 5.6 + 3.5 us, this 7.2.
+template <int VPT>
+__global__ void __launch_bounds__(kDigThreads, 2)
+    k_rmsnorm_digits(const uint4* __restrict__ x, const uint4* __restrict__ residual, const uint4* __restrict__ gamma,
+                     uint4* __restrict__ out, uint4* __restrict__ residual_out, int vpr, float eps,
+                     const float* __restrict__ partials, int nsplit, size_t slab, int tb, int8_t* __restrict__ xq,
+                     float* __restrict__ xs) {
+  pdl_launch_dependents();
+  pdl_wait();
+  uint4 v[VPT];
+  norm_row<VPT>(v, x, residual, gamma, out, residual_out, vpr, eps, partials, nsplit, slab);
+  digits_of_row<false, VPT, 1>(v, blockIdx.x, gridDim.x, 0, vpr, vpr, vpr * 8, tb, xq, xs);
 }
 
 // fp32 slabs [split][m][pitch] -> bf16 [m][n]: sum in split order, then what the epilogue of the unsplit product
@@ -970,6 +1082,33 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: quant_digits launch failed: %s", cudaGetErrorString(e));
+    return -1;
+  }
+  return 0;
+}
+
+extern "C" int bl_rmsnorm_digits(const void* x, const void* residual, const void* gamma, void* out, void* residual_out,
+                                 int rows, int hidden, float eps, const void* partials, int nsplit, size_t slab, void* xq,
+                                 void* xs, void* stream, char* err, size_t errlen) {
+  const uintptr_t ends = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(residual) |
+                         reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(out) |
+                         reinterpret_cast<uintptr_t>(residual_out) | reinterpret_cast<uintptr_t>(partials);
+  if (rows < 1 || rows > BL_QLIN_MAX_TOKENS || hidden < 8 || (hidden & 7) || hidden > 16 * kDigThreads || (!x && !partials) ||
+      !gamma || !out || !xq || !xs || (ends & 15u)) {
+    set_err(err, errlen, "barlink: rmsnorm_digits is for 1..%d rows of up to %d elements, a multiple of 8, on 16-byte boundaries",
+            BL_QLIN_MAX_TOKENS, 16 * kDigThreads);
+    return -1;
+  }
+  auto go = [&](auto kern) {
+    return launch_k(kern, dim3(rows), dim3(kDigThreads), 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x),
+                    static_cast<const uint4*>(residual), static_cast<const uint4*>(gamma), static_cast<uint4*>(out),
+                    static_cast<uint4*>(residual_out), hidden / 8, eps, static_cast<const float*>(partials), nsplit, slab,
+                    bl_qlin_tile_tokens(rows), static_cast<int8_t*>(xq), static_cast<float*>(xs));
+  };
+  cudaError_t e = hidden <= 8 * kDigThreads ? go(k_rmsnorm_digits<1>) : go(k_rmsnorm_digits<2>);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: rmsnorm_digits launch failed: %s", cudaGetErrorString(e));
     return -1;
   }
   return 0;

@@ -104,13 +104,13 @@ class W4Weight:
         return ops.ref.w4_dequant(self.qw, self.sc, self.qz, self.group).to(torch.bfloat16)
 
 
-def qlinear(x, w, bias=None, silu_mul=False, split=False):
+def qlinear(x, w, bias=None, silu_mul=False, split=False, digits=None):
     """x @ w.T for any stored form of w (plain / tiled bf16, W8Weight, W4Weight).
-    split=True allows the k-split slab output of the decode linears."""
+    split=True allows the k-split slab output of the decode linears.  digits: see `ops.rmsnorm_digits`."""
     if isinstance(w, W8Weight):
         if split and not silu_mul:
-            return ops.w8a16_linear_split(x, w.wq, w.scale, bias)
-        return ops.w8a16_linear(x, w.wq, w.scale, bias, silu_mul)
+            return ops.w8a16_linear_split(x, w.wq, w.scale, bias, digits)
+        return ops.w8a16_linear(x, w.wq, w.scale, bias, silu_mul, digits=digits)
     if isinstance(w, W4Weight):
         if bias is None:
             if split and not silu_mul:
@@ -289,21 +289,29 @@ class Qwen2Model:
         """ids [T] int32 -> final normed hidden [T, hidden] (replicated on every rank)."""
         cfg, c, w = self.cfg, self.comm, self.w
         h = ops.embedding(ids, w.embed)
-        res = torch.zeros_like(h)
         split_k = split_k and h.is_cuda
         # prefill sizes on the link: the row-parallel linears scatter their output tiles into the
         # owners' staging inboxes from the GEMM epilogue and one kernel finishes the all-reduce
         pushed = (not split_k and h.is_cuda and w.quant == "none" and c.world > 1 and c.use_link
                   and h.shape[0] > 128 and h.shape[0] % c.world == 0 and not w.tiled)
+        res = None
         pending = False  # h holds a partial sum that still needs the all-reduce
+        # decode on int8 weights, no all-reduce in between: the norm writes the digits that the linear behind it reads
+        digits_too = split_k and (c.world == 1 or c.no_comm)
         for li, L in enumerate(w.layers):
-            if pending:
+            dig = None
+            if li == 0:
+                normed, _ = ops.rmsnorm(h, L["ln1"], cfg.eps)
+                res = h  # the residual stream starts as the embedding
+            elif digits_too and isinstance(L["wqkv"], W8Weight):
+                normed, res, dig = ops.rmsnorm_digits(h, L["ln1"], cfg.eps, res)
+            elif pending:
                 normed, res = c.allreduce_rmsnorm(h, res, L["ln1"], cfg.eps)
             else:
                 normed, res = ops.rmsnorm(h, L["ln1"], cfg.eps, res)
             if w.quant != "none":
                 # decode: as below, a k-split leaves fp32 slabs for the next kernel (which adds the bias)
-                qkv = qlinear(normed, L["wqkv"], L["bqkv"], split=split_k)
+                qkv = qlinear(normed, L["wqkv"], L["bqkv"], split=split_k, digits=dig)
                 a = attn_factory(li)(qkv, L["bqkv"] if qkv.dim() == 3 else None)
                 h = qlinear(a, L["wo"], split=split_k)
             elif split_k:
@@ -324,7 +332,10 @@ class Qwen2Model:
                 qkv = ops.linear(normed, L["wqkv"], L["bqkv"])
                 a = attn_factory(li)(qkv, None)
                 h = ops.linear(a, L["wo"])
-            if pushed:
+            dig = None
+            if digits_too and isinstance(L["wgu"], W8Weight):
+                normed, res, dig = ops.rmsnorm_digits(h, L["ln2"], cfg.eps, res)
+            elif pushed:
                 normed, res = ops.rmsnorm(h, L["ln2"], cfg.eps, res)
             else:
                 normed, res = c.allreduce_rmsnorm(h, res, L["ln2"], cfg.eps)
@@ -333,7 +344,7 @@ class Qwen2Model:
                 # SiLU*mul then runs over the slabs (one small kernel) instead of in the epilogue
                 act = ops.silu_mul(ops.linear_split(normed, L["wgu"]), interleaved=True)
             else:
-                act = qlinear(normed, L["wgu"], silu_mul=True)
+                act = qlinear(normed, L["wgu"], silu_mul=True, digits=dig)
             if pushed:
                 h = c.row_parallel(torch.empty_like(res), [(act, L["wdown"], None, None, False, 0)])
                 pending = False

@@ -127,6 +127,17 @@ def rmsnorm(x, gamma, eps, residual=None, out=None):
     return ref.rmsnorm(x, gamma, eps, residual)
 
 
+def rmsnorm_digits(x, gamma, eps, residual=None):
+    """`rmsnorm`, and the int8 digits of the normed rows that `w8a16_linear` / `w8a16_linear_split` take as `digits`, in one
+    launch: (normed, residual, digits).  digits is None where those linears make no use of them."""
+    rows, hidden = x.shape[-2], x.shape[-1]
+    if x.is_cuda and 1 <= rows <= 128 and hidden % 16 == 0 and hidden <= 8192 and w8_act_mode() == "bf16":
+        _count()
+        normed, res, xq, xs = _C().rmsnorm_digits(x, gamma, eps, residual)
+        return normed, res, (xq, xs)
+    return (*rmsnorm(x, gamma, eps, residual), None)
+
+
 def rope_kv_write(qkv, positions, slots, k_cache, v_cache, nq, nkv, hd, block_size, theta, bias=None):
     """qkv: bf16 [rows, width] rotated in place, or fp32 split-K slabs of the
     QKV linear (then `bias` is added and a new bf16 buffer is returned)."""
@@ -281,7 +292,7 @@ def w8_act_mode():
     return v
 
 
-def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
+def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None, digits=None):
     """scale [n]: per output channel.  scale [n, k/group] or a W8GroupScales: per group, the
     reference's granularity (torch_ext/barlink_sm86/w8a16.cu:119-142 applies group scales inside
     its K loop).  Up to 128 tokens the int8 weights go to the tensor cores as they are, against three
@@ -291,6 +302,8 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
     weights may come from a kernel just ahead in the stream.  Groups of 64 and
     129..256 tokens widen the tile inside the main loop; other groups, and more than 256 tokens,
     widen the weight once and run the bf16 GEMM.
+
+    digits: those of x as `rmsnorm_digits` left them (up to 128 tokens, act="bf16").
 
     act="int8": the activations are quantised per token to int8 first, as the reference does
     (w8a16.cu:37-92 there), one digit instead of three, for any number of tokens with per-channel
@@ -316,12 +329,14 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None):
             else:
                 w = ref.w8_dequant(wq, scale).to(torch.bfloat16)
                 return linear(x, w, bias, silu_mul=silu_mul, dynamic_weights=True)
-        _count(2 if _qlin_rows(x) else 1)
+        _count(2 if _qlin_rows(x) and digits is None else 1)
         if gs is not None:
             if x.shape[0] > 256:
                 w = (ref.w8_dequant(wq, gs.rel.float() * gs.row.float()[:, None])).to(torch.bfloat16)
                 return linear(x, w, bias, silu_mul=silu_mul, dynamic_weights=True)
             return _C().w8a16_linear(x, wq, gs.row, bias, silu_mul, group_rel=gs.rel)
+        if digits is not None:
+            return _C().w8a16_linear(x, wq, scale, bias, silu_mul, xq=digits[0], xs=digits[1])
         return _C().w8a16_linear(x, wq, scale, bias, silu_mul)
     if isinstance(scale, W8GroupScales):
         scale = scale.rel.float() * scale.row.float()[:, None]
@@ -334,17 +349,18 @@ def _qlin_rows(x):
             and x.shape[1] % 16 == 0 and x.shape[1] <= 32768)
 
 
-def w8a16_linear_split(x, wq, scale, bias=None):
+def w8a16_linear_split(x, wq, scale, bias=None, digits=None):
     """Decode-path form of `w8a16_linear` (per-channel scales): when the shape wants a k-split, fp32 slabs
     [splits, tokens, n] whose sum is the product WITHOUT the bias, which the consumer adds (see
     `linear_split`); else the bf16 result with the bias."""
     if x.is_cuda and _qlin_rows(x):
-        _count(2)
-        return _C().w8a16_linear_split(x, wq, scale, bias, w8_act_mode() == "int8")
+        xq, xs = digits if digits is not None else (None, None)
+        _count(2 if xq is None else 1)
+        return _C().w8a16_linear_split(x, wq, scale, bias, w8_act_mode() == "int8", xq, xs)
     return w8a16_linear(x, wq, scale, bias)
 
 
 __all__ = [
-    "linear", "linear_split", "k_splits", "TiledWeight", "tile_weight", "untile_weight", "rmsnorm", "rope_kv_write", "rope", "silu_mul", "embedding", "argmax",
+    "linear", "linear_split", "k_splits", "TiledWeight", "tile_weight", "untile_weight", "rmsnorm", "rmsnorm_digits", "rope_kv_write", "rope", "silu_mul", "embedding", "argmax",
     "paged_attn_decode", "rope_attn_decode", "attention", "w8a16_linear", "w8a16_linear_split", "W8GroupScales", "prepare_w8_scales", "w4a16_linear", "w4a16_linear_split", "qknorm_rope", "layernorm_modulate", "gate_residual", "ref",
 ]

@@ -425,3 +425,26 @@ def test_quant_act_is_the_stated_arithmetic(ext, m, k):
     s = (amax / torch.full_like(amax, 127)).clamp_min(1e-12)  # (a division by a Python number multiplies by 1 / 127)
     assert torch.equal(xs, s)
     assert torch.equal(xq, torch.round(x.float() * (1.0 / s)[:, None]).clamp(-127, 127).to(torch.int8))
+
+
+@pytest.mark.parametrize("hidden", [16, 3584, 4096, 4112, 5120, 8192])
+@pytest.mark.parametrize("m", [1, 16, 17, 128])
+def test_norm_that_leaves_digits(ext, m, hidden):
+    """The same normed rows, residual and products, bit for bit, as the norm and a linear that makes the digits itself."""
+    gamma = _x(1, hidden, 2)[0].contiguous()
+    wq, sc = _w8(96, hidden, 3)
+    slabs = torch.randn(3, m, hidden, generator=_g(4), device="cuda")
+    if hidden > 64:
+        slabs[0, m - 1, hidden - 1] = 1e9  # outweighs its row: the rest has no digits but in the outliers' scale
+    for x in (slabs, slabs.sum(0).bfloat16()):
+        for res in (None, _x(m, hidden, 6)):
+            r0, r1 = (res.clone(), res.clone()) if res is not None else (None, None)
+            n0, _ = ext.rmsnorm(x, gamma, 1e-6, r0)
+            n1, _, xq, xs = ext.rmsnorm_digits(x, gamma, 1e-6, r1)
+            assert torch.equal(n0, n1) and (res is None or torch.equal(r0, r1))
+            assert torch.equal(ext.w8a16_linear(n0, wq, sc), ext.w8a16_linear(n1, wq, sc, xq=xq, xs=xs))
+            assert torch.equal(ext.w8a16_linear_split(n0, wq, sc), ext.w8a16_linear_split(n1, wq, sc, xq=xq, xs=xs))
+    with pytest.raises(RuntimeError):
+        ext.w8a16_linear(n1, wq, sc, xq=xq, xs=xs[:-1])
+    torch.cuda.synchronize()
+    assert ext.w8_error_flag(0) == 0

@@ -448,3 +448,14 @@ def test_norm_that_leaves_digits(ext, m, hidden):
         ext.w8a16_linear(n1, wq, sc, xq=xq, xs=xs[:-1])
     torch.cuda.synchronize()
     assert ext.w8_error_flag(0) == 0
+
+
+@pytest.mark.parametrize("n,k", [(300, 24), (256, 1040), (5, 18944), (300, 3592)])
+def test_widened_weights(ext, n, k):
+    """bl_w8_dequant behind a prefill linear: weights whose rows and whole are no multiple of a block's share."""
+    wq, sc = _w8(n, k, 3)
+    x = torch.zeros(300, k, device="cuda").bfloat16()
+    idx = torch.arange(min(300, k), device="cuda")
+    x[idx, idx] = 1  # rows of the widened weight itself
+    want = (wq.float() * sc.float()[:, None]).bfloat16().t()[: len(idx)]
+    assert torch.equal(ext.w8a16_linear(x, wq, sc)[: len(idx)], want)

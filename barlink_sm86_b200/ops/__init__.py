@@ -165,8 +165,8 @@ def w4a16_linear(x, qweight, scales, qzeros, group_size=128, silu_mul=False):
     over interleaved (gate, up) columns.  Groups of 128: mma.sync up to 16 rows, the digit kernel up to 128;
     else a GEMV up to 16 rows; else widen + GEMM."""
     if x.is_cuda:
-        _count(2)
         x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
+        _count(1 if group_size == 128 and x2.shape[0] <= 16 else 2)
         y = _C().w4a16_linear(x2.contiguous(), qweight, scales, qzeros, group_size, silu_mul=silu_mul)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     y = ref.w4a16_linear(x, qweight, scales, qzeros, group_size)
@@ -177,7 +177,7 @@ def w4a16_linear_split(x, qweight, scales, qzeros, group_size=128):
     """Decode-path form of `w4a16_linear`: fp32 slabs [splits, tokens, n] for the consumer to sum when the
     shape wants a k-split (see `linear_split`), else the bf16 result."""
     if x.is_cuda and x.dim() == 2:
-        _count(2)
+        _count(1 if group_size == 128 and x.shape[0] <= 16 else 2)
         return _C().w4a16_linear(x.contiguous(), qweight, scales, qzeros, group_size, want_slabs=True)
     return w4a16_linear(x, qweight, scales, qzeros, group_size)
 

@@ -134,9 +134,25 @@ class MMDiTWeights:
         self.t1_w, self.t1_b = dev(gen(h, cfg.time_dim)), dev(gen.vec(h))
         self.t2_w, self.t2_b = dev(gen(h, h)), dev(gen.vec(h))
 
+        # The adaLN linears of all blocks see the same vector, so their weights lie in one matrix: one product of a few
+        # rows that streams it, where one a block (57 MB on half of the SMs, 113 MB) took 22 us each.
+        mod_rows = cfg.double_blocks * 12 * h + cfg.single_blocks * 3 * h
+        self.mod_w = torch.empty(mod_rows, h, dtype=dtype, device=device)
+        self.mod_b = torch.empty(mod_rows, dtype=dtype, device=device)
+        self.mod_of = []  # (block's dict, its first row, rows), in forward order
+        filled = [0]
+
+        def mod(s, rows):
+            lo = filled[0]
+            s["mod_w"], s["mod_b"] = self.mod_w[lo:lo + rows], self.mod_b[lo:lo + rows]
+            s["mod_w"].copy_(gen(rows, h, 0.5 / math.sqrt(h)))
+            s["mod_b"].copy_(gen.vec(rows))
+            self.mod_of.append((s, lo, rows))
+            filled[0] += rows
+
         def stream():
             s = {}
-            s["mod_w"], s["mod_b"] = dev(gen(6 * h, h, 0.5 / math.sqrt(h))), dev(gen.vec(6 * h))
+            mod(s, 6 * h)
             s["qkv_w"] = dev(_head_rows(gen(3 * attn, h), nh, hd, tp, rank))
             s["qkv_b"] = dev(_head_rows(gen.vec(3 * attn)[:, None], nh, hd, tp, rank)[:, 0])
             s["gq"], s["gk"] = dev(gen.vec(hd, 0.05, 1.0)), dev(gen.vec(hd, 0.05, 1.0))
@@ -151,7 +167,7 @@ class MMDiTWeights:
         self.single = []
         for _ in range(cfg.single_blocks):
             s = {}
-            s["mod_w"], s["mod_b"] = dev(gen(3 * h, h, 0.5 / math.sqrt(h))), dev(gen.vec(3 * h))
+            mod(s, 3 * h)
             s["qkv_w"] = dev(_head_rows(gen(3 * attn, h), nh, hd, tp, rank))
             s["qkv_b"] = dev(_head_rows(gen.vec(3 * attn)[:, None], nh, hd, tp, rank)[:, 0])
             s["mlp_w"], s["mlp_b"] = dev(_rows(gen(cfg.mlp, h), tp, rank)), dev(_rows(gen.vec(cfg.mlp), tp, rank))
@@ -166,13 +182,17 @@ class MMDiTWeights:
 
     def nbytes(self):
         total = 0
+        seen = set()  # (the blocks' modulation weights are rows of one matrix)
         stack = [self.__dict__]
         while stack:
             o = stack.pop()
             for v in (o.values() if isinstance(o, dict) else o):
                 if isinstance(v, torch.Tensor):
-                    total += v.numel() * v.element_size()
-                elif isinstance(v, (dict, list)):
+                    store = v.untyped_storage()
+                    if store.data_ptr() not in seen:
+                        seen.add(store.data_ptr())
+                        total += store.nbytes()
+                elif isinstance(v, (dict, list, tuple)):
                     stack.append(v)
         return total
 
@@ -202,15 +222,26 @@ class MMDiTModel:
         self.scale = 1.0 / math.sqrt(cfg.head_dim)
 
     # ---- pieces ------------------------------------------------------------
-    def _attention(self, qkv, batch, seq):
+    def _modulations(self, svec):
+        """id of a block's dict -> its modulation vectors [batch, rows]."""
+        w = self.w
+        of = getattr(w, "mod_of", None)
+        # (weights that someone has put in place of the matrix's rows are used as they are)
+        if of and all(s["mod_w"].data_ptr() == w.mod_w[lo].data_ptr() and s["mod_b"].data_ptr() == w.mod_b[lo].data_ptr()
+                      and s["mod_w"].shape[0] == rows for s, lo, rows in of):
+            m = ops.linear(svec, w.mod_w, w.mod_b)
+            return {id(s): m[:, lo:lo + rows] for s, lo, rows in of}
+        blocks = [blk[name] for blk in w.double for name in ("txt", "img")] + list(w.single)
+        return {id(s): ops.linear(svec, s["mod_w"], s["mod_b"]) for s in blocks}
+
+    def _attention(self, qkv, batch, seq, cu):
         """qkv [batch*seq, >= 3*hl*128] with rows laid out [q | k | v]."""
         hl, hd = self.hl, self.cfg.head_dim
         v3 = qkv[:, : 3 * hl * hd].unflatten(1, (3 * hl, hd))
-        cu = torch.arange(0, (batch + 1) * seq, seq, dtype=torch.int32, device=qkv.device)
         o = ops.attention(v3[:, :hl], v3[:, hl:2 * hl], v3[:, 2 * hl:], cu, cu, seq, self.scale, False, max_k=seq)
         return o.reshape(batch * seq, hl * hd)
 
-    def _double(self, blk, h, nt, ni, batch, svec, pos_t, pos_i):
+    def _double(self, blk, h, nt, ni, batch, modulations, pos_t, pos_i, cu):
         """h: [batch*nt + batch*ni, hidden], text rows first (stream-major)."""
         cfg, hl, hd = self.cfg, self.hl, self.cfg.head_dim
         H = cfg.hidden
@@ -219,7 +250,7 @@ class MMDiTModel:
         L = nt + ni
         mods = {}
         for name in ("txt", "img"):
-            m = ops.linear(svec, blk[name]["mod_w"], blk[name]["mod_b"])
+            m = modulations[id(blk[name])]
             mods[name] = [m[:, j * H:(j + 1) * H] for j in range(6)]
 
         W = 3 * hl * hd
@@ -234,7 +265,7 @@ class MMDiTModel:
                 qkv = ops.linear(xm, s["qkv_w"], s["qkv_b"])
                 ops.qknorm_rope(qkv, s["gq"], s["gk"], pos, hl, cfg.eps, cfg.rope_theta, 2)
                 joint.view(batch, L, W)[:, lo:lo + n] = qkv.view(batch, n, W)
-        att = self._attention(joint, batch, L)
+        att = self._attention(joint, batch, L, cu)
         if batch == 1:
             at, ai = att[:nt], att[nt:]
         else:
@@ -257,16 +288,15 @@ class MMDiTModel:
         ops.gate_residual(ht, o[:rt], mods["txt"][5], nt)
         ops.gate_residual(hi, o[rt:], mods["img"][5], ni)
 
-    def _single(self, s, x, L, batch, svec, pos):
+    def _single(self, s, x, L, batch, m, pos, cu):
         cfg, hl, hd = self.cfg, self.hl, self.cfg.head_dim
         H = cfg.hidden
-        m = ops.linear(svec, s["mod_w"], s["mod_b"])
         sh, sc, gt = m[:, :H], m[:, H:2 * H], m[:, 2 * H:]
         xm = ops.layernorm_modulate(x, sh, sc, L, cfg.eps)
         qkv = ops.linear(xm, s["qkv_w"], s["qkv_b"])
         ops.qknorm_rope(qkv, s["gq"], s["gk"], pos, hl, cfg.eps, cfg.rope_theta, 2)
         f = ops.linear(xm, s["mlp_w"], s["mlp_b"], gelu=True)
-        att = self._attention(qkv, batch, L)
+        att = self._attention(qkv, batch, L, cu)
         o_attn = ops.linear(att, s["out_attn_w"], s["out_b"])
         o = torch.empty_like(o_attn)
         self.comm.row_parallel(o, [(f, s["out_mlp_w"], None, o_attn, False, 0)])
@@ -298,8 +328,10 @@ class MMDiTModel:
         h = torch.empty(batch * L, H, dtype=dt, device=dev)
         ops.linear(txt.reshape(rt, cfg.txt_dim).to(dt), w.txt_in_w, w.txt_in_b, out=h[:rt])
         ops.linear(img.reshape(batch * ni, cfg.in_channels).to(dt), w.img_in_w, w.img_in_b, out=h[rt:])
+        modulations = self._modulations(svec)
+        cu = torch.arange(0, (batch + 1) * L, L, dtype=torch.int32, device=dev)
         for blk in w.double:
-            self._double(blk, h, nt, ni, batch, svec, pos_t, pos_i)
+            self._double(blk, h, nt, ni, batch, modulations, pos_t, pos_i, cu)
 
         if batch == 1:
             x = h
@@ -309,7 +341,7 @@ class MMDiTModel:
             x3[:, :nt] = h[:rt].view(batch, nt, H)
             x3[:, nt:] = h[rt:].view(batch, ni, H)
         for s in w.single:
-            self._single(s, x, L, batch, svec, pos_j)
+            self._single(s, x, L, batch, modulations[id(s)], pos_j, cu)
 
         xi = x.view(batch, L, H)[:, nt:].reshape(batch * ni, H)
         m = ops.linear(svec, w.final_mod_w, w.final_mod_b)

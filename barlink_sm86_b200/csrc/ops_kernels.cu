@@ -511,6 +511,10 @@ constexpr int kHd = 128;
 constexpr int kRowPitch = kHd * 2 + 16;               // bytes, padded against bank conflicts
 constexpr int kPageBytes = kPageTokens * kRowPitch;   // one K or V page in shared memory
 constexpr int kAttnStages = 3;                        // pages in flight per warp: kAttnStages - 1
+// The same where an SM has one block at most: three pages in flight a warp instead of two, 139 KB a block.  Decode steps, us, with
+// three and with four buffers: 7B one sequence 2940 and 2887, 32B int8 16 sequences (128 blocks) 8337 and 8095; with
+// more blocks than SMs, where the second no longer fits, 64 x 4 blocks 3783 and 3833.  Five and six: as four or slower.
+constexpr int kAttnDeep = 4;
 constexpr int kWarpSmem = kAttnStages * 2 * kPageBytes;  // (K, V) x stages
 constexpr int kAttnWarps = 4;
 
@@ -549,11 +553,12 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
 }
 
 // grid (nkv, batch, splits), 128 threads.  Each warp walks its own pages with
-// a private ring of kAttnStages page buffers (cp.async, two pages in flight
+// a private ring of STAGES page buffers (cp.async, STAGES - 1 pages in flight
 // while one is consumed); the warp's block-table entries are fetched 32 at a
 // time into registers so that no page address waits on a dependent load.  The
 // four warps are merged through shared memory, splits through `scratch` and
 // k_attn_merge.
+template <int STAGES>
 __global__ void __launch_bounds__(kAttnWarps * 32)
     k_paged_attn_decode(const __nv_bfloat16* __restrict__ q, int q_stride,
                         const __nv_bfloat16* __restrict__ k_cache,
@@ -593,7 +598,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
   for (int d = 0; d < kHd / 8; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
 
-  const uint32_t wbase = smem_u32(smem) + warp * kWarpSmem;
+  const uint32_t wbase = smem_u32(smem) + warp * (STAGES * 2 * kPageBytes);
   // pages of this warp: p0 + warp + i * kAttnWarps, i in [0, count)
   const int count = p1 > p0 + warp ? (p1 - p0 - warp + kAttnWarps - 1) / kAttnWarps : 0;
   int tbl = 0;        // lane l holds the table entry of page index (chunk * 32 + l)
@@ -619,9 +624,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
     }
   };
 
-  // prologue: kAttnStages - 1 pages in flight (one commit group per slot, empty when past the end)
+  // prologue: STAGES - 1 pages in flight (one commit group per slot, empty when past the end)
 #pragma unroll
-  for (int i = 0; i < kAttnStages - 1; ++i) {
+  for (int i = 0; i < STAGES - 1; ++i) {
     if (i < count) issue(i, i);
     cp_async_commit();
   }
@@ -629,12 +634,12 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
   for (int i = 0; i < count; ++i) {
     const int page = p0 + warp + i * kAttnWarps;
     {
-      const int nxt = i + kAttnStages - 1;
-      int nbuf = buf + kAttnStages - 1;
-      if (nbuf >= kAttnStages) nbuf -= kAttnStages;
+      const int nxt = i + STAGES - 1;
+      int nbuf = buf + STAGES - 1;
+      if (nbuf >= STAGES) nbuf -= STAGES;
       if (nxt < count) issue(nxt, nbuf);
       cp_async_commit();
-      cp_async_wait<kAttnStages - 1>();
+      cp_async_wait<STAGES - 1>();
     }
     __syncwarp();
     const uint32_t kd = wbase + buf * 2 * kPageBytes, vd = kd + kPageBytes;
@@ -722,7 +727,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
       }
     }
     __syncwarp();
-    if (++buf == kAttnStages) buf = 0;
+    if (++buf == STAGES) buf = 0;
   }
   cp_async_wait<0>();
   // row sums live spread over the quad
@@ -732,7 +737,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
   l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
 
   // ---- merge the four warps ----------------------------------------------
-  float* wo = reinterpret_cast<float*>(smem + warp * kWarpSmem);  // [16][128] + m[16] + l[16]
+  float* wo = reinterpret_cast<float*>(smem + warp * (STAGES * 2 * kPageBytes));  // [16][128] + m[16] + l[16]
   float* wm = wo + 16 * kHd;
   float* wl = wm + 16;
 #pragma unroll
@@ -752,11 +757,11 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < kAttnWarps; ++w)
-      M = fmaxf(M, reinterpret_cast<const float*>(smem + w * kWarpSmem)[16 * kHd + r]);
+      M = fmaxf(M, reinterpret_cast<const float*>(smem + w * (STAGES * 2 * kPageBytes))[16 * kHd + r]);
     float L = 0.f, acc = 0.f;
 #pragma unroll
     for (int w = 0; w < kAttnWarps; ++w) {
-      const float* base = reinterpret_cast<const float*>(smem + w * kWarpSmem);
+      const float* base = reinterpret_cast<const float*>(smem + w * (STAGES * 2 * kPageBytes));
       const float mw = base[16 * kHd + r];
       const float sc = mw == -INFINITY ? 0.f : exp2f(mw - M);
       L += base[16 * kHd + 16 + r] * sc;
@@ -1437,10 +1442,11 @@ extern "C" int bl_paged_attn_decode(const void* q, int q_stride, const void* k_c
     return -1;
   }
   if (splits <= 0) {
-    // enough CTAs to fill the GPU once; more splits only add merge traffic.  From 64 CTAs
+    // as many CTAs as SMs at most, so that all have the deep ring (8 sequences x 4 heads of 8000 tokens: five splits
+    // 3548 us a step, four 3491); more splits only add merge traffic.  From 64 CTAs
     // on, splitting measured no faster than one CTA per (sequence, KV head) and costs the
     // merge kernel, so it is not done.
-    const int want = batch * nkv >= 64 ? 1 : (sm_count() + batch * nkv - 1) / (batch * nkv);
+    const int want = batch * nkv >= 64 ? 1 : sm_count() / (batch * nkv);
     const int by_len = max_blocks / (2 * kAttnWarps) > 0 ? max_blocks / (2 * kAttnWarps) : 1;
     splits = want < by_len ? want : by_len;
     if (splits > 32) splits = 32;
@@ -1448,21 +1454,20 @@ extern "C" int bl_paged_attn_decode(const void* q, int q_stride, const void* k_c
   }
   const size_t need = size_t(batch) * nq * splits * (kHd + 2) * sizeof(float);
   if (splits > 1 && (!scratch || scratch_bytes < need)) splits = 1;
-  static bool attr = false;
-  const int smem = kAttnWarps * kWarpSmem;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_paged_attn_decode,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: paged attention shared memory opt-in failed: %s",
-              cudaGetErrorString(e));
-      return -1;
-    }
-    attr = true;
+  // one block an SM: a deep ring; more: blocks of which two fit
+  const bool deep = size_t(batch) * nkv * splits <= size_t(sm_count());
+  const int smem = kAttnWarps * (deep ? kAttnDeep : kAttnStages) * 2 * kPageBytes;
+  static bool attr[2][64] = {};
+  cudaError_t e = deep ? allow_smem(reinterpret_cast<const void*>(k_paged_attn_decode<kAttnDeep>), smem, attr[0])
+                       : allow_smem(reinterpret_cast<const void*>(k_paged_attn_decode<kAttnStages>), smem, attr[1]);
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: paged attention shared memory opt-in failed: %s", cudaGetErrorString(e));
+    return -1;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const float scale_log2 = scale * 1.4426950408889634f;
-  launch_k(k_paged_attn_decode, dim3(nkv, batch, splits), dim3(kAttnWarps * 32), smem, st,
+  launch_k(deep ? k_paged_attn_decode<kAttnDeep> : k_paged_attn_decode<kAttnStages>, dim3(nkv, batch, splits),
+      dim3(kAttnWarps * 32), smem, st,
       static_cast<const __nv_bfloat16*>(q), q_stride, static_cast<const __nv_bfloat16*>(k_cache),
       static_cast<const __nv_bfloat16*>(v_cache), block_tables, ctx_lens,
       static_cast<__nv_bfloat16*>(out), static_cast<float*>(scratch), nq, nkv, max_blocks,

@@ -162,6 +162,23 @@ def test_paged_attention_decode(ext, nq, nkv, splits):
     assert rel_l2(got, want) < 1e-2
 
 
+@pytest.mark.parametrize("batch,nkv,splits", [(37, 4, 1), (38, 4, 1), (4, 1, 37), (2, 2, 38), (8, 4, 0)])
+def test_paged_attention_rings(ext, batch, nkv, splits):
+    """Up to one block an SM (a ring of four pages a warp) and beyond (three): contexts that end on either side of a
+    page, of a warp's first lap and of a ring's."""
+    from barlink_sm86_b200.ops import reference as ref
+    nq, hd, bs, max_blocks = 2 * nkv, 128, 16, 40
+    ends = [1, 15, 16, 17, 64, 65, 193, 256, 257, 320, 511, 640]
+    ctx = torch.tensor([ends[i % len(ends)] for i in range(batch)], dtype=torch.int32, device="cuda")
+    kc, vc = _bf(batch * max_blocks, nkv, bs, hd, seed=1), _bf(batch * max_blocks, nkv, bs, hd, seed=2)
+    perm = torch.randperm(batch * max_blocks, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    bt = perm.to(torch.int32).view(batch, max_blocks).contiguous()
+    qkv = _bf(batch, (nq + 2 * nkv) * hd, seed=4)
+    got = ext.paged_attn_decode(qkv, kc, vc, bt, ctx, nq, nkv, hd, 1.0 / math.sqrt(hd), splits)
+    want = ref.paged_attn_decode(qkv, kc, vc, bt, ctx, nq, nkv, hd, 1.0 / math.sqrt(hd))
+    assert rel_l2(got, want) < 1e-2  # (probabilities and output rounded to bf16: 2^-8 each)
+
+
 @pytest.mark.parametrize("tokens,n,k,splits", [(64, 4608, 3584, 4), (8, 3584, 18944, 5), (1, 512, 1024, 2),
                                                (33, 640, 1024, 3)])
 def test_linear_split_slabs_sum_to_the_product(ext, tokens, n, k, splits):

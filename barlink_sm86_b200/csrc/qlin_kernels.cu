@@ -1070,9 +1070,9 @@ extern "C" int bl_quant_digits(const void* x, int m, int ldx, int k, int permute
   // kernel this short comes from L2 or beyond on every launch)
   const int vpt = (k / 8 + kDigThreads - 1) / kDigThreads;
   cudaError_t e;
-  // a cluster for a row of more than 8192 elements, as long as all blocks are resident at once (a cluster of two for 5120
+  // a cluster for a row of more than 8192 elements, as long as there is an SM for every block (a cluster of two for 5120
   // elements took 3.9 us between the linears around it, one block with two vectors a thread 3.2)
-  if (vpt > 2 && m * (vpt <= 4 ? 4 : 8) <= 2 * sm_count()) {
+  if (vpt > 2 && m * (vpt <= 4 ? 4 : 8) <= sm_count()) {
     if (vpt <= 4) e = permute ? go(k_quant_digits_cluster<true, 4>, 4) : go(k_quant_digits_cluster<false, 4>, 4);
     else e = permute ? go(k_quant_digits_cluster<true, 8>, 8) : go(k_quant_digits_cluster<false, 8>, 8);
   } else if (vpt <= 1) e = permute ? go(k_quant_digits<true, 1>) : go(k_quant_digits<false, 1>);

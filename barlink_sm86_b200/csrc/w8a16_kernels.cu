@@ -137,10 +137,10 @@ extern "C" int bl_w8a16_quant_act(const void* x, int m, int k, void* xq, void* x
     return launch_k(kern, dim3(m * blocks), dim3(threads), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const __nv_bfloat16*>(x), static_cast<int8_t*>(xq), static_cast<float*>(xs), k);
   };
-  // blocks of a row: one vector a thread, as long as all blocks are resident at once
+  // blocks of a row: one vector a thread, as long as there is an SM for every block
   const int need = (k / 8 + kQaThreads - 1) / kQaThreads, cl = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : 8;
   cudaError_t e;
-  if (need > 8 || m * cl > 2 * sm_count()) e = go(k_quant_act, 1, kQThreads);
+  if (need > 8 || m * cl > sm_count()) e = go(k_quant_act, 1, kQThreads);
   else if (cl == 1) e = go(k_quant_act_cluster<1>, 1, kQaThreads);
   else if (cl == 2) e = go(k_quant_act_cluster<2>, 2, kQaThreads);
   else if (cl == 4) e = go(k_quant_act_cluster<4>, 4, kQaThreads);

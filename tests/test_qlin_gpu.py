@@ -408,14 +408,14 @@ def test_long_rows_shared_by_blocks(ext, k):
     for p in (0, k // 8, k // 4 - 1, k // 4, k // 2 - 1, k // 2, k - 1):
         x[3, p] = 2.0 ** 14
     want = x.double() @ (wq.double() * sc.double()[:, None]).t()
-    y = {m: ext.w8a16_linear(x[:m].contiguous(), wq, sc, splits=1) for m in (33, 37, 38)}
+    y = {m: ext.w8a16_linear(x[:m].contiguous(), wq, sc, splits=1) for m in (1, 18, 19, 37, 38)}
     for m in y:
         assert rel_l2(y[m], want[:m]) < TOL
         assert torch.equal(y[m], y[38][:m])
 
 
 @pytest.mark.parametrize("k", [8, 4096, 4104, 8192, 8200, 18944, 32768, 32776])
-@pytest.mark.parametrize("m", [1, 37, 300])
+@pytest.mark.parametrize("m", [1, 18, 37, 300])
 def test_quant_act_is_the_stated_arithmetic(ext, m, k):
     """xs = max |x| / 127 and xq = x / xs to the nearest whole number, whichever kernel a row length goes to."""
     x = _x(m, k, 7) * 3

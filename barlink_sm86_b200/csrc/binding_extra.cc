@@ -8,6 +8,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <map>
 
 #include "backend.h"
@@ -137,6 +138,8 @@ at::Tensor attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& 
               "barlink: cu_q / cu_k must be int32 CUDA tensors of batch + 1 entries");
   const int batch = int(cu_q.numel()) - 1;
   const int nq = int(q.size(1)), nkv = int(k.size(1)), hd = int(q.size(2));
+  TORCH_CHECK(k.size(2) == hd && v.size(2) == hd && v.size(1) >= nkv,
+              "barlink: k and v must have q's head_dim, and v a head for each of k's");
   at::Tensor out = at::empty({q.size(0), nq, hd}, q.options());
   c10::cuda::CUDAGuard guard(q.device());
   void* st = at::cuda::getCurrentCUDAStream(q.device().index()).stream();
@@ -144,10 +147,16 @@ at::Tensor attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& 
     const char* e = getenv("BL_ATTN_TC");
     return !(e && e[0] == '0');
   }();
-  if (q.size(0) > 0 && tc_on && max_k > 0 && hd == 128) {
-    BL_CHECK(bl_attn_fwd_tc(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_q.data_ptr<int>(),
-                            cu_k.data_ptr<int>(), batch, max_q, max_k, int(q.size(0)), int(k.size(0)), nq, nkv,
-                            hd, int(q.stride(0)), int(k.stride(0)), int(v.stride(0)), nq * hd, float(scale),
+  if (q.size(0) > 0 && tc_on && max_k > 0 && hd == 128 && v.size(0) > 0) {
+    // K and V are fetched in boxes of 64 rows whose last one reaches beyond its sequence, so the tensor maps end with the
+    // shorter of the two (K may be a longer preallocated buffer).  A map knows no rows that lie on one another, and the
+    // stride of a single row says nothing.
+    const int rows = int(std::min(k.size(0), v.size(0)));
+    const at::Tensor vm = v.size(0) > 1 && v.stride(0) == 0 ? v.contiguous() : v;
+    const int v_stride = int(v.size(0) > 1 ? vm.stride(0) : vm.size(1) * hd);
+    BL_CHECK(bl_attn_fwd_tc(q.data_ptr(), k.data_ptr(), vm.data_ptr(), out.data_ptr(), cu_q.data_ptr<int>(),
+                            cu_k.data_ptr<int>(), batch, max_q, max_k, int(q.size(0)), rows, nq, nkv,
+                            hd, int(q.stride(0)), int(k.stride(0)), v_stride, nq * hd, float(scale),
                             causal ? 1 : 0, attn_err(q.device().index()).data_ptr(), st, err,
                             errlen));
     return out;

@@ -49,3 +49,30 @@ def test_values_of_the_next_sequence_do_not_leak(ext, l0, bad):
         alone = ops.attention(q[:l0].contiguous(), k[:l0].contiguous(), v[:l0].contiguous(), one, one, l0, 0.088, causal,
                               max_k=l0)
         assert torch.equal(both[:l0], alone) and bool(alone.isfinite().all())
+
+
+def test_values_of_other_shapes_than_the_keys(ext):
+    """Tensor maps end with the shorter of K and V, so that no box reaches beyond either; values that do not belong to
+    the keys are refused before anything is launched."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    l, nq, nkv = 70, 4, 2
+    q, k, v = (torch.randn(n, h, 128, generator=g, device="cuda").bfloat16() for n, h in ((l, nq), (200, nkv), (l, nkv)))
+    cu = torch.tensor([0, l], dtype=torch.int32, device="cuda")
+
+    def run(k, v, cu_k=cu, lk=l):
+        return ext.attn_fwd(q, k, v, cu, cu_k, l, 0.088, False, lk)
+
+    want = run(k[:l].contiguous(), v)
+    more = torch.cat([v, torch.full((9, nkv, 128), float("nan"), device="cuda").bfloat16()])
+    assert torch.equal(run(k, v), want) and torch.equal(run(k[:l], more), want)
+    wide = torch.cat([v, v[:, :1]], 1)  # more heads than the keys have
+    assert torch.equal(run(k, wide), want)
+    # all rows at one address, and a single row of any stride
+    assert torch.equal(run(k, v[:1].expand(l, -1, -1)), run(k, v[:1].repeat(l, 1, 1)))
+    one = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    row = torch.as_strided(v, (1, nkv, 128), (3, 128, 1))
+    assert torch.equal(run(k, row, one, 1), run(k, v[:1].contiguous(), one, 1))
+    for bad_k, bad_v in ((k, v[:, :1].contiguous()), (k, v[..., :64].contiguous()), (k[..., :64].contiguous(), v)):
+        for lk in (l, 0):
+            with pytest.raises(RuntimeError, match="head_dim"):
+                run(bad_k, bad_v, lk=lk)

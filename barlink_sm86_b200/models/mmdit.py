@@ -139,7 +139,6 @@ class MMDiTWeights:
         mod_rows = cfg.double_blocks * 12 * h + cfg.single_blocks * 3 * h
         self.mod_w = torch.empty(mod_rows, h, dtype=dtype, device=device)
         self.mod_b = torch.empty(mod_rows, dtype=dtype, device=device)
-        self.mod_of = []  # (block's dict, its first row, rows), in forward order
         filled = [0]
 
         def mod(s, rows):
@@ -147,7 +146,6 @@ class MMDiTWeights:
             s["mod_w"], s["mod_b"] = self.mod_w[lo:lo + rows], self.mod_b[lo:lo + rows]
             s["mod_w"].copy_(gen(rows, h, 0.5 / math.sqrt(h)))
             s["mod_b"].copy_(gen.vec(rows))
-            self.mod_of.append((s, lo, rows))
             filled[0] += rows
 
         def stream():
@@ -211,6 +209,21 @@ def grid_positions(height, width, device):
     return torch.stack([ys.reshape(-1), xs.reshape(-1)], -1).to(torch.int32).to(device)
 
 
+def _rows_in_place(parts, rows, whole):
+    """Whether `parts` are the consecutive rows of `whole`, as `MMDiTWeights` lays them out, and not something that has been
+    put in their place since (another tensor or form of weight, a block's dict, a bias that is None)."""
+    if not parts or type(whole) is not torch.Tensor or not whole.is_contiguous() or sum(rows) > whole.shape[0]:
+        return False
+    at, pitch = whole.data_ptr(), whole[:1].numel() * whole.element_size()
+    for t, n in zip(parts, rows):
+        if type(t) is not torch.Tensor or t.shape != (n, *whole.shape[1:]) or \
+                t.dtype != whole.dtype or t.device != whole.device or not t.is_contiguous() or \
+                t.data_ptr() != at:
+            return False
+        at += n * pitch
+    return True
+
+
 class MMDiTModel:
     def __init__(self, cfg, weights, comm=None):
         self.cfg, self.w = cfg, weights
@@ -225,13 +238,13 @@ class MMDiTModel:
     def _modulations(self, svec):
         """id of a block's dict -> its modulation vectors [batch, rows]."""
         w = self.w
-        of = getattr(w, "mod_of", None)
-        # (weights that someone has put in place of the matrix's rows are used as they are)
-        if of and all(s["mod_w"].data_ptr() == w.mod_w[lo].data_ptr() and s["mod_b"].data_ptr() == w.mod_b[lo].data_ptr()
-                      and s["mod_w"].shape[0] == rows for s, lo, rows in of):
-            m = ops.linear(svec, w.mod_w, w.mod_b)
-            return {id(s): m[:, lo:lo + rows] for s, lo, rows in of}
-        blocks = [blk[name] for blk in w.double for name in ("txt", "img")] + list(w.single)
+        blocks = [s for blk in w.double for s in (blk["img"], blk["txt"])] + list(w.single)
+        rows = [6 * self.cfg.hidden] * (2 * len(w.double)) + [3 * self.cfg.hidden] * len(w.single)
+        total = sum(rows)
+        if _rows_in_place([s["mod_w"] for s in blocks], rows, getattr(w, "mod_w", None)) and \
+                _rows_in_place([s["mod_b"] for s in blocks], rows, getattr(w, "mod_b", None)):
+            m = ops.linear(svec, w.mod_w[:total], w.mod_b[:total])
+            return {id(s): v for s, v in zip(blocks, m.split(rows, 1))}
         return {id(s): ops.linear(svec, s["mod_w"], s["mod_b"]) for s in blocks}
 
     def _attention(self, qkv, batch, seq, cu):

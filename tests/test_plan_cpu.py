@@ -128,6 +128,41 @@ def test_mmdit_batches_are_independent_and_sampler_runs():
     assert m.flops_per_forward(1, 4096, 512) > 0
 
 
+@pytest.mark.parametrize("put", ["nothing", "tensor", "dict", "pair", "no_bias", "strided", "same_block", "one_less"])
+def test_mmdit_modulation_weights_that_were_put_in_place(put):
+    """Blocks whose modulation weights are not the rows they were made with give what a product for each block gives."""
+    from barlink_sm86_b200.models import MMDiTConfig, MMDiTModel, MMDiTWeights, grid_positions
+    cfg = MMDiTConfig.tiny()
+    g = torch.Generator().manual_seed(1)
+    img, txt = torch.randn(1, 16, cfg.in_channels, generator=g), torch.randn(1, 8, cfg.txt_dim, generator=g)
+    new = torch.randn(3 * cfg.hidden, cfg.hidden, generator=g) / cfg.hidden ** 0.5
+
+    def forward(single_products):
+        w = MMDiTWeights(cfg, "cpu", torch.float32, 3)
+        if put == "tensor":
+            w.single[-1]["mod_w"] = new
+        elif put == "dict":
+            w.single[0] = dict(w.single[0], mod_w=new)
+        elif put == "pair":
+            w.double[0] = {name: dict(w.double[-1][name]) for name in ("img", "txt")}
+        elif put == "no_bias":
+            w.double[0]["txt"]["mod_b"] = None
+        elif put == "strided":  # starts where the rows start
+            rows = w.single[0]["mod_w"]
+            w.single[0]["mod_w"] = rows.as_strided(rows.shape, (1, 2))
+        elif put == "same_block":
+            w.single[-1] = w.single[0]
+        elif put == "one_less":
+            w.single.pop()
+        if single_products:
+            for s in [s for blk in w.double for s in blk.values()] + w.single:
+                s["mod_w"] = s["mod_w"].clone()
+        return MMDiTModel(cfg, w).forward(img, txt, torch.tensor([0.4]), grid_positions(4, 4, "cpu"))
+
+    # (fp32 sums of one product in another order)
+    assert torch.allclose(forward(False), forward(True), atol=1e-4, rtol=1e-4)
+
+
 def test_no_comm_control_skips_collectives():
     from barlink_sm86_b200.parallel import TPComm
     c = TPComm.single()

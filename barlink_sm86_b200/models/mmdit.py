@@ -179,18 +179,16 @@ class MMDiTWeights:
         self.final_w, self.final_b = dev(gen(cfg.in_channels, h)), dev(gen.vec(cfg.in_channels))
 
     def nbytes(self):
+        """Bytes of the tensors that the model reads (of a shard: the shard's, whatever they are views of)."""
         total = 0
-        seen = set()  # (the blocks' modulation weights are rows of one matrix)
-        stack = [self.__dict__]
+        # (mod_w and mod_b are the blocks' own modulation weights once more)
+        stack = [{name: v for name, v in self.__dict__.items() if name not in ("mod_w", "mod_b")}]
         while stack:
             o = stack.pop()
             for v in (o.values() if isinstance(o, dict) else o):
                 if isinstance(v, torch.Tensor):
-                    store = v.untyped_storage()
-                    if store.data_ptr() not in seen:
-                        seen.add(store.data_ptr())
-                        total += store.nbytes()
-                elif isinstance(v, (dict, list, tuple)):
+                    total += v.numel() * v.element_size()
+                elif isinstance(v, (dict, list)):
                     stack.append(v)
         return total
 

@@ -163,6 +163,25 @@ def test_mmdit_modulation_weights_that_were_put_in_place(put):
     assert torch.allclose(forward(False), forward(True), atol=1e-4, rtol=1e-4)
 
 
+def test_mmdit_weight_bytes():
+    """Every parameter once; a rank of two has half of what is cut and all of the rest."""
+    from barlink_sm86_b200.models import MMDiTConfig, MMDiTWeights
+    cfg = MMDiTConfig.tiny()
+    h, f, a = cfg.hidden, cfg.mlp, cfg.heads * cfg.head_dim
+
+    def numbers(tp):
+        qkv, mlp, out = (3 * a * h + 3 * a) // tp, (f * h + f) // tp, (h * a) // tp
+        stream = 6 * h * h + 6 * h + qkv + 2 * cfg.head_dim + out + h + mlp + h * f // tp + h
+        single = 3 * h * h + 3 * h + qkv + mlp + 2 * cfg.head_dim + out + h * f // tp + h
+        ends = sum(h * n + h for n in (cfg.in_channels, cfg.txt_dim, cfg.time_dim, h)) \
+            + 2 * h * h + 2 * h + cfg.in_channels * h + cfg.in_channels
+        return 2 * cfg.double_blocks * stream + cfg.single_blocks * single + ends
+
+    assert MMDiTWeights(cfg, "cpu", torch.float32, 3).nbytes() == 4 * numbers(1)
+    for rank in range(2):
+        assert MMDiTWeights(cfg, "cpu", torch.float32, 3, 2, rank).nbytes() == 4 * numbers(2)
+
+
 def test_no_comm_control_skips_collectives():
     from barlink_sm86_b200.parallel import TPComm
     c = TPComm.single()

@@ -10,6 +10,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -638,6 +639,7 @@ __global__ void __launch_bounds__(GemmSmem<BN, 1, true>::kThreads, 1)
               GemmShape g, LocalSink<BN> sink, uint64_t hint_a, uint64_t hint_b) {
   gemm_body<BN, 1, true>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
 }
+constexpr size_t kW8DequantMost = 0xfffff000u;  // eights of weights in a launch
 // Eight weights a thread and vector (16-byte stores side by side), four vectors requested together, 32-bit row numbers:
 // the weights of a 7B layer 146 us, 137 so (37888 x 3584: 79 and 74; a 64-bit division per vector and one request at a time
 // before).  16 weights a thread, two stores 32 bytes apart in every lane, took 173.
@@ -1152,20 +1154,18 @@ extern "C" int bl_w8_dequant(const void* wq, const void* scale, void* out, int n
     set_err(err, errlen, "barlink: w8_dequant needs K a multiple of 8");
     return -1;
   }
-  const size_t total = size_t(n) * k / 8;
-  if (total > 0xfffff000u) {
-    set_err(err, errlen, "barlink: w8_dequant: %d x %d weights are too many", n, k);
-    return -1;
-  }
-  size_t blocks = (total + 1023) / 1024;
-  if (blocks > size_t(148) * 8) blocks = size_t(148) * 8;
-  cudaError_t e = launch_k(k_w8_dequant, dim3(unsigned(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                           static_cast<const int8_t*>(wq), static_cast<const __nv_bfloat16*>(scale),
-                           static_cast<__nv_bfloat16*>(out), uint32_t(total), uint32_t(k / 8));
-  if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_err(err, errlen, "barlink: w8_dequant launch failed: %s", cudaGetErrorString(e));
-    return -1;
+  // the kernel numbers eight weights with 32 bits: rows in launches of fewer than 2^32 of them
+  const size_t per_row = size_t(k) / 8, rows_most = kW8DequantMost / per_row;
+  for (size_t r = 0; r < size_t(n); r += rows_most) {
+    const size_t vecs = std::min(rows_most, size_t(n) - r) * per_row, blocks = std::min((vecs + 1023) / 1024, size_t(148) * 8);
+    cudaError_t e = launch_k(k_w8_dequant, dim3(unsigned(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                             static_cast<const int8_t*>(wq) + r * k, static_cast<const __nv_bfloat16*>(scale) + r,
+                             static_cast<__nv_bfloat16*>(out) + r * k, uint32_t(vecs), uint32_t(per_row));
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) {
+      set_err(err, errlen, "barlink: w8_dequant launch failed: %s", cudaGetErrorString(e));
+      return -1;
+    }
   }
   return 0;
 }

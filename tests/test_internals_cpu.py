@@ -1,7 +1,10 @@
 # SPDX-License-Identifier: MIT
 """Host-side arithmetic of the link core, without a GPU: arena layout, the
 symmetric allocator, the all-reduce algorithm table and the k-split choice."""
+import ctypes
+
 import pytest
+import torch
 
 import barlink_sm86_b200 as bl
 
@@ -96,3 +99,15 @@ def test_an_error_with_a_number_in_it_is_an_error(devices):
             "except RuntimeError as e:\n    print(e)\n" % devices)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "1..8 devices" in r.stdout, (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the pointers are not device memory")
+@pytest.mark.parametrize("n,k", [(16, 64), (1 << 20, 1 << 16), (2147483647, 2147483640)])
+def test_widening_refuses_no_size(n, k):
+    """bl_w8_dequant numbers eights of weights with 32 bits a launch; more of them are more launches (here without a
+    device, so that the first one is the error)."""
+    fn = ctypes.CDLL(C.__file__).bl_w8_dequant
+    fn.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 2 + [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_size_t]
+    err = ctypes.create_string_buffer(512)
+    assert fn(256, 256, 256, n, k, None, err, 512) == -1 and b"launch failed" in err.value
+    assert fn(256, 256, 256, n, k - 4, None, err, 512) == -1 and b"multiple of 8" in err.value

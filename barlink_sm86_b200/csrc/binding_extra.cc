@@ -214,9 +214,22 @@ struct QWeight {
   const void* row_scale = nullptr;
   int group_k = 0;
   const void* zeros = nullptr;
-  // digits that the norm in front has left (bl_rmsnorm_digits)
+  // digits that the norm in front has left (bl_rmsnorm_digits), both or neither
   c10::optional<at::Tensor> xq, xs;
 };
+// digits that a caller hands in for x; `used`: the product reads digits
+void check_digits(const at::Tensor& x, int k, bool used, const c10::optional<at::Tensor>& xq, const c10::optional<at::Tensor>& xs) {
+  if (!xq && !xs) return;
+  TORCH_CHECK(used, "barlink: digits are for bf16 activations of 1..", std::to_string(BL_QLIN_MAX_TOKENS),
+              " 16-byte aligned rows of at most 32768 elements");
+  const int m = int(x.size(0));
+  auto ok = [&](const c10::optional<at::Tensor>& t, at::ScalarType type, size_t bytes) {
+    return t && t->device() == x.device() && t->scalar_type() == type && t->is_contiguous() && t->nbytes() == bytes;
+  };
+  TORCH_CHECK(ok(xq, at::kChar, bl_quant_digits_bytes(m, k)) && ok(xs, at::kFloat, bl_quant_digits_xs_bytes(m)) &&
+                  (reinterpret_cast<uintptr_t>(xq->data_ptr()) & 15u) == 0,
+              "barlink: digits do not belong to these activations (see rmsnorm_digits)");
+}
 // a shape that bl_qlin takes and (three digits) bf16 rows that bl_quant_digits can read; per-channel sums are
 // 32-bit over all of K
 bool qlin_takes(const at::Tensor& x, int k, bool act_int8, bool grouped = false) {
@@ -281,10 +294,7 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
                     bool silu_mul, int splits, bool want_slabs, void* err_flag, void* st) {
   const int m = int(x.size(0));
   at::Tensor xq, xs;
-  if (digits == 3 && q.xq && q.xs) {
-    TORCH_CHECK(q.src != 2 && q.xq->is_cuda() && q.xq->is_contiguous() && q.xs->is_cuda() && q.xs->is_contiguous() &&
-                    q.xq->nbytes() == bl_quant_digits_bytes(m, q.k) && q.xs->nbytes() == bl_quant_digits_xs_bytes(m),
-                "barlink: digits do not belong to these activations (see rmsnorm_digits)");
+  if (q.xq) {
     xq = *q.xq;
     xs = *q.xs;
   } else if (digits == 3) {
@@ -345,6 +355,7 @@ at::Tensor w8a16_linear_split(const at::Tensor& x, const at::Tensor& wq, const a
   TORCH_CHECK(scale.numel() == n, "barlink: scale must have one entry per output channel");
   TORCH_CHECK(qlin_takes(x, k, act_int8), "barlink: w8a16_linear_split is for 1..", std::to_string(BL_QLIN_MAX_TOKENS),
               " 16-byte aligned rows, K % 16 == 0");
+  check_digits(x, k, !act_int8, xq, xs);
   c10::cuda::CUDAGuard guard(x.device());
   void* flag = w8_scratch(dev).err_flag.data_ptr();
   py::gil_scoped_release nogil;
@@ -387,7 +398,9 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   TORCH_CHECK(!(act_int8 && group_rel), "barlink: int8 activations go with per-channel or group_scale weight scales");
   // 1..128 tokens: the weights go to the tensor cores as they are (qlin_kernels.cu).  Group scales need
   // groups of whole 128-wide k-blocks.
-  if (qlin_takes(x, k, act_int8, bool(group_scale)) && (!group_rel || (k / group_rel->size(1)) % 128 == 0)) {
+  const bool by_qlin = qlin_takes(x, k, act_int8, bool(group_scale)) && (!group_rel || (k / group_rel->size(1)) % 128 == 0);
+  check_digits(x, k, by_qlin && !act_int8, xq_in, xs_in);
+  if (by_qlin) {
     QWeight q{wq.data_ptr(), 0, n, k, BL_QSCALE_BF16_N, scale.data_ptr()};
     q.xq = xq_in;
     q.xs = xs_in;

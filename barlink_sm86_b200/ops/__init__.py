@@ -303,12 +303,15 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None, digits=None)
     129..256 tokens widen the tile inside the main loop; other groups, and more than 256 tokens,
     widen the weight once and run the bf16 GEMM.
 
-    digits: those of x as `rmsnorm_digits` left them (up to 128 tokens, act="bf16").
+    digits: those of x as `rmsnorm_digits` left them (up to 128 tokens, act="bf16"; groups of a multiple of 128).
 
     act="int8": the activations are quantised per token to int8 first, as the reference does
     (w8a16.cu:37-92 there), one digit instead of three, for any number of tokens with per-channel
     scales, and for at most 64 tokens and 148 * 128 rows upwards with group scales.  act=None takes
     `w8_act_mode()`."""
+    xq, xs = digits if digits is not None else (None, None)
+    if digits is not None and not (x.is_cuda and (act or w8_act_mode()) == "bf16"):
+        raise ValueError("digits are for bf16 activations on a GPU")
     if x.is_cuda:
         k = wq.shape[1]
         gs = scale if isinstance(scale, W8GroupScales) else None
@@ -322,22 +325,24 @@ def w8a16_linear(x, wq, scale, bias=None, silu_mul=False, act=None, digits=None)
                 # scaled and summed by the epilogue warps
                 _count(2)
                 return _C().w8a16_linear(x, wq, scale, bias, silu_mul, act_int8=True, group_scale=scale.contiguous())
+        widen = None  # group scales of a weight that is widened first
         if gs is None and scale.dim() == 2:
             if (k // scale.shape[1]) % 64 == 0 and x.shape[0] <= 256:
                 _count()
                 gs = prepare_w8_scales(scale, k)
             else:
-                w = ref.w8_dequant(wq, scale).to(torch.bfloat16)
-                return linear(x, w, bias, silu_mul=silu_mul, dynamic_weights=True)
+                widen = scale
+        elif gs is not None and x.shape[0] > 256:
+            widen = gs.rel.float() * gs.row.float()[:, None]
+        if widen is not None:
+            if digits is not None:
+                raise ValueError("digits are of no use to weights that are widened first")
+            w = ref.w8_dequant(wq, widen).to(torch.bfloat16)
+            return linear(x, w, bias, silu_mul=silu_mul, dynamic_weights=True)
         _count(2 if _qlin_rows(x) and digits is None else 1)
         if gs is not None:
-            if x.shape[0] > 256:
-                w = (ref.w8_dequant(wq, gs.rel.float() * gs.row.float()[:, None])).to(torch.bfloat16)
-                return linear(x, w, bias, silu_mul=silu_mul, dynamic_weights=True)
-            return _C().w8a16_linear(x, wq, gs.row, bias, silu_mul, group_rel=gs.rel)
-        if digits is not None:
-            return _C().w8a16_linear(x, wq, scale, bias, silu_mul, xq=digits[0], xs=digits[1])
-        return _C().w8a16_linear(x, wq, scale, bias, silu_mul)
+            return _C().w8a16_linear(x, wq, gs.row, bias, silu_mul, group_rel=gs.rel, xq=xq, xs=xs)
+        return _C().w8a16_linear(x, wq, scale, bias, silu_mul, xq=xq, xs=xs)
     if isinstance(scale, W8GroupScales):
         scale = scale.rel.float() * scale.row.float()[:, None]
     return ref.w8a16_linear(x, wq, scale, bias, silu_mul)
@@ -355,9 +360,9 @@ def w8a16_linear_split(x, wq, scale, bias=None, digits=None):
     `linear_split`); else the bf16 result with the bias."""
     if x.is_cuda and _qlin_rows(x):
         xq, xs = digits if digits is not None else (None, None)
-        _count(2 if xq is None else 1)
+        _count(2 if digits is None else 1)
         return _C().w8a16_linear_split(x, wq, scale, bias, w8_act_mode() == "int8", xq, xs)
-    return w8a16_linear(x, wq, scale, bias)
+    return w8a16_linear(x, wq, scale, bias, digits=digits)
 
 
 __all__ = [

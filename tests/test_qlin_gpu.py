@@ -459,3 +459,30 @@ def test_widened_weights(ext, n, k):
     x[idx, idx] = 1  # rows of the widened weight itself
     want = (wq.float() * sc.float()[:, None]).bfloat16().t()[: len(idx)]
     assert torch.equal(ext.w8a16_linear(x, wq, sc)[: len(idx)], want)
+
+
+def test_digits_that_do_not_belong_are_refused(ext):
+    """Before any launch: half of a pair, other types or sizes, another device, and products that read no digits."""
+    from barlink_sm86_b200 import ops
+    m, k, n = 8, 1024, 96
+    wq, sc = _w8(n, k, 3)
+    x, _, xq, xs = ext.rmsnorm_digits(_x(m, k, 1), _x(1, k, 2)[0].contiguous(), 1e-6, None)
+    want = ext.w8a16_linear(x, wq, sc)
+    assert torch.equal(ext.w8a16_linear(x, wq, sc, xq=xq, xs=xs), want)
+    bad = [(xq, None), (None, xs), (xq.view(torch.uint8), xs), (xq, xs.view(torch.int32)), (xq.cpu(), xs), (xq, xs.cpu()),
+           (xq[1:], xs), (torch.cat([xq[:1], xq])[1:], xs), (torch.stack([xq, xq], 1)[:, 0], xs)]
+    for q, s in bad:
+        for call in (ext.w8a16_linear, ext.w8a16_linear_split):
+            with pytest.raises(RuntimeError, match="digits"):
+                call(x, wq, sc, xq=q, xs=s)
+    with pytest.raises(RuntimeError, match="digits"):
+        ext.w8a16_linear(x, wq, sc, act_int8=True, xq=xq, xs=xs)
+    with pytest.raises(RuntimeError, match="digits"):
+        ext.w8a16_linear(_x(200, k, 1), wq, sc, xq=xq, xs=xs)
+    with pytest.raises(ValueError, match="digits"):
+        ops.w8a16_linear(x, wq, sc, act="int8", digits=(xq, xs))
+    g32 = sc[:, None].expand(n, 32).contiguous()  # groups of 32: the weight is widened
+    with pytest.raises(ValueError, match="digits"):
+        ops.w8a16_linear(x, wq, g32, digits=(xq, xs))
+    gs = ops.prepare_w8_scales(sc[:, None].expand(n, k // 128).contiguous(), k)
+    assert torch.equal(ops.w8a16_linear(x, wq, gs, digits=(xq, xs)), ops.w8a16_linear(x, wq, gs))

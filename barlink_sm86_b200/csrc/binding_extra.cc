@@ -904,6 +904,8 @@ void bind_extra(py::module_& m) {
         py::arg("xq") = py::none(), py::arg("xs") = py::none());
   m.def("w8a16_linear_split", &w8a16_linear_split, py::arg("x"), py::arg("wq"), py::arg("scale"),
         py::arg("bias") = py::none(), py::arg("act_int8") = false, py::arg("xq") = py::none(), py::arg("xs") = py::none());
+  m.def("w4a16_splits", [](int m_, int n, int k) { return bl_w4a16_mma_splits(m_, n, k, 0, 0); }, py::arg("m"), py::arg("n"),
+        py::arg("k"));
   m.def("rmsnorm_digits", &rmsnorm_digits, py::arg("x"), py::arg("gamma"), py::arg("eps"), py::arg("residual") = py::none());
   m.def("w8_group_scales", &w8_group_scales, py::arg("scales"));
   m.def("w8_error_flag", &w8_error_flag, py::arg("device") = 0);

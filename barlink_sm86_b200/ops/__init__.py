@@ -8,6 +8,8 @@ reference's op surface is `w8a16_quant_act` / `w8a16_gemm`
 (torch_ext/barlink_sm86/binding.cpp:434-490); everything else here replaces
 library or eager-framework kernels that its demos call.
 """
+import functools
+
 import torch
 
 from .. import load_extension
@@ -160,14 +162,29 @@ def rope(x, positions, theta, axes=1):
     return ref.rope(x, positions, theta, axes)
 
 
+@functools.lru_cache(maxsize=1024)
+def _w4_splits(m, n, k):
+    return _C().w4a16_splits(m, n, k)
+
+
+def _w4_launches(x, qweight, scales, group, slabs):
+    """Kernels of an int4 linear: one for up to 16 rows in groups of 128 on aligned tensors, unless a k-split has to be
+    summed (no slabs wanted); else two."""
+    if (group == 128 and x.shape[0] <= 16 and (x.data_ptr() | qweight.data_ptr()) % 16 == 0 and scales.data_ptr() % 8 == 0
+            and (slabs or _w4_splits(x.shape[0], qweight.shape[1], x.shape[1]) == 1)):
+        return 1
+    return 2
+
+
 def w4a16_linear(x, qweight, scales, qzeros, group_size=128, silu_mul=False):
     """Weight-only int4 linear on GPTQ-v1 tensors (see `ref.pack_int4`), optionally with SiLU(gate) * up
     over interleaved (gate, up) columns.  Groups of 128: mma.sync up to 16 rows, the digit kernel up to 128;
     else a GEMV up to 16 rows; else widen + GEMM."""
     if x.is_cuda:
         x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
-        _count(1 if group_size == 128 and x2.shape[0] <= 16 else 2)
-        y = _C().w4a16_linear(x2.contiguous(), qweight, scales, qzeros, group_size, silu_mul=silu_mul)
+        x2 = x2.contiguous()
+        _count(_w4_launches(x2, qweight, scales, group_size, False))
+        y = _C().w4a16_linear(x2, qweight, scales, qzeros, group_size, silu_mul=silu_mul)
         return y if x.dim() == 2 else y.view(*x.shape[:-1], y.shape[-1])
     y = ref.w4a16_linear(x, qweight, scales, qzeros, group_size)
     return ref.silu_mul(y, True) if silu_mul else y
@@ -177,8 +194,9 @@ def w4a16_linear_split(x, qweight, scales, qzeros, group_size=128):
     """Decode-path form of `w4a16_linear`: fp32 slabs [splits, tokens, n] for the consumer to sum when the
     shape wants a k-split (see `linear_split`), else the bf16 result."""
     if x.is_cuda and x.dim() == 2:
-        _count(1 if group_size == 128 and x.shape[0] <= 16 else 2)
-        return _C().w4a16_linear(x.contiguous(), qweight, scales, qzeros, group_size, want_slabs=True)
+        x = x.contiguous()
+        _count(_w4_launches(x, qweight, scales, group_size, True))
+        return _C().w4a16_linear(x, qweight, scales, qzeros, group_size, want_slabs=True)
     return w4a16_linear(x, qweight, scales, qzeros, group_size)
 
 

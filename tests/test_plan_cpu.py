@@ -182,6 +182,22 @@ def test_mmdit_weight_bytes():
         assert MMDiTWeights(cfg, "cpu", torch.float32, 3, 2, rank).nbytes() == 4 * numbers(2)
 
 
+@pytest.mark.parametrize("m,n,k,launches", [(1, 37888, 3584, 1), (1, 3584, 18944, 2), (16, 3584, 18944, 1), (4, 8, 128, 1),
+                                            (17, 37888, 3584, 2)])
+def test_launches_of_int4_linears(m, n, k, launches):
+    """A k-split whose slabs nobody asked for is summed by a second kernel, and so is the GEMV that takes what is not aligned."""
+    from barlink_sm86_b200 import ops
+    x, qw, sc = torch.empty(m * k + 8, dtype=torch.bfloat16), torch.empty(k // 8, n, dtype=torch.int32), torch.empty(1).half()
+    at = (-x.data_ptr() % 16) // 2
+    row = x[at:at + m * k].view(m, k)
+    assert (ops._w4_splits(m, n, k) > 1) == (launches == 2) or m > 16
+    assert ops._w4_launches(row, qw, sc, 128, False) == launches
+    assert ops._w4_launches(row, qw, sc, 128, True) == (1 if m <= 16 else 2)
+    assert ops._w4_launches(row, qw, sc, 64, True) == 2
+    off = x[at + 1:at + 1 + m * k].view(m, k)
+    assert ops._w4_launches(off, qw, sc, 128, False) == 2
+
+
 def test_no_comm_control_skips_collectives():
     from barlink_sm86_b200.parallel import TPComm
     c = TPComm.single()

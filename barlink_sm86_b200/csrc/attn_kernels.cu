@@ -13,6 +13,7 @@
 
 #include "bl_ops.h"
 #include "heap.h"
+#include "launch.h"
 #include "ptx.cuh"
 
 namespace bl {
@@ -249,24 +250,20 @@ extern "C" int bl_attn_fwd(const void* q, const void* k, const void* v, void* ou
     return -1;
   }
   if (batch < 1 || max_q < 1) return 0;
-  static bool attr = false;
+  static bool attr[64] = {};
   const int smem = 4 * kATileBytes;
-  if (!attr) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_attn_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: dense attention shared memory opt-in failed: %s",
-              cudaGetErrorString(e));
-      return -1;
-    }
-    attr = true;
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_attn_fwd), smem, attr);
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: dense attention shared memory opt-in failed: %s",
+            cudaGetErrorString(e));
+    return -1;
   }
   dim3 grid((max_q + kQTile - 1) / kQTile, nq, batch);
   k_attn_fwd<<<grid, 128, smem, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
       static_cast<const __nv_bfloat16*>(v), static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq, nkv,
       q_stride, k_stride, v_stride, o_stride, scale * 1.4426950408889634f, causal);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: dense attention launch failed: %s", cudaGetErrorString(e));
     return -1;

@@ -473,21 +473,17 @@ extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void*
       make_tmap_kmajor(k, uint64_t(total_k), uint64_t(nkv) * kTcHD, uint64_t(k_stride), kTcBKV, 2, &tk, err, errlen) ||
       make_tmap_kmajor(v, uint64_t(total_k), uint64_t(nkv) * kTcHD, uint64_t(v_stride), kTcBKV, 2, &tv, err, errlen))
     return -1;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTcSmem));
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: tensor-core attention shared memory opt-in failed: %s", cudaGetErrorString(e));
-      return -1;
-    }
-    attr = true;
+  static bool attr[64] = {};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_attn_tc), int(kTcSmem), attr);
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: tensor-core attention shared memory opt-in failed: %s", cudaGetErrorString(e));
+    return -1;
   }
   const unsigned rblocks = unsigned((max_q + kTcTiles * kTcBM - 1) / (kTcTiles * kTcBM));
   // (a grid has at most 65535 blocks along y and z)
   const dim3 grid = causal ? dim3(nq, batch, rblocks) : dim3(rblocks, nq, batch);
-  cudaError_t e = launch_k(k_attn_tc, grid, dim3(kTcThreads), kTcSmem, st, tq, tk, tv,
-                           static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq, nkv, o_stride,
-                           scale * 1.4426950408889634f, causal, static_cast<uint32_t*>(err_flag));
+  e = launch_k(k_attn_tc, grid, dim3(kTcThreads), kTcSmem, st, tq, tk, tv, static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq,
+               nkv, o_stride, scale * 1.4426950408889634f, causal, static_cast<uint32_t*>(err_flag));
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: tensor-core attention launch failed: %s", cudaGetErrorString(e));

@@ -735,14 +735,11 @@ template <int BN, int CPS>
 static int launch_dlin(const CUtensorMap& tw, const CUtensorMap& tx, const DlinParams& p, int tiles, int cl,
                        cudaStream_t st, char* err, size_t errlen) {
   using S = DlinSmem<BN, CPS>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_dlin<BN, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
-      return -1;
-    }
-    attr_set = true;
+  static bool attr_set[64] = {};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_dlin<BN, CPS>), S::kBytes, attr_set);
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
+    return -1;
   }
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
@@ -759,7 +756,7 @@ static int launch_dlin(const CUtensorMap& tw, const CUtensorMap& tx, const DlinP
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k_dlin<BN, CPS>, tw, tx, p);
+  e = cudaLaunchKernelEx(&cfg, k_dlin<BN, CPS>, tw, tx, p);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: decode linear launch failed (grid %d, cluster %d): %s", tiles * cl, cl,

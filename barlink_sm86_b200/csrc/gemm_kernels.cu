@@ -552,16 +552,12 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
     ps.n = a.ra;
     ps.splits = g.splits;
     ps.tokens = a.rb;
-    static bool attr_q = false;
-    if (!attr_q) {
-      e = cudaFuncSetAttribute(k_gemm_peer<BN, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               S::kBytes);
-      if (e != cudaSuccess) {
-        set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes,
-                cudaGetErrorString(e));
-        return -1;
-      }
-      attr_q = true;
+    static bool attr_q[64] = {};
+    e = allow_smem(reinterpret_cast<const void*>(k_gemm_peer<BN, CPS>), S::kBytes, attr_q);
+    if (e != cudaSuccess) {
+      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes,
+              cudaGetErrorString(e));
+      return -1;
     }
     e = launch_k(k_gemm_peer<BN, CPS>, dim3(grid), dim3(kGemmThreads), size_t(S::kBytes), st, ta, tb,
                  g, ps, hint_w, hint_x);
@@ -574,16 +570,12 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
     ps.ra = a.ra;
     ps.rb = a.rb;
     ps.swap = a.swap;
-    static bool attr_p = false;
-    if (!attr_p) {
-      e = cudaFuncSetAttribute(k_gemm_partial<BN, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               S::kBytes);
-      if (e != cudaSuccess) {
-        set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes,
-                cudaGetErrorString(e));
-        return -1;
-      }
-      attr_p = true;
+    static bool attr_p[64] = {};
+    e = allow_smem(reinterpret_cast<const void*>(k_gemm_partial<BN, CPS>), S::kBytes, attr_p);
+    if (e != cudaSuccess) {
+      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes,
+              cudaGetErrorString(e));
+      return -1;
     }
     e = launch_k(k_gemm_partial<BN, CPS>, dim3(grid), dim3(kGemmThreads), size_t(S::kBytes), st, ta,
                  tb, g, ps, a.swap ? hint_w : hint_x, a.swap ? hint_x : hint_w);
@@ -600,16 +592,12 @@ static int launch_gemm(const blGemmArgs& a, int splits_want, cudaStream_t st, ch
     sink.scale = static_cast<const __nv_bfloat16*>(a.feat_scale);
     sink.xscale = static_cast<const float*>(a.tok_scale);
     fill_push(sink, a.push);
-    static bool attr_set = false;
-    if (!attr_set) {
-      e = cudaFuncSetAttribute(k_gemm<BN, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               S::kBytes);
-      if (e != cudaSuccess) {
-        set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes,
-                cudaGetErrorString(e));
-        return -1;
-      }
-      attr_set = true;
+    static bool attr_set[64] = {};
+    e = allow_smem(reinterpret_cast<const void*>(k_gemm<BN, CPS>), S::kBytes, attr_set);
+    if (e != cudaSuccess) {
+      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes,
+              cudaGetErrorString(e));
+      return -1;
     }
     if (g.i8) {
       using S1 = GemmSmem<BN, 1>;
@@ -717,15 +705,11 @@ static int launch_w8(const blW8A16Args& a, cudaStream_t st, char* err, size_t er
   sink.scale = static_cast<const __nv_bfloat16*>(a.scale);
   sink.xscale = nullptr;
   fill_push(sink, nullptr);
-  static bool attr = false;
-  cudaError_t e;
-  if (!attr) {
-    e = cudaFuncSetAttribute(k_gemm_w8<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
-      return -1;
-    }
-    attr = true;
+  static bool attr[64] = {};
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_gemm_w8<BN>), S::kBytes, attr);
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: cannot raise shared memory to %d B: %s", S::kBytes, cudaGetErrorString(e));
+    return -1;
   }
   e = launch_k(k_gemm_w8<BN>, dim3(grid), dim3(S::kThreads), size_t(S::kBytes), st, ta, tb, g, sink,
                kHintEvictFirst, kHintEvictLast);

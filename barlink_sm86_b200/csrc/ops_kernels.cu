@@ -1541,17 +1541,13 @@ extern "C" int bl_rope_attn_decode(const void* qkv, int q_stride, const void* sl
   src.slab = slab;
   src.bias = static_cast<const __nv_bfloat16*>(bias);
   src.width = (nq + 2 * nkv) * hd;
-  static bool attr = false;
+  static bool attr[64] = {};
   const int smem = kAttnWarps * kWarpSmem;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_rope_attn_decode,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) {
-      set_err(err, errlen, "barlink: paged attention shared memory opt-in failed: %s",
-              cudaGetErrorString(e));
-      return -1;
-    }
-    attr = true;
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(k_rope_attn_decode), smem, attr);
+  if (e != cudaSuccess) {
+    set_err(err, errlen, "barlink: paged attention shared memory opt-in failed: %s",
+            cudaGetErrorString(e));
+    return -1;
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const float scale_log2 = scale * 1.4426950408889634f;

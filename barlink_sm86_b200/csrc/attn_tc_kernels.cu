@@ -452,11 +452,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 
 using namespace bl;
 
-// Tensor-core dense attention.  `total_q` / `total_k` are the row counts of q and k (cu_q[batch], cu_k[batch]).
+extern "C" size_t bl_attn_tc_scratch_bytes(int, int, int) { return 0; }
+
+// Tensor-core dense attention.  `total_q`: rows of q; `total_k`: rows that k and v have (at least cu_k[batch]).
 extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void* out, const int* cu_q,
                               const int* cu_k, int batch, int max_q, int max_k, int total_q, int total_k,
                               int nq, int nkv, int hd, int q_stride, int k_stride, int v_stride,
-                              int o_stride, float scale, int causal, void* err_flag, void* stream,
+                              int o_stride, float scale, int causal, void* /* vt */, void* err_flag, void* stream,
                               char* err, size_t errlen) {
   if (hd != kTcHD || nkv < 1 || nq % nkv) {
     set_err(err, errlen, "barlink: tensor-core attention is built for head_dim %d and nq %% nkv == 0", kTcHD);

@@ -157,7 +157,7 @@ at::Tensor attn_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& 
     BL_CHECK(bl_attn_fwd_tc(q.data_ptr(), k.data_ptr(), vm.data_ptr(), out.data_ptr(), cu_q.data_ptr<int>(),
                             cu_k.data_ptr<int>(), batch, max_q, max_k, int(q.size(0)), rows, nq, nkv,
                             hd, int(q.stride(0)), int(k.stride(0)), v_stride, nq * hd, float(scale),
-                            causal ? 1 : 0, attn_err(q.device().index()).data_ptr(), st, err,
+                            causal ? 1 : 0, nullptr, attn_err(q.device().index()).data_ptr(), st, err,
                             errlen));
     return out;
   }

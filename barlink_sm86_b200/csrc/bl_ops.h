@@ -292,11 +292,13 @@ int bl_attn_fwd(const void* q, const void* k, const void* v, void* out, const in
                 const int* cu_k, int batch, int max_q, int nq, int nkv, int hd, int q_stride,
                 int k_stride, int v_stride, int o_stride, float scale, int causal, void* stream,
                 char* err, size_t errlen);
-/* same contract on the tcgen05 tensor cores (head_dim 128).  total_q / total_k: rows of q and k (and v); err_flag: a
- * device word set to 1 if a bounded wait inside the kernel ran out */
+/* same contract on the tcgen05 tensor cores (head_dim 128).  total_q: rows of q; total_k: rows that k and v both have, none
+ * beyond is read; vt: scratch of bl_attn_tc_scratch_bytes(), which is 0 (V is read as it lies; vt may be null); err_flag:
+ * a device word set to 1 if a bounded wait inside the kernel ran out */
+size_t bl_attn_tc_scratch_bytes(int batch, int max_k, int nkv);
 int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void* out, const int* cu_q, const int* cu_k,
                    int batch, int max_q, int max_k, int total_q, int total_k, int nq, int nkv, int hd,
-                   int q_stride, int k_stride, int v_stride, int o_stride, float scale, int causal,
+                   int q_stride, int k_stride, int v_stride, int o_stride, float scale, int causal, void* vt,
                    void* err_flag, void* stream, char* err, size_t errlen);
 /* arg max over the last dim of [rows x n] bf16 logits -> idx (int32) and
  * value (fp32); `offset` is added to the index (vocab-parallel shards). */

@@ -111,3 +111,17 @@ def test_widening_refuses_no_size(n, k):
     err = ctypes.create_string_buffer(512)
     assert fn(256, 256, 256, n, k, None, err, 512) == -1 and b"launch failed" in err.value
     assert fn(256, 256, 256, n, k - 4, None, err, 512) == -1 and b"multiple of 8" in err.value
+
+
+def test_plain_c_attention_takes_its_scratch_argument():
+    """The interface of bl_attn_fwd_tc has a scratch pointer, of which no bytes are used any more; a head_dim that it is
+    not built for is refused before anything is launched."""
+    lib = ctypes.CDLL(C.__file__)
+    lib.bl_attn_tc_scratch_bytes.restype = ctypes.c_size_t
+    assert lib.bl_attn_tc_scratch_bytes(8, 4096, 4) == 0
+    fn = lib.bl_attn_fwd_tc
+    fn.argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int] * 12 + [ctypes.c_float, ctypes.c_int] + [ctypes.c_void_p] * 3 \
+        + [ctypes.c_char_p, ctypes.c_size_t]
+    err = ctypes.create_string_buffer(512)
+    assert fn(*[None] * 6, 1, 8, 8, 8, 8, 4, 2, 64, 64, 64, 64, 64, 0.1, 1, None, None, None, err, 512) == -1
+    assert b"head_dim 128" in err.value

@@ -57,6 +57,7 @@ constexpr uint32_t kTcOffBar = kTcOffV + kTcStages * kTcVBytes;
 constexpr uint32_t kTcSmem = kTcOffBar + 256 + 1024;       // barriers + alignment slack
 static_assert(kTcSmem <= 232448, "attention tiles do not fit the shared memory of one CTA");
 constexpr uint32_t kTcTmemCols = 512;                      // S of tile t, step parity p: 128 t + 64 p, P in its first half; O of tile t: 256 + 128 t
+constexpr int kTcLastRowsFirst = 2;                        // in `causal`, beside 1
 constexpr float kTcRescale = 8.f;                          // log2 units
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -148,8 +149,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Causal: the later rows have more keys, so their blocks are dealt out first, over all heads and sequences
   // (8 x 1024, 28 heads on 4: 126.7 -> 123.7 us).
-  const int b = causal ? blockIdx.y : blockIdx.z, head = causal ? blockIdx.x : blockIdx.y, kvh = head / (nq / nkv);
-  const int rblock = causal ? int(gridDim.z - 1 - blockIdx.z) : int(blockIdx.x);
+  const bool last_first = causal & kTcLastRowsFirst;
+  const int b = last_first ? blockIdx.y : blockIdx.z, head = last_first ? blockIdx.x : blockIdx.y, kvh = head / (nq / nkv);
+  const int rblock = last_first ? int(gridDim.z - 1 - blockIdx.z) : int(blockIdx.x);
   const int q0 = cu_q[b], lq = cu_q[b + 1] - q0;
   const int k0 = cu_k[b], lk = cu_k[b + 1] - k0;
   const int row0 = rblock * (kTcTiles * kTcBM);   // first query row of this CTA in its sequence
@@ -482,10 +484,12 @@ extern "C" int bl_attn_fwd_tc(const void* q, const void* k, const void* v, void*
     return -1;
   }
   const unsigned rblocks = unsigned((max_q + kTcTiles * kTcBM - 1) / (kTcTiles * kTcBM));
-  // (a grid has at most 65535 blocks along y and z)
-  const dim3 grid = causal ? dim3(nq, batch, rblocks) : dim3(rblocks, nq, batch);
+  // (a grid has at most 65535 blocks along y and z, and max_q may be any bound of the lengths)
+  const bool last_first = causal && rblocks <= 65535;
+  const dim3 grid = last_first ? dim3(nq, batch, rblocks) : dim3(rblocks, nq, batch);
   e = launch_k(k_attn_tc, grid, dim3(kTcThreads), kTcSmem, st, tq, tk, tv, static_cast<__nv_bfloat16*>(out), cu_q, cu_k, nq,
-               nkv, o_stride, scale * 1.4426950408889634f, causal, static_cast<uint32_t*>(err_flag));
+               nkv, o_stride, scale * 1.4426950408889634f, causal ? (last_first ? 1 | kTcLastRowsFirst : 1) : 0,
+               static_cast<uint32_t*>(err_flag));
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_err(err, errlen, "barlink: tensor-core attention launch failed: %s", cudaGetErrorString(e));

@@ -76,3 +76,14 @@ def test_values_of_other_shapes_than_the_keys(ext):
         for lk in (l, 0):
             with pytest.raises(RuntimeError, match="head_dim"):
                 run(bad_k, bad_v, lk=lk)
+
+
+def test_max_q_is_a_bound(ext):
+    """Any bound of the sequence lengths does, also one of more row blocks than a grid has along z."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(700, h, 128, generator=g, device="cuda").bfloat16() for h in (2, 1, 1))
+    cu = torch.tensor([0, 130, 700], dtype=torch.int32, device="cuda")
+    for causal in (False, True):
+        want = ext.attn_fwd(q, k, v, cu, cu, 570, 0.088, causal, 570)
+        for bound in (1024, 256 * 65535 + 1):
+            assert torch.equal(ext.attn_fwd(q, k, v, cu, cu, bound, 0.088, causal, 570), want)

@@ -1175,6 +1175,44 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
   }
 }
 
+// Element d of a head from its splits.  They are read W at a time, the last ones of a count that is no multiple of W too: a
+// loop over the remainder, each load behind the exponential before it, made five to seven splits cost more than eight
+// (7B layer of 5 sequences at 600 tokens, us: 7 splits 100.6, now 99.1, 8 splits 99.4; 32B, 3 sequences, 6 splits
+// 115.9, now 114.7).  Fours for up to four: two splits in eights took 118.3 for 117.8 (7 sequences of the 32B layer).
+template <int W>
+__device__ __forceinline__ float merged_element(const float* __restrict__ base, int d, int nsplit) {
+  float M = -INFINITY;
+#pragma unroll 1
+  for (int s0 = 0; s0 < nsplit; s0 += W) {
+    float m[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i) m[i] = s0 + i < nsplit ? base[(s0 + i) * (kHd + 2) + kHd] : -INFINITY;
+#pragma unroll
+    for (int i = 0; i < W; ++i) M = fmaxf(M, m[i]);
+  }
+  float L = 0.f, acc = 0.f;
+#pragma unroll 1
+  for (int s0 = 0; s0 < nsplit; s0 += W) {
+    float m[W], l[W], a[W];
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      if (s0 + i < nsplit) {
+        const float* p = base + (s0 + i) * (kHd + 2);
+        m[i] = p[kHd];
+        l[i] = p[kHd + 1];
+        a[i] = p[d];
+      }
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      if (s0 + i < nsplit) {
+        const float sc = m[i] == -INFINITY ? 0.f : exp2f(m[i] - M);
+        L += l[i] * sc;
+        acc += a[i] * sc;
+      }
+  }
+  return L > 0.f ? acc / L : 0.f;
+}
+
 __global__ void __launch_bounds__(kHd) k_attn_merge(const float* __restrict__ scratch,
                                                     __nv_bfloat16* __restrict__ out, int nsplit) {
   pdl_launch_dependents();
@@ -1182,16 +1220,7 @@ __global__ void __launch_bounds__(kHd) k_attn_merge(const float* __restrict__ sc
   const size_t bh = blockIdx.x;  // batch*nq + head
   const float* base = scratch + bh * nsplit * (kHd + 2);
   const int d = threadIdx.x;
-  float M = -INFINITY;
-  for (int s = 0; s < nsplit; ++s) M = fmaxf(M, base[s * (kHd + 2) + kHd]);
-  float L = 0.f, acc = 0.f;
-  for (int s = 0; s < nsplit; ++s) {
-    const float mw = base[s * (kHd + 2) + kHd];
-    const float sc = mw == -INFINITY ? 0.f : exp2f(mw - M);
-    L += base[s * (kHd + 2) + kHd + 1] * sc;
-    acc += base[s * (kHd + 2) + d] * sc;
-  }
-  out[bh * kHd + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
+  out[bh * kHd + d] = __float2bfloat16(nsplit <= 4 ? merged_element<4>(base, d, nsplit) : merged_element<8>(base, d, nsplit));
 }
 
 // merge per-rank (value, index) pairs of a vocab-parallel arg max:
@@ -1442,10 +1471,12 @@ extern "C" int bl_paged_attn_decode(const void* q, int q_stride, const void* k_c
     return -1;
   }
   if (splits <= 0) {
-    // as many CTAs as SMs at most, so that all have the deep ring (8 sequences x 4 heads of 8000 tokens: five splits
-    // 3548 us a step, four 3491); more splits only add merge traffic.  From 64 CTAs
-    // on, splitting measured no faster than one CTA per (sequence, KV head) and costs the
-    // merge kernel, so it is not done.
+    // As many CTAs as SMs at most, so that all have the deep ring; more splits only add merge traffic.  Rounded down and
+    // up, us a layer at 600 / 1500 / 8000 tokens: 20 pairs (7 and 8 splits) 99.1 / 100.7 / 111.8 and 99.4 / 101.4 / 113.5,
+    // 32 pairs (4, 5) 100.1 / 102.9 / 119.7 and 100.9 / 104.7 / 121.4, 48 (3, 4) 102.3 / 106.1 / 128.7 and 103.1 / 107.5 / 132.0,
+    // 52 (2, 3: a third of the SMs without work) 102.6 / 108.0 / 135.4 and 104.1 / 109.3 / 135.5, 60 103.0 / 108.4 / 137.7 and
+    // 104.8 / 109.9 / 141.0.  From 64 CTAs on, splitting measured no faster than one CTA per (sequence, KV head) and
+    // costs the merge kernel, so it is not done.
     const int want = batch * nkv >= 64 ? 1 : sm_count() / (batch * nkv);
     const int by_len = max_blocks / (2 * kAttnWarps) > 0 ? max_blocks / (2 * kAttnWarps) : 1;
     splits = want < by_len ? want : by_len;

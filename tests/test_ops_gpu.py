@@ -179,6 +179,20 @@ def test_paged_attention_rings(ext, batch, nkv, splits):
     assert rel_l2(got, want) < 1e-2  # (probabilities and output rounded to bf16: 2^-8 each)
 
 
+@pytest.mark.parametrize("splits", [2, 3, 4, 5, 7, 8, 9, 15, 16, 17, 31, 32])
+def test_paged_attention_merge(ext, splits):
+    """Splits are merged in fours or eights; short contexts leave some of them empty."""
+    from barlink_sm86_b200.ops import reference as ref
+    nq, nkv, hd, bs, max_blocks = 14, 2, 128, 16, 40
+    ctx = torch.tensor([1, 100, 640], dtype=torch.int32, device="cuda")
+    kc, vc = _bf(3 * max_blocks, nkv, bs, hd, seed=1), _bf(3 * max_blocks, nkv, bs, hd, seed=2)
+    bt = torch.arange(3 * max_blocks, dtype=torch.int32, device="cuda").view(3, max_blocks)
+    qkv = _bf(3, (nq + 2 * nkv) * hd, seed=4)
+    got = ext.paged_attn_decode(qkv, kc, vc, bt, ctx, nq, nkv, hd, 1.0 / math.sqrt(hd), splits)
+    want = ref.paged_attn_decode(qkv, kc, vc, bt, ctx, nq, nkv, hd, 1.0 / math.sqrt(hd))
+    assert rel_l2(got, want) < 1e-2  # (probabilities and output rounded to bf16: 2^-8 each)
+
+
 @pytest.mark.parametrize("tokens,n,k,splits", [(64, 4608, 3584, 4), (8, 3584, 18944, 5), (1, 512, 1024, 2),
                                                (33, 640, 1024, 3)])
 def test_linear_split_slabs_sum_to_the_product(ext, tokens, n, k, splits):

@@ -174,6 +174,9 @@ void check_bf16x(const at::Tensor& t, const char* name) {
               " must be a contiguous bfloat16 CUDA tensor");
 }
 
+// kernels that read whole vectors: a tensor that starts between two of them (a view) is copied
+at::Tensor on_16_bytes(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0 ? t : t.clone(); }
+
 struct W8Scratch {
   at::Tensor ws, counters, err_flag;
 };
@@ -303,7 +306,7 @@ at::Tensor qlin_run(const at::Tensor& x, int digits, const QWeight& q, const c10
     BL_CHECK(bl_quant_digits(x.data_ptr(), m, int(x.stride(0)), q.k, q.src == 2 ? 1 : 0, xq.data_ptr(), xs.data_ptr(), st,
                              err, errlen));
   } else {
-    at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    const at::Tensor xc = on_16_bytes(x.contiguous());
     xs = at::empty({m}, x.options().dtype(at::kFloat));
     xq = at::empty({m, q.k}, x.options().dtype(at::kChar));
     BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, q.k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
@@ -423,7 +426,7 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
     // the reference's numerics (w8a16.cu:37-92 there quantises the activations per token and
     // multiplies int8 by int8): both operands go to the tensor cores as int8
     TORCH_CHECK(k % 16 == 0, "barlink: int8 activations need K % 16 == 0");
-    at::Tensor xc = x.is_contiguous() ? x : x.contiguous();
+    const at::Tensor xc = on_16_bytes(x.contiguous());
     at::Tensor xq = at::empty({m, k}, x.options().dtype(at::kChar));
     at::Tensor xs = at::empty({m}, x.options().dtype(at::kFloat));
     BL_CHECK(bl_w8a16_quant_act(xc.data_ptr(), m, k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
@@ -529,11 +532,12 @@ std::vector<at::Tensor> w8a16_quant_act(const at::Tensor& x) {
               "barlink w8a16_quant_act: x must be a contiguous 2-D bfloat16 CUDA tensor");
   const int m = int(x.size(0)), k = int(x.size(1));
   TORCH_CHECK(k % 8 == 0, "barlink w8a16_quant_act: K % 8 must be 0");
+  c10::cuda::CUDAGuard guard(x.device());
+  const at::Tensor xa = on_16_bytes(x);
   at::Tensor xq = at::empty({m, k}, x.options().dtype(at::kChar));
   at::Tensor xs = at::empty({m}, x.options().dtype(at::kFloat));
-  c10::cuda::CUDAGuard guard(x.device());
   void* st = at::cuda::getCurrentCUDAStream(x.device().index()).stream();
-  if (m > 0) BL_CHECK(bl_w8a16_quant_act(x.data_ptr(), m, k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
+  if (m > 0) BL_CHECK(bl_w8a16_quant_act(xa.data_ptr(), m, k, xq.data_ptr(), xs.data_ptr(), st, err, errlen));
   return {xq, xs};
 }
 
@@ -560,7 +564,7 @@ at::Tensor w8a16_gemm(const at::Tensor& xq, const at::Tensor& xs, const at::Tens
   if (splits > K / 128) splits = int(K / 128);
   void* flag = w8_scratch(dev).err_flag.data_ptr();
   py::gil_scoped_release nogil;
-  const at::Tensor xa = (reinterpret_cast<uintptr_t>(xq.data_ptr()) & 15u) == 0 ? xq : xq.clone();
+  const at::Tensor xa = on_16_bytes(xq);
   at::Tensor out = at::empty({m, N}, like), ws;
   if (splits > 1) ws = at::empty({splits, m, N}, like.dtype(at::kFloat));
   BL_CHECK(bl_w8a16_gemm(xa.data_ptr(), xs.data_ptr(), wq_t.data_ptr(), sw_t.data_ptr(), out.data_ptr(), m, int(N), int(K),

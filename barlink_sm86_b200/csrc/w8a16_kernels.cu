@@ -133,6 +133,10 @@ extern "C" int bl_w8a16_quant_act(const void* x, int m, int k, void* xq, void* x
     set_err(err, errlen, "barlink: w8a16_quant_act needs K a multiple of 8");
     return -1;
   }
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(xq) & 7u)) {
+    set_err(err, errlen, "barlink: w8a16_quant_act needs rows on 16-byte boundaries and digits on 8-byte ones");
+    return -1;
+  }
   auto go = [&](auto kern, int blocks, int threads) {
     return launch_k(kern, dim3(m * blocks), dim3(threads), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const __nv_bfloat16*>(x), static_cast<int8_t*>(xq), static_cast<float*>(xs), k);

@@ -486,3 +486,16 @@ def test_digits_that_do_not_belong_are_refused(ext):
         ops.w8a16_linear(x, wq, g32, digits=(xq, xs))
     gs = ops.prepare_w8_scales(sc[:, None].expand(n, k // 128).contiguous(), k)
     assert torch.equal(ops.w8a16_linear(x, wq, gs, digits=(xq, xs)), ops.w8a16_linear(x, wq, gs))
+
+
+@pytest.mark.parametrize("m,k", [(3, 1024), (300, 4104)])
+def test_rows_between_two_vectors_are_quantised(ext, m, k):
+    """Rows that start off a 16-byte boundary give what their copy gives."""
+    buf = _x(1, m * k + 8, 3)[0]
+    wq, sc = _w8(96, k, 3)
+    for off in (1, 4):
+        x = buf[off:off + m * k].view(m, k)
+        (q, s), (q0, s0) = ext.w8a16_quant_act(x), ext.w8a16_quant_act(x.clone())
+        assert torch.equal(q, q0) and torch.equal(s, s0)
+        if k % 16 == 0:
+            assert torch.equal(ext.w8a16_linear(x, wq, sc, act_int8=True), ext.w8a16_linear(x.clone(), wq, sc, act_int8=True))

@@ -645,7 +645,8 @@ at::Tensor w4a16_linear(const at::Tensor& x, const at::Tensor& qweight, const at
     return finish(at::matmul(x, w.t()));  // prefill path, not the decode hot path
   }
   at::Tensor out = at::empty({m, n}, x.options());
-  BL_CHECK(bl_w4a16_gemv(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), out.data_ptr(),
+  const at::Tensor words = on_16_bytes(qweight), sc = on_16_bytes(scales);
+  BL_CHECK(bl_w4a16_gemv(x.data_ptr(), words.data_ptr(), sc.data_ptr(), qzeros.data_ptr(), out.data_ptr(),
                          m, n, k, group, splits, s.ws.data_ptr(), size_t(s.ws.nbytes()), st, err, errlen));
   return finish(out);
 }

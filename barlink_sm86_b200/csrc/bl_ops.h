@@ -321,7 +321,8 @@ int bl_decode_advance(int* positions, int* ctx_lens, int* slots, const int* bloc
 
 /* ---- W4A16: GPTQ-v1 int4 weights, bf16 activations -------------------------- */
 /* y[m, n] = sum_k x[m, k] * (nibble(n, k) - zero(g, n)) * scale(g, n); 1..16 rows;
- * splits <= 0: chosen here; a k-split needs ws of splits*m*n floats.  -2: too many rows */
+ * splits <= 0: chosen here; a k-split needs ws of splits*m*n floats.  qweight and ws on 16-byte
+ * boundaries, scales and out on 8-byte ones.  -2: too many rows */
 int bl_w4a16_gemv(const void* x, const void* qweight, const void* scales, const void* qzeros, void* out,
                   int m, int n, int k, int group, int splits, void* ws, size_t ws_bytes, void* stream,
                   char* err, size_t errlen);

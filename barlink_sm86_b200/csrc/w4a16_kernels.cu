@@ -369,6 +369,11 @@ extern "C" int bl_w4a16_gemv(const void* x, const void* qweight, const void* sca
     return -2;
   }
   if (w4_check(n, k, group, err, errlen)) return -1;
+  if ((reinterpret_cast<uintptr_t>(qweight) | reinterpret_cast<uintptr_t>(ws)) & 15u ||
+      (reinterpret_cast<uintptr_t>(scales) | reinterpret_cast<uintptr_t>(out)) & 7u) {
+    set_err(err, errlen, "barlink: w4a16_gemv needs words and workspace on 16-byte boundaries, scales and output on 8-byte ones");
+    return -1;
+  }
   const int G = k / group;
   const int nblocks = (n / 4 + kW4Threads - 1) / kW4Threads;
   if (splits <= 0) {

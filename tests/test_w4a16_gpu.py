@@ -83,3 +83,20 @@ def test_w4a16_groups_of_128(ext, k, n, m):
         # (SiLU * up of fp32 sums; __expf and the division are good to some 1e-6)
         for splits in (0, 1):
             assert rel_l2(ext.w4a16_linear(x, qw, sc, qz, 128, splits, True), silu) < tol + 1e-5
+
+
+@pytest.mark.parametrize("group,m", [(64, 1), (64, 16), (128, 3), (128, 9), (128, 40)])
+def test_w4a16_words_and_scales_between_two_vectors(ext, group, m):
+    """Weights that are views at an odd offset: the same as their copies (groups of 128: as another kernel's result)."""
+    from barlink_sm86_b200 import ops
+    k, n = 512, 264
+    g = torch.Generator(device="cuda").manual_seed(m)
+    buf = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // 8 * n + 4,), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    qz = torch.randint(-2 ** 31, 2 ** 31 - 1, (k // group, n // 8), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    sbuf = (torch.rand(k // group * n + 4, generator=g, device="cuda") * 0.01 + 1e-3).half()
+    x = torch.randn(m, k, generator=g, device="cuda").bfloat16()
+    for off, soff in ((0, 1), (1, 0), (2, 2), (3, 3)):
+        qw, sc = buf[off:off + k // 8 * n].view(k // 8, n), sbuf[soff:soff + k // group * n].view(k // group, n)
+        got, want = ops.w4a16_linear(x, qw, sc, qz, group), ops.w4a16_linear(x, qw.clone(), sc.clone(), qz, group)
+        # (each result rounded to bf16, and from 17 rows the widened weights too: some 2^-9.2 of the norm apiece)
+        assert torch.equal(got, want) if group == 64 else rel_l2(got, want) < 2.0 ** -8

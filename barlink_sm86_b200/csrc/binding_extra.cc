@@ -481,7 +481,8 @@ at::Tensor w8a16_linear(const at::Tensor& x, const at::Tensor& wq, const at::Ten
   }
   if (m > 256) {
     at::Tensor w = at::empty({n, k}, x.options());
-    BL_CHECK(bl_w8_dequant(wq.data_ptr(), scale.data_ptr(), w.data_ptr(), n, k, st, err, errlen));
+    const at::Tensor wa = (reinterpret_cast<uintptr_t>(wq.data_ptr()) & 7u) == 0 ? wq : wq.clone();  // (read 8 bytes at a time)
+    BL_CHECK(bl_w8_dequant(wa.data_ptr(), scale.data_ptr(), w.data_ptr(), n, k, st, err, errlen));
     py::object lin = py::module_::import("barlink_sm86_b200").attr("load_extension")().attr("linear");
     // `w` was written by the kernel just launched: the GEMM must not fetch weight tiles ahead of
     // that kernel's completion (its producer otherwise requests them before griddepcontrol.wait)

@@ -1138,6 +1138,10 @@ extern "C" int bl_w8_dequant(const void* wq, const void* scale, void* out, int n
     set_err(err, errlen, "barlink: w8_dequant needs K a multiple of 8");
     return -1;
   }
+  if ((reinterpret_cast<uintptr_t>(wq) & 7u) || (reinterpret_cast<uintptr_t>(out) & 15u)) {
+    set_err(err, errlen, "barlink: w8_dequant needs weights on an 8-byte boundary and its output on a 16-byte one");
+    return -1;
+  }
   // the kernel numbers eight weights with 32 bits: rows in launches of fewer than 2^32 of them
   const size_t per_row = size_t(k) / 8, rows_most = kW8DequantMost / per_row;
   for (size_t r = 0; r < size_t(n); r += rows_most) {

@@ -499,3 +499,16 @@ def test_rows_between_two_vectors_are_quantised(ext, m, k):
         assert torch.equal(q, q0) and torch.equal(s, s0)
         if k % 16 == 0:
             assert torch.equal(ext.w8a16_linear(x, wq, sc, act_int8=True), ext.w8a16_linear(x.clone(), wq, sc, act_int8=True))
+
+
+def test_widened_weights_between_two_vectors(ext):
+    """Prefill on int8 weights that are a view at any byte."""
+    n, k = 160, 1024
+    wq, sc = _w8(n, k, 3)
+    x = _x(300, k, 2)
+    want = ext.w8a16_linear(x, wq, sc)
+    for off in (1, 4, 8):
+        buf = torch.empty(n * k + 16, dtype=torch.int8, device="cuda")
+        view = buf[off:off + n * k].view(n, k)
+        view.copy_(wq)
+        assert torch.equal(ext.w8a16_linear(x, view, sc), want)

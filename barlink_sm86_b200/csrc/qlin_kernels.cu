@@ -609,11 +609,17 @@ __device__ __forceinline__ uint32_t bf16x2_absmax_bits(uint32_t m, uint32_t v) {
   m = max(m, v & 0x7fffu);
   return max(m, (v >> 16) & 0x7fffu);
 }
+__device__ __forceinline__ uint32_t bf16x8_absmax_bits(uint32_t m, const uint4& v) {
+  m = bf16x2_absmax_bits(bf16x2_absmax_bits(m, v.x), v.y);
+  return bf16x2_absmax_bits(bf16x2_absmax_bits(m, v.z), v.w);
+}
 // The digits of a row that the blocks of a cluster (CL of them, or one) hold in registers: vector i of a thread is vector
 // threadIdx.x + i * kDigThreads of its block's share, which is `vecs` long and starts at vector `first` of the row; every
-// block but the last has `per` of them.
+// block but the last has `per` of them.  mx: the largest |x| of the thread's vectors as bf16 bits, ordered like the values,
+// NaN above infinity (found while they are loaded: in a loop of its own behind the loads it cost rows of eight vectors a
+// thread half as many spills again, 12.2 us for 11.6).
 template <bool PERMUTE, int VPT, int CL>
-__device__ __forceinline__ void digits_of_row(uint4 (&v)[VPT], int row, int rows, int first, int per, int vecs, int k, int tb,
+__device__ __forceinline__ void digits_of_row(uint4 (&v)[VPT], uint32_t mx, int row, int rows, int first, int per, int vecs, int k, int tb,
                                               int8_t* __restrict__ xq, float* __restrict__ xs) {
   // (little shared memory: a block of these kernels fits beside one of k_qlin, which has nearly all of it)
   __shared__ uint32_t s_red[kDigThreads / 32];
@@ -627,12 +633,6 @@ __device__ __forceinline__ void digits_of_row(uint4 (&v)[VPT], int row, int rows
     cluster_sync_all();
     turn ^= 1;
   };
-  uint32_t mx = 0;  // largest |x| as bf16 bits: ordered like the values, NaN above infinity
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].x), v[i].y);
-    mx = bf16x2_absmax_bits(bf16x2_absmax_bits(mx, v[i].z), v[i].w);
-  }
   mx = __reduce_max_sync(0xffffffffu, mx);
   if (lane == 0) s_red[warp] = mx;
   __syncthreads();
@@ -749,12 +749,14 @@ __device__ __forceinline__ void quant_digits_body(const __nv_bfloat16* __restric
   const int first = CL > 1 ? int(cluster_ctarank()) * per : 0, vecs = max(0, min(per, (k >> 3) - first));
   const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * ldx) + first;
   uint4 v[VPT];
+  uint32_t mx = 0;
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = threadIdx.x + i * kDigThreads;
     v[i] = c < vecs ? xr[c] : make_uint4(0, 0, 0, 0);
+    mx = bf16x8_absmax_bits(mx, v[i]);
   }
-  digits_of_row<PERMUTE, VPT, CL>(v, row, gridDim.x / CL, first, per, vecs, k, tb, xq, xs);
+  digits_of_row<PERMUTE, VPT, CL>(v, mx, row, gridDim.x / CL, first, per, vecs, k, tb, xq, xs);
 }
 template <bool PERMUTE, int VPT>
 __global__ void __launch_bounds__(kDigThreads, 2) k_quant_digits(const __nv_bfloat16* __restrict__ x, int ldx, int k, int tb,
@@ -869,7 +871,10 @@ __global__ void __launch_bounds__(kDigThreads, 2)
   pdl_wait();
   uint4 v[VPT];
   norm_row<VPT>(v, x, residual, gamma, out, residual_out, vpr, eps, partials, nsplit, slab);
-  digits_of_row<false, VPT, 1>(v, blockIdx.x, gridDim.x, 0, vpr, vpr, vpr * 8, tb, xq, xs);
+  uint32_t mx = 0;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) mx = bf16x8_absmax_bits(mx, v[i]);
+  digits_of_row<false, VPT, 1>(v, mx, blockIdx.x, gridDim.x, 0, vpr, vpr, vpr * 8, tb, xq, xs);
 }
 
 // fp32 slabs [split][m][pitch] -> bf16 [m][n]: sum in split order, then what the epilogue of the unsplit product

@@ -141,12 +141,13 @@ extern "C" int bl_w8a16_quant_act(const void* x, int m, int k, void* xq, void* x
     return launch_k(kern, dim3(m * blocks), dim3(threads), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const __nv_bfloat16*>(x), static_cast<int8_t*>(xq), static_cast<float*>(xs), k);
   };
-  // blocks of a row: one vector a thread, as long as there is an SM for every block
-  const int need = (k / 8 + kQaThreads - 1) / kQaThreads, cl = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : 8;
+  // Blocks of a row: one vector a thread, as long as there is an SM for every block.  Not clusters of two: rows of 5120
+  // elements take them longer than one block and two passes (the reference's pair on a 32B layer, 8 tokens: 120.2 us and
+  // 118.2; per-channel scales, 64 tokens: 127.2 and 126.1; group scales 277 and 267).
+  const int need = (k / 8 + kQaThreads - 1) / kQaThreads, cl = need <= 1 ? 1 : need <= 4 ? 4 : 8;
   cudaError_t e;
-  if (need > 8 || m * cl > sm_count()) e = go(k_quant_act, 1, kQThreads);
+  if (need == 2 || need > 8 || m * cl > sm_count()) e = go(k_quant_act, 1, kQThreads);
   else if (cl == 1) e = go(k_quant_act_cluster<1>, 1, kQaThreads);
-  else if (cl == 2) e = go(k_quant_act_cluster<2>, 2, kQaThreads);
   else if (cl == 4) e = go(k_quant_act_cluster<4>, 4, kQaThreads);
   else e = go(k_quant_act_cluster<8>, 8, kQaThreads);
   if (e == cudaSuccess) e = cudaGetLastError();

@@ -87,13 +87,22 @@ struct QlinCfg {
   static constexpr int kScales = GROUPED ? 8 * kQRows * 4 : 0;   // group scales of eight k-blocks
   static constexpr int kFit = (226 * 1024 - 2048 - kScales - kA8 * kQTileA) / kStage;
   static constexpr int kStages = kFit > 10 ? 10 : kFit;
-  static constexpr int kSmem = kStages * kStage + kA8 * kQTileA + kScales + 2048;
+  // Barriers, then the ring on a 1024-byte boundary, and no byte more: the blocks of the kernels before and after (quantisers,
+  // norms, RoPE) fit beside one of this kernel only if it leaves them 1 KB and what they declare.  With 640 bytes more the
+  // stages of 32 tokens left them 1 KB: a norm that writes digits waited for an SM without such a block, and took longer
+  // than norm and quantiser apart.  Norm of four slabs and product of 24 rows, us, apart / together / together now:
+  // 4608 x 3584 11.2 / 11.8 / 10.6, 7168 x 5120 16.0 / 16.6 / 14.4; 5120 x 27648 alone, 20 rows, 41.7 -> 36.4.
+  static constexpr int kBars = 384;
+  static constexpr int kSmem = kStages * kStage + kA8 * kQTileA + kScales + kBars + 1024;
   // per-group mode hands an accumulator over every k-block: four of them where they fit
   static constexpr int kAcc = GROUPED && 4 * BN <= 512 ? 4 : 2;
   static constexpr int kCols = kAcc * BN <= 32 ? 32 : kAcc * BN <= 64 ? 64 : kAcc * BN <= 128 ? 128 : kAcc * BN <= 256 ? 256 : 512;
   static constexpr int kExpand = SRC == kNibbles ? 256 : 0;
   static constexpr int kThreads = 192 + kExpand;
   static_assert(kStages >= 3 && kAcc * BN <= 512 && kStage % 1024 == 0, "stage ring / TMEM do not fit");
+  static_assert((2 * kStages + 16) * 8 + 8 <= kBars, "barriers");
+  // 228 KB an SM, of which every block takes 1 KB itself; up to 256 bytes for a block beside this one
+  static_assert(kSmem + 2 * 1024 + 256 <= 228 * 1024, "nothing fits beside a block");
 };
 
 // K-major tile of 16-byte chunks [chunk][row][16 B], no swizzle: eight rows of one chunk are a 128-byte
@@ -193,7 +202,7 @@ __global__ void __launch_bounds__(QlinCfg<SRC, ND, TB, GROUPED>::kThreads, 1)
   uint64_t* afree_bar = ready_bar + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(afree_bar + 4);
   volatile uint32_t* s_abort = tmem_slot + 1;
-  const uint32_t ring = (smem_u32(smem_raw) + 1024u + 1023u) & ~1023u;
+  const uint32_t ring = (smem_u32(smem_raw) + uint32_t(S::kBars) + 1023u) & ~1023u;
   const uint32_t ring_a8 = ring + S::kStages * S::kStage;
 
   pdl_launch_dependents();

@@ -628,26 +628,28 @@ __global__ void __launch_bounds__(GemmSmem<BN, 1, true>::kThreads, 1)
   gemm_body<BN, 1, true>(&tmap_a, &tmap_b, g, sink, hint_a, hint_b);
 }
 constexpr size_t kW8DequantMost = 0xfffff000u;  // eights of weights in a launch
-// Eight weights a thread and vector (16-byte stores side by side), four vectors requested together, 32-bit row numbers:
-// the weights of a 7B layer 146 us, 137 so (37888 x 3584: 79 and 74; a 64-bit division per vector and one request at a time
-// before).  16 weights a thread, two stores 32 bytes apart in every lane, took 173.
+// Eight weights a thread and vector (16-byte stores side by side), V vectors requested together, 32-bit row numbers.  Bound by
+// memory where the weight is large: the weights of a 7B layer 146 us, 137 with four vectors (37888 x 3584: 79 and 74; a 64-bit
+// division per vector and one request at a time before); 16 weights a thread, two stores 32 bytes apart in every lane, took 173.
+// A small one has too few blocks for that: see w8_dequant_vectors.
+template <int V>
 __global__ void __launch_bounds__(256) k_w8_dequant(const int8_t* __restrict__ wq, const __nv_bfloat16* __restrict__ scale,
                                                     __nv_bfloat16* __restrict__ out, uint32_t vecs, uint32_t per_row) {
   pdl_launch_dependents();
   pdl_wait();
-  for (size_t b = blockIdx.x; b * 1024 < vecs; b += gridDim.x) {
-    uint2 w[4];
-    float sc[4];
+  for (size_t b = blockIdx.x; b * (V * 256) < vecs; b += gridDim.x) {
+    uint2 w[V];
+    float sc[V];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t t = uint32_t(b) * 1024 + i * 256 + threadIdx.x;
+    for (int i = 0; i < V; ++i) {
+      const uint32_t t = uint32_t(b) * (V * 256) + i * 256 + threadIdx.x;
       if (t >= vecs) continue;
       w[i] = __ldcs(reinterpret_cast<const uint2*>(wq) + t);
       sc[i] = __bfloat162float(scale[t / per_row]);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t t = uint32_t(b) * 1024 + i * 256 + threadIdx.x;
+    for (int i = 0; i < V; ++i) {
+      const uint32_t t = uint32_t(b) * (V * 256) + i * 256 + threadIdx.x;
       if (t >= vecs) continue;
       uint32_t p, q, r, s;
       s8x4_to_bf16x4(w[i].x, p, q);
@@ -657,6 +659,13 @@ __global__ void __launch_bounds__(256) k_w8_dequant(const int8_t* __restrict__ w
                                                     pack_bf16x2(f2.x * sc[i], f2.y * sc[i]), pack_bf16x2(f3.x * sc[i], f3.y * sc[i]));
     }
   }
+}
+// Vectors of a thread.  Widening and product of 257 rows, us, with one vector a thread, two and four: 512 x 512 9.6 / 10.1 / 10.7;
+// 1024 x 1024 13.0 / 12.8 / 13.7, 1024 x 2048 15.5 / 15.6 / 17.9, 4096 x 1024 15.1 / 14.8 / 16.3, 3584 x 3584 (1.6 million
+// vectors) 31.6 / 31.2 / 31.4; 5120 x 5120 at 1000 rows 69.9 / 69.3 / 68.9.
+static int w8_dequant_vectors(size_t vecs) {
+  if (vecs <= size_t(148) * 512) return 1;  // with two, an SM would go without a block
+  return vecs <= 2000000 ? 2 : 4;
 }
 
 template <int BN>
@@ -1145,8 +1154,11 @@ extern "C" int bl_w8_dequant(const void* wq, const void* scale, void* out, int n
   // the kernel numbers eight weights with 32 bits: rows in launches of fewer than 2^32 of them
   const size_t per_row = size_t(k) / 8, rows_most = kW8DequantMost / per_row;
   for (size_t r = 0; r < size_t(n); r += rows_most) {
-    const size_t vecs = std::min(rows_most, size_t(n) - r) * per_row, blocks = std::min((vecs + 1023) / 1024, size_t(148) * 8);
-    cudaError_t e = launch_k(k_w8_dequant, dim3(unsigned(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    const size_t vecs = std::min(rows_most, size_t(n) - r) * per_row;
+    const int v = w8_dequant_vectors(vecs);
+    const size_t blocks = std::min((vecs + v * 256 - 1) / (v * 256), size_t(148) * 8);
+    cudaError_t e = launch_k(v == 1 ? k_w8_dequant<1> : v == 2 ? k_w8_dequant<2> : k_w8_dequant<4>, dim3(unsigned(blocks)),
+                             dim3(256), 0, static_cast<cudaStream_t>(stream),
                              static_cast<const int8_t*>(wq) + r * k, static_cast<const __nv_bfloat16*>(scale) + r,
                              static_cast<__nv_bfloat16*>(out) + r * k, uint32_t(vecs), uint32_t(per_row));
     if (e == cudaSuccess) e = cudaGetLastError();

@@ -461,6 +461,17 @@ def test_widened_weights(ext, n, k):
     assert torch.equal(ext.w8a16_linear(x, wq, sc)[: len(idx)], want)
 
 
+@pytest.mark.parametrize("n,k", [(5, 24), (592, 1024), (593, 1024), (4000, 4000), (4001, 4000)])
+def test_widened_weights_by_size(ext, n, k):
+    """One, two and four vectors a thread, on both sides of the lines between them: first and last columns."""
+    wq, sc = _w8(n, k, 3)
+    want = (wq.float() * sc.float()[:, None]).bfloat16().t()
+    for idx in (torch.arange(min(300, k), device="cuda"), torch.arange(max(0, k - 300), k, device="cuda")):
+        x = torch.zeros(300, k, device="cuda").bfloat16()
+        x[torch.arange(len(idx), device="cuda"), idx] = 1
+        assert torch.equal(ext.w8a16_linear(x, wq, sc)[: len(idx)], want[idx])
+
+
 def test_digits_that_do_not_belong_are_refused(ext):
     """Before any launch: half of a pair, other types or sizes, another device, and products that read no digits."""
     from barlink_sm86_b200 import ops

@@ -1175,39 +1175,42 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
   }
 }
 
-// Element d of a head from its splits.  They are read W at a time, the last ones of a count that is no multiple of W too: a
-// loop over the remainder, each load behind the exponential before it, made five to seven splits cost more than eight
-// (7B layer of 5 sequences at 600 tokens, us: 7 splits 100.6, now 99.1, 8 splits 99.4; 32B, 3 sequences, 6 splits
-// 115.9, now 114.7).  Fours for up to four: two splits in eights took 118.3 for 117.8 (7 sequences of the 32B layer).
+// Element d of a head from its splits.  Bound by its trips to memory: a lane fetches maximum and sum of one split (32 of them a
+// lap), and the elements of W splits are on their way meanwhile, so that up to 32 splits take one trip.  Attention and merge,
+// us, with every thread reading all maxima first, then splits one by one or four at a time / in fours and eights / so (all same
+// bits): 28 heads on 4, one sequence of 8000 tokens, 32 splits, 11.2 / 11.7 / 8.1; five of 600, 7 splits 8.1 / 6.6 / 5.9;
+// 40 on 8, seven of 600, 2 splits 8.1 / 7.9 / 7.5.
 template <int W>
 __device__ __forceinline__ float merged_element(const float* __restrict__ base, int d, int nsplit) {
-  float M = -INFINITY;
+  const int lane = threadIdx.x & 31;
+  float a[W];
+  auto load = [&](int s0) {
+#pragma unroll
+    for (int i = 0; i < W; ++i)
+      if (s0 + i < nsplit) a[i] = base[(s0 + i) * (kHd + 2) + d];
+  };
+  float m = -INFINITY, l = 0.f;
+  auto head = [&](int s) {
+    m = s < nsplit ? base[s * (kHd + 2) + kHd] : -INFINITY;
+    l = s < nsplit ? base[s * (kHd + 2) + kHd + 1] : 0.f;
+  };
+  head(lane);
+  load(0);
+  float M = m, L = 0.f, acc = 0.f;
+  for (int s = 32 + lane; s < nsplit; s += 32) M = fmaxf(M, base[s * (kHd + 2) + kHd]);
+  M = warp_max(M);
 #pragma unroll 1
   for (int s0 = 0; s0 < nsplit; s0 += W) {
-    float m[W];
-#pragma unroll
-    for (int i = 0; i < W; ++i) m[i] = s0 + i < nsplit ? base[(s0 + i) * (kHd + 2) + kHd] : -INFINITY;
-#pragma unroll
-    for (int i = 0; i < W; ++i) M = fmaxf(M, m[i]);
-  }
-  float L = 0.f, acc = 0.f;
-#pragma unroll 1
-  for (int s0 = 0; s0 < nsplit; s0 += W) {
-    float m[W], l[W], a[W];
+    if (s0 > 0) load(s0);
+    if (s0 > 0 && (s0 & 31) == 0) head(s0 + lane);
+    const float sc = m == -INFINITY ? 0.f : exp2f(m - M);
 #pragma unroll
     for (int i = 0; i < W; ++i)
       if (s0 + i < nsplit) {
-        const float* p = base + (s0 + i) * (kHd + 2);
-        m[i] = p[kHd];
-        l[i] = p[kHd + 1];
-        a[i] = p[d];
-      }
-#pragma unroll
-    for (int i = 0; i < W; ++i)
-      if (s0 + i < nsplit) {
-        const float sc = m[i] == -INFINITY ? 0.f : exp2f(m[i] - M);
-        L += l[i] * sc;
-        acc += a[i] * sc;
+        const int from = (s0 & 31) + i;
+        const float w = __shfl_sync(0xffffffffu, sc, from);
+        L += __shfl_sync(0xffffffffu, l, from) * w;
+        acc += a[i] * w;
       }
   }
   return L > 0.f ? acc / L : 0.f;
@@ -1220,7 +1223,7 @@ __global__ void __launch_bounds__(kHd) k_attn_merge(const float* __restrict__ sc
   const size_t bh = blockIdx.x;  // batch*nq + head
   const float* base = scratch + bh * nsplit * (kHd + 2);
   const int d = threadIdx.x;
-  out[bh * kHd + d] = __float2bfloat16(nsplit <= 4 ? merged_element<4>(base, d, nsplit) : merged_element<8>(base, d, nsplit));
+  out[bh * kHd + d] = __float2bfloat16(nsplit <= 8 ? merged_element<8>(base, d, nsplit) : merged_element<32>(base, d, nsplit));
 }
 
 // merge per-rank (value, index) pairs of a vocab-parallel arg max:
@@ -1472,10 +1475,10 @@ extern "C" int bl_paged_attn_decode(const void* q, int q_stride, const void* k_c
   }
   if (splits <= 0) {
     // As many CTAs as SMs at most, so that all have the deep ring; more splits only add merge traffic.  Rounded down and
-    // up, us a layer at 600 / 1500 / 8000 tokens: 20 pairs (7 and 8 splits) 99.1 / 100.7 / 111.8 and 99.4 / 101.4 / 113.5,
-    // 32 pairs (4, 5) 100.1 / 102.9 / 119.7 and 100.9 / 104.7 / 121.4, 48 (3, 4) 102.3 / 106.1 / 128.7 and 103.1 / 107.5 / 132.0,
-    // 52 (2, 3: a third of the SMs without work) 102.6 / 108.0 / 135.4 and 104.1 / 109.3 / 135.5, 60 103.0 / 108.4 / 137.7 and
-    // 104.8 / 109.9 / 141.0.  From 64 CTAs on, splitting measured no faster than one CTA per (sequence, KV head) and
+    // up, us from the QKV to the o linear of a 7B layer at 600 / 1500 / 8000 tokens: 20 pairs (7 and 8 splits) 23.0 / 24.4 / 34.5
+    // and 23.9 / 25.6 / 36.7, 32 pairs (4, 5) 23.8 / 25.8 / 42.6 and 24.8 / 27.4 / 44.2, 48 (3, 4) 24.7 / 28.3 / 51.2 and
+    // 25.7 / 29.0 / 53.2, 52 (2, 3: a third of the SMs without work) 25.2 / 29.6 / 57.5 and 26.4 / 30.4 / 57.5, 60
+    // 25.2 / 30.1 / 60.7 and 26.7 / 30.7 / 62.9.  From 64 CTAs on, splitting measured no faster than one CTA per (sequence, KV head) and
     // costs the merge kernel, so it is not done.
     const int want = batch * nkv >= 64 ? 1 : sm_count() / (batch * nkv);
     const int by_len = max_blocks / (2 * kAttnWarps) > 0 ? max_blocks / (2 * kAttnWarps) : 1;

@@ -193,6 +193,20 @@ def test_paged_attention_merge(ext, splits):
     assert rel_l2(got, want) < 1e-2  # (probabilities and output rounded to bf16: 2^-8 each)
 
 
+@pytest.mark.parametrize("splits", [33, 40, 64, 65])
+def test_paged_attention_merge_of_more_than_a_warp(ext, splits):
+    """More splits than lanes, asked for by the caller: maxima and sums are fetched lap by lap."""
+    from barlink_sm86_b200.ops import reference as ref
+    nq, nkv, hd, bs, max_blocks = 14, 2, 128, 16, 70
+    ctx = torch.tensor([1, 600, 1111], dtype=torch.int32, device="cuda")
+    kc, vc = _bf(3 * max_blocks, nkv, bs, hd, seed=1), _bf(3 * max_blocks, nkv, bs, hd, seed=2)
+    bt = torch.arange(3 * max_blocks, dtype=torch.int32, device="cuda").view(3, max_blocks)
+    qkv = _bf(3, (nq + 2 * nkv) * hd, seed=4)
+    got = ext.paged_attn_decode(qkv, kc, vc, bt, ctx, nq, nkv, hd, 1.0 / math.sqrt(hd), splits)
+    want = ref.paged_attn_decode(qkv, kc, vc, bt, ctx, nq, nkv, hd, 1.0 / math.sqrt(hd))
+    assert rel_l2(got, want) < 1e-2  # (probabilities and output rounded to bf16: 2^-8 each)
+
+
 @pytest.mark.parametrize("tokens,n,k,splits", [(64, 4608, 3584, 4), (8, 3584, 18944, 5), (1, 512, 1024, 2),
                                                (33, 640, 1024, 3)])
 def test_linear_split_slabs_sum_to_the_product(ext, tokens, n, k, splits):

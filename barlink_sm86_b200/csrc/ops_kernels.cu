@@ -1177,9 +1177,9 @@ __global__ void __launch_bounds__(kAttnWarps * 32)
 
 // Element d of a head from its splits.  Bound by its trips to memory: a lane fetches maximum and sum of one split (32 of them a
 // lap), and the elements of W splits are on their way meanwhile, so that up to 32 splits take one trip.  Attention and merge,
-// us, with every thread reading all maxima first, then splits one by one or four at a time / in fours and eights / so (all same
-// bits): 28 heads on 4, one sequence of 8000 tokens, 32 splits, 11.2 / 11.7 / 8.1; five of 600, 7 splits 8.1 / 6.6 / 5.9;
-// 40 on 8, seven of 600, 2 splits 8.1 / 7.9 / 7.5.
+// us, with every thread reading all maxima first, then the splits in a plain loop / in fours and eights / so (all same
+// bits): 28 heads on 4, one sequence of 8000 tokens, 32 splits, 11.2 / 11.8 / 8.2; five of up to 600, 7 splits 7.2 / 6.9 / 6.6;
+// 40 on 8, three of up to 1500, 6 splits 8.6 / 7.6 / 7.0.
 template <int W>
 __device__ __forceinline__ float merged_element(const float* __restrict__ base, int d, int nsplit) {
   const int lane = threadIdx.x & 31;

@@ -21,11 +21,12 @@
 // products take) and, before S had two buffers, the chain softmax -> P V -> next S -> softmax of a tile, whose
 // links added up to 2700 cycles a step.  Now S of step j + 2 is issued right behind P V of step j, so a
 // tile's softmax always finds its scores; P has two buffers for the same reason, and a rescale of O waits
-// for the P V before it.  24 heads x 4608 tokens with the transpose: 319 -> 297 us (879 TFLOP/s), 8 x 1024
-// causal, 28 heads on 4: 152 -> 141 us; 2550 cycles a step are left.  P through shared memory and V through a kernel
-// that transposed it (22 us at 24 x 4608, 12 us at 8 x 1024 x 4) gave the same step time, so the tiles in shared
-// memory do not bound it (an SM that always has work: tensor pipe 72 %, special functions 57 %; 24 heads x 4608 tokens 269 us);
-// without them the 4096-token MMDiT forward takes 71.5 ms instead of 73.4.
+// for the P V before it.  S of step j + 2 goes into the columns from which P V of step j, issued just before and not waited
+// for, takes P: one thread issues both, and the tensor pipe works off the products of one CTA in the order in which they are issued,
+// so the scores are written behind the reads of P.  (P is written by the softmax only after s_ready of its own step, so behind
+// both.)  With P in shared memory and V through a kernel that transposed it a step took the same time, so the tiles in
+// shared memory do not bound it; 24 heads x 4608 tokens: 297 us with the transpose (22 of them), 269 without, 2370 cycles a step
+// of an SM that always has work.  The 4096-token MMDiT forward takes 71.5 ms instead of 73.4.
 // The accumulator is rescaled only when the running max has grown by more than
 // 2^8 since the last rescale (the stale max is exact after the final division
 // by the row sum), which takes the TMEM read-modify-write out of the loop.

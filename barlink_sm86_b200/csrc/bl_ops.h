@@ -326,13 +326,13 @@ int bl_decode_advance(int* positions, int* ctx_lens, int* slots, const int* bloc
 int bl_w4a16_gemv(const void* x, const void* qweight, const void* scales, const void* qzeros, void* out,
                   int m, int n, int k, int group, int splits, void* ws, size_t ws_bytes, void* stream,
                   char* err, size_t errlen);
-/* packed tensors -> bf16 [n, k] */
-/* The same for groups of 128 on 16-byte aligned x and qweight and 8-byte aligned scales, 1..16 rows; silu: SiLU(gate) *
+/* The same product for groups of 128 on 16-byte aligned x and qweight and 8-byte aligned scales, 1..16 rows; silu: SiLU(gate) *
  * up over interleaved columns into [m][n / 2].  splits (from bl_w4a16_mma_splits: what suits the shape, or as many of
  * `splits` as there can be) > 1, or slabs given: fp32 [splits][m][n], for the next kernel or bl_slab_finish to sum. */
 int bl_w4a16_mma_splits(int m, int n, int k, int splits, int want_slabs);
 int bl_w4a16_mma(const void* x, const void* qweight, const void* scales, const void* qzeros, void* out, int m,
                  int n, int k, int silu, int splits, void* slabs, void* stream, char* err, size_t errlen);
+/* packed tensors -> bf16 [n, k] */
 int bl_w4_dequant(const void* qweight, const void* scales, const void* qzeros, void* w, int n, int k,
                   int group, void* stream, char* err, size_t errlen);
 

@@ -64,7 +64,7 @@ def main():
     cu = torch.tensor([0, T], dtype=torch.int32, device=dev)
     us = timed(lambda: ops.attention(v3[:, :heads], v3[:, heads:2 * heads], v3[:, 2 * heads:], cu, cu, T,
                                      hd ** -0.5, False, max_k=T))
-    rows.append({"kernel": "joint attention (V transpose + tcgen05)", "shape": [T, heads, hd], "us": us,
+    rows.append({"kernel": "joint attention (tcgen05)", "shape": [T, heads, hd], "us": us,
                  "tflops": 4.0 * T * T * heads * hd / us / 1e6})
     us = timed(lambda: ops.attention(v3[:, :heads], v3[:, heads:2 * heads], v3[:, 2 * heads:], cu, cu, T,
                                      hd ** -0.5, False))
